@@ -16,6 +16,7 @@
 #include "../../include/sdim_gb300.h"
 #include "frame.cuh"
 #include "kernels.cuh"
+#include "rows.cuh"
 #include "trace.cuh"
 #include "variants.cuh"
 
@@ -61,7 +62,10 @@ struct sdim_ctx {
   DevBuf cols;       // record columns of a d = 2 trace program (trace_cols.cuh)
   DevBuf dsnap;      // its x / z pass's deterministic snapshots (TraceDesc::snap)
   DevBuf cdet;       // deterministic slice sums of the odd-d cluster x / z passes (TraceDescU8::dsum)
+  DevBuf rdescs, rows;  // row form of the x / z pass (rows.cuh): descriptors, rows and updates
   cudaStream_t aux = nullptr;                      // coin pass, concurrent with the x / z pass
+  cudaStream_t fast = nullptr;                     // d = 2 row form beside a coin pass: the highest priority
+  cudaEvent_t ev_fast = nullptr;
   cudaStream_t grp = nullptr;                      // shot-group engines of a batch with trace programs
   // sdim_run's device-to-host copy of the records, when the record pass can
   // feed it in chunks (launch_trace_jobs copies each chunk as it is written)
@@ -95,6 +99,7 @@ struct sdim_ctx {
   double pass_ms[2] = {0.0, 0.0};        // x / z passes alone, coin pass alone
   int smem_attr_set[V_COUNT] = {};
   bool trace_smem_set = false;
+  bool rows_smem_set = false;
   bool frame_smem_set = false;
   int trace_threads = kTracePassThreads;  // x / z pass CTA size (SDIM_TRACE_PASS_THREADS: 256 or 512)
   GraphCapture* capture = nullptr;  // set while sdim_graph_create runs on its private context
@@ -147,6 +152,8 @@ struct sdim_circuit {
   int nfops = 0;
   const uint2* d_lay = nullptr;  // odd d: the layered x / z stream (append_layers_u8), inside the blob
   int nlay = 0;
+  RowProgram rows;              // row form of the x / z pass; nops 0 when the program has none
+  const uint2* d_blob = nullptr;  // what the offsets in `rows` count from
   // d = 2 x / z trace kept on the device for SDIM_FLAG_REUSE_XZ: written by a
   // run with the flag, valid once that synchronous run has ended without a
   // device error, then read by the later runs with the flag instead of
@@ -386,6 +393,7 @@ struct Job {
   int64_t shot0, nshots;
   uint8_t* out_dev;
   int index = -1;  // position in the caller's batch (graph capture: whose seed a descriptor holds)
+  bool rows = false;  // trace engine: its x / z pass runs in the row form
 };
 
 // Host -> device copy of `count` descriptors of `each` bytes, each holding a
@@ -410,6 +418,21 @@ int upload_descs(sdim_ctx* ctx, void* dst, const void* src, size_t each, size_t 
     return SDIM_OK;
   }
   if (g) g->need += (bytes + 255) & ~(size_t)255;
+  CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+  return SDIM_OK;
+}
+
+// The same for descriptors that hold no seed.
+int upload_fixed(sdim_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  GraphCapture* g = ctx->capture;
+  if (g && !g->sizing) {
+    if (g->used + bytes > g->cap) return fail(ctx, SDIM_ECUDA, "graph descriptor staging overflow");
+    std::memcpy(g->host + g->used, src, bytes);
+    src = g->host + g->used;
+    g->used += (bytes + 255) & ~(size_t)255;
+  } else if (g) {
+    g->need += (bytes + 255) & ~(size_t)255;
+  }
   CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
   return SDIM_OK;
 }
@@ -515,6 +538,124 @@ bool use_trace_u8(const Job& j, unsigned flags) {
   return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits;
 }
 
+// Whether a trace-engine job's x / z pass runs in the row form (rows.cuh):
+// wherever the encoder built one, unless a flag names a tableau pass.
+bool row_form(const sdim_circuit* c, unsigned flags) {
+  return c->rows.nops > 0 && !(flags & (SDIM_FLAG_FORCE_GMEM | SDIM_FLAG_SPLIT_XZ | SDIM_FLAG_CLUSTER_XZ |
+                                        SDIM_FLAG_U8_XZ | SDIM_FLAG_PACKED_XZ | SDIM_FLAG_UNLAYERED));
+}
+
+// The row-form programs of one d and chain-pass slice in a run: descriptors
+// [b, e) of the array, largest program first.
+struct RowGroup {
+  int d, slice, b, e, tiles, lg, block, ctas, cblock, rawt, xctas;
+  size_t raw_smem, chain_smem, extra_smem;
+};
+
+// Launch shapes of a group of row-form programs (their descriptors' tile_begin
+// and x_begin are set here).
+//   chain pass: a cluster of 8, 4 or 2 CTAs per program while the clusters
+//     leave SMs idle and the program has more than two panels; else one CTA.
+//     With more programs than SMs, CTAs no larger than the elimination needs,
+//     so that several share an SM.
+//   raw pass: in front of the chain pass in the same launch while the clusters
+//     do not fill the SMs and its state fits their shared memory (one launch
+//     less, and a coin pass beside it finds those SMs taken); else its own
+//     launch, a unit (column word) per CTA while that leaves the SMs room, 2
+//     or 4 once there are several CTAs per SM, which read the layers' ops once
+//     for all of them.
+void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vector<const sdim_circuit*>& c) {
+  long long units = 0, tasks = 1;
+  int nmax = 1, nmmax = 0, umax = 1;
+  for (int i = g.b; i < g.e; ++i) {
+    units += row_units(h[i].n, g.d, h[i].nk);
+    umax = std::max(umax, row_units(h[i].n, g.d, h[i].nk));
+    nmax = std::max(nmax, h[i].n);
+    nmmax = std::max(nmmax, h[i].nm);
+    tasks = std::max<long long>(tasks, c[i]->rows.nops / std::max(1, h[i].nlayers));
+  }
+  const size_t optin = (size_t)ctx->smem_optin - 12288;  // less the kernels' static arrays
+  g.ctas = 1;
+  if (nmmax > 2 * kRowPanel)
+    for (int k = 8; k > 1 && g.ctas == 1; k >>= 1)
+      if ((long long)k * (g.e - g.b) <= ctx->num_sms) g.ctas = k;
+  const bool batch = (long long)g.ctas * (g.e - g.b) > ctx->num_sms;
+  g.cblock = !batch ? 32 * kRowWarps : g.slice < 16 ? 128 : g.slice == 17 ? 256 : 32 * kRowWarps;
+  g.chain_smem = row_ops(g.d).chain_smem(nmax, g.cblock);
+  g.extra_smem = row_ops(g.d).extra_smem(nmax);
+  // the raw pass in front of the chain pass, on its CTAs
+  g.rawt = 0;
+  for (g.lg = 0; (g.ctas << g.lg) < umax; ++g.lg) {}
+  const size_t fused = row_ops(g.d).raw_smem(nmax, g.lg);
+  if (!batch && fused <= optin) {
+    g.rawt = 32;
+    while (g.rawt < g.cblock && g.rawt < (tasks << g.lg)) g.rawt <<= 1;
+    g.chain_smem = std::max(g.chain_smem, fused);
+  } else {
+    g.lg = units <= 2LL * ctx->num_sms ? 0 : units <= 8LL * ctx->num_sms ? 1 : 2;
+    while (g.lg > 0 && row_ops(g.d).raw_smem(nmax, g.lg) > optin) --g.lg;
+    g.block = 32;
+    while (g.block < 256 && g.block < (tasks << g.lg)) g.block <<= 1;
+    g.raw_smem = row_ops(g.d).raw_smem(nmax, g.lg);
+  }
+  g.tiles = g.xctas = 0;
+  for (int i = g.b; i < g.e; ++i) {
+    h[i].tile_begin = g.tiles;
+    h[i].x_begin = g.xctas;
+    g.tiles += (row_units(h[i].n, g.d, h[i].nk) + (1 << g.lg) - 1) >> g.lg;
+    const int per = row_ops(g.d).extra_per_cta(h[i].n);
+    g.xctas += (h[i].nx + per - 1) / per;
+  }
+}
+
+RowDesc row_desc(const sdim_circuit* c, uint8_t* mem, uint4* mhdr, uint8_t* mrow, uint8_t* nrow, int rowb) {
+  RowDesc r;
+  std::memset(&r, 0, sizeof(r));
+  const RowProgram& p = c->rows;
+  r.ops = reinterpret_cast<const uint4*>(c->d_blob + p.ops_off);
+  r.lay = reinterpret_cast<const uint32_t*>(c->d_blob + p.lay_off);
+  r.minfo = reinterpret_cast<const uint32_t*>(c->d_blob + p.minfo_off);
+  r.xinfo = c->d_blob + p.xinfo_off;
+  const RowBytes b = row_bytes(c->n, c->d, c->nmeas, p.nx, p.nk);
+  r.raw = mem + b.raw;
+  r.xraw = mem + b.xraw;
+  r.kpart = mem + b.kpart;
+  r.ksign = mem + b.ksign;
+  r.opf = mem + b.opf;
+  r.opm = reinterpret_cast<int4*>(mem + b.opm);
+  r.pop = reinterpret_cast<int*>(mem + b.pop);
+  r.opw = reinterpret_cast<uint32_t*>(mem + b.opw);
+  r.mhdr = mhdr;
+  r.mrow = mrow;
+  r.nrow = nrow;
+  r.n = c->n;
+  r.d = c->d;
+  r.nlayers = p.nlayers;
+  r.nm = c->nmeas;
+  r.nx = p.nx;
+  r.nk = p.nk;
+  r.E = row_elems(c->n);
+  r.EK = (p.nk + (c->d == 2 ? 0 : 1) + kRowLanes - 1) / kRowLanes;
+  r.rowb = rowb;
+  return r;
+}
+
+int launch_row_raw(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s) {
+  if (g.rawt) return SDIM_OK;
+  row_ops(g.d).raw(g.tiles, g.block, g.lg, g.raw_smem, s, rd + g.b, g.e - g.b);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row raw pass launch");
+}
+
+// fence: least shared memory of a chain CTA, 0 for none
+int launch_row_rest(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s, size_t fence) {
+  cudaError_t e = row_ops(g.d).chain(g.slice, g.ctas, g.cblock, g.rawt, g.lg, std::max(g.chain_smem, fence), s, rd + g.b, g.e - g.b);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "row chain pass launch");
+  if (g.xctas > 0) row_ops(g.d).extra(g.xctas, g.extra_smem, s, rd + g.b, g.e - g.b);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row extra pass launch");
+}
+
 // Trace-engine launches: the x / z pass of every program (d = 2 jobs, then
 // odd-d jobs per variant of d), the coin pass of the d = 2 jobs alongside on
 // the second stream, then the phase passes (d = 2 per trace-row width, odd
@@ -542,6 +683,40 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFuncSetAttribute");
     ctx->trace_smem_set = true;
   }
+  if (!ctx->rows_smem_set) {
+    for (int d : {2, 3, 5, 7}) {
+      const cudaError_t e = row_ops(d).set_smem(ctx->smem_optin);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFuncSetAttribute");
+    }
+    ctx->rows_smem_set = true;
+  }
+  // which programs take the row form: those that have one, within the budget
+  // of the slots that the tableau passes would use
+  size_t row_total = 0;
+  for (std::vector<Job>* list : {&jobs, &ujobs})
+    for (Job& j : *list) {
+      if (!row_form(j.c, flags)) continue;
+      const size_t b = row_bytes(j.c->n, j.c->d, j.c->nmeas, j.c->rows.nx, j.c->rows.nk).total;
+      if (row_total + b > ctx->gmem_slot_budget) continue;
+      row_total += b;
+      j.rows = true;
+    }
+  // row-form programs: their descriptors, d = 2 first
+  std::vector<RowDesc> hr;
+  std::vector<const sdim_circuit*> rcirc;
+  std::vector<RowGroup> rgroups;
+  size_t rmem = 0;
+  auto add_row = [&](const sdim_circuit* c, uint4* mhdr, void* mrow, void* nrow, int rowb) {
+    // memory offsets first, the base pointer once the buffer's size is known
+    hr.push_back(row_desc(c, reinterpret_cast<uint8_t*>(rmem), mhdr, static_cast<uint8_t*>(mrow),
+                          static_cast<uint8_t*>(nrow), rowb));
+    rcirc.push_back(c);
+    rmem += row_bytes(c->n, c->d, c->nmeas, c->rows.nx, c->rows.nk).total;
+    const int sl = row_slice(row_elems(c->n));
+    if (rgroups.empty() || rgroups.back().d != c->d || rgroups.back().slice != sl)
+      rgroups.push_back(RowGroup{c->d, sl, (int)hr.size() - 1, 0});
+    rgroups.back().e = (int)hr.size();
+  };
   // ---- d = 2 descriptors
   // largest first: the x / z passes of a batch start with the longest ones
   std::stable_sort(jobs.begin(), jobs.end(), [](const Job& a, const Job& b) { return a.c->n > b.c->n; });
@@ -653,7 +828,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
         td.nchunk = (j.c->nn1_used + kCoinChunk - 1) / kCoinChunk;
         td.cmap = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(td.masks) +
                                               coin_mask_bytes(td.nchunk, j.nshots));
-        coins += (long long)((td.nchunk + kCoinChunksPerItem - 1) / kCoinChunksPerItem) * j.nshots;
+        coins += coin_blocks(td.nchunk, j.nshots);
       }
       td.nm = j.c->nmeas;
       td.nn1 = j.c->nn1;
@@ -661,7 +836,11 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       td.wn = (j.c->n + 31) >> 5;
       td.nused = j.c->nn1_used;
     }
-    if (k == 1 && !skip_xz && jobs[0].c->nmeas > 0) {
+    for (size_t i = 0; i < k; ++i) {
+      hd[i].rows = jobs[i].rows ? 1 : 0;
+      if (hd[i].rows && !skip_xz) add_row(jobs[i].c, hd[i].mhdr, hd[i].mrow, hd[i].nrow, 4 * hd[i].tw);
+    }
+    if (k == 1 && !skip_xz && !hd[0].rows && jobs[0].c->nmeas > 0) {
       // one program: the x / z pass leaves the deterministic cross terms to
       // the header pass, a snapshot per run of deterministic measurements
       const sdim_circuit* c0 = jobs[0].c;
@@ -700,16 +879,18 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   // ---- odd-d descriptors
   std::stable_sort(ujobs.begin(), ujobs.end(), [](const Job& a, const Job& b) {
     const int va = trace_u8_variant(a.c->d), vb = trace_u8_variant(b.c->d);
-    return va != vb ? va < vb : a.c->n > b.c->n;
+    if (va != vb) return va < vb;
+    return a.rows != b.rows ? a.rows : a.c->n > b.c->n;
   });
   const size_t ku = ujobs.size();
   std::vector<TraceDescU8> hu(ku);
+  std::vector<int> xmode(ku);
+  constexpr int kRowMode = 9;
   TraceDescU8* du = nullptr;
   if (ku) {
     // per program its trace, and for a cluster x / z pass (odd_xz_mode 3, 4)
     // its deterministic slice sums
     std::vector<size_t> off(ku), doff(ku, SIZE_MAX);
-    std::vector<int> xmode(ku);
     size_t total = 0, dtotal = 0;
     for (size_t i = 0; i < ku; ++i) {
       const Job& j = ujobs[i];
@@ -717,7 +898,9 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       trace_offsets_u8(j.c->nmeas, j.c->nn1, trace_row_bytes_u8(j.c->n), o);
       off[i] = total;
       total += o[4];
-      const int mode = odd_xz_mode(j.c->n, j.c->d, (long long)ku, flags, (size_t)ctx->smem_optin, ctx->num_sms);
+      const int mode = j.rows ? kRowMode
+                                            : odd_xz_mode(j.c->n, j.c->d, (long long)ku, flags,
+                                                          (size_t)ctx->smem_optin, ctx->num_sms);
       xmode[i] = mode;
       if (mode == 3 || mode == 4) {
         doff[i] = dtotal;
@@ -763,17 +946,37 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
         td.lay = j.c->d_lay;
         td.nlay = j.c->nlay;
       }
+      if (xm == kRowMode) {
+        td.nhdr = const_cast<uint2*>(j.c->d_blob + j.c->rows.nhdr_off);
+        add_row(j.c, td.mhdr, td.mrow, td.nrow, td.sw);
+      }
     }
     du = static_cast<TraceDescU8*>(ctx->tdescs_u8.p);
     if ((rc = upload_descs(ctx, du, hu.data(), sizeof(TraceDescU8), ku, offsetof(TraceDescU8, c),
                            [&](size_t i) { return ujobs[i].index; }, s)) != SDIM_OK)
       return rc;
   }
+  RowDesc* dr = nullptr;
+  if (!hr.empty()) {
+    if ((rc = ensure(ctx, ctx->rows, std::max<size_t>(rmem, 256))) != SDIM_OK) return rc;
+    if ((rc = ensure(ctx, ctx->rdescs, sizeof(RowDesc) * hr.size())) != SDIM_OK) return rc;
+    const size_t base = reinterpret_cast<size_t>(ctx->rows.p);
+    for (RowDesc& r : hr) {
+      uint8_t** ptrs[] = {&r.raw, &r.xraw, &r.kpart, &r.ksign, &r.opf};
+      for (uint8_t** p : ptrs) *p += base;
+      r.opm = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(r.opm) + base);
+      r.pop = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(r.pop) + base);
+      r.opw = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(r.opw) + base);
+    }
+    for (RowGroup& g : rgroups) plan_row_group(ctx, g, hr.data(), rcirc);
+    dr = static_cast<RowDesc*>(ctx->rdescs.p);
+    if ((rc = upload_fixed(ctx, dr, hr.data(), sizeof(RowDesc) * hr.size(), s)) != SDIM_OK) return rc;
+  }
+  const bool d2_tab = k && !skip_xz && std::any_of(hd.begin(), hd.end(), [](const TraceDesc& t) { return !t.rows; });
   if (coins) CK(cudaEventRecord(ctx->ev_fork, s));
   // odd d: the x / z pass form of each program (odd_xz_mode)
   const size_t optin = (size_t)ctx->smem_optin;
   const size_t win = trace_u8_window_bytes();
-  auto xz_mode = [&](int n, int d) { return odd_xz_mode(n, d, (long long)ku, flags, optin, ctx->num_sms); };
   // clusters of a mode-4 run: one per kTraceClusterCtas SMs, each CTA alone
   // on its SM, so the programs in flight keep their columns in L2
   auto stream_clusters = [&](size_t programs) {
@@ -786,9 +989,11 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   size_t slot_total = 0;
   for (size_t b = 0; b < ku;) {
     const int v = trace_u8_variant(hu[b].c.d);
-    const int mode = xz_mode(hu[b].c.n, hu[b].c.d);
+    const int mode = xmode[b];
     size_t e = b;
-    while (e < ku && trace_u8_variant(hu[e].c.d) == v && xz_mode(hu[e].c.n, hu[e].c.d) == mode) ++e;
+    auto slice = [&](size_t i) { return row_slice(row_elems(hu[i].c.n)); };
+    while (e < ku && trace_u8_variant(hu[e].c.d) == v && xmode[e] == mode && (mode != kRowMode || slice(e) == slice(b)))
+      ++e;
     runs.push_back(Run{b, e, v, mode, slot_total});
     if (mode == 2) {
       const size_t grid = std::min<size_t>(e - b, 2 * (size_t)ctx->num_sms);
@@ -815,9 +1020,31 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   const bool d2_xz = k && !skip_xz;
   const bool fan = runs.size() > 1 || (d2_xz && !runs.empty());
   if (fan) CK(cudaEventRecord(ctx->ev_xzf, s));
-  // ---- x / z passes: one CTA per program (none when a kept trace is valid)
-  if (d2_xz) {
-    const int nmax = jobs[0].c->n;
+  // ---- d = 2 x / z passes (none when a kept trace is valid).  One program in
+  // row form with a coin pass beside it: on the stream of highest priority, up
+  // to its column pass, since the coin pass's blocks take every SM that the
+  // short chain leaves and the passes after it would wait for them to drain
+  // (the L = 7 step: 381 us with them on the caller's stream)
+  const bool d2_fast = k == 1 && coins && d2_xz && hd[0].rows;
+  const cudaStream_t xs = d2_fast ? ctx->fast : s;
+  if (d2_fast) CK(cudaStreamWaitEvent(xs, ctx->ev_fork, 0));
+  for (const RowGroup& g : rgroups)
+    if (g.d == 2 && (rc = launch_row_raw(ctx, g, dr, xs)) != SDIM_OK) return rc;
+  // shared-memory fence: a few x / z CTAs claim enough shared memory that no
+  // coin-pass block fits beside them, so the coin warps do not take the issue
+  // slots of the latency-bound x / z pass on its SM
+  auto coin_fence = [&](int ctas) -> size_t {
+    if (!coins || ctas > ctx->num_sms / 8) return 0;
+    const long long fence = (long long)ctx->smem_per_sm - 2LL * ctx->smem_reserved - (long long)kCoinFenceSmem + 16;
+    const long long cap = (long long)ctx->smem_optin - 4096;  // room for the kernel's static arrays
+    return (size_t)std::max(0LL, std::min(fence, cap));
+  };
+  for (const RowGroup& g : rgroups)
+    if (g.d == 2 && (rc = launch_row_rest(ctx, g, dr, xs, coin_fence(g.ctas * (g.e - g.b)))) != SDIM_OK) return rc;
+  if (d2_tab) {
+    int nmax = 1;
+    for (size_t i = 0; i < k; ++i)
+      if (!hd[i].rows) nmax = std::max(nmax, jobs[i].c->n);
     const size_t hot = trace_pass_hot_bytes(nmax), xz = trace_pass_xz_bytes(nmax);
     // after the tableau: the schedule window; about 3.2 KB of static shared memory besides
     const size_t win = trace_pass_window_bytes();
@@ -828,14 +1055,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       if ((rc = ensure(ctx, ctx->gslots_xz, xz * (size_t)grid)) != SDIM_OK) return rc;
     }
     size_t smem = hot + (in_smem ? xz : 0) + win;
-    if (coins && grid <= ctx->num_sms / 8) {
-      // shared-memory fence: a few x / z CTAs claim enough shared memory that
-      // no coin-pass block fits beside them, so the coin warps do not take
-      // the issue slots of the latency-bound x / z pass on its SM
-      const long long fence = (long long)ctx->smem_per_sm - 2LL * ctx->smem_reserved - (long long)kCoinFenceSmem + 16;
-      const long long cap = (long long)ctx->smem_optin - 4096;  // room for the kernel's static arrays
-      smem = std::max<size_t>(smem, (size_t)std::max(0LL, std::min(fence, cap)));
-    }
+    smem = std::max(smem, coin_fence(grid));
     launch_trace_pass(ctx->trace_threads, grid, smem, s, dd, (int)k, static_cast<uint8_t*>(ctx->gslots_xz.p), xz, hot,
                       in_smem ? 1 : 0, status);
     const cudaError_t le = cudaGetLastError();
@@ -854,7 +1074,13 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       used[si] = true;
     }
     const int nmax = hu[b].c.n;
-    if (mode >= 7) {
+    if (mode == kRowMode) {
+      for (const RowGroup& g : rgroups)
+        if (g.d == hu[b].c.d && g.slice == row_slice(row_elems(nmax)))
+          if ((rc = launch_row_raw(ctx, g, dr, rs)) != SDIM_OK ||
+              (rc = launch_row_rest(ctx, g, dr, rs, 0)) != SDIM_OK)
+            return rc;
+    } else if (mode >= 7) {
       // d = 5, 7 on 4-bit lanes: one CTA per program, largest first
       const bool in_smem = mode == 7;
       const int dd = hu[b].c.d;
@@ -909,34 +1135,31 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       CK(cudaEventRecord(ctx->ev_xzj[i], ctx->xzs[i]));
       CK(cudaStreamWaitEvent(s, ctx->ev_xzj[i], 0));
     }
-  if (timed) CK(cudaEventRecord(ctx->ev_xzo, s));
+  if (timed) CK(cudaEventRecord(ctx->ev_xzo, xs));
   // ---- header and column passes: after the x / z pass, beside the rest of
-  // the coin pass.  (On a stream of the highest priority their blocks shared
-  // SMs with the coin pass's and the latency-bound column pass took twice as
-  // long: 0.389 against 0.370 ms on the L = 7 step.)
-  if (k == 1 && d2_xz && hd[0].snap) {
-    launch_header_pass((jobs[0].c->nmeas + 3) / 4, s, dd, status);
+  // the coin pass
+  if (k == 1 && d2_xz && (hd[0].snap || (hd[0].rows && (colform || keep)))) {
+    launch_header_pass((jobs[0].c->nmeas + 3) / 4, xs, dd, status);
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return cuda_fail(ctx, le, "header pass launch");
   }
   if (colform && !skip_cols) {
-    if (!launch_column_pass(hd[0].tw, (int)((ncols + 32 * kColumnWarps - 1) / (32 * kColumnWarps)), s, dd, status))
+    if (!launch_column_pass(hd[0].tw, (int)((ncols + 32 * kColumnWarps - 1) / (32 * kColumnWarps)), xs, dd, status))
       return fail(ctx, SDIM_EINVAL, "no column pass for trace rows of " + std::to_string(hd[0].tw) + " words");
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return cuda_fail(ctx, le, "column pass launch");
     if (timed) {
-      CK(cudaEventRecord(ctx->ev_cols, s));
+      CK(cudaEventRecord(ctx->ev_cols, xs));
       ctx->cols_recorded = true;
     }
   }
+  if (d2_fast) CK(cudaEventRecord(ctx->ev_fast, xs));
   // ---- coin pass on the second stream, alongside the x / z passes (independent work)
   if (coins) {
     CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
-    const int block = 256;
-    const long long grid = (coins + block - 1) / block;
-    if (grid > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one coin pass");
+    if (coins > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one coin pass");
     if (timed) CK(cudaEventRecord(ctx->ev_c0, ctx->aux));
-    launch_coin_pass((int)grid, block, kCoinFenceSmem, ctx->aux, dd, (int)k, coins);
+    launch_coin_pass((int)coins, ctx->aux, dd, (int)k);
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return cuda_fail(ctx, le, "coin pass launch");
     if (timed) {
@@ -946,6 +1169,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     CK(cudaEventRecord(ctx->ev_join, ctx->aux));
     CK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
   }
+  if (d2_fast) CK(cudaStreamWaitEvent(s, ctx->ev_fast, 0));
   if (timed) CK(cudaEventRecord(ctx->ev_xz, s));
   // ---- phase passes (the record pass for record columns)
   if (colform) {
@@ -998,7 +1222,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       items = hu[e].c.item_begin + (hu[e].c.nshots + 31) / 32;
       ++e;
     }
-    const int nmax = hu[b].c.n;
+    int nmax = 1;
+    for (size_t i = b; i < e; ++i) nmax = std::max(nmax, hu[i].c.n);
     // (shot, chunk) threads: about 64 generators per thread, 32 to 512 threads
     const int nch = std::max(1, std::min(16, (2 * nmax + 63) / 64));
     if (items > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one phase pass");
@@ -1450,6 +1675,147 @@ void append_schedule(std::vector<uint2>& dev, size_t op_begin, size_t nops, int 
   if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
 }
 
+// Row program (rows.cuh) of a program's instruction words, appended to dev:
+// every op goes one layer after the last op on one of its qudits, whatever
+// the program order between qudits, so a measurement holds no other qudit's
+// gates up.  None (out.nops = 0) for a program without measurements, with a
+// two-qudit gate on one qudit twice (not a symplectic map), or whose rows
+// would take more than kRowBytesMost or kRowWorkMost: there the cost of
+// carrying every row through every earlier update (quadratic in the
+// measurements) passes that of the tableau passes.
+constexpr size_t kRowBytesMost = (size_t)256 << 20;
+constexpr double kRowWorkMost = 4e9;
+
+void append_rows(std::vector<uint2>& dev, size_t op_begin, size_t nops, int n, int d, int nmeas, RowProgram& out) {
+  out = RowProgram();
+  if (!row_dim(d) || n > 2048 || nmeas < 1) return;
+  struct Entry {
+    uint4 o;
+    int level;
+  };
+  std::vector<Entry> ops;
+  ops.reserve(nops);
+  std::vector<int> last(n, -1), slot(n, -1);  // level of the last op on a qudit; 2 entry + (0: z, 1: w) of a free N1 slot
+  std::vector<uint32_t> minfo;
+  std::vector<uint2> xinfo, nhdr;
+  uint32_t mord = 0, nord = 0, gated = 0;  // gated: measurements before the last gate so far
+  int nk = 0, levels = 0;
+  auto put_op = [&](const uint4& o, int lv) {
+    ops.push_back(Entry{o, lv});
+    levels = std::max(levels, lv + 1);
+    return (int)ops.size() - 1;
+  };
+  for (size_t i = op_begin; i < op_begin + nops && mord < (uint32_t)nmeas; ++i) {
+    const uint2 w = dev[i];
+    const uint32_t op = w.x & kOpMask;
+    const int q = (int)(w.x >> 8);
+    if (op == OP_NOP) continue;
+    if (op == OP_N1OFF) {
+      nhdr.push_back(make_uint2(0xffffffffu, op));
+      ++nord;
+      continue;
+    }
+    if (op == OP_N1D || op == OP_N1F || op == OP_N1P) {
+      nhdr.push_back(make_uint2(w.y, op));
+      const uint32_t r = (uint32_t)xinfo.size() + 1u;
+      xinfo.push_back(make_uint2(mord, (1u << 30) | nord));
+      xinfo.push_back(make_uint2(mord, (2u << 30) | nord));
+      nk = std::max(nk, (int)mord);
+      ++nord;
+      if (slot[q] >= 0) {
+        uint4& o = ops[slot[q] >> 1].o;
+        ((slot[q] & 1) ? o.w : o.z) = r;
+        o.x |= kRopN;
+        slot[q] = -1;
+      } else {
+        last[q] += 1;
+        put_op(make_uint4((uint32_t)q | ((uint32_t)q << 11) | kRopN, 0u, r, 0u), last[q]);
+      }
+      continue;
+    }
+    if (op == OP_M || op == OP_RESET) {
+      last[q] += 1;
+      uint32_t z = 0u;
+      nk = std::max(nk, (int)gated);
+      if (op == OP_RESET) {
+        z = (uint32_t)xinfo.size() + 1u;
+        xinfo.push_back(make_uint2(mord + 1u, mord));
+        nk = std::max(nk, (int)mord + 1);
+      }
+      minfo.push_back(nord | (op == OP_RESET ? 0x80000000u : 0u));
+      const uint32_t f = kRopM | (op == OP_RESET ? kRopReset : 0u);
+      slot[q] = 2 * put_op(make_uint4((uint32_t)q | ((uint32_t)q << 11) | f, mord, z, 0u), last[q]) + 1;
+      ++mord;
+      continue;
+    }
+    const bool two = op == OP_CNOT || op == OP_CNOT_INV;
+    const int t = (int)w.y;
+    if (two && t == q) return;
+    gated = mord;
+    const int lv = two ? std::max(last[q], last[t]) + 1 : last[q] + 1;
+    // what the constants of x_q and z_q gain: d = 2 sign exponents, else the
+    // linear phase of the gate
+    const int half = (d + 1) / 2;
+    uint32_t f = 0u, cx = 0u, cz = 0u;
+    switch (op) {
+      case OP_X: cx = d == 2 ? 2 : 1; break;
+      case OP_X_INV: cx = d == 2 ? 2 : d - 1; break;
+      case OP_Z: cz = d == 2 ? 2 : 1; break;
+      case OP_Z_INV: cz = d == 2 ? 2 : d - 1; break;
+      case OP_H: f = kRopH; break;
+      case OP_H_INV: f = kRopHInv; break;
+      case OP_P: f = kRopP; cz = d == 2 ? 3 : d - half; break;
+      case OP_P_INV: f = kRopPInv; cz = d == 2 ? 1 : half; break;
+      case OP_CNOT: f = kRopC; break;
+      default: f = kRopCInv; break;
+    }
+    if (cx | cz) f |= kRopK;
+    const uint32_t tq = two ? (uint32_t)t : (uint32_t)q;
+    const int e = put_op(make_uint4((uint32_t)q | (tq << 11) | f, cx | (cz << 3), 0u, 0u), lv);
+    last[q] = lv;
+    slot[q] = 2 * e;
+    if (two) {
+      last[t] = lv;
+      slot[t] = 2 * e + 1;
+    }
+  }
+  const double rows = (double)nmeas + (double)xinfo.size();
+  if (xinfo.size() >= (size_t)1 << 30 ||
+      row_bytes(n, d, nmeas, (int)xinfo.size(), nk).total > kRowBytesMost ||
+      rows * nmeas * 2 * row_elems(n) > kRowWorkMost)
+    return;
+  // layer by layer
+  std::vector<uint32_t> lay(levels + 1, 0u);
+  for (const Entry& e : ops) ++lay[e.level + 1];
+  for (int l = 0; l < levels; ++l) lay[l + 1] += lay[l];
+  std::vector<uint32_t> at(lay.begin(), lay.end() - 1);
+  std::vector<uint4> sorted(ops.size());
+  for (const Entry& e : ops) sorted[at[e.level]++] = e.o;
+  if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
+  out.ops_off = (int64_t)dev.size();
+  for (const uint4& o : sorted) {
+    dev.push_back(make_uint2(o.x, o.y));
+    dev.push_back(make_uint2(o.z, o.w));
+  }
+  auto put32 = [&](std::vector<uint32_t>& v) {
+    const int64_t off = (int64_t)dev.size();
+    if (v.size() & 1) v.push_back(0u);
+    for (size_t k = 0; k < v.size(); k += 2) dev.push_back(make_uint2(v[k], v[k + 1]));
+    return off;
+  };
+  out.lay_off = put32(lay);
+  out.minfo_off = put32(minfo);
+  out.xinfo_off = (int64_t)dev.size();
+  dev.insert(dev.end(), xinfo.begin(), xinfo.end());
+  out.nhdr_off = (int64_t)dev.size();
+  dev.insert(dev.end(), nhdr.begin(), nhdr.end());
+  out.nops = (int)ops.size();
+  out.nlayers = levels;
+  out.nx = (int)xinfo.size();
+  out.nk = nk;
+  if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
+}
+
 // Frame instruction stream (frame.cuh) of rows already checked by
 // encode_rows, appended to dev: one word per instruction other than the
 // identity (sdim/program.py:479-480 leaves I out of the frame walk).
@@ -1590,6 +1956,8 @@ int sdim_ctx_create(int device, sdim_ctx** out) {
   sdim_ctx* ctx = new sdim_ctx();
   ctx->device = device;
   cudaSetDevice(device);
+  int least = 0, greatest = 0;
+  cudaDeviceGetStreamPriorityRange(&least, &greatest);
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1598,6 +1966,8 @@ int sdim_ctx_create(int device, sdim_ctx** out) {
       cudaEventCreate(&ctx->ev_xzo) != cudaSuccess || cudaEventCreate(&ctx->ev_c0) != cudaSuccess ||
       cudaEventCreate(&ctx->ev_c1) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&ctx->fast, cudaStreamNonBlocking, greatest) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->ev_fast, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_xzf, cudaEventDisableTiming) != cudaSuccess ||
@@ -1642,12 +2012,13 @@ int sdim_ctx_destroy(sdim_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   cudaStreamSynchronize(ctx->aux);
+  cudaStreamSynchronize(ctx->fast);
   cudaStreamSynchronize(ctx->grp);
   cudaStreamSynchronize(ctx->cps);
   for (int i = 0; i < sdim_ctx::kXzStreams; ++i) cudaStreamSynchronize(ctx->xzs[i]);
   DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap, &ctx->arena,
                     &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8, &ctx->xz_u8,
-                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet};
+                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rdescs, &ctx->rows};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   if (ctx->staging) cudaFreeHost(ctx->staging);
@@ -1674,6 +2045,8 @@ int sdim_ctx_destroy(sdim_ctx* ctx) {
     cudaEventDestroy(ctx->ev_xzj[i]);
     cudaStreamDestroy(ctx->xzs[i]);
   }
+  cudaEventDestroy(ctx->ev_fast);
+  cudaStreamDestroy(ctx->fast);
   cudaStreamDestroy(ctx->aux);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -1700,7 +2073,8 @@ int sdim_memory_info(sdim_ctx* ctx, int64_t info[3]) {
   info[1] = (int64_t)total_b;
   const DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap,
                           &ctx->arena, &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8,
-                          &ctx->xz_u8, &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet};
+                          &ctx->xz_u8, &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet,
+                          &ctx->rdescs, &ctx->rows};
   int64_t held = 0;
   for (const DevBuf* b : bufs) held += (int64_t)b->cap;
   info[2] = held;
@@ -1731,6 +2105,8 @@ int sdim_encode_circuit(sdim_ctx* ctx, const int32_t* ops, int64_t nops, const d
   int64_t lay_off = -1;
   int nlay = 0;
   if (d != 2) append_layers_u8(dev, 0, ndev, n, lay_off, nlay);
+  RowProgram rows;
+  append_rows(dev, 0, ndev, n, d, nmeas, rows);
   int64_t fops_off = 0;
   int nfops = 0;
   append_frame_ops(ops, nops, noise_prob, dev, fops_off, nfops);
@@ -1778,6 +2154,8 @@ int sdim_encode_circuit(sdim_ctx* ctx, const int32_t* ops, int64_t nops, const d
     c->d_lay = c->d_ops + lay_off;
     c->nlay = nlay;
   }
+  c->rows = rows;
+  c->d_blob = c->d_ops;
   c->fops_off = fops_off;
   c->nfops = nfops;
   *out = c;
@@ -2180,6 +2558,7 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
     if (d[i] == 2 && trace_words(n[i]))
       append_schedule(dev, op_off[i], (size_t)c.nops, n[i], kTraceWinSteps, kTraceWinOps, sch[i]);
     if (d[i] != 2 && layered) append_layers_u8(dev, op_off[i], (size_t)c.nops, n[i], lay_off[i], nlay[i]);
+    append_rows(dev, op_off[i], (size_t)c.nops, n[i], d[i], nmeas, c.rows);
     c.variant = variant_for(d[i]);
     c.gvariant = group_variant_for(d[i], n[i], 0);
     c.gblock = variant_ops(c.gvariant).cta ? cta_block_for(n[i]) : 32;
@@ -2203,6 +2582,7 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
   uint2* base = static_cast<uint2*>(ctx->arena.p);
   for (int i = 0; i < ncirc; ++i) {
     circs[i].d_ops = base + op_off[i];
+    circs[i].d_blob = base;
     if (sch[i].steps_off >= 0) {
       circs[i].d_steps = reinterpret_cast<const uint4*>(base + sch[i].steps_off);
       circs[i].d_lops = reinterpret_cast<const uint4*>(base + sch[i].lops_off);

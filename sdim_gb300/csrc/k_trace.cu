@@ -21,6 +21,7 @@ __global__ void __launch_bounds__(THREADS) k_trace_pass(const TraceDesc* __restr
   uint4* win = reinterpret_cast<uint4*>(smem + hot_bytes + (xz_in_smem ? xz_bytes : 0));
   for (int i = blockIdx.x; i < ndesc; i += gridDim.x) {
     const TraceDesc td = descs[i];
+    if (td.rows) continue;
     TraceTab e(xz, hot, td.c.n, 2, CtaTeam(red));
     trace_program(td, e, win, sc, tacc, pacc, status);
     __syncthreads();
@@ -143,16 +144,15 @@ __global__ void __launch_bounds__(32, NW >= 32 ? 16 : 32)
   record_group<NW>(descs, g0 + blockIdx.x, threadIdx.x, rec);
 }
 
-// One thread per (chunk group, shot) item of the coin pass; descs with
-// masks only, numbered through coin_begin.  Three blocks per SM leave 80
-// registers a thread: the eight interleaved Philox chains and their round
-// keys fit without spills.
-__global__ void __launch_bounds__(256, 3) k_coin_pass(const TraceDesc* __restrict__ descs, int ndesc,
-                                                      long long total) {
-  const long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= total) return;
-  const int i = find_coin_desc(descs, ndesc, it);
-  coin_item(descs + i, it - descs[i].coin_begin);
+// Blocks of the coin pass; descs with masks only, numbered through coin_begin.
+// Bound by the multiply pipe: 15 of a Philox block's 20 multiplies are left.
+// Three blocks per SM leave 80 registers a thread: the eight interleaved
+// chains and their round keys fit without spills.
+__global__ void __launch_bounds__(kCoinThreads, 3) k_coin_pass(const TraceDesc* __restrict__ descs, int ndesc) {
+  __shared__ CoinSmem sm;
+  static_assert(sizeof(CoinSmem) >= kCoinFenceSmem, "the fence counts on it");
+  const int i = find_coin_desc(descs, ndesc, blockIdx.x);
+  coin_tile(descs + i, (long long)blockIdx.x - descs[i].coin_begin, sm);
 }
 
 // Philox throughput probe: every thread draws iters x 8 blocks (eight
@@ -186,9 +186,8 @@ void launch_header_pass(int grid, cudaStream_t s, const TraceDesc* descs, const 
   k_header_pass<<<grid, 128, 0, s>>>(descs, status);
 }
 
-void launch_coin_pass(int grid, int block, size_t smem, cudaStream_t s, const TraceDesc* descs, int ndesc,
-                      long long total) {
-  k_coin_pass<<<grid, block, smem, s>>>(descs, ndesc, total);
+void launch_coin_pass(int grid, cudaStream_t s, const TraceDesc* descs, int ndesc) {
+  k_coin_pass<<<grid, kCoinThreads, 0, s>>>(descs, ndesc);
 }
 
 size_t trace_pass_hot_bytes(int n) { return round16(TraceTab::hot_bytes(n)); }

@@ -1,0 +1,1355 @@
+// Row form of the x / z pass (rows.cuh), device side: the raw, chain and extra
+// passes.  Instantiated for d = 2, 3, 5 and 7 in k_rows_<d>.cu.
+#pragma once
+#include "planes3.cuh"
+#include "rows.cuh"
+#include "trace_split_u8.cuh"
+#include "variants.cuh"
+
+#include <type_traits>
+
+namespace sdim {
+namespace {
+
+constexpr int L = kRowLanes;
+
+// ---------------------------------------------------------------- elements
+// T: the residues of 32 generators in bit planes (rows.cuh).  Every operation
+// is a few three-input logic instructions for all 32.
+
+__device__ __forceinline__ uint32_t mux(uint32_t m, uint32_t a, uint32_t b) { return (m & a) | (~m & b); }
+__device__ __forceinline__ uint32_t maj(uint32_t a, uint32_t b, uint32_t c) { return (a & b) | (a & c) | (b & c); }
+__device__ __forceinline__ uint32_t lane_mask(bool b) { return b ? 0xffffffffu : 0u; }
+
+// Three planes (d = 5, 7): bit 0 in x, bit 1 in y, bit 2 in z; w unused.
+template <int D>
+struct El {
+  using T = uint4;
+  static __device__ __forceinline__ T zero() { return make_uint4(0u, 0u, 0u, 0u); }
+  // d = 7 keeps 0 as 000 or 111: a sum is a three-bit one with its carry added
+  // back in, a negative the complement, twice a value its rotation
+  static __device__ __forceinline__ uint32_t nzw(T a) {
+    const uint32_t any = a.x | a.y | a.z;
+    return D == 7 ? any & ~(a.x & a.y & a.z) : any;
+  }
+  static __device__ __forceinline__ T add(T a, T b) {
+    const uint32_t s0 = a.x ^ b.x, c0 = a.x & b.x;
+    const uint32_t s1 = a.y ^ b.y ^ c0, c1 = maj(a.y, b.y, c0);
+    const uint32_t s2 = a.z ^ b.z ^ c1, c2 = maj(a.z, b.z, c1);
+    if constexpr (D == 7) {
+      const uint32_t k = s0 & c2;
+      return make_uint4(s0 ^ c2, s1 ^ k, s2 ^ (s1 & k), 0u);
+    } else {  // the sum is at most 8: subtract 5 from 5 on
+      const uint32_t ge = c2 | (s2 & (s1 | s0));
+      return make_uint4(s0 ^ ge, mux(ge, (s1 & s0) | c2, s1), s2 & ~ge, 0u);
+    }
+  }
+  static __device__ __forceinline__ T neg(T a) {
+    if constexpr (D == 7) return make_uint4(~a.x, ~a.y, ~a.z, 0u);
+    return make_uint4(a.z | (a.y & ~a.x), a.y, a.x & ~a.y, 0u);
+  }
+  static __device__ __forceinline__ T sub(T a, T b) { return add(a, neg(b)); }
+  static __device__ __forceinline__ T dbl(T a) {
+    if constexpr (D == 7) return make_uint4(a.z, a.x, a.y, 0u);
+    return make_uint4((a.x & a.y) | a.z, (a.x & ~a.y) | a.z, a.y & ~a.x, 0u);
+  }
+  static __device__ __forceinline__ T mulc(T a, int c) {  // c uniform
+    switch (c) {
+      case 0: return zero();
+      case 1: return a;
+      case 2: return dbl(a);
+      case 3: return D == 7 ? neg(dbl(dbl(a))) : neg(dbl(a));
+      case 4: return D == 7 ? dbl(dbl(a)) : neg(a);
+      case 5: return neg(dbl(a));
+      default: return neg(a);
+    }
+  }
+  // v + c f with c a lane's own
+  static __device__ __forceinline__ T muladd(T v, T f, int c) {
+    const uint32_t nz = lane_mask(c != 0);
+    if constexpr (D == 7) {  // c = +- 2^k: 1 2 4 | 6 5 3
+      const uint32_t m1 = lane_mask(c == 2 || c == 5), m2 = lane_mask(c == 4 || c == 3);
+      const uint32_t mn = lane_mask(c == 3 || c >= 5);
+      const uint32_t x = mux(m1, f.z, mux(m2, f.y, f.x)), y = mux(m1, f.x, mux(m2, f.z, f.y)),
+                     z = mux(m1, f.y, mux(m2, f.x, f.z));
+      return add(v, make_uint4((x ^ mn) & nz, (y ^ mn) & nz, (z ^ mn) & nz, 0u));
+    } else {
+      const uint32_t md = lane_mask(c == 2 || c == 3), mn = lane_mask(c >= 3);
+      const T g = dbl(f);
+      const T t = make_uint4(mux(md, g.x, f.x) & nz, mux(md, g.y, f.y) & nz, mux(md, g.z, f.z) & nz, 0u);
+      const T u = neg(t);
+      return add(v, make_uint4(mux(mn, u.x, t.x), t.y, mux(mn, u.z, t.z), 0u));
+    }
+  }
+  // v + c f, c uniform and not 0
+  static __device__ __forceinline__ T addmul(T v, T f, int c) {
+    if constexpr (D == 7) {
+      switch (c) {
+        case 1: return add(v, f);
+        case 2: return add(v, dbl(f));
+        case 3: return sub(v, dbl(dbl(f)));
+        case 4: return add(v, dbl(dbl(f)));
+        case 5: return sub(v, dbl(f));
+        default: return sub(v, f);
+      }
+    } else {
+      switch (c) {
+        case 1: return add(v, f);
+        case 2: return add(v, dbl(f));
+        case 3: return sub(v, dbl(f));
+        default: return sub(v, f);
+      }
+    }
+  }
+  static __device__ __forceinline__ int get(T a, int j) {
+    const int v = (int)((a.x >> j) & 1u) | (int)(((a.y >> j) & 1u) << 1) | (int)(((a.z >> j) & 1u) << 2);
+    return D == 7 && v == 7 ? 0 : v;
+  }
+  static __device__ __forceinline__ T set(T a, int j, int v) {
+    const uint32_t m = ~(1u << j);
+    return make_uint4((a.x & m) | ((uint32_t)(v & 1) << j), (a.y & m) | ((uint32_t)((v >> 1) & 1) << j),
+                      (a.z & m) | ((uint32_t)(v >> 2) << j), 0u);
+  }
+  // lanes m set to v
+  static __device__ __forceinline__ T put_at(T a, uint32_t m, int v) {
+    return make_uint4(mux(m, lane_mask(v & 1), a.x), mux(m, lane_mask(v & 2), a.y), mux(m, lane_mask(v & 4), a.z), 0u);
+  }
+  static __device__ __forceinline__ int dot(T a, T b) {  // sum of the products (d = 7: mod 7)
+    const int p0 = __popc(a.x & b.x), p1 = __popc(a.x & b.y) + __popc(a.y & b.x);
+    const int p2 = __popc(a.x & b.z) + __popc(a.y & b.y) + __popc(a.z & b.x);
+    const int p3 = __popc(a.y & b.z) + __popc(a.z & b.y), p4 = __popc(a.z & b.z);
+    return p0 + 2 * p1 + 4 * p2 + 8 * p3 + 16 * p4;
+  }
+  static __device__ __forceinline__ T shfl(T a, int l) {
+    return make_uint4(__shfl_sync(0xffffffffu, a.x, l), __shfl_sync(0xffffffffu, a.y, l),
+                      __shfl_sync(0xffffffffu, a.z, l), 0u);
+  }
+  static __device__ __forceinline__ T shfl_xor(T a, int o) {
+    return make_uint4(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
+                      __shfl_xor_sync(0xffffffffu, a.z, o), 0u);
+  }
+  static __device__ __forceinline__ void clear(T* p, int j) {
+    atomicAnd(&p->x, ~(1u << j));
+    atomicAnd(&p->y, ~(1u << j));
+    atomicAnd(&p->z, ~(1u << j));
+  }
+  static __device__ __forceinline__ void put(T* p, int j, int v) {
+    if (v & 1) atomicOr(&p->x, 1u << j);
+    if (v & 2) atomicOr(&p->y, 1u << j);
+    if (v & 4) atomicOr(&p->z, 1u << j);
+  }
+  // residues 4 i .. 4 i + 3 as bytes
+  static __device__ __forceinline__ uint32_t bytes(T a, int i) {
+    if constexpr (D == 7) {
+      const uint32_t k = ~(a.x & a.y & a.z);
+      a = make_uint4(a.x & k, a.y & k, a.z & k, 0u);
+    }
+    auto spread = [&](uint32_t w) { return (((w >> (4 * i)) & 15u) * 0x00204081u) & 0x01010101u; };
+    return spread(a.x) + 2u * spread(a.y) + 4u * spread(a.z);
+  }
+};
+
+template <>
+struct El<3> {  // two planes (planes3.cuh)
+  using T = uint2;
+  static __device__ __forceinline__ P3 p(T a) { return p3(a.x, a.y); }
+  static __device__ __forceinline__ T t(P3 a) { return make_uint2(a.p0, a.p1); }
+  static __device__ __forceinline__ T zero() { return make_uint2(0u, 0u); }
+  static __device__ __forceinline__ uint32_t nzw(T a) { return a.x | a.y; }
+  static __device__ __forceinline__ T add(T a, T b) { return t(p3_add(p(a), p(b))); }
+  static __device__ __forceinline__ T sub(T a, T b) { return t(p3_sub(p(a), p(b))); }
+  static __device__ __forceinline__ T neg(T a) { return make_uint2(a.y, a.x); }
+  static __device__ __forceinline__ T mulc(T a, int c) { return c == 0 ? zero() : c == 1 ? a : neg(a); }
+  static __device__ __forceinline__ T muladd(T v, T f, int c) {
+    const uint32_t m1 = lane_mask(c == 1), m2 = lane_mask(c == 2);
+    return add(v, make_uint2((f.x & m1) | (f.y & m2), (f.y & m1) | (f.x & m2)));
+  }
+  static __device__ __forceinline__ T addmul(T v, T f, int c) { return c == 1 ? add(v, f) : sub(v, f); }
+  static __device__ __forceinline__ int get(T a, int j) { return p3_get(p(a), j); }
+  static __device__ __forceinline__ T set(T a, int j, int v) { return t(p3_set(p(a), j, v)); }
+  static __device__ __forceinline__ T put_at(T a, uint32_t m, int v) {
+    return make_uint2(mux(m, lane_mask(v == 1), a.x), mux(m, lane_mask(v == 2), a.y));
+  }
+  static __device__ __forceinline__ int dot(T a, T b) { return p3_rsum(p3_mul(p(a), p(b))); }
+  static __device__ __forceinline__ T shfl(T a, int l) {
+    return make_uint2(__shfl_sync(0xffffffffu, a.x, l), __shfl_sync(0xffffffffu, a.y, l));
+  }
+  static __device__ __forceinline__ T shfl_xor(T a, int o) {
+    return make_uint2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
+  }
+  static __device__ __forceinline__ void clear(T* q, int j) {
+    atomicAnd(&q->x, ~(1u << j));
+    atomicAnd(&q->y, ~(1u << j));
+  }
+  static __device__ __forceinline__ void put(T* q, int j, int v) {
+    if (v == 1) atomicOr(&q->x, 1u << j);
+    if (v == 2) atomicOr(&q->y, 1u << j);
+  }
+  static __device__ __forceinline__ uint32_t bytes(T a, int i) {
+    auto spread = [&](uint32_t w) { return (((w >> (4 * i)) & 15u) * 0x00204081u) & 0x01010101u; };
+    return spread(a.x) + 2u * spread(a.y);
+  }
+};
+
+template <>
+struct El<2> {  // one plane
+  using T = uint32_t;
+  static __device__ __forceinline__ T zero() { return 0u; }
+  static __device__ __forceinline__ uint32_t nzw(T a) { return a; }
+  static __device__ __forceinline__ T add(T a, T b) { return a ^ b; }
+  static __device__ __forceinline__ T neg(T a) { return a; }
+  static __device__ __forceinline__ T mulc(T a, int c) { return c ? a : 0u; }
+  static __device__ __forceinline__ T muladd(T v, T f, int c) { return v ^ (f & (0u - (uint32_t)c)); }
+  static __device__ __forceinline__ int get(T a, int j) { return (int)((a >> j) & 1u); }
+  static __device__ __forceinline__ T set(T a, int j, int v) { return (a & ~(1u << j)) | ((uint32_t)v << j); }
+  static __device__ __forceinline__ T put_at(T a, uint32_t m, int v) { return mux(m, lane_mask(v), a); }
+  static __device__ __forceinline__ int dot(T a, T b) { return __popc(a & b); }
+  static __device__ __forceinline__ T shfl(T a, int l) { return __shfl_sync(0xffffffffu, a, l); }
+};
+
+// Rows written by one CTA of a cluster and read by another in the same launch:
+// past L1, which is not coherent between SMs.
+__device__ __forceinline__ uint32_t ldc(const uint32_t* p) { return __ldcg(p); }
+__device__ __forceinline__ uint2 ldc(const uint2* p) { return __ldcg(p); }
+__device__ __forceinline__ uint4 ldc(const uint4* p) { return __ldcg(p); }
+__device__ __forceinline__ void stc(uint32_t* p, uint32_t v) { __stcg(p, v); }
+__device__ __forceinline__ void stc(uint2* p, uint2 v) { __stcg(p, v); }
+__device__ __forceinline__ void stc(uint4* p, uint4 v) { __stcg(p, v); }
+
+template <int D>
+__device__ __forceinline__ int inverse(int x) {  // of x in [1, D)
+  if constexpr (D == 2) return 1;
+  if constexpr (D == 3) return x;
+  if constexpr (D == 5) return (0x42310 >> (4 * x)) & 15;    // 1, 3, 2, 4
+  return (0x6325410 >> (4 * x)) & 15;                         // 1, 4, 5, 2, 3, 6
+}
+
+__device__ __forceinline__ int find_tile(const RowDesc* descs, int nd, int b, bool extra) {
+  int lo = 0, hi = nd - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if ((extra ? descs[mid].x_begin : descs[mid].tile_begin) <= b) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// ---------------------------------------------------------------- raw pass
+
+// A column word of one qudit's row x_q or z_q.  Odd d: an element.  d = 2: the
+// S and T words of one position (x, y) and the row's sign exponent as far as
+// these words make it (z): a product of rows adds twice the parity of T . S'.
+template <int D>
+struct Unit : El<D> {
+  using T = typename El<D>::T;
+  static __device__ __forceinline__ T mask(T a, uint32_t m) {
+    a.x &= m;
+    a.y &= m;
+    if constexpr (D != 3) a.z &= m;
+    return a;
+  }
+  static __device__ __forceinline__ T pick(uint32_t m, T a, T b) {  // m ? a : b
+    a.x = mux(m, a.x, b.x);
+    a.y = mux(m, a.y, b.y);
+    if constexpr (D != 3) a.z = mux(m, a.z, b.z);
+    return a;
+  }
+  static __device__ __forceinline__ T bump(T a, int v) {  // the constant lane
+    return El<D>::set(a, 0, (El<D>::get(a, 0) + v) % D);
+  }
+};
+template <>
+struct Unit<2> {
+  using T = uint4;
+  static __device__ __forceinline__ T zero() { return make_uint4(0u, 0u, 0u, 0u); }
+  static __device__ __forceinline__ T add(T a, T b) {
+    return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z + b.z + 2u * (uint32_t)__popc(a.y & b.x), 0u);
+  }
+  static __device__ __forceinline__ T neg(T a) { return a; }
+  static __device__ __forceinline__ T mask(T a, uint32_t m) { return make_uint4(a.x & m, a.y & m, a.z & m, 0u); }
+  static __device__ __forceinline__ T pick(uint32_t m, T a, T b) {
+    return make_uint4(mux(m, a.x, b.x), mux(m, a.y, b.y), mux(m, a.z, b.z), 0u);
+  }
+  static __device__ __forceinline__ T bump(T a, int v) { return make_uint4(a.x, a.y, a.z + (uint32_t)v, 0u); }
+};
+
+// Element of extra row r at unit u.
+template <int D>
+__device__ __forceinline__ void dump_extra(const RowDesc& rd, int r, int u, typename Unit<D>::T v) {
+  using T = typename El<D>::T;
+  T* row = reinterpret_cast<T*>(rd.xraw) + (size_t)r * (rd.E + rd.EK);
+  if constexpr (D == 2) {
+    row[u] = v.x;
+  } else {
+    if (u < rd.E) row[u] = v;
+    else if (u >= 2 * rd.E) row[u - rd.E] = v;
+  }
+}
+
+// One op (rows.cuh: RowProgram) on unit u, the CTA's unit c (of 2^lg) of every
+// qudit.  The gates are one formula without branches -- nx = H ? +-z : x, nz =
+// H ? +-x : z + t, x_t += +-x with t = +-x (P) or +-z_t (CNOT) or 0 -- since
+// the lanes of a warp hold different gates.
+template <int D>
+__device__ __forceinline__ void raw_op(const RowDesc& rd, const uint4* o, int u, int c, int lg,
+                                       typename Unit<D>::T* x, typename Unit<D>::T* z, bool konst) {
+  using U = Unit<D>;
+  using T = typename U::T;
+  const uint32_t w = o->x;
+  const int i = ((int)(w & 0x7ffu) << lg) + c, j = ((int)((w >> 11) & 0x7ffu) << lg) + c;
+  const T xa = x[i], za = z[i], xb = x[j], zb = z[j];
+  const uint32_t mh = lane_mask(w & (kRopH | kRopHInv)), mc = lane_mask(w & (kRopC | kRopCInv));
+  const uint32_t mt = lane_mask(w & (kRopC | kRopCInv | kRopP | kRopPInv));
+  T nx, nz, nt;
+  if constexpr (D == 2) {
+    nt = U::add(U::mask(xa, mc), xb);  // A_c A_t and B_c B_t, B A for a P
+    const T t = U::mask(U::pick(mc, zb, xa), mt);
+    nz = U::pick(mh, xa, U::add(za, t));
+    nx = U::pick(mh, za, xa);
+  } else {
+    const uint32_t mneg = lane_mask(w & (kRopC | kRopPInv));
+    const T t0 = U::pick(mc, zb, xa);
+    const T t = U::mask(U::pick(mneg, U::neg(t0), t0), mt);
+    const T xn = U::neg(xa), zn = U::neg(za);
+    nt = U::add(xb, U::mask(U::pick(lane_mask(w & kRopCInv), xn, xa), mc));
+    nz = U::pick(mh, U::pick(lane_mask(w & kRopHInv), xn, xa), U::add(za, t));
+    nx = U::pick(mh, U::pick(lane_mask(w & kRopH), zn, za), xa);
+  }
+  if (konst && (w & kRopK)) {
+    nx = U::bump(nx, (int)(o->y & 7u));
+    nz = U::bump(nz, (int)((o->y >> 3) & 7u));
+  }
+  if (w & kRopM) {  // a measurement dumps its row, and leaves the generator Z_q
+    using E = typename El<D>::T;
+    const int m = (int)o->y;
+    E* row = reinterpret_cast<E*>(rd.raw) + (size_t)m * (2 * rd.E + rd.EK);
+    const int kbase = D == 2 ? rd.E : 2 * rd.E;
+    if constexpr (D == 2) {
+      if (u < rd.E) {
+        row[u] = nx.x;
+        row[rd.E + u] = nx.y;
+        rd.kpart[(size_t)m * rd.E + u] = (uint8_t)(nx.z & 3u);
+        if (u == 0) rd.ksign[m] = 0;
+      } else {
+        row[rd.E + u] = nx.x;
+      }
+    } else {
+      row[u] = nx;
+    }
+    const int v = m + (D == 2 ? 0 : 1);
+    if (m < rd.nk && u == kbase + v / L) {
+      if constexpr (D == 2)
+        nz.x |= 1u << (v % L);
+      else
+        nz = El<D>::set(nz, v % L, 1);
+    }
+    if (w & kRopReset) dump_extra<D>(rd, (int)o->z - 1, u, nz);
+  }
+  x[i] = nx;
+  z[i] = nz;
+  if (mc) x[j] = nt;
+  if (w & kRopN) {  // N1 rows of the qudit, of a CNOT's target
+    const uint32_t r = (w & kRopM) ? o->w : o->z;
+    if (r) {
+      dump_extra<D>(rd, (int)r - 1, u, nx);
+      dump_extra<D>(rd, (int)r, u, nz);
+    }
+    if (mc && o->w) {
+      dump_extra<D>(rd, (int)o->w - 1, u, nt);
+      dump_extra<D>(rd, (int)o->w, u, zb);
+    }
+  }
+}
+
+// Gates move no data between column words, so a CTA walks the layers on its
+// 2^lg units (u0 on) of every qudit alone; a layer's ops are on disjoint
+// qudits, so its (op, unit) tasks run in any order and one barrier ends it.
+// Bound by the chain of layers (two shared-memory reads, a gate and a barrier
+// each).  Threads 0 .. nt - 1 of the block; mem: raw_bytes(n, lg).
+constexpr int kRawOps = 768, kRawLayers = 255;
+
+template <int D>
+__host__ __device__ inline size_t raw_bytes(int n, int lg) {
+  return 2 * ((size_t)n << lg) * sizeof(typename Unit<D>::T) + kRawOps * sizeof(uint4) + 4 * (kRawLayers + 1);
+}
+
+template <int D>
+__device__ void raw_program(const RowDesc& rd, int u0, int lg, int nt, uint8_t* mem) {
+  using UT = typename Unit<D>::T;
+  const int t = threadIdx.x;
+  if (t >= nt) return;
+  const int n = rd.n, E = rd.E, cw = 1 << lg;
+  const int units = (D == 2 ? E : 2 * E) + rd.EK;
+  uint4* wops = reinterpret_cast<uint4*>(mem);
+  UT* x = reinterpret_cast<UT*>(wops + kRawOps);
+  UT* z = x + ((size_t)n << lg);
+  uint32_t* wlay = reinterpret_cast<uint32_t*>(z + ((size_t)n << lg));
+  auto sync = [&]() { asm volatile("bar.sync 2, %0;" ::"r"(nt) : "memory"); };
+  // stabilizer g = Z_g, destabilizer n + g = X_g
+  for (int i = t; i < (n << lg); i += nt) {
+    const int q = i >> lg, u = u0 + (i & (cw - 1)), g = q / L;
+    UT xv = Unit<D>::zero(), zv = Unit<D>::zero();
+    if constexpr (D == 2) {
+      if (u == g) xv.y = zv.x = 1u << (q % L);
+    } else {
+      if (u == E + g) xv = El<D>::set(xv, q % L, 1);
+      if (u == g) zv = El<D>::set(zv, q % L, 1);
+    }
+    x[i] = xv;
+    z[i] = zv;
+  }
+  const int c = t & (cw - 1), u = u0 + c, k0 = t >> lg, dk = nt >> lg;
+  const bool mine = u < units, konst = u == (D == 2 ? 0 : 2 * E);
+  // the ops of the layers that fit the window, in shared memory (a layer that
+  // does not fit by itself is read in place)
+  int l = 0;
+  while (l < rd.nlayers) {
+    const int nl = min(kRawLayers, rd.nlayers - l);
+    for (int i = t; i <= nl; i += nt) wlay[i] = __ldg(rd.lay + l + i);
+    sync();
+    const uint32_t w0 = wlay[0], wend = min(wlay[nl], w0 + (uint32_t)kRawOps);
+    for (uint32_t i0 = w0 + t; i0 < wend; i0 += 4 * nt) {
+      uint4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * nt < wend) v[j] = __ldg(rd.ops + i0 + j * nt);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j * nt < wend) wops[i0 + j * nt - w0] = v[j];
+    }
+    sync();
+    int i = 0;
+    uint32_t b = w0;
+    for (; i < nl; ++i) {
+      const uint32_t e = wlay[i + 1];
+      if (e > wend) {
+        if (i > 0) break;
+        if (mine)
+          for (uint32_t k = b + k0; k < e; k += dk) raw_op<D>(rd, rd.ops + k, u, c, lg, x, z, konst);
+      } else if (mine) {
+        for (uint32_t k = b + k0; k < e; k += dk) raw_op<D>(rd, wops + (k - w0), u, c, lg, x, z, konst);
+      }
+      b = e;
+      sync();
+    }
+    l += i;
+    sync();
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(256) k_rows_raw(const RowDesc* __restrict__ descs, int nd, int lg) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const RowDesc rd = descs[find_tile(descs, nd, (int)blockIdx.x, false)];
+  raw_program<D>(rd, ((int)blockIdx.x - rd.tile_begin) << lg, lg, (int)blockDim.x, smem);
+}
+
+// ---------------------------------------------------------------- panels
+
+// x mod D for x in [0, 36 * 32 + 6], without a division.
+template <int D>
+__device__ __forceinline__ int small_mod(int x) {
+  constexpr uint32_t m = (65536u + D - 1) / D;  // exact: the error x (m D - 65536) / (65536 D) stays below 1 / D
+  return x - D * (int)(((uint32_t)x * m) >> 16);
+}
+
+// The updates of one panel, staged in shared memory.
+struct PanelOps {
+  int nops;
+  int p[32], e[32], mord[32];
+  int dup[32];   // the last earlier op of the panel with the same pivot, -1 for none
+  int last[32];  // 1 when no later op of the panel has this pivot
+  uint8_t G[32][32];  // extra pass: G[h][k], what op h's factor adds at op k's pivot (0 where it does not count)
+  // chain pass: byte h of Wt[k] = W[h][k] with a = a0 W, a0 the row's entries
+  // at the pivots before the panel: W = (1 - G)^-1
+  __align__(16) uint32_t Wt[32][8];
+};
+
+// cnt elements from global memory (past L1), several loads in flight a thread.
+template <class T, class Put>
+__device__ __forceinline__ void copy_elems(const T* src, int cnt, int t, int nt, Put put) {
+  constexpr int U = sizeof(T) == 16 ? 4 : 8;
+  for (int i0 = t; i0 < cnt; i0 += U * nt) {
+    T v[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (i0 + j * nt < cnt) v[j] = ldc(src + i0 + j * nt);
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+      if (i0 + j * nt < cnt) put(i0 + j * nt, v[j]);
+  }
+}
+
+// The panel's factor rows (whole rows, kFull, or their stabilizer halves)
+// into Fs[h][cnt], cnt = 2 E or E, with the columns that a later op of the
+// panel replaces cleared (odd d), so that a row's update by the whole panel is
+// one linear combination of these rows.  The extra pass gets the pivot
+// products G first, the chain pass the matrix W from the panel's elimination.
+template <int D, bool kFull>
+__device__ void stage_panel(PanelOps& po, typename El<D>::T* Fs, const RowDesc& rd, int panel, int first,
+                            int nops) {
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int t = threadIdx.x, nt = blockDim.x;
+  const int E = rd.E, cnt = kFull ? 2 * E : E;
+  const T* opf = reinterpret_cast<const T*>(rd.opf) + (size_t)first * 2 * E;
+  if (t == 0) po.nops = nops;
+  if (t < nops) {
+    const int4 m = __ldcg(rd.opm + first + t);
+    po.p[t] = m.x;
+    po.e[t] = m.y;
+    po.mord[t] = m.z;
+  }
+  if constexpr (kFull) {
+    if constexpr (D != 2) {
+      const uint32_t* w = rd.opw + (size_t)panel * 256;
+      for (int i = t; i < nops * 8; i += nt) (&po.Wt[0][0])[i] = ldc(w + i);
+    }
+    copy_elems(opf, nops * cnt, t, nt, [&](int i, T v) { Fs[i] = v; });
+  } else {
+    for (int h = t >> 5; h < nops; h += nt >> 5)
+      copy_elems(opf + (size_t)h * 2 * E, E, t & 31, 32, [&](int i, T v) { Fs[h * E + i] = v; });
+  }
+  __syncthreads();
+  if constexpr (D != 2) {
+    if (t < nops) {
+      int dup = -1, last = 1;
+      for (int h = 0; h < nops; ++h)
+        if (po.p[h] == po.p[t]) {
+          if (h < t) dup = h;
+          if (h > t) last = 0;
+        }
+      po.dup[t] = dup;
+      po.last[t] = last;
+    }
+    if constexpr (!kFull) {
+      __syncthreads();
+      for (int i = t; i < 1024; i += nt) {
+        const int h = i >> 5, k = i & 31;
+        int g = 0;
+        if (h < k && k < nops && h > po.dup[k]) g = E_::get(Fs[h * cnt + po.p[k] / L], po.p[k] % L);
+        po.G[h][k] = (uint8_t)g;
+      }
+      __syncthreads();
+    }
+    // op h keeps nothing at the pivots of ops k >= h: those entries are
+    // replaced after it (its own are zero already)
+    for (int i = t; i < 1024; i += nt) {
+      const int h = i >> 5, k = i & 31;
+      if (h >= k || k >= nops) continue;
+      const int pe = po.p[k] / L, pl = po.p[k] % L;
+#pragma unroll
+      for (int half = 0; half < (kFull ? 2 : 1); ++half) {
+        E_::clear(&Fs[h * cnt + (half ? E + pe : pe)], pl);
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Odd d: buf[0, cnt) += sum of the panel's factor rows times ab[0, nops).  A
+// row of at most 16 elements leaves lanes over: they take their share of the
+// ops, and the partial sums meet by shuffles.
+template <int D>
+__device__ __forceinline__ void combine_row(const PanelOps& po, const typename El<D>::T* Fs, typename El<D>::T* buf,
+                                            int cnt, const int* ab) {
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int lane = threadIdx.x & 31, nops = po.nops;
+  int G = 32;
+  while (G > 1 && (G >> 1) >= cnt) G >>= 1;
+  const int K = 32 / G, part = lane / G;
+  for (int e0 = 0; e0 < cnt; e0 += G) {
+    const int e = e0 + (lane & (G - 1));
+    const bool in = e < cnt;
+    const T* f = Fs + (in ? e : 0);
+    T v = in && part == 0 ? buf[e] : E_::zero();
+    if (K == 1) {  // the multiples are uniform over the warp
+#pragma unroll 2
+      for (int h = 0; h < nops; ++h) {
+        const int a = ab[h];
+        if (a != 0) v = E_::addmul(v, f[h * cnt], a);
+      }
+    } else {
+      for (int h = part; h < nops; h += K) v = E_::muladd(v, f[h * cnt], ab[h]);
+      for (int o = G; o < 32; o <<= 1) v = E_::add(v, E_::shfl_xor(v, o));
+    }
+    if (in && part == 0) buf[e] = v;
+  }
+  __syncwarp();
+}
+
+// Odd d, one warp: a whole row in buf[0, 2 E) (shared memory) through the
+// panel's ops; kraw: its raw K elements, ab: 32 ints and 32 bytes of this warp.
+template <int D>
+__device__ __forceinline__ void update_row(const PanelOps& po, const typename El<D>::T* Fs,
+                                           typename El<D>::T* buf, const typename El<D>::T* kraw, int E, int nk,
+                                           int* ab) {
+  using E_ = El<D>;
+  const int lane = threadIdx.x & 31;
+  const int nops = po.nops;
+  int a0 = 0, om = 0;
+  if (lane < nops) {
+    const int v = po.mord[lane] + 1;
+    if (v <= nk) om = E_::get(ldc(kraw + v / L), v % L);
+  }
+  const int dup = lane < nops ? po.dup[lane] : -1;
+  const int omd = __shfl_sync(0xffffffffu, om, dup < 0 ? 0 : dup);
+  if (lane < nops) a0 = dup < 0 ? E_::get(buf[po.p[lane] / L], po.p[lane] % L) : omd;
+  uint8_t* a0b = reinterpret_cast<uint8_t*>(ab + 32);
+  a0b[lane] = (uint8_t)a0;
+  __syncwarp();
+  int av = 0;
+  if (lane < nops) {
+    const uint4* x = reinterpret_cast<const uint4*>(a0b);
+    const uint4* w = reinterpret_cast<const uint4*>(po.Wt[lane]);
+    const uint4 x0 = x[0], x1 = x[1], w0 = w[0], w1 = w[1];
+    uint32_t s = 0u;
+    s = __dp4a(x0.x, w0.x, s);
+    s = __dp4a(x0.y, w0.y, s);
+    s = __dp4a(x0.z, w0.z, s);
+    s = __dp4a(x0.w, w0.w, s);
+    s = __dp4a(x1.x, w1.x, s);
+    s = __dp4a(x1.y, w1.y, s);
+    s = __dp4a(x1.z, w1.z, s);
+    s = __dp4a(x1.w, w1.w, s);
+    av = small_mod<D>((int)s);
+    // the replaced entries: S[p] from measurement h's K column, T[p] = e a
+    if (po.last[lane]) {
+      const int pe = po.p[lane] / L, pl = po.p[lane] % L;
+      E_::clear(buf + pe, pl);
+      E_::put(buf + pe, pl, om);
+      E_::clear(buf + E + pe, pl);
+      E_::put(buf + E + pe, pl, small_mod<D>(po.e[lane] * av));
+    }
+  }
+  ab[lane] = av;
+  __syncwarp();
+  combine_row<D>(po, Fs, buf, 2 * E, ab);
+}
+
+// The same for the stabilizer half alone, through the panel's ops with
+// ordinal below `after` (the first `non` ops).
+template <int D>
+__device__ __forceinline__ void update_half_row(const PanelOps& po, const typename El<D>::T* Fs,
+                                                typename El<D>::T* buf, const typename El<D>::T* kraw, int E, int nk,
+                                                int after, int* ab) {
+  using E_ = El<D>;
+  const int lane = threadIdx.x & 31;
+  const int nops = po.nops;
+  const unsigned onm = __ballot_sync(0xffffffffu, lane < nops && po.mord[lane] < after);
+  const int non = __popc(onm);
+  int av = 0, om = 0;
+  if (lane < non) {
+    const int v = po.mord[lane] + 1;
+    if (v <= nk) om = E_::get(ldc(kraw + v / L), v % L);
+  }
+  const int dup = lane < nops ? po.dup[lane] : -1;
+  const int omd = __shfl_sync(0xffffffffu, om, dup < 0 ? 0 : dup);
+  if (lane < nops) av = dup < 0 ? E_::get(buf[po.p[lane] / L], po.p[lane] % L) : omd;
+  __syncwarp();
+  // a_h = the row's entry at op h's pivot once the ops before it are applied
+  for (int h = 0; h < non; ++h) {
+    const int a = small_mod<D>(__shfl_sync(0xffffffffu, av, h));
+    av = lane == h ? a : av + a * po.G[h][lane];
+  }
+  ab[lane] = lane < non ? av : 0;
+  // S[p] from measurement h's K column.  An op past `after` replaces nothing,
+  // but its pivot's entry is missing in the combination below (cleared): it is
+  // the value gathered above.
+  if (lane < non ? po.last[lane] != 0 : lane < nops && dup < non) {
+    const int pe = po.p[lane] / L, pl = po.p[lane] % L;
+    E_::clear(buf + pe, pl);
+    E_::put(buf + pe, pl, lane < non ? om : small_mod<D>(av));
+  }
+  __syncwarp();
+  combine_row<D>(po, Fs, buf, E, ab);
+}
+
+// d = 2: lanes of a row's group (a power of two of at least E words, at most
+// a warp), each holding the words gl, gl + G, ...
+__host__ __device__ inline int row_group(int E) {
+  int g = 1;
+  while (g < E && g < 32) g <<= 1;
+  return g;
+}
+constexpr int kRowGroupWords = 2;  // words per lane: n <= 2048
+
+// d = 2: the words of a row (S, T) in a group's registers through the panel's
+// ops with ordinal below `after`, in order; kword: the row's raw K bits of the
+// panel's ordinals (m0 on); returns what the row's sign exponent gains (T only).
+template <bool kFull>
+__device__ __forceinline__ int update_row2(const PanelOps& po, const uint32_t* Fs, uint32_t (&S)[kRowGroupWords],
+                                           uint32_t (&T)[kRowGroupWords], uint32_t kword, int m0, int E, int cnt,
+                                           int after, int gl, int G) {
+  uint32_t acc = 0u;
+  int kk = 0;
+  for (int h = 0; h < po.nops; ++h) {
+    const int mord = po.mord[h];
+    const int p = po.p[h], pw = p >> 5;
+    const uint32_t sw = pw >= G ? S[1] : S[0];
+    const uint32_t word = __shfl_sync(0xffffffffu, sw, pw & (G - 1), G);
+    if (mord >= after) continue;  // uniform over the group only: the shuffle comes first
+    const uint32_t a = (word >> (p & 31)) & 1u, om = (kword >> (mord - m0)) & 1u, mk = 0u - a;
+#pragma unroll
+    for (int i = 0; i < kRowGroupWords; ++i) {
+      const int w = gl + i * G;
+      if (w >= E) break;
+      S[i] ^= Fs[h * cnt + w] & mk;
+      if constexpr (kFull) {
+        const uint32_t ft = Fs[h * cnt + E + w] & mk;
+        T[i] ^= ft;
+        acc ^= S[i] & ft;
+      }
+      if (w == pw) {
+        S[i] = El<2>::set(S[i], p & 31, (int)om);
+        if constexpr (kFull) T[i] = El<2>::set(T[i], p & 31, (int)a);
+      }
+    }
+    if constexpr (kFull) kk += (int)a * ((po.e[h] >> 8) + 2 * (int)om);
+  }
+  if constexpr (kFull) {
+    int par = __popc(acc) & 1;
+    for (int o = G >> 1; o > 0; o >>= 1) par ^= __shfl_xor_sync(0xffffffffu, par, o);
+    kk += 2 * par;
+  }
+  return kk;
+}
+
+// d = 2: bits [m0, m0 + 31) of a row's raw K words.
+__device__ __forceinline__ uint32_t k_bits(const uint32_t* kraw, int EK, int m0) {
+  const int q = m0 >> 5;
+  const uint32_t lo = q < EK ? ldc(kraw + q) : 0u, hi = q + 1 < EK ? ldc(kraw + q + 1) : 0u;
+  return __funnelshift_r(lo, hi, m0 & 31);
+}
+
+// ---------------------------------------------------------------- chain pass
+
+template <int D>
+struct ChainSmem {
+  using T = typename El<D>::T;
+  // rows of the panel 2 E + 1 apart, so that a warp reading one word of all of
+  // them meets no bank twice
+  static __host__ __device__ size_t rows(int E) { return round_up((size_t)32 * (2 * E + 1) * sizeof(T), 16); }
+  static __host__ __device__ size_t staged(int E) { return round_up((size_t)kRowPanel * 2 * E * sizeof(T), 16); }
+  static __host__ __device__ size_t total(int E, int warps) {
+    return rows(E) + staged(E) + (size_t)E * sizeof(T) + warps * 40 * sizeof(int) + 64;
+  }
+};
+
+// State of a panel while it is eliminated.
+struct PanelState {
+  uint32_t rand;  // its random rows
+  int pv[32];     // pivot | its residue << 16 of a random row
+  int orow[32];   // the random rows in order
+  int kk[32];     // constant lane (odd d), sign exponent (d = 2)
+  int kq[32];     // d = 2: parities that the updates add to it
+  int tp[32];     // d = 2: parity of S . T of a random row
+  int dsum[32];   // T . V of a deterministic row
+  uint8_t om[32][32];  // om[j][i]: raw entry of row i in row j's K column
+  // what a warp offers for the next random row, by parity: the first
+  // generator of the row in the warp's words (x: | residue << 16, -1 for none)
+  // and its rows with a non-zero S (y), all rows' entries at that generator,
+  // d = 2: the row's parities
+  int2 cp[2][kRowWarps];
+  int ct[2][kRowWarps];
+  uint8_t ca[2][kRowWarps][32];
+  __align__(16) uint32_t Wt[32][8];  // as PanelOps::Wt
+  __align__(16) uint32_t Gt[32][8];  // byte h of Gt[o]: G[h][o]
+};
+
+__device__ __forceinline__ void bar_threads(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
+
+// The panel's rows (P, row i at i (2 E + 1), up to date) one after the other:
+// lane i holds words of row i and lane 31 those of V, so one update serves all
+// rows after a random one and V alike; warp w the words [w CE, (w + 1) CE) of
+// S and of T.  Before the barrier of a step every warp offers what it knows of
+// the next row, should that be random: its first generator there and all rows'
+// entries at it; after it the first warp with one has the pivot.  When that
+// row turns out deterministic and a later one is random, one more barrier
+// offers that one.  Deterministic rows cost a dot product and no step.
+// kSolo: one warp holds whole rows (E <= CE) and needs neither offers nor
+// barriers.
+// Bound by the step's chain of dependent instructions, not by their number.
+template <int D, int CE, bool kSolo>
+__device__ __forceinline__ void eliminate(const RowDesc& rd, int cnt, typename El<D>::T* P, typename El<D>::T* V,
+                                          PanelState& ps) {
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int E = rd.E, nw = kSolo ? 1 : (E + CE - 1) / CE, e0 = kSolo ? 0 : warp * CE;
+  if (warp >= nw) return;
+  T s[CE], t[CE];
+#pragma unroll
+  for (int i = 0; i < CE; ++i) {
+    const int e = e0 + i;
+    s[i] = t[i] = E_::zero();
+    if (e < E && lane < cnt) {
+      s[i] = P[(size_t)lane * (2 * E + 1) + e];
+      t[i] = P[(size_t)lane * (2 * E + 1) + E + e];
+    }
+    if (e < E && lane == 31) s[i] = V[e];
+  }
+  int kb = lane < cnt ? ps.kk[lane] : 0;
+  uint32_t kacc = 0u;  // d = 2: words whose parity the sign exponent gains
+  uint32_t randm = 0u;
+  int j = -1, buf = 0;
+  const uint32_t live = cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u;
+  // this lane's first generator in the warp's words, -1 for none
+  auto first = [&]() {
+    int k = -1;
+#pragma unroll
+    for (int i = CE - 1; i >= 0; --i) {
+      const uint32_t x = E_::nzw(s[i]);
+      k = x ? 32 * i + __ffs(x) - 1 : k;
+    }
+    return k;
+  };
+  // this lane's entry at generator k (uniform) of the warp's words
+  auto entry = [&](int k) {
+    T x = s[0];
+#pragma unroll
+    for (int i = 1; i < CE; ++i)
+      if ((k >> 5) == i) x = s[i];
+    return E_::get(x, k & 31);
+  };
+  // d = 2: parity of S . T | parity of kacc << 1, of row r
+  auto parities = [&](int r) {
+    int w = 0;
+    if constexpr (D == 2) {
+      uint32_t x = 0u;
+#pragma unroll
+      for (int i = 0; i < CE; ++i) x ^= s[i] & t[i];
+      w = __shfl_sync(0xffffffffu, (__popc(x) & 1) | ((__popc(kacc) & 1) << 1), r);
+    }
+    return w;
+  };
+  auto offer = [&](int key, uint32_t nzm, int r) {
+    const int k = __shfl_sync(0xffffffffu, key, r);
+    const int a = entry(k & 0x7ff);
+    ps.ca[buf][warp][lane] = (uint8_t)a;
+    const int v = __shfl_sync(0xffffffffu, a, r), ct = parities(r);
+    if (lane == 0) {
+      ps.cp[buf][warp] = make_int2(k < 0 ? -1 : (e0 * 32 + k) | (v << 16), (int)nzm);
+      if constexpr (D == 2) ps.ct[buf][warp] = ct;
+    }
+    bar_threads(32 * nw);
+  };
+  for (int step = 0; step <= cnt; ++step) {  // a random row each, the last without one
+    const uint32_t after = j < 0 ? 0xffffffffu : ~((2u << j) - 1u);
+    const int key = first();
+    const uint32_t nzm = __ballot_sync(0xffffffffu, key >= 0) & live;
+    uint32_t rnd;
+    int2 got = make_int2(-1, 0);  // lane w: warp w's offer
+    if constexpr (kSolo) {
+      rnd = nzm & after;
+    } else {
+      offer(key, nzm, (j + 1) & 31);
+      got = lane < nw ? ps.cp[buf][lane] : make_int2(-1, 0);
+      rnd = __reduce_or_sync(0xffffffffu, (uint32_t)got.y) & after;
+    }
+    const int jn = rnd ? __ffs(rnd) - 1 : cnt;
+    if (jn > j + 1) {  // deterministic rows up to it: T . V
+      int d = 0;
+#pragma unroll
+      for (int i = 0; i < CE; ++i) d += E_::dot(t[i], E_::shfl(s[i], 31));
+      if (lane > j && lane < jn) atomicAdd(&ps.dsum[lane], d);
+    }
+    if (jn >= cnt) break;
+    if (!kSolo && jn > j + 1) {
+      buf ^= 1;
+      offer(key, nzm, jn);
+      got = lane < nw ? ps.cp[buf][lane] : make_int2(-1, 0);
+    }
+    int p, val, a, tp = 0, kpar = 0;
+    if constexpr (kSolo) {
+      p = __shfl_sync(0xffffffffu, key, jn);
+      a = entry(p);
+      val = __shfl_sync(0xffffffffu, a, jn);
+      if constexpr (D == 2) {
+        const int w = parities(jn);
+        tp = w & 1;
+        kpar = w >> 1;
+      }
+    } else {
+      const int ws = __ffs(__ballot_sync(0xffffffffu, got.x >= 0)) - 1;
+      const int pv = __shfl_sync(0xffffffffu, got.x, ws);
+      a = ps.ca[buf][ws][lane];
+      p = pv & 0xffff;
+      val = pv >> 16;
+      if constexpr (D == 2) {
+        const int w = lane < nw ? ps.ct[buf][lane] : 0;
+        tp = __popc(__ballot_sync(0xffffffffu, w & 1)) & 1;
+        kpar = __popc(__ballot_sync(0xffffffffu, w & 2)) & 1;
+      }
+    }
+    const int e = inverse<D>(val), pe = p / L, pl = p % L;
+    const int kj = __shfl_sync(0xffffffffu, kb, jn);
+    const int nv = D == 2 ? ((kj + 2 * kpar + tp) >> 1) & 1 : kj;
+    const int om = lane == 31 ? nv : ps.om[jn][lane];
+    const bool act = lane > jn && (lane < cnt || lane == 31);
+    const int c = !act ? 0 : D == 2 ? a : small_mod<D>((D - e) * a);
+    const int ta = D == 2 ? a : small_mod<D>(e * a);
+    if (D == 2 && c) kb += tp + 2 * om;
+#pragma unroll
+    for (int i = 0; i < CE; ++i) {
+      const T fs = E_::shfl(s[i], jn), ft = E_::shfl(t[i], jn);
+      T ns = E_::muladd(s[i], fs, c), nt = E_::muladd(t[i], ft, c);
+      const uint32_t at = e0 + i == pe ? 1u << pl : 0u;  // the pivot's lane
+      if constexpr (D == 2) kacc ^= ns & ft & ~at & (0u - (uint32_t)c);
+      s[i] = E_::put_at(ns, act ? at : 0u, om);
+      t[i] = E_::put_at(nt, act ? at : 0u, ta);
+    }
+    if (warp == 0 && lane == 0) {
+      ps.pv[jn] = p | (val << 16);
+      ps.orow[__popc(randm)] = jn;
+      if constexpr (D == 2) ps.tp[jn] = tp;
+    }
+    randm |= 1u << jn;
+    j = jn;
+    buf ^= 1;
+  }
+#pragma unroll
+  for (int i = 0; i < CE; ++i) {
+    const int e = e0 + i;
+    if (e < E && lane < cnt) {
+      P[(size_t)lane * (2 * E + 1) + e] = s[i];
+      P[(size_t)lane * (2 * E + 1) + E + e] = t[i];
+    }
+    if (e < E && lane == 31) V[e] = s[i];
+  }
+  if constexpr (D == 2) {
+    if (__popc(kacc) & 1) atomicAdd(&ps.kq[lane], 1);
+  }
+  if (warp == 0) {
+    if (lane < cnt) ps.kk[lane] = kb;
+    if (lane == 0) ps.rand = randm;
+  }
+}
+
+// Element e of a trace row of rowb bytes: a word (d = 2) or 32 bytes.
+template <int D>
+__device__ __forceinline__ void trace_elem(uint8_t* row, int e, typename El<D>::T v, int rowb) {
+  if constexpr (D == 2) {
+    reinterpret_cast<uint32_t*>(row)[e] = v;
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (32 * e + 16 * h < rowb)
+        reinterpret_cast<uint4*>(row)[2 * e + h] =
+            make_uint4(El<D>::bytes(v, 4 * h), El<D>::bytes(v, 4 * h + 1), El<D>::bytes(v, 4 * h + 2),
+                       El<D>::bytes(v, 4 * h + 3));
+  }
+}
+
+// The rest of a trace row after E elements.
+template <int D>
+__device__ __forceinline__ void trace_pad(uint8_t* row, int E, int rowb, int lane) {
+  constexpr int kB = D == 2 ? 4 : L;  // bytes written per element
+  for (int b = E * kB + 4 * lane; b < rowb; b += 128) *reinterpret_cast<uint32_t*>(row + b) = 0u;
+}
+
+// Eliminates panel k (its rows in P, up to date) and writes its trace records
+// and the updates that its random rows are to later rows.
+template <int D, int CE, bool kSolo>
+__device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typename El<D>::T* V, PanelState& ps,
+                             int& nopsum) {
+  const int nwp = (int)(blockDim.x >> 5);
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int E = rd.E, m0 = k * kRowPanel, cnt = min(kRowPanel, rd.nm - m0);
+  eliminate<D, CE, kSolo>(rd, cnt, P, V, ps);
+  __syncthreads();
+  const uint32_t randm = ps.rand;
+  const int nops = __popc(randm);
+  if constexpr (D != 2) {
+    // G[h][o] = -e_h times op h's entry at op o's pivot, nothing where an op
+    // from h on has replaced it before o (rows by op number: orow)
+    for (int i = threadIdx.x; i < 1024; i += 32 * nwp) {
+      const int o = i >> 5, h = i & 31;
+      int g = 0;
+      if (h < o && o < nops) {
+        const int ro = ps.orow[o], rh = ps.orow[h];
+        const int p = ps.pv[ro] & 0xffff;
+        bool kept = true;
+        for (int q = h; q < o; ++q) kept &= (ps.pv[ps.orow[q]] & 0xffff) != p;
+        if (kept)
+          g = small_mod<D>((D - inverse<D>(ps.pv[rh] >> 16)) * E_::get(P[(size_t)rh * (2 * E + 1) + p / L], p % L));
+      }
+      reinterpret_cast<uint8_t*>(ps.Gt[o])[h] = (uint8_t)g;
+    }
+    __syncthreads();
+    // W = (1 - G)^-1 by columns, in the last warp: W[i][o] = sum_h W[i][h] G[h][o]
+    if (warp == nwp - 1) {
+      uint32_t wr[8] = {};
+      for (int o = 0; o < nops; ++o) {
+        const uint4 g0 = *reinterpret_cast<const uint4*>(ps.Gt[o]), g1 = *reinterpret_cast<const uint4*>(ps.Gt[o] + 4);
+        uint32_t a = __dp4a(wr[0], g0.x, 0u), b = __dp4a(wr[4], g1.x, 0u);
+        a = __dp4a(wr[1], g0.y, a);
+        b = __dp4a(wr[5], g1.y, b);
+        a = __dp4a(wr[2], g0.z, a);
+        b = __dp4a(wr[6], g1.z, b);
+        a = __dp4a(wr[3], g0.w, a);
+        b = __dp4a(wr[7], g1.w, b);
+        const int v = lane == o ? 1 : lane < o ? small_mod<D>((int)(a + b)) : 0;
+        const uint32_t vb = (uint32_t)v << (8 * (o & 3));
+#pragma unroll
+        for (int q = 0; q < 8; ++q) wr[q] |= q == o >> 2 ? vb : 0u;
+        reinterpret_cast<uint8_t*>(ps.Wt[o])[lane] = (uint8_t)v;
+      }
+      __syncwarp();
+      uint32_t* w = rd.opw + (size_t)k * 256;
+      for (int i = lane; i < 8 * nops; i += 32) stc(w + i, (&ps.Wt[0][0])[i]);
+    }
+  }
+  // the panel's trace records and updates
+  const int writers = D == 2 ? nwp : nwp - 1;
+  for (int i = warp; i < cnt && warp < writers; i += writers) {
+    const int m = m0 + i;
+    const T* row = P + (size_t)i * (2 * E + 1);
+    uint8_t* out = rd.mrow + (size_t)m * 2 * rd.rowb;
+    const uint32_t info = __ldg(rd.minfo + m);
+    const uint32_t nord = info & 0x7fffffffu, reset = info >> 31;
+    if ((randm >> i) & 1u) {
+      const int p = ps.pv[i] & 0xffff, e = inverse<D>(ps.pv[i] >> 16), pe = p / L, pl = p % L;
+      const int h = nopsum + __popc(randm & ((1u << i) - 1u));
+      T* f = reinterpret_cast<T*>(rd.opf) + (size_t)h * 2 * E;
+      for (int w = lane; w < 2 * E; w += 32) {
+        T v = row[w];
+        if (w == pe || w == E + pe) v = E_::set(v, pl, 0);
+        stc(f + w, E_::mulc(v, D == 2 ? 1 : D - e));
+        if (w < E) trace_elem<D>(out, w, E_::neg(v), rd.rowb);
+      }
+      if (lane == 0) {
+        __stcg(rd.opm + h, make_int4(p, D == 2 ? 1 | (ps.tp[i] << 8) : e, m, 0));
+        rd.mhdr[m] = make_uint4(2u * reset | (D == 2 ? 0u : (uint32_t)e << 8), (uint32_t)p, nord, 0u);
+      }
+    } else {
+      for (int w = lane; w < E; w += 32) trace_elem<D>(out, w, row[E + w], rd.rowb);
+      const int det = D == 2 ? 2 * (((ps.kk[i] + 2 * ps.kq[i]) >> 1) + ps.dsum[i] & 1)
+                             : (ps.dsum[i] - ps.kk[i] + D) % D;
+      if (lane == 0) rd.mhdr[m] = make_uint4(2u * reset | 1u, 0u, nord, (uint32_t)det);
+    }
+    trace_pad<D>(out, E, rd.rowb, lane);
+  }
+  if (threadIdx.x == 0) {
+    if (k == 0) __stcg(rd.pop, 0);
+    __stcg(rd.pop + k + 1, nopsum + __popc(randm));
+  }
+  nopsum += __popc(randm);
+  __syncthreads();
+}
+
+// One program per cluster of C CTAs.  rawt > 0: the raw pass first, 2^lg units
+// a CTA on rawt threads.  CTA 0 eliminates panel after panel (32
+// rows in shared memory); the panel's updates then go to the rows after it:
+// with C = 1 by this CTA itself, with more the next panel's rows by CTA 0 (it
+// eliminates them next) and the others' by the other CTAs meanwhile, so one
+// cluster barrier per panel is all they wait for.
+template <int D, int CE, bool kSolo>
+__global__ void __launch_bounds__(32 * kRowWarps) k_rows_chain(const RowDesc* __restrict__ descs, int nd, int C, int rawt,
+                                                               int lg) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ PanelOps po;
+  __shared__ PanelState ps;
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int r = C > 1 ? (int)cluster_rank() : 0;
+  const int pi = (int)blockIdx.x / C;
+  if (pi >= nd) return;  // the whole cluster
+  const RowDesc rd = descs[pi];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwp = (int)(blockDim.x >> 5);
+  const int E = rd.E, RS = 2 * E + rd.EK;
+  T* P = reinterpret_cast<T*>(smem);
+  T* Fs = reinterpret_cast<T*>(smem + ChainSmem<D>::rows(E));
+  T* V = reinterpret_cast<T*>(smem + ChainSmem<D>::rows(E) + ChainSmem<D>::staged(E));
+  int* ab = reinterpret_cast<int*>(smem + round_up(ChainSmem<D>::rows(E) + ChainSmem<D>::staged(E) +
+                                                  (size_t)E * sizeof(T), 16)) + 40 * warp;
+  T* raw = reinterpret_cast<T*>(rd.raw);
+  if (rawt > 0) {
+    raw_program<D>(rd, r << lg, lg, rawt, smem);
+    __syncthreads();
+    if (C > 1) cluster_sync_all();
+  }
+  const int panels = (rd.nm + kRowPanel - 1) / kRowPanel;
+  const int G = row_group(E), gl = lane & (G - 1), gpw = 32 / G;  // d = 2: rows per warp
+  int nops = 0;
+  const int PS = 2 * E + 1;
+  // panel k's rows into P, with their entries in each other's K columns and
+  // their constants (odd d) or sign exponents (d = 2)
+  auto load_panel = [&](int k) {
+    const int m0 = k * kRowPanel, cnt = min(kRowPanel, rd.nm - m0);
+    for (int i = warp; i < 32; i += nwp) {
+      int om = 0, kk = 0;
+      if (i < cnt) {
+        const T* src = raw + (size_t)(m0 + i) * RS;
+        const int v = m0 + lane + (D == 2 ? 0 : 1);
+        T kw = E_::zero();
+        if (m0 + lane < rd.nk && lane < i) kw = ldc(src + 2 * E + v / L);
+        if constexpr (D == 2) {
+          for (int w = lane; w < E; w += 32) kk += __ldcg(rd.kpart + (size_t)(m0 + i) * E + w);
+          kk = __reduce_add_sync(0xffffffffu, kk) + (int)__ldcg(rd.ksign + m0 + i);
+        } else {
+          kk = E_::get(ldc(src + 2 * E), 0);
+        }
+        copy_elems(src, 2 * E, lane, 32, [&](int e, T x) { P[(size_t)i * PS + e] = x; });
+        om = E_::get(kw, v % L);
+      }
+      ps.om[lane][i] = (uint8_t)om;
+      if (lane == 0) {
+        ps.kk[i] = D == 2 ? kk & 3 : kk;
+        ps.kq[i] = ps.dsum[i] = 0;
+      }
+    }
+    __syncthreads();
+  };
+  if (r == 0) {
+    for (int e = threadIdx.x; e < E; e += blockDim.x) V[e] = E_::zero();
+    load_panel(0);
+    factor_panel<D, CE, kSolo>(rd, 0, P, V, ps, nops);
+  }
+  for (int k = 0; k + 1 < panels; ++k) {
+    if (C > 1) cluster_sync_all(); else __syncthreads();
+    const int first = __ldcg(rd.pop + k), cnt = __ldcg(rd.pop + k + 1) - first;
+    const int b1 = (k + 1) * kRowPanel;
+    if (cnt > 0) stage_panel<D, true>(po, Fs, rd, k, first, cnt);
+    if (C > 1 && r == 0) {
+      load_panel(k + 1);
+      if (cnt > 0) {
+        const int rows = min(kRowPanel, rd.nm - b1);
+        if constexpr (D == 2) {
+          for (int i0 = warp * gpw; i0 < rows; i0 += nwp * gpw) {
+            const int i = i0 + lane / G;
+            const bool in = i < rows;
+            uint32_t S[kRowGroupWords] = {}, Tt[kRowGroupWords] = {};
+            T* buf = P + (size_t)i * PS;
+#pragma unroll
+            for (int h = 0; h < kRowGroupWords; ++h) {
+              const int w = gl + h * G;
+              if (in && w < E) {
+                S[h] = buf[w];
+                Tt[h] = buf[E + w];
+              }
+            }
+            const uint32_t kw = in ? k_bits(raw + (size_t)(b1 + i) * RS + 2 * E, rd.EK, k * kRowPanel) : 0u;
+            const int dk = update_row2<true>(po, Fs, S, Tt, kw, k * kRowPanel, E, 2 * E, INT_MAX, gl, G);
+#pragma unroll
+            for (int h = 0; h < kRowGroupWords; ++h) {
+              const int w = gl + h * G;
+              if (in && w < E) {
+                buf[w] = S[h];
+                buf[E + w] = Tt[h];
+              }
+            }
+            if (in && gl == 0) ps.kk[i] = (ps.kk[i] + dk) & 3;
+          }
+        } else {
+          for (int i = warp; i < rows; i += nwp)
+            update_row<D>(po, Fs, P + (size_t)i * PS, raw + (size_t)(b1 + i) * RS + 2 * E, E, rd.nk, ab);
+        }
+        __syncthreads();
+      }
+      factor_panel<D, CE, kSolo>(rd, k + 1, P, V, ps, nops);
+    } else {
+      if (cnt > 0) {
+        // rows of the panels after the next (of all later ones with C = 1)
+        const int m0 = C > 1 ? b1 + kRowPanel : b1;
+        const int w0 = C > 1 ? (r - 1) * nwp + warp : warp, dw = C > 1 ? (C - 1) * nwp : nwp;
+        if constexpr (D == 2) {
+          for (int i0 = m0 + w0 * gpw; i0 < rd.nm; i0 += dw * gpw) {
+            const int i = i0 + lane / G;
+            const bool in = i < rd.nm;
+            uint32_t S[kRowGroupWords] = {}, Tt[kRowGroupWords] = {};
+            T* row = raw + (size_t)i * RS;
+#pragma unroll
+            for (int h = 0; h < kRowGroupWords; ++h) {
+              const int w = gl + h * G;
+              if (in && w < E) {
+                S[h] = ldc(row + w);
+                Tt[h] = ldc(row + E + w);
+              }
+            }
+            const uint32_t kw = in ? k_bits(row + 2 * E, rd.EK, k * kRowPanel) : 0u;
+            const int dk = update_row2<true>(po, Fs, S, Tt, kw, k * kRowPanel, E, 2 * E, INT_MAX, gl, G);
+#pragma unroll
+            for (int h = 0; h < kRowGroupWords; ++h) {
+              const int w = gl + h * G;
+              if (in && w < E) {
+                stc(row + w, S[h]);
+                stc(row + E + w, Tt[h]);
+              }
+            }
+            if (in && gl == 0) __stcg(rd.ksign + i, (uint8_t)((__ldcg(rd.ksign + i) + dk) & 3));
+          }
+        } else {
+          T* buf = P + (size_t)warp * PS;
+          for (int i = m0 + w0; i < rd.nm; i += dw) {
+            T* row = raw + (size_t)i * RS;
+            copy_elems(row, 2 * E, lane, 32, [&](int e, T x) { buf[e] = x; });
+            __syncwarp();
+            update_row<D>(po, Fs, buf, row + 2 * E, E, rd.nk, ab);
+            for (int e = lane; e < 2 * E; e += 32) stc(row + e, buf[e]);
+            __syncwarp();
+          }
+        }
+      }
+      if (C == 1) {
+        __syncthreads();
+        load_panel(k + 1);
+        factor_panel<D, CE, kSolo>(rd, k + 1, P, V, ps, nops);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------- extra pass
+
+// Rows of an extra-pass CTA: d = 2 one per lane group, odd d one per warp.
+template <int D>
+__host__ __device__ inline int extra_rows(int E) {
+  return D == 2 ? kRowWarps * (32 / row_group(E)) : kRowWarps;
+}
+
+template <int D>
+struct ExtraSmem {
+  using T = typename El<D>::T;
+  static __host__ __device__ size_t staged(int E) { return (size_t)kRowPanel * E * sizeof(T); }
+  static __host__ __device__ size_t total(int E) {
+    return staged(E) + (size_t)kRowWarps * E * sizeof(T) + kRowWarps * 40 * sizeof(int) + 64;
+  }
+};
+
+__device__ __forceinline__ uint8_t* extra_row(const RowDesc& rd, uint32_t who) {
+  const uint32_t kind = who >> 30, i = who & 0x3fffffffu;
+  if (kind == 0) return rd.mrow + ((size_t)i * 2 + 1) * rd.rowb;
+  return rd.nrow + ((size_t)i * 2 + (kind == 2 ? 1 : 0)) * rd.rowb;
+}
+
+// Stabilizer halves of the rows that only the phase pass reads, through every
+// update that precedes them.
+template <int D>
+__global__ void __launch_bounds__(32 * kRowWarps) k_rows_extra(const RowDesc* __restrict__ descs, int nd) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ PanelOps po;
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const RowDesc rd = descs[find_tile(descs, nd, (int)blockIdx.x, true)];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int E = rd.E, XS = E + rd.EK;
+  const int G = D == 2 ? row_group(E) : 32, gl = lane & (G - 1);
+  const int x0 = ((int)blockIdx.x - rd.x_begin) * extra_rows<D>(E);
+  const int i = x0 + warp * (32 / G) + lane / G;
+  const bool in = i < rd.nx;
+  const uint2 info = in ? __ldg(rd.xinfo + i) : make_uint2(0u, 0u);
+  const int after = (int)info.x;
+  const T* src = reinterpret_cast<const T*>(rd.xraw) + (size_t)(in ? i : 0) * XS;
+  T* Fs = reinterpret_cast<T*>(smem);
+  T* buf = reinterpret_cast<T*>(smem + ExtraSmem<D>::staged(E)) + (size_t)warp * E;
+  int* ab = reinterpret_cast<int*>(smem + round_up(ExtraSmem<D>::staged(E) + (size_t)kRowWarps * E * sizeof(T), 16)) +
+            40 * warp;
+  uint32_t S[kRowGroupWords] = {}, none[kRowGroupWords] = {};
+  if constexpr (D == 2) {
+#pragma unroll
+    for (int h = 0; h < kRowGroupWords; ++h)
+      if (in && gl + h * G < E) S[h] = src[gl + h * G];
+  } else {
+    for (int e = lane; e < E; e += 32) buf[e] = in ? src[e] : E_::zero();
+    __syncwarp();
+  }
+  // rows are in program order: the CTA's last row takes the most updates
+  const int most = (int)__ldg(&rd.xinfo[min(rd.nx, x0 + extra_rows<D>(E)) - 1].x);
+  for (int k = 0; k * kRowPanel < most; ++k) {
+    const int first = rd.pop[k], cnt = rd.pop[k + 1] - first;
+    if (cnt == 0) continue;
+    __syncthreads();
+    stage_panel<D, false>(po, Fs, rd, k, first, cnt);
+    if constexpr (D == 2) {
+      const uint32_t kw = in ? k_bits(src + E, rd.EK, k * kRowPanel) : 0u;
+      update_row2<false>(po, Fs, S, none, kw, k * kRowPanel, E, E, after, gl, G);
+    } else {
+      if (in && after > k * kRowPanel) update_half_row<D>(po, Fs, buf, src + E, E, rd.nk, after, ab);
+    }
+  }
+  if (!in) return;
+  uint8_t* out = extra_row(rd, info.y);
+  if constexpr (D == 2) {
+#pragma unroll
+    for (int h = 0; h < kRowGroupWords; ++h)
+      if (gl + h * G < E) reinterpret_cast<uint32_t*>(out)[gl + h * G] = S[h];
+    for (int w = E + gl; 4 * w < rd.rowb; w += G) reinterpret_cast<uint32_t*>(out)[w] = 0u;
+  } else {
+    for (int e = lane; e < E; e += 32) trace_elem<D>(out, e, buf[e], rd.rowb);
+    trace_pad<D>(out, E, rd.rowb, lane);
+  }
+}
+
+template <int D>
+size_t raw_smem(int n, int lg) {
+  return round16(raw_bytes<D>(n, lg));
+}
+
+// Chain-pass instances, by row_slice.
+template <class Fn>
+cudaError_t for_slice(int slice, Fn fn) {
+  using std::integral_constant;
+  switch (slice) {
+    case 1: return fn(integral_constant<int, 1>(), std::true_type());
+    case 2: return fn(integral_constant<int, 2>(), std::true_type());
+    case 4: return fn(integral_constant<int, 4>(), std::true_type());
+    case 17: return fn(integral_constant<int, 1>(), std::false_type());
+    case 18: return fn(integral_constant<int, 2>(), std::false_type());
+    default: return fn(integral_constant<int, 4>(), std::false_type());
+  }
+}
+constexpr int kSlices[] = {1, 2, 4, 17, 18, 20};
+
+template <int D>
+cudaError_t set_smem(int optin) {
+  cudaError_t e = set_dynamic_smem(k_rows_raw<D>, optin);
+  for (int sl : kSlices)
+    if (e == cudaSuccess)
+      e = for_slice(sl, [&](auto c, auto solo) { return set_dynamic_smem(k_rows_chain<D, c.value, solo.value>, optin); });
+  return e != cudaSuccess ? e : set_dynamic_smem(k_rows_extra<D>, optin);
+}
+
+template <int D>
+cudaError_t chain(int slice, int C, int block, int rawt, int lg, size_t smem, cudaStream_t s, const RowDesc* descs,
+                  int nd) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(C * nd));
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute a;
+  a.id = cudaLaunchAttributeClusterDimension;
+  a.val.clusterDim.x = (unsigned)C;
+  a.val.clusterDim.y = a.val.clusterDim.z = 1;
+  cfg.attrs = &a;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return for_slice(slice, [&](auto c, auto solo) {
+    return cudaLaunchKernelEx(&cfg, k_rows_chain<D, c.value, solo.value>, descs, nd, C, rawt, lg);
+  });
+}
+
+}  // namespace
+
+// The instance of one d, as rows.cuh's launchers see it.
+template <int D>
+RowOps row_ops() {
+  RowOps o;
+  o.set_smem = set_smem<D>;
+  o.raw_smem = raw_smem<D>;
+  o.chain_smem = [](int n, int block) { return (size_t)round16(ChainSmem<D>::total(row_elems(n), block / 32)); };
+  o.extra_smem = [](int n) { return (size_t)round16(ExtraSmem<D>::total(row_elems(n))); };
+  o.extra_per_cta = [](int n) { return extra_rows<D>(row_elems(n)); };
+  o.raw = [](int tiles, int block, int lg, size_t smem, cudaStream_t s, const RowDesc* descs, int nd) {
+    k_rows_raw<D><<<tiles, block, smem, s>>>(descs, nd, lg);
+  };
+  o.chain = chain<D>;
+  o.extra = [](int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd) {
+    k_rows_extra<D><<<ctas, 32 * kRowWarps, smem, s>>>(descs, nd);
+  };
+  return o;
+}
+
+}  // namespace sdim

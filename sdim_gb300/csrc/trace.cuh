@@ -49,7 +49,7 @@ struct TraceDesc {
   // carry flag 4 and the slot until the header pass adds the cross term
   uint32_t* snap;
   int nsnap;
-  long long coin_begin;  // first coin-pass item of this program
+  long long coin_begin;  // first coin-pass block of this program
   int nsteps;
   int nwins;
   int nm;      // measurements (M and RESET)
@@ -60,6 +60,7 @@ struct TraceDesc {
   int spl;     // shots per lane of the phase pass (item_begin counts groups of 32 spl)
   int nw;      // words per record column (a power of two >= 2)
   int nused;   // N1 ordinals before the last measurement
+  int rows;    // 1: the row form (rows.cuh) writes this trace, the tableau pass skips it
 };
 
 __host__ __device__ inline size_t round_up(size_t b, size_t a) { return (b + a - 1) / a * a; }
@@ -83,6 +84,12 @@ __host__ __device__ inline size_t trace_bytes(int nm, int nn1, int tw) {
 constexpr int kCoinChunk = 32;
 // Chunks one coin-pass thread fills (one byte of the chunk map).
 constexpr int kCoinChunksPerItem = 8;
+// Threads (shots) of a coin-pass block.
+constexpr int kCoinThreads = 256;
+// Coin-pass blocks of a program: a tile of shots by a byte of chunks each.
+inline long long coin_blocks(long long nchunk, long long nshots) {
+  return (nchunk + kCoinChunksPerItem - 1) / kCoinChunksPerItem * ((nshots + kCoinThreads - 1) / kCoinThreads);
+}
 
 // Bytes of the fire masks and of the chunk map of one program (each
 // 256-byte aligned).
@@ -164,14 +171,12 @@ void launch_trace_pass(int threads, int grid, size_t smem, cudaStream_t s, const
 // iters x 8 blocks keyed by seeds[thread % 256]; results folded into sink[256].
 void launch_philox_probe(int grid, cudaStream_t s, const unsigned long long* seeds, int iters, uint4* sink);
 
-// Coin pass: the fire masks of every program of descs with masks (items:
-// (chunk group, shot) pairs numbered through coin_begin).
-void launch_coin_pass(int grid, int block, size_t smem, cudaStream_t s, const TraceDesc* descs, int ndesc,
-                      long long total);
+// Coin pass: the fire masks of every program of descs with masks (blocks
+// numbered through coin_begin).
+void launch_coin_pass(int grid, cudaStream_t s, const TraceDesc* descs, int ndesc);
 
-// Dynamic shared memory every coin-pass block requests (and leaves unused):
-// with a few x / z CTAs running alongside, those claim the rest of their SM's
-// shared memory so that no coin block lands beside them.
+// Shared memory of a coin-pass block, which keeps it off an SM whose shared
+// memory an x / z CTA has claimed.
 constexpr size_t kCoinFenceSmem = 8192;
 
 // Phase pass: spl (1 or 2) shots per lane, one warp per group of 32 spl

@@ -987,43 +987,128 @@ __device__ __forceinline__ void phase_program_multi(const TraceDesc* __restrict_
   }
 }
 
-// Coin pass item it of td: shot it % nshots, chunks kCoinChunksPerItem *
-// (it / nshots) onwards.  For every fired N1 (rare) the Pauli is drawn here,
-// so masks[c * nshots + s] = (x mask, z mask): bit i of .x set when ordinal
-// 32 c + i applies X^a with a odd (the phase update reads z_q), of .y when it
-// applies Z^b with b odd (reads x_q); an N1 with probability 0 never fires.
-// The item's byte of the chunk map (byte cg % 4 of word cg / 4) marks which
-// of its chunks have a non-zero pair.
-__device__ __forceinline__ void coin_item(const TraceDesc* __restrict__ tdp, long long it) {
-  const int nshots = tdp->c.nshots;
-  const long long cg = it / nshots;
-  const int rel = (int)(it - cg * nshots);
-  const long long shot = tdp->c.shot0 + rel;
+// Philox rounds shared between the (ordinal, shot) pairs of a coin-pass block.
+// With the counter (ordinal, shot_lo, shot_hi, domain) the first round's
+// multiplies see the ordinal and shot_hi alone, the second's the shot alone and
+// the ordinal alone, and one of the third's the ordinal alone: five of a
+// block's twenty multiplies, which are what bounds the pass.  They are made
+// once per ordinal (CoinOrdinal, in shared memory) and once per shot.
+struct CoinOrdinal {
+  uint32_t c3;      // what the ordinal adds to c2 of round 3
+  uint32_t r0, r2;  // what it adds to round 3's first and third word
+  uint32_t r3;      // round 3's fourth word
+};
+__device__ __forceinline__ CoinOrdinal coin_ordinal(const PhiloxKeys& K, uint32_t ord, uint32_t shot_hi, uint32_t domain) {
+  const uint32_t kM0 = 0xD2511F53u, kM1 = 0xCD9E8D57u;
+  const uint32_t c2 = __umulhi(kM0, ord) ^ domain ^ K.k1[0];           // round 1
+  const uint32_t c0 = __umulhi(kM1, c2) ^ (kM1 * shot_hi) ^ K.k0[1];   // round 2
+  CoinOrdinal o;
+  o.c3 = (kM0 * ord) ^ K.k1[1];
+  o.r0 = (kM1 * c2) ^ K.k0[2];
+  o.r2 = __umulhi(kM0, c0) ^ K.k1[2];
+  o.r3 = kM0 * c0;
+  return o;
+}
+// The shot's part: (hi, lo) of round 2's product.
+__device__ __forceinline__ uint2 coin_shot(const PhiloxKeys& K, uint32_t shot_lo, uint32_t shot_hi) {
+  const uint32_t c0 = __umulhi(0xCD9E8D57u, shot_hi) ^ shot_lo ^ K.k0[0];
+  return make_uint2(__umulhi(0xD2511F53u, c0), 0xD2511F53u * c0);
+}
+// Block (ordinal, shot): rounds 3 (one multiply) to 10.
+__device__ __forceinline__ uint4 coin_block(const PhiloxKeys& K, const CoinOrdinal& o, uint2 sh) {
+  unsigned long long p0, p1;
+  asm("mul.wide.u32 %0, %1, %2;" : "=l"(p1) : "r"(sh.x ^ o.c3), "r"(0xCD9E8D57u));
+  uint4 c = make_uint4((uint32_t)(p1 >> 32) ^ o.r0, (uint32_t)p1, o.r2 ^ sh.y, o.r3);
+#pragma unroll
+  for (int r = 3; r < 10; ++r) {
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(p0) : "r"(c.x), "r"(0xD2511F53u));
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(p1) : "r"(c.z), "r"(0xCD9E8D57u));
+    c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ K.k0[r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ K.k1[r],
+                   (uint32_t)p0);
+  }
+  return c;
+}
+
+// Shared memory of a coin-pass block: per Philox block of its ordinals the
+// shared rounds and the four thresholds, and each thread's fire masks.
+struct CoinSmem {
+  CoinOrdinal ord[kCoinChunksPerItem * kCoinChunk / 4];
+  uint4 thr[kCoinChunksPerItem * kCoinChunk / 4];
+  uint32_t fire[kCoinChunksPerItem][kCoinThreads];
+};
+
+// Coin-pass block `blk` of td: kCoinThreads shots from kCoinThreads (blk %
+// tiles) on, chunks kCoinChunksPerItem (blk / tiles) onwards.  For every fired
+// N1 (rare) the Pauli is drawn here, so masks[c * nshots + s] = (x mask, z
+// mask): bit i of .x set when ordinal 32 c + i applies X^a with a odd (the
+// phase update reads z_q), of .y when it applies Z^b with b odd (reads x_q);
+// an N1 with probability 0 never fires.  The thread's byte of the chunk map
+// (byte cg % 4 of word cg / 4) marks which of its chunks have a non-zero pair.
+// The Paulis are drawn after all chunks' coins: a warp then runs as many
+// draws as its busiest lane has fires, not one per chunk with a fire in it.
+__device__ __forceinline__ void coin_tile(const TraceDesc* __restrict__ tdp, long long blk, CoinSmem& sm) {
+  const int nshots = tdp->c.nshots, t = threadIdx.x;
+  const int tiles = (nshots + kCoinThreads - 1) / kCoinThreads;
+  const int cg = (int)(blk / tiles), rel = (int)(blk - (long long)cg * tiles) * kCoinThreads + t;
+  const unsigned long long shot = (unsigned long long)(tdp->c.shot0 + rel);
   const unsigned long long seed = tdp->c.seed;
   const PhiloxKeys K(seed);
-  const uint32_t* nthr = tdp->nthr;
-  uint2* out = reinterpret_cast<uint2*>(tdp->masks) + rel;
   const int nchunk = tdp->nchunk;
-  const int c0 = (int)cg * kCoinChunksPerItem;
-  const int c1 = min(nchunk, c0 + kCoinChunksPerItem);
+  const int c0 = cg * kCoinChunksPerItem, nc = min(nchunk - c0, kCoinChunksPerItem);
+  const unsigned long long first = shot - t;
+  // one shot_hi in the tile, or (a tile across a multiple of 2^32) every block whole
+  const bool same = (first >> 32) == ((first + kCoinThreads - 1) >> 32);
+  for (int i = t; i < nc * (kCoinChunk / 4); i += kCoinThreads) {
+    sm.ord[i] = coin_ordinal(K, (uint32_t)c0 * (kCoinChunk / 4) + i, (uint32_t)(first >> 32), 1u);
+    sm.thr[i] = __ldg(reinterpret_cast<const uint4*>(tdp->nthr + (size_t)c0 * kCoinChunk) + i);
+  }
+  __syncthreads();
+  if (rel >= nshots) return;
+  const uint2 sh = coin_shot(K, (uint32_t)shot, (uint32_t)(shot >> 32));
+  uint2* out = reinterpret_cast<uint2*>(tdp->masks) + rel;
   uint32_t any = 0u;
-  for (int c = c0; c < c1; ++c) {
-    const uint32_t cb = (uint32_t)c * kCoinChunk;
-    uint32_t f = coin_mask(K, nthr, cb, (uint32_t)(unsigned long long)shot, (uint32_t)((unsigned long long)shot >> 32));
-    uint32_t ax = 0u, bz = 0u;
-    while (f) {
-      const int i = __ffs(f) - 1;
-      f &= f - 1u;
-      const uint2 nh = __ldg(tdp->nhdr + cb + i);
-      if (nh.y == OP_N1OFF) continue;  // threshold 0xffffffff: a coin of 0xffffffff is not a fire
-      const int2 ab = noise_choice(nh.y, 2, seed, shot, cb + i);
+  for (int c = 0; c < nc; ++c) {
+    uint32_t m = 0u;
+    if (same) {
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const uint4 w = coin_block(K, sm.ord[8 * c + b], sh);
+        const uint4 th = sm.thr[8 * c + b];
+        if ((w.x >= th.x) | (w.y >= th.y) | (w.z >= th.z) | (w.w >= th.w))
+          m |= ((uint32_t)(w.x >= th.x) | ((uint32_t)(w.y >= th.y) << 1) | ((uint32_t)(w.z >= th.z) << 2) |
+                ((uint32_t)(w.w >= th.w) << 3)) << (4 * b);
+      }
+    } else {
+      m = coin_mask(K, tdp->nthr, (uint32_t)(c0 + c) * kCoinChunk, (uint32_t)shot, (uint32_t)(shot >> 32));
+    }
+    sm.fire[c][t] = m;
+    any |= (uint32_t)(m != 0u) << c;
+    out[(size_t)(c0 + c) * nshots] = make_uint2(0u, 0u);
+  }
+  uint32_t map = 0u, f = 0u, ax = 0u, bz = 0u;
+  int c = 0;
+  while (f | any) {  // one fire a turn
+    if (!f) {
+      c = __ffs(any) - 1;
+      any &= any - 1u;
+      f = sm.fire[c][t];
+      ax = bz = 0u;
+    }
+    const int i = __ffs(f) - 1;
+    f &= f - 1u;
+    const uint32_t j = (uint32_t)(c0 + c) * kCoinChunk + i;
+    const uint2 nh = __ldg(tdp->nhdr + j);
+    if (nh.y != OP_N1OFF) {  // threshold 0xffffffff: a coin of 0xffffffff is not a fire
+      const int2 ab = noise_choice(nh.y, 2, seed, (long long)shot, j);
       ax |= (uint32_t)(ab.x & 1) << i;
       bz |= (uint32_t)(ab.y & 1) << i;
     }
-    out[(size_t)c * nshots] = make_uint2(ax, bz);
-    any |= (uint32_t)((ax | bz) != 0u) << (c - c0);
+    if (!f && (ax | bz)) {
+      out[(size_t)(c0 + c) * nshots] = make_uint2(ax, bz);
+      map |= 1u << c;
+    }
   }
-  reinterpret_cast<uint8_t*>(tdp->cmap + (size_t)(cg >> 2) * nshots + rel)[cg & 3] = (uint8_t)any;
+  reinterpret_cast<uint8_t*>(tdp->cmap + (size_t)(cg >> 2) * nshots + rel)[cg & 3] = (uint8_t)map;
 }
 
 __device__ __forceinline__ int find_coin_desc(const TraceDesc* descs, int ndesc, long long it) {

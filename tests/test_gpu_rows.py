@@ -1,0 +1,62 @@
+"""GPU: the row form of the x / z pass (the trace engines' default for d = 2,
+3, 5, 7) against the oracle, bit for bit: qudit counts on both sides of a
+packed element and of a lane group, one to several panels of 32 measurements
+(one CTA and clusters), pivots used again within a panel, every gate, RESET
+and N1 rows; programs in one batch; and two-qudit gates on one qudit, which
+keep the tableau pass."""
+import numpy as np
+import pytest
+
+from sdim_gb300 import Program, workloads
+from sdim_gb300.batch import BatchRunner
+from tests.conftest import oracle_run
+
+pytestmark = pytest.mark.gpu
+
+
+def _sweeps(n, d, seed, sweeps):
+    """Random gates, then M / RESET on a part of the qudits, several times; M on all."""
+    rng = np.random.default_rng(seed)
+    ops = []
+    for _ in range(sweeps):
+        ops += workloads.all_gates_random(n, d, 3 * n + 6, seed=rng, noise_probs=(0.0, 0.4, 1.0)).ops[:-n]
+        for q in rng.permutation(n)[: max(1, n // 2)]:
+            ops.append((("M", "RESET")[int(rng.integers(2))], int(q), None, {}))
+    ops += [("M", q, None, {}) for q in range(n)] * 2
+    return workloads.CircuitSpec(n, d, ops, "sweeps")
+
+
+def _check(spec, shots, seed):
+    got = Program(spec.build()).sample(shots, seed=seed, engine="trace")
+    want = oracle_run([spec], seed, 0, shots)["records"]
+    assert np.array_equal(got, want), (spec.num_qudits, spec.dimension)
+
+
+@pytest.mark.parametrize("d", [2, 3, 5, 7])
+@pytest.mark.parametrize("n,sweeps", [(1, 3), (2, 20), (7, 12), (8, 1), (9, 8), (31, 3), (33, 5), (64, 3), (65, 2),
+                                      (130, 2)])
+def test_rows_match_oracle(n, d, sweeps):
+    _check(_sweeps(n, d, 1000 * n + d, sweeps), 40, seed=5 + n)
+
+
+@pytest.mark.parametrize("n,d", [(300, 2), (1030, 2), (257, 3), (200, 5), (290, 7)])
+def test_rows_match_oracle_wide(n, d):
+    _check(workloads.random_hpc(n, d, 5 * n, seed=n, mr_every=n, mr_fraction=0.1), 3, seed=2)
+
+
+@pytest.mark.parametrize("d", [2, 3, 5, 7])
+def test_rows_batch_matches_oracle(d):
+    br = BatchRunner()
+    items = [(_sweeps(n, d, 7 * n + d, s), 33 + n) for n, s in ((3, 4), (40, 3), (17, 6), (90, 2), (33, 1))]
+    for k, (spec, shots) in enumerate(items):
+        br.add_spec(spec, shots, 50 + k)
+    for k, ((spec, shots), out) in enumerate(zip(items, br.run(engine="trace"))):
+        assert np.array_equal(out, oracle_run([spec], 50 + k, 0, shots)["records"]), k
+
+
+@pytest.mark.parametrize("d", [2, 3, 5])
+def test_gates_on_one_qudit_twice(d):
+    spec = _sweeps(6, d, 3, 2)
+    ops = list(spec.ops)
+    ops[5:5] = [("CNOT", 2, 2, {}), ("CZ", 1, 1, {}), ("SWAP", 3, 3, {})]
+    _check(workloads.CircuitSpec(6, d, ops, "aliased"), 40, seed=9)

@@ -63,6 +63,7 @@ struct sdim_ctx {
   DevBuf dsnap;      // its x / z pass's deterministic snapshots (TraceDesc::snap)
   DevBuf cdet;       // deterministic slice sums of the odd-d cluster x / z passes (TraceDescU8::dsum)
   DevBuf rdescs, rows;  // row form of the x / z pass (rows.cuh): descriptors, rows and updates
+  DevBuf pdescs;        // its phase pass's descriptors
   cudaStream_t aux = nullptr;                      // coin pass, concurrent with the x / z pass
   cudaStream_t fast = nullptr;                     // d = 2 row form beside a coin pass: the highest priority
   cudaEvent_t ev_fast = nullptr;
@@ -608,6 +609,15 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
   }
 }
 
+// Warps in one phase-pass launch up to which a lane holds one element: about
+// six per scheduler.
+constexpr long long kRowPhaseWarps = 152LL * 4 * 6;
+
+int row_phase_blocks(const RowPhaseDesc& p) {
+  const int per = 4 * (32 >> p.lg);  // shots of a CTA
+  return (p.c.nshots + per - 1) / per;
+}
+
 RowDesc row_desc(const sdim_circuit* c, uint8_t* mem, uint4* mhdr, uint8_t* mrow, uint8_t* nrow, int rowb) {
   RowDesc r;
   std::memset(&r, 0, sizeof(r));
@@ -876,6 +886,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
                            [&](size_t i) { return jobs[i].index; }, s)) != SDIM_OK)
       return rc;
   }
+  // a d = 2 program in row form without fires: replayed by the row form's phase pass
+  auto d2_packed = [&](size_t i) { return hd[i].rows && hd[i].nused == 0; };
   // ---- odd-d descriptors
   std::stable_sort(ujobs.begin(), ujobs.end(), [](const Job& a, const Job& b) {
     const int va = trace_u8_variant(a.c->d), vb = trace_u8_variant(b.c->d);
@@ -883,6 +895,9 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     return a.rows != b.rows ? a.rows : a.c->n > b.c->n;
   });
   const size_t ku = ujobs.size();
+  auto odd_row_bytes = [](const Job& j) {
+    return j.rows ? row_trace_bytes(row_elems(j.c->n), j.c->d) : trace_row_bytes_u8(j.c->n);
+  };
   std::vector<TraceDescU8> hu(ku);
   std::vector<int> xmode(ku);
   constexpr int kRowMode = 9;
@@ -895,7 +910,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     for (size_t i = 0; i < ku; ++i) {
       const Job& j = ujobs[i];
       size_t o[5];
-      trace_offsets_u8(j.c->nmeas, j.c->nn1, trace_row_bytes_u8(j.c->n), o);
+      trace_offsets_u8(j.c->nmeas, j.c->nn1, odd_row_bytes(j), o);
       off[i] = total;
       total += o[4];
       const int mode = j.rows ? kRowMode
@@ -913,7 +928,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     long long groups = 0;
     for (size_t i = 0; i < ku; ++i) {
       const Job& j = ujobs[i];
-      if (i > 0 && trace_u8_variant(j.c->d) != trace_u8_variant(ujobs[i - 1].c->d)) groups = 0;
+      // the row form's programs come first in a variant, and have a phase pass of their own
+      if (i > 0 && (trace_u8_variant(j.c->d) != trace_u8_variant(ujobs[i - 1].c->d) || ujobs[i - 1].rows)) groups = 0;
       TraceDescU8& td = hu[i];
       std::memset(&td, 0, sizeof(td));
       td.c.ops = j.c->d_ops;
@@ -927,7 +943,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       td.c.nmeas = j.c->nmeas;
       td.c.nshots = (int)j.nshots;
       groups += (j.nshots + 31) / 32;
-      td.sw = trace_row_bytes_u8(j.c->n);
+      td.sw = odd_row_bytes(j);
       size_t o[5];
       trace_offsets_u8(j.c->nmeas, j.c->nn1, td.sw, o);
       uint8_t* b = static_cast<uint8_t*>(ctx->trace_u8.p) + off[i];
@@ -971,6 +987,64 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     for (RowGroup& g : rgroups) plan_row_group(ctx, g, hr.data(), rcirc);
     dr = static_cast<RowDesc*>(ctx->rdescs.p);
     if ((rc = upload_fixed(ctx, dr, hr.data(), sizeof(RowDesc) * hr.size(), s)) != SDIM_OK) return rc;
+  }
+  // the row form's phase pass: odd d, and d = 2 without fires to apply.  One
+  // element a lane up to kRowPhaseWarps warps in a launch, else two or four
+  std::vector<RowPhaseDesc> phr;
+  std::vector<int> phwpl, phjob;
+  auto add_phase = [&](const CircuitDesc& c, const uint4* mhdr, const void* mrow, const void* nrow, const uint2* nhdr,
+                       int nm, int nn1, int rowb, bool resets, int job) {
+    RowPhaseDesc p;
+    std::memset(&p, 0, sizeof(p));
+    p.c = c;
+    p.mhdr = mhdr;
+    p.mrow = static_cast<const uint8_t*>(mrow);
+    p.nrow = static_cast<const uint8_t*>(nrow);
+    p.nhdr = nhdr;
+    p.nm = nm;
+    p.nn1 = nn1;
+    p.E = row_elems(c.n);
+    p.rowb = rowb;
+    p.pitch = resets || rowb % 16 ? 2 * rowb : rowb;
+    phr.push_back(p);
+    phjob.push_back(job);
+  };
+  if (!colform)
+    for (size_t i = 0; i < k; ++i)
+      if (d2_packed(i))
+        add_phase(hd[i].c, hd[i].mhdr, hd[i].mrow, nullptr, nullptr, hd[i].nm, 0, 4 * hd[i].tw,
+                  jobs[i].c->rows.nx > 0, jobs[i].index);
+  for (size_t i = 0; i < ku; ++i)
+    if (ujobs[i].rows)
+      add_phase(hu[i].c, hu[i].mhdr, hu[i].mrow, hu[i].nrow, hu[i].nhdr, hu[i].nm, hu[i].nn1, hu[i].sw,
+                ujobs[i].c->rows.nx > 0, ujobs[i].index);
+  if (!phr.empty()) {
+    for (size_t b = 0; b < phr.size();) {
+      size_t e = b;
+      int wpl = 1;
+      for (; wpl <= 4; wpl <<= 1) {
+        long long warps = 0;
+        bool fits = true;
+        for (e = b; e < phr.size() && phr[e].c.d == phr[b].c.d; ++e) {
+          const int lg = row_phase_lg(phr[e].E, wpl);
+          fits &= (wpl << lg) >= phr[e].E;
+          warps += ((long long)phr[e].c.nshots * (1 << lg) + 31) / 32;
+        }
+        if (fits && (wpl == 4 || warps <= kRowPhaseWarps)) break;
+      }
+      int blocks = 0;
+      for (size_t i = b; i < e; ++i) {
+        phr[i].lg = row_phase_lg(phr[i].E, wpl);
+        phr[i].block_begin = blocks;
+        blocks += row_phase_blocks(phr[i]);
+        phwpl.push_back(wpl);
+      }
+      b = e;
+    }
+    if ((rc = ensure(ctx, ctx->pdescs, sizeof(RowPhaseDesc) * phr.size())) != SDIM_OK) return rc;
+    if ((rc = upload_descs(ctx, ctx->pdescs.p, phr.data(), sizeof(RowPhaseDesc), phr.size(), offsetof(RowPhaseDesc, c),
+                           [&](size_t i) { return phjob[i]; }, s)) != SDIM_OK)
+      return rc;
   }
   const bool d2_tab = k && !skip_xz && std::any_of(hd.begin(), hd.end(), [](const TraceDesc& t) { return !t.rows; });
   if (coins) CK(cudaEventRecord(ctx->ev_fork, s));
@@ -1197,11 +1271,32 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return cuda_fail(ctx, le, "record pass launch");
   }
+  // row form: one launch per d and elements a lane
+  if (!phr.empty()) {
+    for (size_t b = 0; b < phr.size();) {
+      size_t e = b;
+      size_t smem = 0;
+      int blocks = 0;
+      for (; e < phr.size() && phr[e].c.d == phr[b].c.d && phwpl[e] == phwpl[b]; ++e) {
+        smem = std::max(smem, row_phase_smem(phr[e].pitch));
+        blocks = phr[e].block_begin + row_phase_blocks(phr[e]);
+      }
+      row_ops(phr[b].c.d).phase(phwpl[b], blocks, smem, s, static_cast<const RowPhaseDesc*>(ctx->pdescs.p) + b,
+                                (int)(e - b));
+      const cudaError_t le = cudaGetLastError();
+      if (le != cudaSuccess) return cuda_fail(ctx, le, "row phase pass launch");
+      b = e;
+    }
+  }
   for (size_t b = colform ? k : 0; b < k;) {
+    if (d2_packed(b)) {
+      ++b;
+      continue;
+    }
     const int tw = hd[b].tw, sp = hd[b].spl;
     size_t e = b;
     long long items = 0;
-    while (e < k && hd[e].tw == tw) {
+    while (e < k && hd[e].tw == tw && !d2_packed(e)) {
       items = hd[e].c.item_begin + (hd[e].c.nshots + 32 * sp - 1) / (32 * sp);
       ++e;
     }
@@ -1215,6 +1310,10 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     b = e;
   }
   for (size_t b = 0; b < ku;) {
+    if (ujobs[b].rows) {
+      ++b;
+      continue;
+    }
     const int v = trace_u8_variant(hu[b].c.d);
     size_t e = b;
     long long items = 0;
@@ -2018,7 +2117,7 @@ int sdim_ctx_destroy(sdim_ctx* ctx) {
   for (int i = 0; i < sdim_ctx::kXzStreams; ++i) cudaStreamSynchronize(ctx->xzs[i]);
   DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap, &ctx->arena,
                     &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8, &ctx->xz_u8,
-                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rdescs, &ctx->rows};
+                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rdescs, &ctx->rows, &ctx->pdescs};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   if (ctx->staging) cudaFreeHost(ctx->staging);
@@ -2074,7 +2173,7 @@ int sdim_memory_info(sdim_ctx* ctx, int64_t info[3]) {
   const DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap,
                           &ctx->arena, &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8,
                           &ctx->xz_u8, &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet,
-                          &ctx->rdescs, &ctx->rows};
+                          &ctx->rdescs, &ctx->rows, &ctx->pdescs};
   int64_t held = 0;
   for (const DevBuf* b : bufs) held += (int64_t)b->cap;
   info[2] = held;

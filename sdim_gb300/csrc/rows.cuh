@@ -27,10 +27,12 @@
 // a vector V of the stabilizers' phases, updated like a row.  d = 2: the rows
 // are signed Pauli strings i^k prod X^S Z^T over the initial generators; k
 // follows the gates word by word and the updates row by row, and V holds the
-// stabilizers' signs.  The trace written is that of trace_bits.cuh and
-// trace_u8.cuh over the stabilizer half (same pivots, factors and phases);
-// the destabilizer half of a random measurement's factor row is zero, since
-// no record depends on the destabilizers' deltas.
+// stabilizers' signs.  The trace written is that of trace_bits.cuh (d = 2, the
+// destabilizer half of factor rows zero) or of trace_u8.cuh (odd d, rows
+// packed) over the stabilizer half, with the same pivots, factors and phases:
+// no record depends on the destabilizers' deltas.  The row form's phase pass
+// replays it, for d = 2 the programs without N1 before their last measurement
+// (the others keep the passes that read the coin pass's masks).
 #pragma once
 #include <cstddef>
 #include <cuda_runtime.h>
@@ -134,6 +136,30 @@ inline int row_units(int n, int d, int nk) {
 // holds whole rows, and a step needs no barrier.
 inline int row_slice(int E) { return E <= 1 ? 1 : E <= 2 ? 2 : E <= 4 ? 4 : 16 + (E <= 8 ? 1 : E <= 24 ? 2 : 4); }
 
+// A program in the row form's phase pass.
+struct RowPhaseDesc {
+  CircuitDesc c;
+  const uint4* mhdr;
+  const uint8_t* mrow;  // rowb bytes each: factor row, z_q row of a RESET
+  const uint8_t* nrow;  // odd d: rowb bytes each: x_q, z_q at an N1
+  const uint2* nhdr;    // odd d: N1 (coin threshold, opcode)
+  int nm, nn1, E, rowb;
+  int pitch;        // bytes of a measurement's rows that a window stages: both, or the factor row alone
+  int lg;           // a shot is 2^lg lanes
+  int block_begin;  // first CTA (4 warps) of this program
+};
+// Elements a lane of the phase pass holds: one while the launch's warps stay
+// below a few per scheduler (the chain of a measurement bounds it), up to four
+// for many shots (the issue of the per-lane overhead bounds it).
+inline int row_phase_lg(int E, int wpl) {
+  int lg = 0;
+  while ((wpl << lg) < E && lg < 5) ++lg;
+  return lg;
+}
+inline size_t row_phase_smem(int pitch) { return (size_t)2 * 32 * (16 + pitch) + 4 * 2 * 32 * 36; }
+// Bytes of a packed trace row over E elements (a multiple of 16).
+inline int row_trace_bytes(int E, int d) { return (E * row_elem_bytes(d) + 15) / 16 * 16; }
+
 // The launchers of one d (k_rows_<d>.cu).
 struct RowOps {
   cudaError_t (*set_smem)(int optin);
@@ -149,6 +175,8 @@ struct RowOps {
   cudaError_t (*chain)(int slice, int ctas, int block, int rawt, int lg, size_t smem, cudaStream_t s, const RowDesc* descs, int nd);
   // extra pass: `ctas` CTAs, extra_per_cta rows each
   void (*extra)(int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd);
+  // phase pass: `blocks` CTAs of 128 threads, wpl (1, 2 or 4) elements a lane
+  void (*phase)(int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd);
 };
 const RowOps& row_ops_2();
 const RowOps& row_ops_3();

@@ -138,15 +138,6 @@ struct El {
     if (v & 2) atomicOr(&p->y, 1u << j);
     if (v & 4) atomicOr(&p->z, 1u << j);
   }
-  // residues 4 i .. 4 i + 3 as bytes
-  static __device__ __forceinline__ uint32_t bytes(T a, int i) {
-    if constexpr (D == 7) {
-      const uint32_t k = ~(a.x & a.y & a.z);
-      a = make_uint4(a.x & k, a.y & k, a.z & k, 0u);
-    }
-    auto spread = [&](uint32_t w) { return (((w >> (4 * i)) & 15u) * 0x00204081u) & 0x01010101u; };
-    return spread(a.x) + 2u * spread(a.y) + 4u * spread(a.z);
-  }
 };
 
 template <>
@@ -184,10 +175,6 @@ struct El<3> {  // two planes (planes3.cuh)
   static __device__ __forceinline__ void put(T* q, int j, int v) {
     if (v == 1) atomicOr(&q->x, 1u << j);
     if (v == 2) atomicOr(&q->y, 1u << j);
-  }
-  static __device__ __forceinline__ uint32_t bytes(T a, int i) {
-    auto spread = [&](uint32_t w) { return (((w >> (4 * i)) & 15u) * 0x00204081u) & 0x01010101u; };
-    return spread(a.x) + 2u * spread(a.y);
   }
 };
 
@@ -926,26 +913,10 @@ __device__ __forceinline__ void eliminate(const RowDesc& rd, int cnt, typename E
   }
 }
 
-// Element e of a trace row of rowb bytes: a word (d = 2) or 32 bytes.
-template <int D>
-__device__ __forceinline__ void trace_elem(uint8_t* row, int e, typename El<D>::T v, int rowb) {
-  if constexpr (D == 2) {
-    reinterpret_cast<uint32_t*>(row)[e] = v;
-  } else {
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (32 * e + 16 * h < rowb)
-        reinterpret_cast<uint4*>(row)[2 * e + h] =
-            make_uint4(El<D>::bytes(v, 4 * h), El<D>::bytes(v, 4 * h + 1), El<D>::bytes(v, 4 * h + 2),
-                       El<D>::bytes(v, 4 * h + 3));
-  }
-}
-
 // The rest of a trace row after E elements.
 template <int D>
 __device__ __forceinline__ void trace_pad(uint8_t* row, int E, int rowb, int lane) {
-  constexpr int kB = D == 2 ? 4 : L;  // bytes written per element
-  for (int b = E * kB + 4 * lane; b < rowb; b += 128) *reinterpret_cast<uint32_t*>(row + b) = 0u;
+  for (int b = E * row_elem_bytes(D) + 4 * lane; b < rowb; b += 128) *reinterpret_cast<uint32_t*>(row + b) = 0u;
 }
 
 // Eliminates panel k (its rows in P, up to date) and writes its trace records
@@ -1018,14 +989,14 @@ __device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typ
         T v = row[w];
         if (w == pe || w == E + pe) v = E_::set(v, pl, 0);
         stc(f + w, E_::mulc(v, D == 2 ? 1 : D - e));
-        if (w < E) trace_elem<D>(out, w, E_::neg(v), rd.rowb);
+        if (w < E) reinterpret_cast<T*>(out)[w] = E_::neg(v);
       }
       if (lane == 0) {
         __stcg(rd.opm + h, make_int4(p, D == 2 ? 1 | (ps.tp[i] << 8) : e, m, 0));
         rd.mhdr[m] = make_uint4(2u * reset | (D == 2 ? 0u : (uint32_t)e << 8), (uint32_t)p, nord, 0u);
       }
     } else {
-      for (int w = lane; w < E; w += 32) trace_elem<D>(out, w, row[E + w], rd.rowb);
+      for (int w = lane; w < E; w += 32) reinterpret_cast<T*>(out)[w] = row[E + w];
       const int det = D == 2 ? 2 * (((ps.kk[i] + 2 * ps.kq[i]) >> 1) + ps.dsum[i] & 1)
                              : (ps.dsum[i] - ps.kk[i] + D) % D;
       if (lane == 0) rd.mhdr[m] = make_uint4(2u * reset | 1u, 0u, nord, (uint32_t)det);
@@ -1278,9 +1249,169 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_extra(const RowDesc* __
       if (gl + h * G < E) reinterpret_cast<uint32_t*>(out)[gl + h * G] = S[h];
     for (int w = E + gl; 4 * w < rd.rowb; w += G) reinterpret_cast<uint32_t*>(out)[w] = 0u;
   } else {
-    for (int e = lane; e < E; e += 32) trace_elem<D>(out, e, buf[e], rd.rowb);
+    for (int e = lane; e < E; e += 32) reinterpret_cast<T*>(out)[e] = buf[e];
     trace_pad<D>(out, E, rd.rowb, lane);
   }
+}
+
+// ---------------------------------------------------------------- phase pass
+
+// Every shot's deltas from the trace (trace_bits.cuh, trace_u8.cuh: the same
+// updates with the same streams, over the stabilizer half).  A shot is LG =
+// 2^lg lanes, element e in lane e mod LG, and a warp 32 / LG shots; the four
+// warps of a CTA share the measurements' headers and rows, staged 32 at a time
+// while the 32 before them run, and a window's outcomes are drawn at its start
+// with every lane on another draw.  A measurement then needs no barrier: a
+// shuffle for the pivot's delta or log LG for a factor sum.
+// Bound by a measurement's chain of about 60 instructions where the warps are
+// few, by their issue where they are many (then WPL elements a lane).
+template <int D, int WPL>
+__global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restrict__ descs, int nd) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  using E_ = El<D>;
+  using T = typename E_::T;
+  int di = 0;
+  {
+    int hi = nd - 1;
+    while (di < hi) {
+      const int mid = (di + hi + 1) >> 1;
+      if (descs[mid].block_begin <= (int)blockIdx.x) di = mid; else hi = mid - 1;
+    }
+  }
+  const RowPhaseDesc td = descs[di];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int lg = td.lg, LG = 1 << lg, SPW = 32 >> lg, gl = lane & (LG - 1), sl = lane >> lg;
+  const int E = td.E, nm = td.nm, nmeas = td.c.nmeas;
+  const int first = (((int)blockIdx.x - td.block_begin) * 4 + warp) * SPW;  // this warp's first shot
+  const int rel = first + sl;
+  const bool live = rel < td.c.nshots;
+  const long long shot = td.c.shot0 + rel;
+  const unsigned long long seed = td.c.seed;
+  constexpr int WIN = 32;
+  const int pitch = td.pitch;  // staged bytes of a measurement, a multiple of 16
+  uint4* hdr = reinterpret_cast<uint4*>(smem);  // [2][WIN]
+  uint8_t* rows = smem + 2 * WIN * 16;          // [2][WIN][pitch]
+  uint8_t* mo = rows + 2 * (size_t)WIN * pitch + warp * (2 * 32 * 36) + sl * 36;  // this shot's outcomes
+  uint8_t* rec0 = mo - sl * 36 + 32 * 36;                                         // the warp's records
+  auto stage = [&](int wb, int b) {
+    const int cnt = min(WIN, nm - wb);
+    if (t < cnt) {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(hdr + b * WIN + t);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(td.mhdr + wb + t) : "memory");
+    }
+    const int per = pitch >> 4;
+    for (int i = t; i < cnt * per; i += 128) {
+      const int m = i / per, q = i - m * per;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(rows + ((size_t)b * WIN + m) * pitch + 16 * q);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                   "l"(td.mrow + (size_t)(wb + m) * 2 * td.rowb + 16 * q)
+                   : "memory");
+    }
+  };
+  T d[WPL];
+#pragma unroll
+  for (int i = 0; i < WPL; ++i) d[i] = E_::zero();
+  uint32_t nord = 0;
+  if (nm > 0) stage(0, 0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int wb = 0, b = 0; wb < nm; wb += WIN, b ^= 1) {
+    const int cnt = min(WIN, nm - wb);
+    if (wb + WIN < nm) stage(wb + WIN, b ^ 1);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const uint4* hw = hdr + b * WIN;
+    const uint8_t* rw = rows + (size_t)b * WIN * pitch;
+    const uint32_t rnd = __ballot_sync(0xffffffffu, lane < cnt && !(hw[lane].x & 1u));
+    for (int k = gl; k < cnt; k += LG)
+      if ((rnd >> k) & 1u) mo[k] = (uint8_t)mulshift(stream_block(seed, shot, (uint32_t)(wb + k), 0u).x, D);
+    __syncwarp();
+    for (int k = 0; k < cnt; ++k) {
+      const uint4 h = hw[k];
+      const T* row = reinterpret_cast<const T*>(rw + (size_t)k * pitch);
+      if constexpr (D != 2) {
+        // N1 before the measurement: four coins a lane at a time; a group
+        // applies one fire a turn
+        const uint32_t nend = min(h.z, (uint32_t)td.nn1);
+        for (; nord < nend; nord = min(nend, (nord / 4u + LG) * 4u)) {
+          const uint32_t blk = nord / 4u + gl;
+          uint32_t f = 0u;
+          if (live && blk * 4u < nend) {
+            const uint4 w = stream_block(seed, shot, blk, 1u);
+            const uint32_t cw[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t j = 4u * blk + q;
+              if (j >= nord && j < nend) {
+                const uint2 nh = __ldg(td.nhdr + j);
+                if (nh.y != OP_N1OFF && cw[q] >= nh.x) f |= 1u << q;
+              }
+            }
+          }
+          while (true) {
+            const uint32_t pend = __ballot_sync(0xffffffffu, f != 0u);
+            if (!pend) break;
+            const uint32_t mine = (pend >> (lane & ~(LG - 1))) & (LG == 32 ? 0xffffffffu : (1u << LG) - 1u);
+            const int src = mine ? (lane & ~(LG - 1)) + __ffs(mine) - 1 : lane;
+            const uint32_t sf = __shfl_sync(0xffffffffu, f, src);
+            const uint32_t j = 4u * (nord / 4u + (uint32_t)(src & (LG - 1))) + (uint32_t)(__ffs(sf | 16u) - 1);
+            if (mine) {
+              const int2 ab = noise_choice(__ldg(&td.nhdr[j].y), D, seed, shot, j);
+              const int cz = ab.x ? D - ab.x : 0, cx = ab.y;  // delta += -a z_q + b x_q
+              const T* xr = reinterpret_cast<const T*>(td.nrow + (size_t)j * 2 * td.rowb);
+              const T* zr = reinterpret_cast<const T*>(td.nrow + ((size_t)j * 2 + 1) * td.rowb);
+#pragma unroll
+              for (int i = 0; i < WPL; ++i) {
+                const int e = gl + i * LG;
+                if (e < E) d[i] = E_::muladd(E_::muladd(d[i], zr[e], cz), xr[e], cx);
+              }
+              if (src == lane) f &= f - 1u;
+            }
+          }
+        }
+      }
+      int m;
+      if (!(h.x & 1u)) {
+        const int p = (int)h.y, pe = p / L, pl = p % L;
+        T x = d[0];
+#pragma unroll
+        for (int i = 1; i < WPL; ++i)
+          if ((pe >> lg) == i) x = d[i];
+        int dp = __shfl_sync(0xffffffffu, E_::get(x, pl), pe & (LG - 1), LG);
+        if constexpr (D != 2) dp = small_mod<D>(dp * (int)(h.x >> 8));
+        m = mo[k];
+        const int nv = D == 2 ? m : m ? D - m : 0;
+#pragma unroll
+        for (int i = 0; i < WPL; ++i) {
+          const int e = gl + i * LG;
+          if (e < E) d[i] = E_::put_at(E_::muladd(d[i], row[e], dp), e == pe ? 1u << pl : 0u, nv);
+        }
+      } else {
+        int s = 0;
+#pragma unroll
+        for (int i = 0; i < WPL; ++i) {
+          const int e = gl + i * LG;
+          if (e < E) s += E_::dot(row[e], d[i]);
+        }
+        for (int o = LG >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        m = D == 2 ? (((((int)h.w + 2 * s) & 3) + 1) >> 1) & 1 : (D - ((int)h.w + s) % D) % D;
+      }
+      if (h.x & 2u) {
+        const T* zr = reinterpret_cast<const T*>(rw + (size_t)k * pitch + td.rowb);
+#pragma unroll
+        for (int i = 0; i < WPL; ++i) {
+          const int e = gl + i * LG;
+          if (e < E) d[i] = E_::muladd(d[i], zr[e], m);
+        }
+      }
+      if (gl == 0) rec0[sl * 36 + k] = (uint8_t)(m | (int)((h.x & 1u) << 7));
+    }
+    __syncwarp();
+    if (lane < cnt)
+      for (int q = 0; q < SPW && first + q < td.c.nshots; ++q)
+        td.c.out[(size_t)(first + q) * nmeas + wb + lane] = rec0[q * 36 + lane];
+    __syncthreads();  // the window's buffers and outcomes are free
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 template <int D>
@@ -1309,6 +1440,9 @@ cudaError_t set_smem(int optin) {
   for (int sl : kSlices)
     if (e == cudaSuccess)
       e = for_slice(sl, [&](auto c, auto solo) { return set_dynamic_smem(k_rows_chain<D, c.value, solo.value>, optin); });
+  if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 1>, optin);
+  if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 2>, optin);
+  if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 4>, optin);
   return e != cudaSuccess ? e : set_dynamic_smem(k_rows_extra<D>, optin);
 }
 
@@ -1348,6 +1482,11 @@ RowOps row_ops() {
   o.chain = chain<D>;
   o.extra = [](int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd) {
     k_rows_extra<D><<<ctas, 32 * kRowWarps, smem, s>>>(descs, nd);
+  };
+  o.phase = [](int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd) {
+    if (wpl == 1) k_rows_phase<D, 1><<<blocks, 128, smem, s>>>(descs, nd);
+    else if (wpl == 2) k_rows_phase<D, 2><<<blocks, 128, smem, s>>>(descs, nd);
+    else k_rows_phase<D, 4><<<blocks, 128, smem, s>>>(descs, nd);
   };
   return o;
 }

@@ -79,7 +79,7 @@ struct sdim_ctx {
   bool d2h_done = false;             // the copies are enqueued on cps
   cudaEvent_t ev_gf = nullptr, ev_gj = nullptr;    // fork to and join from grp
   cudaEvent_t ev_g0 = nullptr, ev_g1 = nullptr;    // shot-group engines' span on grp (SDIM_FLAG_TIME)
-  static constexpr int kXzStreams = 3;
+  static constexpr int kXzStreams = 8;
   cudaStream_t xzs[kXzStreams] = {};               // odd-d x / z passes of different runs, concurrently
   cudaEvent_t ev_xzf = nullptr, ev_xzj[kXzStreams] = {};
   DevBuf xz_queue;                                 // program counters of the dynamic x / z passes
@@ -447,7 +447,14 @@ int job_variant(const sdim_circuit* c, unsigned flags) {
   return c->gvariant;
 }
 
-// Below this many shots a program runs on the shot-group engine: one x / z
+// Whether a trace-engine job's x / z pass runs in the row form (rows.cuh):
+// wherever the encoder built one, unless a flag names a tableau pass.
+bool row_form(const sdim_circuit* c, unsigned flags) {
+  return c->rows.nops > 0 && !(flags & (SDIM_FLAG_FORCE_GMEM | SDIM_FLAG_SPLIT_XZ | SDIM_FLAG_CLUSTER_XZ |
+                                        SDIM_FLAG_U8_XZ | SDIM_FLAG_PACKED_XZ | SDIM_FLAG_UNLAYERED));
+}
+
+// Below this many shots a program without a row form runs on the shot-group engine: one x / z
 // pass per program plus a phase pass only pays once there are several 32-shot
 // groups to share it, and in a batch of small programs the group engine's
 // single persistent launch keeps every SM busy.
@@ -467,7 +474,7 @@ bool use_trace(const Job& j, unsigned flags) {
                SDIM_FLAG_NO_TRACE))
     return false;
   if (j.c->d != 2 || trace_words(j.c->n) == 0 || !j.c->d_steps || j.nshots <= 0) return false;
-  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits;
+  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || row_form(j.c, flags);
 }
 
 // Odd-d programs above this many qudits stay on the shot-group engine (the
@@ -536,14 +543,7 @@ bool use_trace_u8(const Job& j, unsigned flags) {
                SDIM_FLAG_NO_TRACE))
     return false;
   if (j.c->d == 2 || j.c->n > kTraceU8MaxQudits || j.nshots <= 0) return false;
-  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits;
-}
-
-// Whether a trace-engine job's x / z pass runs in the row form (rows.cuh):
-// wherever the encoder built one, unless a flag names a tableau pass.
-bool row_form(const sdim_circuit* c, unsigned flags) {
-  return c->rows.nops > 0 && !(flags & (SDIM_FLAG_FORCE_GMEM | SDIM_FLAG_SPLIT_XZ | SDIM_FLAG_CLUSTER_XZ |
-                                        SDIM_FLAG_U8_XZ | SDIM_FLAG_PACKED_XZ | SDIM_FLAG_UNLAYERED));
+  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || row_form(j.c, flags);
 }
 
 // The row-form programs of one d and chain-pass slice in a run: descriptors
@@ -729,7 +729,14 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   };
   // ---- d = 2 descriptors
   // largest first: the x / z passes of a batch start with the longest ones
-  std::stable_sort(jobs.begin(), jobs.end(), [](const Job& a, const Job& b) { return a.c->n > b.c->n; });
+  // (a program in row form without fires to apply is replayed by the row form's
+  // phase pass: those come last, so that the other phase passes number the
+  // shot groups of consecutive descriptors)
+  auto packed_job = [](const Job& j) { return j.rows && j.c->nn1_used == 0; };
+  std::stable_sort(jobs.begin(), jobs.end(), [&](const Job& a, const Job& b) {
+    const bool pa = packed_job(a), pb = packed_job(b);
+    return pa != pb ? pb : a.c->n > b.c->n;
+  });
   const size_t k = jobs.size();
   std::vector<TraceDesc> hd(k);
   long long coins = 0;
@@ -886,8 +893,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
                            [&](size_t i) { return jobs[i].index; }, s)) != SDIM_OK)
       return rc;
   }
-  // a d = 2 program in row form without fires: replayed by the row form's phase pass
-  auto d2_packed = [&](size_t i) { return hd[i].rows && hd[i].nused == 0; };
+  auto d2_packed = [&](size_t i) { return packed_job(jobs[i]); };
   // ---- odd-d descriptors
   std::stable_sort(ujobs.begin(), ujobs.end(), [](const Job& a, const Job& b) {
     const int va = trace_u8_variant(a.c->d), vb = trace_u8_variant(b.c->d);

@@ -60,3 +60,20 @@ def test_gates_on_one_qudit_twice(d):
     ops = list(spec.ops)
     ops[5:5] = [("CNOT", 2, 2, {}), ("CZ", 1, 1, {}), ("SWAP", 3, 3, {})]
     _check(workloads.CircuitSpec(6, d, ops, "aliased"), 40, seed=9)
+
+
+def test_mixed_batch_matches_oracle():
+    """Programs with and without fires, in row form and not, of one trace-row
+    width, in one launch: each kind has its own replay."""
+    twice = workloads.CircuitSpec(9, 2, [("H", 0, None, {}), ("CNOT", 3, 3, {})] + [("M", q, None, {}) for q in range(9)],
+                                  "aliased")
+    odd = workloads.CircuitSpec(8, 5, [("H", 0, None, {}), ("CNOT", 3, 3, {})] + [("M", q, None, {}) for q in range(8)],
+                                "aliased")
+    specs = [workloads.random_hpc(30, 2, 100, seed=3), workloads.surface_memory(3, 2, prob=0.05), twice,
+             workloads.random_hpc(12, 5, 60, seed=1), odd, workloads.random_hpc(21, 2, 80, seed=4),
+             workloads.random_hpc(9, 5, 60, seed=6)]
+    br = BatchRunner()
+    for k, spec in enumerate(specs):
+        br.add_spec(spec, 150 + 40 * k, 60 + k)
+    for k, (spec, out) in enumerate(zip(specs, br.run())):
+        assert np.array_equal(out, oracle_run([spec], 60 + k, 0, 150 + 40 * k)["records"]), k

@@ -64,6 +64,7 @@ struct sdim_ctx {
   DevBuf cdet;       // deterministic slice sums of the odd-d cluster x / z passes (TraceDescU8::dsum)
   DevBuf rdescs, rows;  // row form of the x / z pass (rows.cuh): descriptors, rows and updates
   DevBuf pdescs;        // its phase pass's descriptors
+  DevBuf fdescs;        // the frame route's coin pass
   cudaStream_t aux = nullptr;                      // coin pass, concurrent with the x / z pass
   cudaStream_t fast = nullptr;                     // d = 2 row form beside a coin pass: the highest priority
   cudaEvent_t ev_fast = nullptr;
@@ -476,6 +477,9 @@ bool use_trace(const Job& j, unsigned flags) {
   if (j.c->d != 2 || trace_words(j.c->n) == 0 || !j.c->d_steps || j.nshots <= 0) return false;
   return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || row_form(j.c, flags);
 }
+
+// Device memory of the fire masks of one part of the frame route's shots.
+constexpr size_t kFrameMaskBudget = (size_t)512 << 20;
 
 // Odd-d programs above this many qudits stay on the shot-group engine (the
 // phase pass keeps 32 shots' deltas in shared memory).
@@ -1805,6 +1809,7 @@ void append_rows(std::vector<uint2>& dev, size_t op_begin, size_t nops, int n, i
   std::vector<uint2> xinfo, nhdr;
   uint32_t mord = 0, nord = 0, gated = 0;  // gated: measurements before the last gate so far
   int nk = 0, levels = 0;
+  double fires = 0.0;
   auto put_op = [&](const uint4& o, int lv) {
     ops.push_back(Entry{o, lv});
     levels = std::max(levels, lv + 1);
@@ -1822,6 +1827,7 @@ void append_rows(std::vector<uint2>& dev, size_t op_begin, size_t nops, int n, i
     }
     if (op == OP_N1D || op == OP_N1F || op == OP_N1P) {
       nhdr.push_back(make_uint2(w.y, op));
+      fires += 1.0 - std::pow((double)w.y / 4294967296.0, 32.0);
       const uint32_t r = (uint32_t)xinfo.size() + 1u;
       xinfo.push_back(make_uint2(mord, (1u << 30) | nord));
       xinfo.push_back(make_uint2(mord, (2u << 30) | nord));
@@ -1918,6 +1924,8 @@ void append_rows(std::vector<uint2>& dev, size_t op_begin, size_t nops, int n, i
   out.nlayers = levels;
   out.nx = (int)xinfo.size();
   out.nk = nk;
+  out.nn1 = (int)nhdr.size();
+  out.fires = fires;
   if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
 }
 
@@ -2123,7 +2131,7 @@ int sdim_ctx_destroy(sdim_ctx* ctx) {
   for (int i = 0; i < sdim_ctx::kXzStreams; ++i) cudaStreamSynchronize(ctx->xzs[i]);
   DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap, &ctx->arena,
                     &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8, &ctx->xz_u8,
-                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rdescs, &ctx->rows, &ctx->pdescs};
+                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rdescs, &ctx->rows, &ctx->pdescs, &ctx->fdescs};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   if (ctx->staging) cudaFreeHost(ctx->staging);
@@ -2179,7 +2187,7 @@ int sdim_memory_info(sdim_ctx* ctx, int64_t info[3]) {
   const DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap,
                           &ctx->arena, &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8,
                           &ctx->xz_u8, &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet,
-                          &ctx->rdescs, &ctx->rows, &ctx->pdescs};
+                          &ctx->rdescs, &ctx->rows, &ctx->pdescs, &ctx->fdescs};
   int64_t held = 0;
   for (const DevBuf* b : bufs) held += (int64_t)b->cap;
   info[2] = held;
@@ -2389,28 +2397,110 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
                        ctx->stream));
   }
   cudaStream_t s = ctx->stream;
-  // shot 0: the noiseless tableau shot, into row 0, on the trace engines
-  // (one x / z pass) where they take the program: the shot-group engine
-  // spends a whole group's latency on a single shot
-  std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
-  if ((rc = launch_jobs(ctx, jobs, s, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE)) != SDIM_OK) return rc;
-  // shots 1 .. nshots - 1: frames against row 0
-  if (nshots > 1 && c->nmeas > 0) {
-    FrameDesc fd;
-    fd.ops = c->d_ops + c->fops_off;
-    fd.ref = dst;
-    fd.out = dst + c->nmeas;
-    fd.seed = seed;
-    fd.shot0 = 1;
-    fd.nops = c->nfops;
-    fd.n = c->n;
-    fd.d = c->d;
-    fd.nmeas = c->nmeas;
-    fd.nshots = (int)(nshots - 1);
-    const long long grid = (nshots - 1 + 31) / 32;
-    launch_frame_pass((int)grid, smem, s, fd, static_cast<int*>(ctx->status.p));
-    const cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) return cuda_fail(ctx, le, "frame pass launch");
+  // shots 1 .. nshots - 1 on bit planes where the program has a row form that
+  // fits: frames against row 0
+  RowFrameDesc rf;
+  std::memset(&rf, 0, sizeof(rf));
+  int warps = 0;  // of a frame-pass CTA; 0: the byte-per-shot kernel
+  size_t fsmem = 0;
+  if (nshots > 1 && c->rows.nops > 0 && !(flags & SDIM_FLAG_FORCE_GMEM)) {
+    rf.ops = reinterpret_cast<const uint4*>(c->d_blob + c->rows.ops_off);
+    rf.lay = reinterpret_cast<const uint32_t*>(c->d_blob + c->rows.lay_off);
+    rf.xinfo = c->d_blob + c->rows.xinfo_off;
+    rf.nhdr = c->d_blob + c->rows.nhdr_off;
+    rf.ref = dst;
+    rf.seed = seed;
+    rf.nlayers = c->rows.nlayers;
+    rf.n = c->n;
+    rf.nm = c->nmeas;
+    rf.nused = c->rows.nn1;
+    rf.nchunk = c->d == 2 ? (rf.nused + kCoinChunk - 1) / kCoinChunk : 0;
+    // fired ordinals of a warp: the mean and six deviations; past that the pass
+    // gathers a word from the masks
+    rf.cap = (int)std::min<double>(rf.nused, c->rows.fires + 6.0 * std::sqrt(c->rows.fires) + 32.0);
+    for (warps = 4; warps > 0; warps >>= 1)
+      if ((fsmem = row_ops(c->d).frame_smem(rf, warps)) + 1024 <= (size_t)ctx->smem_optin) break;
+  }
+  if (warps) {
+    for (int d : {2, 3, 5, 7})
+      if (!ctx->rows_smem_set) {
+        const cudaError_t e = row_ops(d).set_smem(ctx->smem_optin);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFuncSetAttribute");
+      }
+    ctx->rows_smem_set = true;
+    // the reference shot on the stream of highest priority, beside the coin
+    // pass of the first part of the shots; parts bound the masks' memory
+    const long long frames = nshots - 1;
+    const size_t per_shot = c->d == 2 ? coin_mask_bytes(rf.nchunk, 1024) / 1024 + coin_map_bytes(rf.nchunk, 1024) / 1024 : 0;
+    long long part = frames;
+    if (per_shot) part = std::min<long long>(part, std::max<long long>(32768, (long long)(kFrameMaskBudget / per_shot)));
+    CK(cudaEventRecord(ctx->ev_gf, s));
+    CK(cudaStreamWaitEvent(ctx->fast, ctx->ev_gf, 0));
+    std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
+    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE);
+    ctx->last_stream = s;
+    if (rc != SDIM_OK) return rc;
+    CK(cudaEventRecord(ctx->ev_fast, ctx->fast));
+    TraceDesc td;
+    std::memset(&td, 0, sizeof(td));
+    if (rf.nchunk) {
+      if ((rc = ensure(ctx, ctx->masks, coin_mask_bytes(rf.nchunk, part) + coin_map_bytes(rf.nchunk, part))) != SDIM_OK)
+        return rc;
+      if ((rc = ensure(ctx, ctx->fdescs, sizeof(TraceDesc))) != SDIM_OK) return rc;
+      td.c.seed = seed;
+      td.nthr = c->d_nthr;
+      td.nhdr = c->d_nhdr;
+      td.nchunk = rf.nchunk;
+      td.masks = static_cast<uint32_t*>(ctx->masks.p);
+      td.cmap = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ctx->masks.p) + coin_mask_bytes(rf.nchunk, part));
+      rf.masks = static_cast<const uint2*>(ctx->masks.p);
+    }
+    for (long long f0 = 0; f0 < frames; f0 += part) {
+      const long long fn = std::min(part, frames - f0);
+      if (rf.nchunk) {
+        td.c.shot0 = 1 + f0;
+        td.c.nshots = (int)fn;
+        CK(cudaMemcpyAsync(ctx->fdescs.p, &td, sizeof(td), cudaMemcpyHostToDevice, s));
+        const long long blocks = coin_blocks(rf.nchunk, fn);
+        if (blocks > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one coin pass");
+        launch_coin_pass((int)blocks, s, static_cast<const TraceDesc*>(ctx->fdescs.p), 1);
+        const cudaError_t le = cudaGetLastError();
+        if (le != cudaSuccess) return cuda_fail(ctx, le, "coin pass launch");
+      }
+      if (f0 == 0) CK(cudaStreamWaitEvent(s, ctx->ev_fast, 0));
+      rf.out = dst + (size_t)(1 + f0) * c->nmeas;
+      rf.shot0 = 1 + f0;
+      rf.nshots = (int)fn;
+      rf.mshots = fn;
+      rf.mrel = 0;
+      row_ops(c->d).frame((int)((fn + 32 * warps - 1) / (32 * warps)), warps, fsmem, s, rf);
+      const cudaError_t le = cudaGetLastError();
+      if (le != cudaSuccess) return cuda_fail(ctx, le, "frame pass launch");
+    }
+  } else {
+    // shot 0: the noiseless tableau shot, into row 0, on the trace engines
+    // (one x / z pass) where they take the program: the shot-group engine
+    // spends a whole group's latency on a single shot
+    std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
+    if ((rc = launch_jobs(ctx, jobs, s, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE)) != SDIM_OK) return rc;
+    // shots 1 .. nshots - 1: frames against row 0
+    if (nshots > 1 && c->nmeas > 0) {
+      FrameDesc fd;
+      fd.ops = c->d_ops + c->fops_off;
+      fd.ref = dst;
+      fd.out = dst + c->nmeas;
+      fd.seed = seed;
+      fd.shot0 = 1;
+      fd.nops = c->nfops;
+      fd.n = c->n;
+      fd.d = c->d;
+      fd.nmeas = c->nmeas;
+      fd.nshots = (int)(nshots - 1);
+      const long long grid = (nshots - 1 + 31) / 32;
+      launch_frame_pass((int)grid, smem, s, fd, static_cast<int*>(ctx->status.p));
+      const cudaError_t le = cudaGetLastError();
+      if (le != cudaSuccess) return cuda_fail(ctx, le, "frame pass launch");
+    }
   }
   if (dev_out) return finish(ctx, s, flags & ~SDIM_FLAG_ASYNC);
   if (flags & SDIM_FLAG_TIME) {

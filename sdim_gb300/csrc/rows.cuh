@@ -78,6 +78,8 @@ struct RowProgram {
   int64_t ops_off = -1, lay_off = -1, minfo_off = -1, xinfo_off = -1, nhdr_off = -1;  // uint2 words of the blob
   int nops = 0, nlayers = 0, nx = 0;
   int nk = 0;  // measurements with a K column
+  int nn1 = 0;           // N1 ordinals before the last measurement
+  double fires = 0.0;    // expected number of them that any of 32 shots fires
 };
 
 struct RowDesc {
@@ -160,6 +162,24 @@ inline size_t row_phase_smem(int pitch) { return (size_t)2 * 32 * (16 + pitch) +
 // Bytes of a packed trace row over E elements (a multiple of 16).
 inline int row_trace_bytes(int E, int d) { return (E * row_elem_bytes(d) + 15) / 16 * 16; }
 
+// The frame pass of one program (k_frame.cu has the frame rules).
+struct RowFrameDesc {
+  const uint4* ops;      // its row program
+  const uint32_t* lay;
+  const uint2* xinfo;
+  const uint2* nhdr;     // odd d: N1 (coin threshold, opcode)
+  const uint8_t* ref;    // records of the reference shot
+  uint8_t* out;          // nshots x nm records
+  const uint2* masks;    // d = 2: the coin pass's fire masks, mshots shots a chunk, from shot mrel on
+  unsigned long long seed;
+  long long shot0;       // stream index of the first shot, below 2^32
+  long long mshots, mrel;
+  int nlayers, n, nm, nshots;
+  int nused;   // N1 ordinals before the last measurement
+  int nchunk;  // d = 2: chunks of 32 of them
+  int cap;     // d = 2: entries of a warp for fired ordinals
+};
+
 // The launchers of one d (k_rows_<d>.cu).
 struct RowOps {
   cudaError_t (*set_smem)(int optin);
@@ -177,6 +197,9 @@ struct RowOps {
   void (*extra)(int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd);
   // phase pass: `blocks` CTAs of 128 threads, wpl (1, 2 or 4) elements a lane
   void (*phase)(int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd);
+  // frame pass: `blocks` CTAs of `warps` (1 to 4) warps, 32 shots each
+  size_t (*frame_smem)(const RowFrameDesc& f, int warps);
+  void (*frame)(int blocks, int warps, size_t smem, cudaStream_t s, const RowFrameDesc& f);
 };
 const RowOps& row_ops_2();
 const RowOps& row_ops_3();

@@ -1,6 +1,7 @@
 // Row form of the x / z pass (rows.cuh), device side: the raw, chain and extra
 // passes.  Instantiated for d = 2, 3, 5 and 7 in k_rows_<d>.cu.
 #pragma once
+#include "philox.cuh"
 #include "planes3.cuh"
 #include "rows.cuh"
 #include "trace_split_u8.cuh"
@@ -1414,6 +1415,260 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// ---------------------------------------------------------------- frame pass
+
+// Pauli frames (k_frame.cu: the rules) of 32 shots a warp, as bit planes: the
+// frame of a shot is one more column under the gates, so the words X[q], Z[q]
+// of 32 shots walk the row program's layers, a lane to an op.  Frame draws are
+// made by lanes as shots and turned into words by ballots; N1 samples likewise,
+// for d = 2 from the coin pass's masks (the few ordinals that any of the 32
+// shots fires, behind a bitmap), else by atomics into a word per ordinal.  The
+// record words stay in shared memory and leave as bytes at the end, a lane to
+// a measurement.
+// Bound by the Philox blocks of the draws.
+template <int D>
+struct FrameSmem {
+  using T = typename El<D>::T;
+  int fb, cb;              // Philox blocks of the frame draws, of the coins (odd d)
+  size_t ordf, ordc, warp0, x, z, rec, fire, warp;
+  __host__ __device__ FrameSmem(int n, int nm, int nused, int nchunk, int cap) {
+    auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    fb = (n + nm + 3) / 4;
+    cb = D == 2 ? 0 : (nused + 3) / 4;
+    ordf = kRawOps * 16 + up(4 * (kRawLayers + 1));
+    ordc = ordf + (size_t)fb * sizeof(CoinOrdinal);
+    warp0 = ordc + (size_t)cb * sizeof(CoinOrdinal);
+    x = 0;
+    z = x + up((size_t)n * sizeof(T));
+    rec = z + up((size_t)n * sizeof(T));
+    fire = rec + up((size_t)nm * sizeof(T));
+    warp = fire + up(D == 2 ? (size_t)nchunk * 8 + (size_t)cap * 8 : (size_t)nused * 2 * sizeof(T));
+  }
+};
+
+template <int D>
+__global__ void __launch_bounds__(128) k_rows_frame(const RowFrameDesc fd) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const FrameSmem<D> L_(fd.n, fd.nm, fd.nused, fd.nchunk, fd.cap);
+  const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5;
+  const int n = fd.n, nm = fd.nm;
+  uint4* wops = reinterpret_cast<uint4*>(smem);
+  uint32_t* wlay = reinterpret_cast<uint32_t*>(smem + kRawOps * 16);
+  CoinOrdinal* ordf = reinterpret_cast<CoinOrdinal*>(smem + L_.ordf);
+  CoinOrdinal* ordc = reinterpret_cast<CoinOrdinal*>(smem + L_.ordc);
+  uint8_t* mem = smem + L_.warp0 + warp * L_.warp;
+  T* X = reinterpret_cast<T*>(mem + L_.x);
+  T* Z = reinterpret_cast<T*>(mem + L_.z);
+  T* rec = reinterpret_cast<T*>(mem + L_.rec);  // the z drawn after a measurement, then its record word
+  uint32_t* bm = reinterpret_cast<uint32_t*>(mem + L_.fire);  // d = 2: fired ordinals, entries before the chunk, entries
+  uint2* ent = reinterpret_cast<uint2*>(bm + 2 * fd.nchunk);
+  T* fire = reinterpret_cast<T*>(mem + L_.fire);  // odd d: x and z words of every ordinal
+  const PhiloxKeys K(fd.seed);
+  for (int i = t; i < L_.fb; i += nt) ordf[i] = coin_ordinal(K, (uint32_t)i, 0u, 3u);
+  for (int i = t; i < L_.cb; i += nt) ordc[i] = coin_ordinal(K, (uint32_t)i, 0u, 1u);
+  __syncthreads();
+  const long long first = ((long long)blockIdx.x * (nt >> 5) + warp) * 32;  // of the launch's shots
+  const long long rel = first + lane;
+  const bool live = rel < fd.nshots;
+  const uint32_t shot = (uint32_t)(fd.shot0 + rel);  // shots are below 2^32: shot_hi 0
+  const uint2 sh = coin_shot(K, shot, 0u);
+  // frame draws: z of qudit e at the start (e < n), after measurement e - n
+  for (int b = 0; b < L_.fb; ++b) {
+    const uint4 w = coin_block(K, ordf[b], sh);
+    const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+    T mine = E_::zero();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = mulshift(v[q], D);
+      T word;
+      if constexpr (D == 2) {
+        word = __ballot_sync(0xffffffffu, r);
+      } else if constexpr (D == 3) {
+        word = make_uint2(__ballot_sync(0xffffffffu, r == 1), __ballot_sync(0xffffffffu, r == 2));
+      } else {
+        word = make_uint4(__ballot_sync(0xffffffffu, r & 1), __ballot_sync(0xffffffffu, r & 2),
+                          __ballot_sync(0xffffffffu, r & 4), 0u);
+      }
+      if (lane == q) mine = word;
+    }
+    const int e = 4 * b + lane;
+    if (lane < 4 && e < n + nm) {
+      if (e < n) Z[e] = mine; else rec[e - n] = mine;
+    }
+  }
+  for (int q = lane; q < n; q += 32) X[q] = E_::zero();
+  // N1 samples
+  if constexpr (D == 2) {
+    int total = 0;
+    for (int c0 = 0; c0 < fd.nchunk; c0 += 8) {  // eight loads in flight
+      uint2 mq[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        mq[q] = make_uint2(0u, 0u);
+        if (live && c0 + q < fd.nchunk) mq[q] = __ldcs(fd.masks + (size_t)(c0 + q) * fd.mshots + fd.mrel + rel);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint2 m = mq[q];
+        const uint32_t any = __reduce_or_sync(0xffffffffu, m.x | m.y);
+        if (lane == 0 && c0 + q < fd.nchunk) {
+          bm[c0 + q] = any;
+          bm[fd.nchunk + c0 + q] = (uint32_t)total;
+        }
+        for (uint32_t a = any; a; a &= a - 1u, ++total) {
+          const int i = __ffs(a) - 1;
+          const uint32_t fx = __ballot_sync(0xffffffffu, (m.x >> i) & 1u);
+          const uint32_t fz = __ballot_sync(0xffffffffu, (m.y >> i) & 1u);
+          if (lane == 0 && total < fd.cap) ent[total] = make_uint2(fx, fz);
+        }
+      }
+    }
+  } else {
+    for (int i = lane; i < 2 * fd.nused; i += 32) fire[i] = E_::zero();
+    __syncwarp();
+    for (int b = 0; b < L_.cb; ++b) {
+      const uint4 w = coin_block(K, ordc[b], sh);
+      const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+      uint32_t f = 0u;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = 4 * b + q;
+        if (j < fd.nused) {
+          const uint2 nh = __ldg(fd.nhdr + j);
+          if (v[q] >= nh.x && nh.y != OP_N1OFF) f |= 1u << q;
+        }
+      }
+      while (live && f) {
+        const int j = 4 * b + __ffs(f) - 1;
+        f &= f - 1u;
+        const int2 ab = noise_choice(__ldg(&fd.nhdr[j].y), D, fd.seed, (long long)shot, (uint32_t)j);
+        E_::put(fire + 2 * j, lane, ab.x);
+        E_::put(fire + 2 * j + 1, lane, ab.y);
+      }
+    }
+  }
+  __syncwarp();
+  // words (x, z) of N1 ordinal j
+  auto sample = [&](uint32_t j, T& fx, T& fz) {
+    if constexpr (D == 2) {
+      const uint32_t b = bm[j >> 5], i = j & 31u;
+      fx = fz = 0u;
+      if (!((b >> i) & 1u)) return;
+      const uint32_t k = bm[fd.nchunk + (j >> 5)] + (uint32_t)__popc(b & ((1u << i) - 1u));
+      if (k < (uint32_t)fd.cap) {
+        fx = ent[k].x;
+        fz = ent[k].y;
+      } else {  // more fires than entries: gather the word from the masks
+        for (int s = 0; s < 32 && first + s < fd.nshots; ++s) {
+          const uint2 m = __ldg(fd.masks + (size_t)(j >> 5) * fd.mshots + fd.mrel + first + s);
+          fx |= ((m.x >> i) & 1u) << s;
+          fz |= ((m.y >> i) & 1u) << s;
+        }
+      }
+    } else {
+      fx = fire[2 * j];
+      fz = fire[2 * j + 1];
+    }
+  };
+  // the layers; a window's ops are staged for all warps, their N1 riders turned
+  // from row numbers into ordinals + 1
+  auto ordinal = [&](uint32_t r) { return r ? (__ldg(&fd.xinfo[r - 1u].y) & 0x3fffffffu) + 1u : 0u; };
+  auto staged = [&](uint32_t k) {
+    uint4 o = __ldg(fd.ops + k);
+    if (o.x & kRopN) {
+      if (!(o.x & kRopM)) o.z = ordinal(o.z);
+      o.w = ordinal(o.w);
+    }
+    return o;
+  };
+  auto step = [&](const uint4 o) {
+    const uint32_t w = o.x;
+    const int i = (int)(w & 0x7ffu), j = (int)((w >> 11) & 0x7ffu);
+    const T xa = X[i], za = Z[i], xb = X[j], zb = Z[j];
+    const bool mh = w & (kRopH | kRopHInv), mc = w & (kRopC | kRopCInv);
+    T nx, nz, nt = xb, zt = zb;
+    if constexpr (D == 2) {
+      nx = mh ? za : xa;
+      nz = mh ? xa : za ^ (mc ? zb : (w & (kRopP | kRopPInv)) ? xa : 0u);
+      nt = xb ^ (mc ? xa : 0u);
+    } else {
+      using U = Unit<D>;
+      const uint32_t vh = lane_mask(mh), vc = lane_mask(mc);
+      const uint32_t mt = lane_mask(w & (kRopC | kRopCInv | kRopP | kRopPInv)), mn = lane_mask(w & (kRopC | kRopPInv));
+      const T t0 = U::pick(vc, zb, xa);
+      const T tt = U::mask(U::pick(mn, U::neg(t0), t0), mt);
+      const T xn = U::neg(xa), zn = U::neg(za);
+      nt = U::add(xb, U::mask(U::pick(lane_mask(w & kRopCInv), xn, xa), vc));
+      nz = U::pick(vh, U::pick(lane_mask(w & kRopHInv), xn, xa), U::add(za, tt));
+      nx = U::pick(vh, U::pick(lane_mask(w & kRopH), zn, za), xa);
+    }
+    if (w & kRopM) {
+      const bool reset = w & kRopReset;
+      nz = rec[o.y];
+      rec[o.y] = reset ? E_::zero() : nx;  // RESET records the reference value itself
+      if (reset) nx = E_::zero();
+    }
+    if (w & kRopN) {
+      T fx, fz;
+      const uint32_t a = (w & kRopM) ? o.w : o.z;
+      if (a) {
+        sample(a - 1u, fx, fz);
+        nx = E_::add(nx, fx);
+        nz = E_::add(nz, fz);
+      }
+      if (mc && o.w) {
+        sample(o.w - 1u, fx, fz);
+        nt = E_::add(nt, fx);
+        zt = E_::add(zb, fz);
+      }
+    }
+    X[i] = nx;
+    Z[i] = nz;
+    if (mc) {
+      X[j] = nt;
+      Z[j] = zt;
+    }
+  };
+  int l = 0;
+  while (l < fd.nlayers) {
+    __syncthreads();
+    const int nl = min(kRawLayers, fd.nlayers - l);
+    for (int i = t; i <= nl; i += nt) wlay[i] = __ldg(fd.lay + l + i);
+    __syncthreads();
+    const uint32_t w0 = wlay[0], wend = min(wlay[nl], w0 + (uint32_t)kRawOps);
+    for (uint32_t i = w0 + t; i < wend; i += nt) wops[i - w0] = staged(i);
+    __syncthreads();
+    int i = 0;
+    uint32_t b = w0;
+    for (; i < nl; ++i) {
+      const uint32_t e = wlay[i + 1];
+      const bool in = e <= wend;
+      if (!in && i > 0) break;
+      for (uint32_t k = b + lane; k < e; k += 32) step(in ? wops[k - w0] : staged(k));
+      b = e;
+      __syncwarp();
+    }
+    l += i;
+  }
+  // records: 32 measurements a turn, a byte per shot and lane
+  const int rows = (int)min(32LL, (long long)fd.nshots - first);
+  for (int k0 = 0; k0 < nm; k0 += 32) {
+    const int k = k0 + lane;
+    if (k < nm) {
+      const T x = rec[k];
+      const int rv = __ldg(fd.ref + k), det = rv & 0x80, v0 = rv & 0x7f;
+      uint8_t* o = fd.out + first * (long long)nm + k;
+      for (int s = 0; s < rows; ++s, o += nm) {
+        int v = v0 + E_::get(x, s);
+        if (v >= D) v -= D;
+        *o = (uint8_t)(v | det);
+      }
+    }
+  }
+}
+
 template <int D>
 size_t raw_smem(int n, int lg) {
   return round16(raw_bytes<D>(n, lg));
@@ -1443,6 +1698,7 @@ cudaError_t set_smem(int optin) {
   if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 1>, optin);
   if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 2>, optin);
   if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 4>, optin);
+  if (e == cudaSuccess) e = set_dynamic_smem(k_rows_frame<D>, optin);
   return e != cudaSuccess ? e : set_dynamic_smem(k_rows_extra<D>, optin);
 }
 
@@ -1487,6 +1743,13 @@ RowOps row_ops() {
     if (wpl == 1) k_rows_phase<D, 1><<<blocks, 128, smem, s>>>(descs, nd);
     else if (wpl == 2) k_rows_phase<D, 2><<<blocks, 128, smem, s>>>(descs, nd);
     else k_rows_phase<D, 4><<<blocks, 128, smem, s>>>(descs, nd);
+  };
+  o.frame_smem = [](const RowFrameDesc& f, int warps) {
+    const FrameSmem<D> l(f.n, f.nm, f.nused, f.nchunk, f.cap);
+    return l.warp0 + (size_t)warps * l.warp;
+  };
+  o.frame = [](int blocks, int warps, size_t smem, cudaStream_t s, const RowFrameDesc& f) {
+    k_rows_frame<D><<<blocks, 32 * warps, smem, s>>>(f);
   };
   return o;
 }

@@ -554,6 +554,7 @@ bool use_trace_u8(const Job& j, unsigned flags) {
 // [b, e) of the array, largest program first.
 struct RowGroup {
   int d, slice, b, e, tiles, lg, block, ctas, cblock, rawt, xctas;
+  int pb, pe;  // its programs in the row form's phase pass
   size_t raw_smem, chain_smem, extra_smem;
 };
 
@@ -662,11 +663,15 @@ int launch_row_raw(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStre
 }
 
 // fence: least shared memory of a chain CTA, 0 for none
-int launch_row_rest(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s, size_t fence) {
+int launch_row_chain(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s, size_t fence) {
   cudaError_t e = row_ops(g.d).chain(g.slice, g.ctas, g.cblock, g.rawt, g.lg, std::max(g.chain_smem, fence), s, rd + g.b, g.e - g.b);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "row chain pass launch");
-  if (g.xctas > 0) row_ops(g.d).extra(g.xctas, g.extra_smem, s, rd + g.b, g.e - g.b);
-  e = cudaGetLastError();
+  return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row chain pass launch");
+}
+
+int launch_row_extra(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s) {
+  if (g.xctas == 0) return SDIM_OK;
+  row_ops(g.d).extra(g.xctas, g.extra_smem, s, rd + g.b, g.e - g.b);
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row extra pass launch");
 }
 
@@ -720,7 +725,9 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   std::vector<const sdim_circuit*> rcirc;
   std::vector<RowGroup> rgroups;
   size_t rmem = 0;
-  auto add_row = [&](const sdim_circuit* c, uint4* mhdr, void* mrow, void* nrow, int rowb) {
+  std::vector<int> rjob;  // their indices in jobs (d = 2) or ujobs
+  auto add_row = [&](const sdim_circuit* c, uint4* mhdr, void* mrow, void* nrow, int rowb, size_t job) {
+    rjob.push_back((int)job);
     // memory offsets first, the base pointer once the buffer's size is known
     hr.push_back(row_desc(c, reinterpret_cast<uint8_t*>(rmem), mhdr, static_cast<uint8_t*>(mrow),
                           static_cast<uint8_t*>(nrow), rowb));
@@ -859,7 +866,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     }
     for (size_t i = 0; i < k; ++i) {
       hd[i].rows = jobs[i].rows ? 1 : 0;
-      if (hd[i].rows && !skip_xz) add_row(jobs[i].c, hd[i].mhdr, hd[i].mrow, hd[i].nrow, 4 * hd[i].tw);
+      if (hd[i].rows && !skip_xz) add_row(jobs[i].c, hd[i].mhdr, hd[i].mrow, hd[i].nrow, 4 * hd[i].tw, i);
     }
     if (k == 1 && !skip_xz && !hd[0].rows && jobs[0].c->nmeas > 0) {
       // one program: the x / z pass leaves the deterministic cross terms to
@@ -974,7 +981,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       }
       if (xm == kRowMode) {
         td.nhdr = const_cast<uint2*>(j.c->d_blob + j.c->rows.nhdr_off);
-        add_row(j.c, td.mhdr, td.mrow, td.nrow, td.sw);
+        add_row(j.c, td.mhdr, td.mrow, td.nrow, td.sw, i);
       }
     }
     du = static_cast<TraceDescU8*>(ctx->tdescs_u8.p);
@@ -998,10 +1005,14 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     dr = static_cast<RowDesc*>(ctx->rdescs.p);
     if ((rc = upload_fixed(ctx, dr, hr.data(), sizeof(RowDesc) * hr.size(), s)) != SDIM_OK) return rc;
   }
-  // the row form's phase pass: odd d, and d = 2 without fires to apply.  One
-  // element a lane up to kRowPhaseWarps warps in a launch, else two or four
+  // the row form's phase pass: odd d, and d = 2 without fires to apply, each row
+  // group's programs in a launch (those of a kept trace last, in one of their
+  // own).  One element a lane up to kRowPhaseWarps warps in a launch, else two
+  // or four
   std::vector<RowPhaseDesc> phr;
-  std::vector<int> phwpl, phjob;
+  std::vector<int> phjob;
+  struct PhaseRun { int b, e, wpl; };
+  std::vector<PhaseRun> pruns;
   auto add_phase = [&](const CircuitDesc& c, const uint4* mhdr, const void* mrow, const void* nrow, const uint2* nhdr,
                        int nm, int nn1, int rowb, bool resets, int job) {
     RowPhaseDesc p;
@@ -1019,43 +1030,69 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     phr.push_back(p);
     phjob.push_back(job);
   };
-  if (!colform)
-    for (size_t i = 0; i < k; ++i)
-      if (d2_packed(i))
-        add_phase(hd[i].c, hd[i].mhdr, hd[i].mrow, nullptr, nullptr, hd[i].nm, 0, 4 * hd[i].tw,
-                  jobs[i].c->rows.nx > 0, jobs[i].index);
-  for (size_t i = 0; i < ku; ++i)
-    if (ujobs[i].rows)
-      add_phase(hu[i].c, hu[i].mhdr, hu[i].mrow, hu[i].nrow, hu[i].nhdr, hu[i].nm, hu[i].nn1, hu[i].sw,
-                ujobs[i].c->rows.nx > 0, ujobs[i].index);
-  if (!phr.empty()) {
-    for (size_t b = 0; b < phr.size();) {
-      size_t e = b;
-      int wpl = 1;
-      for (; wpl <= 4; wpl <<= 1) {
-        long long warps = 0;
-        bool fits = true;
-        for (e = b; e < phr.size() && phr[e].c.d == phr[b].c.d; ++e) {
-          const int lg = row_phase_lg(phr[e].E, wpl);
-          fits &= (wpl << lg) >= phr[e].E;
-          warps += ((long long)phr[e].c.nshots * (1 << lg) + 31) / 32;
-        }
-        if (fits && (wpl == 4 || warps <= kRowPhaseWarps)) break;
+  auto end_phase_run = [&](int b) {
+    const int e = (int)phr.size();
+    if (b == e) return;
+    int wpl = 1;
+    for (; wpl < 4; wpl <<= 1) {
+      long long warps = 0;
+      bool fits = true;
+      for (int i = b; i < e; ++i) {
+        const int lg = row_phase_lg(phr[i].E, wpl);
+        fits &= (wpl << lg) >= phr[i].E;
+        warps += ((long long)phr[i].c.nshots * (1 << lg) + 31) / 32;
       }
-      int blocks = 0;
-      for (size_t i = b; i < e; ++i) {
-        phr[i].lg = row_phase_lg(phr[i].E, wpl);
-        phr[i].block_begin = blocks;
-        blocks += row_phase_blocks(phr[i]);
-        phwpl.push_back(wpl);
-      }
-      b = e;
+      if (fits && warps <= kRowPhaseWarps) break;
     }
+    int blocks = 0;
+    for (int i = b; i < e; ++i) {
+      phr[i].lg = row_phase_lg(phr[i].E, wpl);
+      phr[i].block_begin = blocks;
+      blocks += row_phase_blocks(phr[i]);
+    }
+    pruns.push_back(PhaseRun{b, e, wpl});
+  };
+  for (RowGroup& g : rgroups) {
+    g.pb = (int)phr.size();
+    for (int i = g.b; i < g.e; ++i) {
+      const size_t j = (size_t)rjob[i];
+      if (g.d != 2)
+        add_phase(hu[j].c, hu[j].mhdr, hu[j].mrow, hu[j].nrow, hu[j].nhdr, hu[j].nm, hu[j].nn1, hu[j].sw,
+                  ujobs[j].c->rows.nx > 0, ujobs[j].index);
+      else if (!colform && d2_packed(j))
+        add_phase(hd[j].c, hd[j].mhdr, hd[j].mrow, nullptr, nullptr, hd[j].nm, 0, 4 * hd[j].tw,
+                  jobs[j].c->rows.nx > 0, jobs[j].index);
+    }
+    g.pe = (int)phr.size();
+    end_phase_run(g.pb);
+  }
+  const bool kept_phase = skip_xz && !colform && d2_packed(0);
+  if (kept_phase) {
+    const int b = (int)phr.size();
+    add_phase(hd[0].c, hd[0].mhdr, hd[0].mrow, nullptr, nullptr, hd[0].nm, 0, 4 * hd[0].tw, jobs[0].c->rows.nx > 0,
+              jobs[0].index);
+    end_phase_run(b);
+  }
+  if (!phr.empty()) {
     if ((rc = ensure(ctx, ctx->pdescs, sizeof(RowPhaseDesc) * phr.size())) != SDIM_OK) return rc;
     if ((rc = upload_descs(ctx, ctx->pdescs.p, phr.data(), sizeof(RowPhaseDesc), phr.size(), offsetof(RowPhaseDesc, c),
                            [&](size_t i) { return phjob[i]; }, s)) != SDIM_OK)
       return rc;
   }
+  // the phase pass of descriptors [b, e) of phr (a run), none when empty
+  auto launch_row_phase = [&](int b, int e, cudaStream_t st) -> int {
+    for (const PhaseRun& r : pruns) {
+      if (r.b != b || r.e != e) continue;
+      size_t smem = 0;
+      for (int i = b; i < e; ++i) smem = std::max(smem, row_phase_smem(phr[i].pitch));
+      const RowPhaseDesc& last = phr[e - 1];
+      row_ops(last.c.d).phase(r.wpl, last.block_begin + row_phase_blocks(last), smem, st,
+                              static_cast<const RowPhaseDesc*>(ctx->pdescs.p) + b, e - b);
+      const cudaError_t le = cudaGetLastError();
+      if (le != cudaSuccess) return cuda_fail(ctx, le, "row phase pass launch");
+    }
+    return SDIM_OK;
+  };
   const bool d2_tab = k && !skip_xz && std::any_of(hd.begin(), hd.end(), [](const TraceDesc& t) { return !t.rows; });
   if (coins) CK(cudaEventRecord(ctx->ev_fork, s));
   // odd d: the x / z pass form of each program (odd_xz_mode)
@@ -1074,10 +1111,12 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   for (size_t b = 0; b < ku;) {
     const int v = trace_u8_variant(hu[b].c.d);
     const int mode = xmode[b];
+    if (mode == kRowMode) {
+      ++b;
+      continue;
+    }
     size_t e = b;
-    auto slice = [&](size_t i) { return row_slice(row_elems(hu[i].c.n)); };
-    while (e < ku && trace_u8_variant(hu[e].c.d) == v && xmode[e] == mode && (mode != kRowMode || slice(e) == slice(b)))
-      ++e;
+    while (e < ku && trace_u8_variant(hu[e].c.d) == v && xmode[e] == mode) ++e;
     runs.push_back(Run{b, e, v, mode, slot_total});
     if (mode == 2) {
       const size_t grid = std::min<size_t>(e - b, 2 * (size_t)ctx->num_sms);
@@ -1102,18 +1141,44 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   // the d = 2 x / z passes run on s: all x / z passes of the batch start
   // together (the uneven batch: x / z stage 295 -> 229 ms)
   const bool d2_xz = k && !skip_xz;
-  const bool fan = runs.size() > 1 || (d2_xz && !runs.empty());
+  const bool fan = runs.size() + rgroups.size() + (d2_tab ? 1 : 0) > 1;
   if (fan) CK(cudaEventRecord(ctx->ev_xzf, s));
-  // ---- d = 2 x / z passes (none when a kept trace is valid).  One program in
-  // row form with a coin pass beside it: on the stream of highest priority, up
-  // to its column pass, since the coin pass's blocks take every SM that the
-  // short chain leaves and the passes after it would wait for them to drain
-  // (the L = 7 step: 381 us with them on the caller's stream)
+  bool used[sdim_ctx::kXzStreams] = {};
+  int next_stream = 0;
+  auto fan_stream = [&](cudaStream_t& st) -> int {
+    const int si = next_stream++ % sdim_ctx::kXzStreams;
+    st = ctx->xzs[si];
+    if (!used[si]) CK(cudaStreamWaitEvent(st, ctx->ev_xzf, 0));
+    used[si] = true;
+    return SDIM_OK;
+  };
+  // ---- coin pass on the second stream, alongside the x / z passes (independent work)
+  auto launch_coins = [&]() -> int {
+    CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
+    if (coins > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one coin pass");
+    if (timed) CK(cudaEventRecord(ctx->ev_c0, ctx->aux));
+    launch_coin_pass((int)coins, ctx->aux, dd, (int)k);
+    const cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) return cuda_fail(ctx, le, "coin pass launch");
+    if (timed) {
+      CK(cudaEventRecord(ctx->ev_c1, ctx->aux));
+      ctx->coin_recorded = true;
+    }
+    CK(cudaEventRecord(ctx->ev_join, ctx->aux));
+    return SDIM_OK;
+  };
+  // ---- x / z passes in row form, each group with its phase pass on a stream of
+  // its own where there are several.  One d = 2 program with a coin pass beside
+  // it: on the stream of highest priority, up to its column pass, since the
+  // coin pass's blocks take every SM that the short chain leaves and the passes
+  // after it would wait for them to drain (the L = 7 step: 381 us with them on
+  // the caller's stream)
   const bool d2_fast = k == 1 && coins && d2_xz && hd[0].rows;
-  const cudaStream_t xs = d2_fast ? ctx->fast : s;
-  if (d2_fast) CK(cudaStreamWaitEvent(xs, ctx->ev_fork, 0));
-  for (const RowGroup& g : rgroups)
-    if (g.d == 2 && (rc = launch_row_raw(ctx, g, dr, xs)) != SDIM_OK) return rc;
+  cudaStream_t xs = s;
+  if (d2_fast) {
+    xs = ctx->fast;
+    CK(cudaStreamWaitEvent(xs, ctx->ev_fork, 0));
+  }
   // shared-memory fence: a few x / z CTAs claim enough shared memory that no
   // coin-pass block fits beside them, so the coin warps do not take the issue
   // slots of the latency-bound x / z pass on its SM
@@ -1123,8 +1188,20 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     const long long cap = (long long)ctx->smem_optin - 4096;  // room for the kernel's static arrays
     return (size_t)std::max(0LL, std::min(fence, cap));
   };
-  for (const RowGroup& g : rgroups)
-    if (g.d == 2 && (rc = launch_row_rest(ctx, g, dr, xs, coin_fence(g.ctas * (g.e - g.b)))) != SDIM_OK) return rc;
+  bool coins_out = false;
+  for (const RowGroup& g : rgroups) {
+    cudaStream_t st = g.d == 2 ? xs : s;
+    if (fan && !(g.d == 2 && d2_fast) && (rc = fan_stream(st)) != SDIM_OK) return rc;
+    if ((rc = launch_row_raw(ctx, g, dr, st)) != SDIM_OK ||
+        (rc = launch_row_chain(ctx, g, dr, st, g.d == 2 ? coin_fence(g.ctas * (g.e - g.b)) : 0)) != SDIM_OK)
+      return rc;
+    if (g.d == 2 && d2_fast && !coins_out) {  // behind the chain, ahead of the passes after it
+      if ((rc = launch_coins()) != SDIM_OK) return rc;
+      coins_out = true;
+    }
+    if ((rc = launch_row_extra(ctx, g, dr, st)) != SDIM_OK) return rc;
+    if (fan && (rc = launch_row_phase(g.pb, g.pe, st)) != SDIM_OK) return rc;
+  }
   if (d2_tab) {
     int nmax = 1;
     for (size_t i = 0; i < k; ++i)
@@ -1145,26 +1222,14 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return cuda_fail(ctx, le, "trace pass launch");
   }
-  bool used[sdim_ctx::kXzStreams] = {};
   for (size_t r = 0; r < runs.size(); ++r) {
     const Run& run = runs[r];
     const size_t b = run.b, e = run.e;
     const int v = run.v, mode = run.mode;
     cudaStream_t rs = s;
-    if (fan) {
-      const int si = (int)(r % sdim_ctx::kXzStreams);
-      rs = ctx->xzs[si];
-      if (!used[si]) CK(cudaStreamWaitEvent(rs, ctx->ev_xzf, 0));
-      used[si] = true;
-    }
+    if (fan && (rc = fan_stream(rs)) != SDIM_OK) return rc;
     const int nmax = hu[b].c.n;
-    if (mode == kRowMode) {
-      for (const RowGroup& g : rgroups)
-        if (g.d == hu[b].c.d && g.slice == row_slice(row_elems(nmax)))
-          if ((rc = launch_row_raw(ctx, g, dr, rs)) != SDIM_OK ||
-              (rc = launch_row_rest(ctx, g, dr, rs, 0)) != SDIM_OK)
-            return rc;
-    } else if (mode >= 7) {
+    if (mode >= 7) {
       // d = 5, 7 on 4-bit lanes: one CTA per program, largest first
       const bool in_smem = mode == 7;
       const int dd = hu[b].c.d;
@@ -1238,19 +1303,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     }
   }
   if (d2_fast) CK(cudaEventRecord(ctx->ev_fast, xs));
-  // ---- coin pass on the second stream, alongside the x / z passes (independent work)
   if (coins) {
-    CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
-    if (coins > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one coin pass");
-    if (timed) CK(cudaEventRecord(ctx->ev_c0, ctx->aux));
-    launch_coin_pass((int)coins, ctx->aux, dd, (int)k);
-    const cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) return cuda_fail(ctx, le, "coin pass launch");
-    if (timed) {
-      CK(cudaEventRecord(ctx->ev_c1, ctx->aux));
-      ctx->coin_recorded = true;
-    }
-    CK(cudaEventRecord(ctx->ev_join, ctx->aux));
+    if (!coins_out && (rc = launch_coins()) != SDIM_OK) return rc;
     CK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
   }
   if (d2_fast) CK(cudaStreamWaitEvent(s, ctx->ev_fast, 0));
@@ -1281,23 +1335,10 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return cuda_fail(ctx, le, "record pass launch");
   }
-  // row form: one launch per d and elements a lane
-  if (!phr.empty()) {
-    for (size_t b = 0; b < phr.size();) {
-      size_t e = b;
-      size_t smem = 0;
-      int blocks = 0;
-      for (; e < phr.size() && phr[e].c.d == phr[b].c.d && phwpl[e] == phwpl[b]; ++e) {
-        smem = std::max(smem, row_phase_smem(phr[e].pitch));
-        blocks = phr[e].block_begin + row_phase_blocks(phr[e]);
-      }
-      row_ops(phr[b].c.d).phase(phwpl[b], blocks, smem, s, static_cast<const RowPhaseDesc*>(ctx->pdescs.p) + b,
-                                (int)(e - b));
-      const cudaError_t le = cudaGetLastError();
-      if (le != cudaSuccess) return cuda_fail(ctx, le, "row phase pass launch");
-      b = e;
-    }
-  }
+  if (!fan)
+    for (const RowGroup& g : rgroups)
+      if ((rc = launch_row_phase(g.pb, g.pe, s)) != SDIM_OK) return rc;
+  if (kept_phase && (rc = launch_row_phase(pruns.back().b, pruns.back().e, s)) != SDIM_OK) return rc;
   for (size_t b = colform ? k : 0; b < k;) {
     if (d2_packed(b)) {
       ++b;

@@ -57,13 +57,12 @@ struct sdim_ctx {
   int64_t gmem_bytes = 0;
   size_t gmem_slot_budget = (size_t)8 << 30;
   std::string err;
-  DevBuf descs, counters, status, gslots, out, snap, arena, tdescs, trace, masks, tdescs_u8, trace_u8, xz_u8;
+  DevBuf descs, counters, status, gslots, out, snap, arena, tdescs, trace, masks, trace_u8, xz_u8;
   DevBuf gslots_xz;  // d = 2 x / z pass tableaux in global memory (gslots: the shot-group engines')
   DevBuf cols;       // record columns of a d = 2 trace program (trace_cols.cuh)
   DevBuf dsnap;      // its x / z pass's deterministic snapshots (TraceDesc::snap)
   DevBuf cdet;       // deterministic slice sums of the odd-d cluster x / z passes (TraceDescU8::dsum)
-  DevBuf rdescs, rows;  // row form of the x / z pass (rows.cuh): descriptors, rows and updates
-  DevBuf pdescs;        // its phase pass's descriptors
+  DevBuf rows;          // row form of the x / z pass (rows.cuh): rows and updates
   DevBuf fdescs;        // the frame route's coin pass
   cudaStream_t aux = nullptr;                      // coin pass, concurrent with the x / z pass
   cudaStream_t fast = nullptr;                     // d = 2 row form beside a coin pass: the highest priority
@@ -99,6 +98,8 @@ struct sdim_ctx {
   double last_ms = 0.0;
   double stage_ms[3] = {0.0, 0.0, 0.0};  // x / z passes, phase passes, other engines
   double pass_ms[2] = {0.0, 0.0};        // x / z passes alone, coin pass alone
+  int* h_status = nullptr;      // page-locked copy of the status word, fetched behind a run's kernels
+  bool status_fetched = false;  // ... of the last run
   int smem_attr_set[V_COUNT] = {};
   bool trace_smem_set = false;
   bool rows_smem_set = false;
@@ -299,9 +300,22 @@ Plan plan_launch(const sdim_ctx* ctx, int variant, size_t hot, size_t big, long 
   return p;
 }
 
+// The status word into page-locked memory, behind the run's kernels on s: the
+// run's own synchronisation then covers it (a blocking copy of its own took
+// about 8 us).
+int fetch_status(sdim_ctx* ctx, cudaStream_t s) {
+  CK(cudaMemcpyAsync(ctx->h_status, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  ctx->status_fetched = true;
+  return SDIM_OK;
+}
+
+// The last run's status, after its stream was synchronised.
 int read_status(sdim_ctx* ctx) {
   int st = 0;
-  CK(cudaMemcpy(&st, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost));
+  if (ctx->status_fetched)
+    st = *static_cast<volatile int*>(ctx->h_status);
+  else
+    CK(cudaMemcpy(&st, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost));
   if (st == DEV_OK) return SDIM_OK;
   const char* why = st == DEV_BAD_OPCODE ? "bad opcode" : st == DEV_BAD_QUDIT ? "qudit index out of range"
                                                                                  : "slot too small";
@@ -359,6 +373,8 @@ int finish(sdim_ctx* ctx, cudaStream_t s, unsigned flags) {
   }
   cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) return cuda_fail(ctx, le, "kernel launch");
+  const int frc = fetch_status(ctx, s);
+  if (frc != SDIM_OK) return frc;
   if (flags & SDIM_FLAG_ASYNC) {
     ctx->xz_pending = nullptr;  // not checked, so a trace written now is not kept valid
     ctx->pend_trace = ctx->pend_cols = false;
@@ -424,18 +440,43 @@ int upload_descs(sdim_ctx* ctx, void* dst, const void* src, size_t each, size_t 
   return SDIM_OK;
 }
 
-// The same for descriptors that hold no seed.
-int upload_fixed(sdim_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+// The trace engines' descriptor arrays of one run, uploaded together.
+struct DescPack {
+  struct Seeded { size_t at; int job; };  // a CircuitDesc's byte offset and its job's batch index
+  std::vector<uint8_t> host;
+  std::vector<Seeded> seeded;
+  // appends an array (256-byte aligned) and returns its offset; cdesc_off:
+  // where each descriptor holds its CircuitDesc, SIZE_MAX for none
+  template <class T, class JobIndex>
+  size_t add(const std::vector<T>& v, size_t cdesc_off, JobIndex job) {
+    const size_t off = (host.size() + 255) & ~(size_t)255;
+    host.resize(off + sizeof(T) * v.size());
+    if (!v.empty()) std::memcpy(host.data() + off, v.data(), sizeof(T) * v.size());
+    for (size_t i = 0; cdesc_off != SIZE_MAX && i < v.size(); ++i)
+      seeded.push_back(Seeded{off + i * sizeof(T) + cdesc_off, job(i)});
+    return off;
+  }
+};
+
+int upload_pack(sdim_ctx* ctx, DescPack& p, DevBuf& buf, cudaStream_t s) {
+  if (p.host.empty()) return SDIM_OK;
+  int rc = ensure(ctx, buf, p.host.size());
+  if (rc != SDIM_OK) return rc;
+  const void* src = p.host.data();
   GraphCapture* g = ctx->capture;
   if (g && !g->sizing) {
-    if (g->used + bytes > g->cap) return fail(ctx, SDIM_ECUDA, "graph descriptor staging overflow");
-    std::memcpy(g->host + g->used, src, bytes);
+    if (g->used + p.host.size() > g->cap) return fail(ctx, SDIM_ECUDA, "graph descriptor staging overflow");
+    std::memcpy(g->host + g->used, src, p.host.size());
     src = g->host + g->used;
-    g->used += (bytes + 255) & ~(size_t)255;
+    for (const DescPack::Seeded& d : p.seeded) {
+      g->seed_at.emplace_back(g->used + d.at + offsetof(CircuitDesc, seed), d.job);
+      g->shot0_at.emplace_back(g->used + d.at + offsetof(CircuitDesc, shot0), d.job);
+    }
+    g->used += (p.host.size() + 255) & ~(size_t)255;
   } else if (g) {
-    g->need += (bytes + 255) & ~(size_t)255;
+    g->need += (p.host.size() + 255) & ~(size_t)255;
   }
-  CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(buf.p, src, p.host.size(), cudaMemcpyHostToDevice, s));
   return SDIM_OK;
 }
 
@@ -474,7 +515,7 @@ bool use_trace(const Job& j, unsigned flags) {
   if (flags & (SDIM_FLAG_PLAIN | SDIM_FLAG_PER_SHOT | SDIM_FLAG_TEAM_WARP | SDIM_FLAG_TEAM_CTA |
                SDIM_FLAG_NO_TRACE))
     return false;
-  if (j.c->d != 2 || trace_words(j.c->n) == 0 || !j.c->d_steps || j.nshots <= 0) return false;
+  if (j.c->d != 2 || trace_words(j.c->n) == 0 || j.nshots <= 0 || !(j.c->d_steps || row_form(j.c, flags))) return false;
   return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || row_form(j.c, flags);
 }
 
@@ -716,7 +757,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     for (Job& j : *list) {
       if (!row_form(j.c, flags)) continue;
       const size_t b = row_bytes(j.c->n, j.c->d, j.c->nmeas, j.c->rows.nx, j.c->rows.nk).total;
-      if (row_total + b > ctx->gmem_slot_budget) continue;
+      const bool other = j.c->d != 2 || j.c->d_steps;  // sdim_run_tables builds schedules when the rows exceed the budget
+      if (other && row_total + b > ctx->gmem_slot_budget) continue;
       row_total += b;
       j.rows = true;
     }
@@ -787,7 +829,6 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       total += trace_bytes(jobs[i].c->nmeas, jobs[i].c->nn1, trace_words(jobs[i].c->n));
     }
     if (!keep && (rc = ensure(ctx, ctx->trace, std::max<size_t>(total, 256))) != SDIM_OK) return rc;
-    if ((rc = ensure(ctx, ctx->tdescs, sizeof(TraceDesc) * k)) != SDIM_OK) return rc;
     // fire masks: a word pair per 32 N1 ordinals per shot and the chunk map,
     // within a budget
     constexpr size_t kMaskBudget = (size_t)1 << 30;
@@ -899,10 +940,6 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       hd[0].cols = static_cast<uint32_t*>(cb.p);
       hd[0].nw = cnw;
     }
-    dd = static_cast<TraceDesc*>(ctx->tdescs.p);
-    if ((rc = upload_descs(ctx, dd, hd.data(), sizeof(TraceDesc), k, offsetof(TraceDesc, c),
-                           [&](size_t i) { return jobs[i].index; }, s)) != SDIM_OK)
-      return rc;
   }
   auto d2_packed = [&](size_t i) { return packed_job(jobs[i]); };
   // ---- odd-d descriptors
@@ -941,7 +978,6 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     }
     if ((rc = ensure(ctx, ctx->trace_u8, std::max<size_t>(total, 256))) != SDIM_OK) return rc;
     if (dtotal && (rc = ensure(ctx, ctx->cdet, dtotal)) != SDIM_OK) return rc;
-    if ((rc = ensure(ctx, ctx->tdescs_u8, sizeof(TraceDescU8) * ku)) != SDIM_OK) return rc;
     long long groups = 0;
     for (size_t i = 0; i < ku; ++i) {
       const Job& j = ujobs[i];
@@ -984,15 +1020,10 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
         add_row(j.c, td.mhdr, td.mrow, td.nrow, td.sw, i);
       }
     }
-    du = static_cast<TraceDescU8*>(ctx->tdescs_u8.p);
-    if ((rc = upload_descs(ctx, du, hu.data(), sizeof(TraceDescU8), ku, offsetof(TraceDescU8, c),
-                           [&](size_t i) { return ujobs[i].index; }, s)) != SDIM_OK)
-      return rc;
   }
   RowDesc* dr = nullptr;
   if (!hr.empty()) {
     if ((rc = ensure(ctx, ctx->rows, std::max<size_t>(rmem, 256))) != SDIM_OK) return rc;
-    if ((rc = ensure(ctx, ctx->rdescs, sizeof(RowDesc) * hr.size())) != SDIM_OK) return rc;
     const size_t base = reinterpret_cast<size_t>(ctx->rows.p);
     for (RowDesc& r : hr) {
       uint8_t** ptrs[] = {&r.raw, &r.xraw, &r.kpart, &r.ksign, &r.opf};
@@ -1002,8 +1033,6 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       r.opw = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(r.opw) + base);
     }
     for (RowGroup& g : rgroups) plan_row_group(ctx, g, hr.data(), rcirc);
-    dr = static_cast<RowDesc*>(ctx->rdescs.p);
-    if ((rc = upload_fixed(ctx, dr, hr.data(), sizeof(RowDesc) * hr.size(), s)) != SDIM_OK) return rc;
   }
   // the row form's phase pass: odd d, and d = 2 without fires to apply, each row
   // group's programs in a launch (those of a kept trace last, in one of their
@@ -1073,11 +1102,20 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
               jobs[0].index);
     end_phase_run(b);
   }
-  if (!phr.empty()) {
-    if ((rc = ensure(ctx, ctx->pdescs, sizeof(RowPhaseDesc) * phr.size())) != SDIM_OK) return rc;
-    if ((rc = upload_descs(ctx, ctx->pdescs.p, phr.data(), sizeof(RowPhaseDesc), phr.size(), offsetof(RowPhaseDesc, c),
-                           [&](size_t i) { return phjob[i]; }, s)) != SDIM_OK)
-      return rc;
+  // ---- every descriptor array in one upload
+  const RowPhaseDesc* dp = nullptr;
+  {
+    DescPack pack;
+    const size_t od = pack.add(hd, offsetof(TraceDesc, c), [&](size_t i) { return jobs[i].index; });
+    const size_t ou = pack.add(hu, offsetof(TraceDescU8, c), [&](size_t i) { return ujobs[i].index; });
+    const size_t orow = pack.add(hr, SIZE_MAX, [](size_t) { return 0; });
+    const size_t op = pack.add(phr, offsetof(RowPhaseDesc, c), [&](size_t i) { return phjob[i]; });
+    if ((rc = upload_pack(ctx, pack, ctx->tdescs, s)) != SDIM_OK) return rc;
+    uint8_t* base = static_cast<uint8_t*>(ctx->tdescs.p);
+    dd = reinterpret_cast<TraceDesc*>(base + od);
+    du = reinterpret_cast<TraceDescU8*>(base + ou);
+    dr = reinterpret_cast<RowDesc*>(base + orow);
+    dp = reinterpret_cast<const RowPhaseDesc*>(base + op);
   }
   // the phase pass of descriptors [b, e) of phr (a run), none when empty
   auto launch_row_phase = [&](int b, int e, cudaStream_t st) -> int {
@@ -1087,7 +1125,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       for (int i = b; i < e; ++i) smem = std::max(smem, row_phase_smem(phr[i].pitch));
       const RowPhaseDesc& last = phr[e - 1];
       row_ops(last.c.d).phase(r.wpl, last.block_begin + row_phase_blocks(last), smem, st,
-                              static_cast<const RowPhaseDesc*>(ctx->pdescs.p) + b, e - b);
+                              dp + b, e - b);
       const cudaError_t le = cudaGetLastError();
       if (le != cudaSuccess) return cuda_fail(ctx, le, "row phase pass launch");
     }
@@ -1404,8 +1442,9 @@ int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsig
   std::vector<Job> jobs, tjobs, ujobs;
   for (const Job& j : all_jobs) (use_trace(j, flags) ? tjobs : use_trace_u8(j, flags) ? ujobs : jobs).push_back(j);
   int rc;
+  ctx->status_fetched = false;
   if ((rc = ensure(ctx, ctx->status, sizeof(int))) != SDIM_OK) return rc;
-  if ((rc = ensure(ctx, ctx->counters, sizeof(unsigned long long) * V_COUNT)) != SDIM_OK) return rc;
+  if (!jobs.empty() && (rc = ensure(ctx, ctx->counters, sizeof(unsigned long long) * V_COUNT)) != SDIM_OK) return rc;
   if ((rc = ensure(ctx, ctx->descs, sizeof(CircuitDesc) * std::max<size_t>(jobs.size(), 1))) != SDIM_OK)
     return rc;
   std::vector<int> var(jobs.size());
@@ -1449,7 +1488,7 @@ int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsig
                                         [&](size_t k) { return jobs[order[k]].index; }, s)) != SDIM_OK)
     return rc;
   CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(int), s));
-  CK(cudaMemsetAsync(ctx->counters.p, 0, sizeof(unsigned long long) * V_COUNT, s));
+  if (!jobs.empty()) CK(cudaMemsetAsync(ctx->counters.p, 0, sizeof(unsigned long long) * V_COUNT, s));
   if (flags & SDIM_FLAG_TIME) CK(cudaEventRecord(ctx->ev0, s));
   int* status = static_cast<int*>(ctx->status.p);
   // with trace programs in the batch the shot-group engines run on a stream
@@ -1685,6 +1724,31 @@ void append_layers_u8(std::vector<uint2>& dev, size_t op_begin, size_t nops, int
   dev.insert(dev.end(), out.begin(), out.end());
 }
 
+// N1 coin thresholds of a d = 2 program (dense, 64-ordinal padded, 16-byte
+// aligned) and its (threshold, opcode) pairs, appended to dev.
+void append_coins(std::vector<uint2>& dev, size_t op_begin, size_t nops, TraceSchedule& out) {
+  if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
+  std::vector<uint32_t> thr;
+  std::vector<uint2> hdr;
+  int used = 0;
+  for (size_t i = op_begin; i < op_begin + nops; ++i) {
+    const uint32_t op = dev[i].x & kOpMask;
+    if (op == OP_M || op == OP_RESET) used = (int)thr.size();
+    if (op == OP_N1D || op == OP_N1F || op == OP_N1P || op == OP_N1OFF) {
+      const uint32_t t = op == OP_N1OFF ? 0xffffffffu : dev[i].y;
+      thr.push_back(t);
+      hdr.push_back(make_uint2(t, op));
+    }
+  }
+  out.nn1_used = used;
+  while (thr.size() % 64) thr.push_back(0xffffffffu);
+  out.nthr_off = (int64_t)dev.size();
+  for (size_t i = 0; i < thr.size(); i += 2) dev.push_back(make_uint2(thr[i], thr[i + 1]));
+  out.nhdr_off = (int64_t)dev.size();
+  dev.insert(dev.end(), hdr.begin(), hdr.end());
+  if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
+}
+
 // Layered schedule of a d = 2 program for the trace engine's x / z pass,
 // appended to dev after the instruction words (16-byte aligned):
 //   steps[s] = {kind, first, count, 0}: kind 0 is a gate layer -- ops on
@@ -1803,26 +1867,7 @@ void append_schedule(std::vector<uint2>& dev, size_t op_begin, size_t nops, int 
   out.wins_off = put(wins);
   out.nsteps = (int)steps.size();
   out.nwins = (int)wins.size();
-  // N1 coin thresholds (dense, 64-ordinal padded, 16-byte aligned) and (threshold, opcode) pairs
-  std::vector<uint32_t> thr;
-  std::vector<uint2> hdr;
-  int used = 0;
-  for (size_t i = op_begin; i < op_begin + nops; ++i) {
-    const uint32_t op = dev[i].x & kOpMask;
-    if (op == OP_M || op == OP_RESET) used = (int)thr.size();
-    if (op == OP_N1D || op == OP_N1F || op == OP_N1P || op == OP_N1OFF) {
-      const uint32_t t = op == OP_N1OFF ? 0xffffffffu : dev[i].y;
-      thr.push_back(t);
-      hdr.push_back(make_uint2(t, op));
-    }
-  }
-  out.nn1_used = used;
-  while (thr.size() % 64) thr.push_back(0xffffffffu);
-  out.nthr_off = (int64_t)dev.size();
-  for (size_t i = 0; i < thr.size(); i += 2) dev.push_back(make_uint2(thr[i], thr[i + 1]));
-  out.nhdr_off = (int64_t)dev.size();
-  dev.insert(dev.end(), hdr.begin(), hdr.end());
-  if (dev.size() & 1) dev.push_back(make_uint2(0u, 0u));
+  append_coins(dev, op_begin, nops, out);
 }
 
 // Row program (rows.cuh) of a program's instruction words, appended to dev:
@@ -2149,6 +2194,12 @@ int sdim_ctx_create(int device, sdim_ctx** out) {
       delete ctx;
       return SDIM_ECUDA;
     }
+  if (cudaMallocHost(reinterpret_cast<void**>(&ctx->h_status), sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    delete ctx;
+    return SDIM_ECUDA;
+  }
+  *ctx->h_status = 0;
   ctx->num_sms = prop.multiProcessorCount;
   ctx->smem_optin = (int)prop.sharedMemPerBlockOptin;
   ctx->smem_per_sm = (int)prop.sharedMemPerMultiprocessor;
@@ -2171,11 +2222,12 @@ int sdim_ctx_destroy(sdim_ctx* ctx) {
   cudaStreamSynchronize(ctx->cps);
   for (int i = 0; i < sdim_ctx::kXzStreams; ++i) cudaStreamSynchronize(ctx->xzs[i]);
   DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap, &ctx->arena,
-                    &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8, &ctx->xz_u8,
-                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rdescs, &ctx->rows, &ctx->pdescs, &ctx->fdescs};
+                    &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->trace_u8, &ctx->xz_u8,
+                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rows, &ctx->fdescs};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   if (ctx->staging) cudaFreeHost(ctx->staging);
+  if (ctx->h_status) cudaFreeHost(ctx->h_status);
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);
   cudaEventDestroy(ctx->ev_xz);
@@ -2226,9 +2278,9 @@ int sdim_memory_info(sdim_ctx* ctx, int64_t info[3]) {
   info[0] = (int64_t)free_b;
   info[1] = (int64_t)total_b;
   const DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap,
-                          &ctx->arena, &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->tdescs_u8, &ctx->trace_u8,
+                          &ctx->arena, &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->trace_u8,
                           &ctx->xz_u8, &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet,
-                          &ctx->rdescs, &ctx->rows, &ctx->pdescs, &ctx->fdescs};
+                          &ctx->rows, &ctx->fdescs};
   int64_t held = 0;
   for (const DevBuf* b : bufs) held += (int64_t)b->cap;
   info[2] = held;
@@ -2399,6 +2451,7 @@ int sdim_run(sdim_ctx* ctx, const sdim_circuit* c, uint64_t seed, int64_t shot0,
   } else if (bytes && !direct) {
     CK(cudaMemcpyAsync(out, ctx->out.p, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   }
+  if ((rc = fetch_status(ctx, ctx->stream)) != SDIM_OK) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   if (ctx->timing_pending) {
     const int trc = collect_times(ctx);
@@ -2549,6 +2602,7 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
     ctx->timing_pending = true;
   }
   if (bytes) CK(cudaMemcpyAsync(out, dst, bytes, cudaMemcpyDeviceToHost, s));
+  if ((rc = fetch_status(ctx, s)) != SDIM_OK) return rc;
   CK(cudaStreamSynchronize(s));
   if (ctx->timing_pending) {
     const int trc = collect_times(ctx);
@@ -2603,6 +2657,7 @@ int sdim_run_batch(sdim_ctx* ctx, int ncirc, const sdim_circuit* const* circs, c
     if (b && !direct[i])
       CK(cudaMemcpyAsync(outs[i], static_cast<uint8_t*>(ctx->out.p) + offs[i], b, cudaMemcpyDeviceToHost, s));
   }
+  if ((rc = fetch_status(ctx, s)) != SDIM_OK) return rc;
   if (flags & SDIM_FLAG_ASYNC) {
     // the caller keeps the (pinned) host buffers alive until sdim_query / sdim_sync
     ctx->last_stream = s;
@@ -2674,6 +2729,7 @@ int sdim_graph_create(sdim_ctx* parent, int ncirc, const sdim_circuit* const* ci
   cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
   if (e != cudaSuccess) return bail(cuda_fail(ctx, e, "cudaStreamBeginCapture"));
   rc = launch_jobs(ctx, jobs, ctx->stream, f);
+  if (rc == SDIM_OK) rc = fetch_status(ctx, ctx->stream);
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(ctx->stream, &graph);
   ctx->capture = nullptr;
@@ -2767,14 +2823,8 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
   std::vector<TraceSchedule> sch(ncirc);
   std::vector<int64_t> lay_off(ncirc, -1);
   std::vector<int> nlay(ncirc, 0);
-  // layered streams only serve the cluster x / z pass, which a batch takes
-  // only with fewer than num_sms / 2 odd-d programs (odd_xz_mode); larger
-  // batches skip building them (SDIM_FLAG_CLUSTER_XZ then walks the
-  // instructions as written)
-  int odd = 0;
-  for (int i = 0; i < ncirc; ++i) odd += d[i] != 2 ? 1 : 0;
-  const bool layered = 2 * odd < ctx->num_sms;
   std::vector<sdim_circuit> circs(ncirc);
+  size_t row_total = 0;
   int rc;
   for (int i = 0; i < ncirc; ++i) {
     op_off[i] = dev.size();
@@ -2791,13 +2841,29 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
     c.nn1 = nn1;
     c.nops_user = r1 - r0;
     c.nops = (int)(dev.size() - op_off[i]);
-    if (d[i] == 2 && trace_words(n[i]))
-      append_schedule(dev, op_off[i], (size_t)c.nops, n[i], kTraceWinSteps, kTraceWinOps, sch[i]);
-    if (d[i] != 2 && layered) append_layers_u8(dev, op_off[i], (size_t)c.nops, n[i], lay_off[i], nlay[i]);
     append_rows(dev, op_off[i], (size_t)c.nops, n[i], d[i], nmeas, c.rows);
+    if (row_form(&c, flags)) row_total += row_bytes(n[i], d[i], nmeas, c.rows.nx, c.rows.nk).total;
     c.variant = variant_for(d[i]);
     c.gvariant = group_variant_for(d[i], n[i], 0);
     c.gblock = variant_ops(c.gvariant).cta ? cta_block_for(n[i]) : 32;
+  }
+  // the tableau passes' streams where the row form does not take the program:
+  // the d = 2 schedule, and the layered stream of the cluster x / z pass, which
+  // a batch takes only with fewer than num_sms / 2 odd-d programs
+  // (odd_xz_mode; SDIM_FLAG_CLUSTER_XZ in a larger batch walks the instructions
+  // as written)
+  int odd = 0;
+  const bool rows_fit = row_total <= ctx->gmem_slot_budget;
+  auto by_rows = [&](int i) { return rows_fit && row_form(&circs[i], flags); };
+  for (int i = 0; i < ncirc; ++i) odd += d[i] != 2 && !by_rows(i) ? 1 : 0;
+  for (int i = 0; i < ncirc; ++i) {
+    const size_t ops = (size_t)circs[i].nops;
+    if (d[i] == 2 && trace_words(n[i])) {
+      if (by_rows(i)) append_coins(dev, op_off[i], ops, sch[i]);
+      else append_schedule(dev, op_off[i], ops, n[i], kTraceWinSteps, kTraceWinOps, sch[i]);
+    }
+    if (d[i] != 2 && !by_rows(i) && 2 * odd < ctx->num_sms)
+      append_layers_u8(dev, op_off[i], ops, n[i], lay_off[i], nlay[i]);
   }
   // instruction streams: pinned staging -> device arena, both owned by the context
   const size_t ob = std::max<size_t>(dev.size(), 1) * sizeof(uint2);
@@ -2819,15 +2885,17 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
   for (int i = 0; i < ncirc; ++i) {
     circs[i].d_ops = base + op_off[i];
     circs[i].d_blob = base;
+    if (sch[i].nthr_off >= 0) {
+      circs[i].d_nthr = reinterpret_cast<const uint32_t*>(base + sch[i].nthr_off);
+      circs[i].d_nhdr = base + sch[i].nhdr_off;
+      circs[i].nn1_used = sch[i].nn1_used;
+    }
     if (sch[i].steps_off >= 0) {
       circs[i].d_steps = reinterpret_cast<const uint4*>(base + sch[i].steps_off);
       circs[i].d_lops = reinterpret_cast<const uint4*>(base + sch[i].lops_off);
       circs[i].d_wins = reinterpret_cast<const uint4*>(base + sch[i].wins_off);
-      circs[i].d_nthr = reinterpret_cast<const uint32_t*>(base + sch[i].nthr_off);
-      circs[i].d_nhdr = base + sch[i].nhdr_off;
       circs[i].nsteps = sch[i].nsteps;
       circs[i].nwins = sch[i].nwins;
-      circs[i].nn1_used = sch[i].nn1_used;
     }
     if (lay_off[i] >= 0) {
       circs[i].d_lay = base + lay_off[i];
@@ -2871,6 +2939,7 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
     if (b && !direct[i])
       CK(cudaMemcpyAsync(outs[i], static_cast<uint8_t*>(ctx->out.p) + offs[i], b, cudaMemcpyDeviceToHost, s));
   }
+  if ((rc = fetch_status(ctx, s)) != SDIM_OK) return rc;
   if (flags & SDIM_FLAG_ASYNC) return SDIM_OK;
   CK(cudaStreamSynchronize(s));
   if (ctx->timing_pending) {
@@ -2979,6 +3048,7 @@ int sdim_snapshot(sdim_ctx* ctx, const sdim_circuit* c, uint64_t seed, int64_t s
   cudaStream_t s = ctx->stream;
   CK(cudaMemcpyAsync(ctx->descs.p, &dsc, sizeof(dsc), cudaMemcpyHostToDevice, s));
   CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(int), s));
+  ctx->status_fetched = false;
   const int block = ops.cta ? cta_block_for(c->n) : 32;
   ops.snapshot(dim3(block), hot + (in_smem ? big : 0), s, static_cast<const CircuitDesc*>(ctx->descs.p), 0,
                static_cast<uint8_t*>(ctx->gslots.p), big, hot, in_smem ? 1 : 0, static_cast<int8_t*>(ctx->snap.p),

@@ -126,18 +126,21 @@ class Program:
                     (p.get("noise_channel"), p.get("channel"), p.get("prob")))
         return (gid, ins.qudit_index, ins.target_index)
 
+    def _program_content(self) -> tuple:
+        """The content of every instruction of every circuit (and each
+        circuit's qudit count)."""
+        content = self._instruction_content
+        circuits = self.circuits + ([self._applied_circuit()] if self._applied else [])
+        return tuple((c.num_qudits, tuple([content(o) for o in c.operations])) for c in circuits)
+
     def _program_key(self, noise: bool):
-        """Cache key of the encoded program: the content of every instruction
-        of every circuit (and each circuit's qudit count), read afresh on
+        """Cache key of the encoded program: its content, read afresh on
         every call as the reference re-reads ``circuit.operations`` on every
         simulate (sdim/program.py:311-320).  Added, removed, replaced,
         reordered or edited-in-place instructions all change it; object
         identities play no part, so a new instruction that reuses a freed
         object's address cannot alias an old one."""
-        content = self._instruction_content
-        circuits = self.circuits + ([self._applied_circuit()] if self._applied else [])
-        return (tuple((c.num_qudits, tuple([content(o) for o in c.operations])) for c in circuits),
-                bool(noise))
+        return (self._program_content(), bool(noise))
 
     def _applied_circuit(self) -> Circuit:
         c = Circuit(self.num_qudits, self.dimension)
@@ -147,7 +150,10 @@ class Program:
     def compile(self, noise: bool = True) -> DeviceProgram:
         """Encoded program on the device (cached while the circuits' content
         stays the same)."""
-        key = self._program_key(noise)
+        return self._compile(self._program_key(noise))
+
+    def _compile(self, key: tuple) -> DeviceProgram:
+        noise = key[1]
         hit = self._cache.get(key[1])
         if hit is not None and hit[0] == key[0]:
             return hit[1]
@@ -227,8 +233,9 @@ class Program:
         tableau shot 0, rows 1 .. shots-1 are Pauli-frame shots
         (sdim/program.py:45-165, 244-265); ``noise=False`` leaves N1 out of
         the frames too."""
-        ref = self.compile(False)
-        dp = self.compile(noise)
+        content = self._program_content()  # read once for both programs of this call
+        ref = self._compile((content, False))
+        dp = self._compile((content, bool(noise)))
         s = self._seed(seed)
         if out is None:
             out = np.empty((int(shots), dp.num_records), dtype=np.uint8)

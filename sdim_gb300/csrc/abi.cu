@@ -1223,7 +1223,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   auto coin_fence = [&](int ctas) -> size_t {
     if (!coins || ctas > ctx->num_sms / 8) return 0;
     const long long fence = (long long)ctx->smem_per_sm - 2LL * ctx->smem_reserved - (long long)kCoinFenceSmem + 16;
-    const long long cap = (long long)ctx->smem_optin - 4096;  // room for the kernel's static arrays
+    const long long cap = (long long)ctx->smem_optin - 12288;  // room for the kernel's static arrays
     return (size_t)std::max(0LL, std::min(fence, cap));
   };
   bool coins_out = false;

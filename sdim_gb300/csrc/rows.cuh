@@ -92,7 +92,8 @@ struct RowDesc {
   uint8_t* kpart;  // d = 2: sign exponents per measurement and word, [nm][E]
   uint8_t* ksign;  // d = 2: sign exponents gathered from the updates, [nm]
   uint8_t* opf;    // factor rows F of the random measurements, [..][2 E]
-  int4* opm;       // their {pivot, exponent | commute parity << 8, ordinal, 0}
+  int4* opm;       // their {pivot, exponent | commute parity << 8, ordinal, 1 + last op of the panel
+                   // before it with its pivot (0: none) | no later one has it << 6}
   int* pop;        // first op of each panel, [panels + 1]
   uint32_t* opw;   // odd d: each panel's matrix W, [panels][32][8] words (k_rows.cu: PanelOps::Wt)
   uint4* mhdr;     // the trace

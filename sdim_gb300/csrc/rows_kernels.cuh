@@ -486,6 +486,8 @@ __device__ void stage_panel(PanelOps& po, typename El<D>::T* Fs, const RowDesc& 
     po.p[t] = m.x;
     po.e[t] = m.y;
     po.mord[t] = m.z;
+    po.dup[t] = (m.w & 63) - 1;
+    po.last[t] = m.w >> 6;
   }
   if constexpr (kFull) {
     if constexpr (D != 2) {
@@ -499,18 +501,7 @@ __device__ void stage_panel(PanelOps& po, typename El<D>::T* Fs, const RowDesc& 
   }
   __syncthreads();
   if constexpr (D != 2) {
-    if (t < nops) {
-      int dup = -1, last = 1;
-      for (int h = 0; h < nops; ++h)
-        if (po.p[h] == po.p[t]) {
-          if (h < t) dup = h;
-          if (h > t) last = 0;
-        }
-      po.dup[t] = dup;
-      po.last[t] = last;
-    }
     if constexpr (!kFull) {
-      __syncthreads();
       for (int i = t; i < 1024; i += nt) {
         const int h = i >> 5, k = i & 31;
         int g = 0;
@@ -534,33 +525,49 @@ __device__ void stage_panel(PanelOps& po, typename El<D>::T* Fs, const RowDesc& 
   __syncthreads();
 }
 
-// Odd d: buf[0, cnt) += sum of the panel's factor rows times ab[0, nops).  A
-// row of at most 16 elements leaves lanes over: they take their share of the
-// ops, and the partial sums meet by shuffles.
+// Odd d: the elements [e0, cnt) of a row, buf, += sum of the panel's factor
+// rows times ab[0, nops), 32 elements a turn, up to the last whole turn or one
+// that is more than half full; returns the elements done.  The multiples are
+// uniform over the warp, so each takes its cheapest form.
 template <int D>
-__device__ __forceinline__ void combine_row(const PanelOps& po, const typename El<D>::T* Fs, typename El<D>::T* buf,
-                                            int cnt, const int* ab) {
+__device__ __forceinline__ int combine_row(const PanelOps& po, const typename El<D>::T* Fs, typename El<D>::T* buf,
+                                           int cnt, const int* ab) {
   using E_ = El<D>;
   using T = typename E_::T;
   const int lane = threadIdx.x & 31, nops = po.nops;
-  int G = 32;
-  while (G > 1 && (G >> 1) >= cnt) G >>= 1;
-  const int K = 32 / G, part = lane / G;
-  for (int e0 = 0; e0 < cnt; e0 += G) {
-    const int e = e0 + (lane & (G - 1));
+  int e0 = 0;
+  for (; cnt - e0 > 16; e0 += 32) {
+    const int e = e0 + lane;
+    const bool in = e < cnt;
+    const T* f = Fs + (in ? e : 0);
+    T v = in ? buf[e] : E_::zero();
+#pragma unroll 2
+    for (int h = 0; h < nops; ++h) {
+      const int a = ab[h];
+      if (a != 0) v = E_::addmul(v, f[h * cnt], a);
+    }
+    if (in) buf[e] = v;
+  }
+  return min(e0, cnt);
+}
+
+// The rest of a row, at most 16 elements from e0 on: lanes to spare take their
+// share of the ops, and the partial sums meet by shuffles.
+template <int D>
+__device__ __forceinline__ void combine_tail(const PanelOps& po, const typename El<D>::T* Fs, typename El<D>::T* buf,
+                                             int e0, int cnt, const int* ab) {
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int lane = threadIdx.x & 31, nops = po.nops;
+  if (e0 < cnt) {
+    int G = 16;
+    while (G > 1 && (G >> 1) >= cnt - e0) G >>= 1;
+    const int K = 32 / G, part = lane / G, e = e0 + (lane & (G - 1));
     const bool in = e < cnt;
     const T* f = Fs + (in ? e : 0);
     T v = in && part == 0 ? buf[e] : E_::zero();
-    if (K == 1) {  // the multiples are uniform over the warp
-#pragma unroll 2
-      for (int h = 0; h < nops; ++h) {
-        const int a = ab[h];
-        if (a != 0) v = E_::addmul(v, f[h * cnt], a);
-      }
-    } else {
-      for (int h = part; h < nops; h += K) v = E_::muladd(v, f[h * cnt], ab[h]);
-      for (int o = G; o < 32; o <<= 1) v = E_::add(v, E_::shfl_xor(v, o));
-    }
+    for (int h = part; h < nops; h += K) v = E_::muladd(v, f[h * cnt], ab[h]);
+    for (int o = G; o < 32; o <<= 1) v = E_::add(v, E_::shfl_xor(v, o));
     if (in && part == 0) buf[e] = v;
   }
   __syncwarp();
@@ -612,7 +619,7 @@ __device__ __forceinline__ void update_row(const PanelOps& po, const typename El
   }
   ab[lane] = av;
   __syncwarp();
-  combine_row<D>(po, Fs, buf, 2 * E, ab);
+  combine_tail<D>(po, Fs, buf, combine_row<D>(po, Fs, buf, 2 * E, ab), 2 * E, ab);
 }
 
 // The same for the stabilizer half alone, through the panel's ops with
@@ -650,7 +657,7 @@ __device__ __forceinline__ void update_half_row(const PanelOps& po, const typena
     E_::put(buf + pe, pl, lane < non ? om : small_mod<D>(av));
   }
   __syncwarp();
-  combine_row<D>(po, Fs, buf, E, ab);
+  combine_tail<D>(po, Fs, buf, combine_row<D>(po, Fs, buf, E, ab), E, ab);
 }
 
 // d = 2: lanes of a row's group (a power of two of at least E words, at most
@@ -728,7 +735,8 @@ struct ChainSmem {
 struct PanelState {
   uint32_t rand;  // its random rows
   int pv[32];     // pivot | its residue << 16 of a random row
-  int orow[32];   // the random rows in order
+  int orow[32];   // the random rows in order: the panel's ops
+  int dup[32], last[32];  // of an op, as in PanelOps
   int kk[32];     // constant lane (odd d), sign exponent (d = 2)
   int kq[32];     // d = 2: parities that the updates add to it
   int tp[32];     // d = 2: parity of S . T of a random row
@@ -935,18 +943,22 @@ __device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typ
   const uint32_t randm = ps.rand;
   const int nops = __popc(randm);
   if constexpr (D != 2) {
+    if (threadIdx.x < 32) {  // ops with one pivot; idle lanes have one of their own
+      const int o = threadIdx.x;
+      const uint32_t same = __match_any_sync(0xffffffffu, o < nops ? ps.pv[ps.orow[o]] & 0xffff : -1 - o);
+      ps.dup[o] = 31 - __clz((int)(same & ((1u << o) - 1u)));
+      ps.last[o] = (same >> o) == 1u;
+    }
+    __syncthreads();
     // G[h][o] = -e_h times op h's entry at op o's pivot, nothing where an op
-    // from h on has replaced it before o (rows by op number: orow)
-    for (int i = threadIdx.x; i < 1024; i += 32 * nwp) {
+    // from h on has replaced it before o
+    for (int i = threadIdx.x; i < 1024; i += (int)blockDim.x) {
       const int o = i >> 5, h = i & 31;
       int g = 0;
-      if (h < o && o < nops) {
+      if (h < o && o < nops && h > ps.dup[o]) {
         const int ro = ps.orow[o], rh = ps.orow[h];
         const int p = ps.pv[ro] & 0xffff;
-        bool kept = true;
-        for (int q = h; q < o; ++q) kept &= (ps.pv[ps.orow[q]] & 0xffff) != p;
-        if (kept)
-          g = small_mod<D>((D - inverse<D>(ps.pv[rh] >> 16)) * E_::get(P[(size_t)rh * (2 * E + 1) + p / L], p % L));
+        g = small_mod<D>((D - inverse<D>(ps.pv[rh] >> 16)) * E_::get(P[(size_t)rh * (2 * E + 1) + p / L], p % L));
       }
       reinterpret_cast<uint8_t*>(ps.Gt[o])[h] = (uint8_t)g;
     }
@@ -993,7 +1005,9 @@ __device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typ
         if (w < E) reinterpret_cast<T*>(out)[w] = E_::neg(v);
       }
       if (lane == 0) {
-        __stcg(rd.opm + h, make_int4(p, D == 2 ? 1 | (ps.tp[i] << 8) : e, m, 0));
+        const int o = h - nopsum;
+        __stcg(rd.opm + h, make_int4(p, D == 2 ? 1 | (ps.tp[i] << 8) : e, m,
+                                         D == 2 ? 0 : (ps.dup[o] + 1) | (ps.last[o] << 6)));
         rd.mhdr[m] = make_uint4(2u * reset | (D == 2 ? 0u : (uint32_t)e << 8), (uint32_t)p, nord, 0u);
       }
     } else {

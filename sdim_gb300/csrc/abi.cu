@@ -664,6 +664,21 @@ int row_phase_blocks(const RowPhaseDesc& p) {
   return (p.c.nshots + per - 1) / per;
 }
 
+// Every pointer into the passes' memory, which begins at mem (and at r.raw).
+void row_memory(RowDesc& r, uint8_t* mem) {
+  const RowBytes b = row_bytes(r.n, r.d, r.nm, r.nx, r.nk);
+  r.raw = mem + b.raw;
+  r.xraw = mem + b.xraw;
+  r.kpart = mem + b.kpart;
+  r.ksign = mem + b.ksign;
+  r.nz = mem + b.nz;
+  r.vg = mem + b.vg;
+  r.opf = mem + b.opf;
+  r.opm = reinterpret_cast<int4*>(mem + b.opm);
+  r.pop = reinterpret_cast<int*>(mem + b.pop);
+  r.opw = reinterpret_cast<uint32_t*>(mem + b.opw);
+}
+
 RowDesc row_desc(const sdim_circuit* c, uint8_t* mem, uint4* mhdr, uint8_t* mrow, uint8_t* nrow, int rowb) {
   RowDesc r;
   std::memset(&r, 0, sizeof(r));
@@ -672,15 +687,6 @@ RowDesc row_desc(const sdim_circuit* c, uint8_t* mem, uint4* mhdr, uint8_t* mrow
   r.lay = reinterpret_cast<const uint32_t*>(c->d_blob + p.lay_off);
   r.minfo = reinterpret_cast<const uint32_t*>(c->d_blob + p.minfo_off);
   r.xinfo = c->d_blob + p.xinfo_off;
-  const RowBytes b = row_bytes(c->n, c->d, c->nmeas, p.nx, p.nk);
-  r.raw = mem + b.raw;
-  r.xraw = mem + b.xraw;
-  r.kpart = mem + b.kpart;
-  r.ksign = mem + b.ksign;
-  r.opf = mem + b.opf;
-  r.opm = reinterpret_cast<int4*>(mem + b.opm);
-  r.pop = reinterpret_cast<int*>(mem + b.pop);
-  r.opw = reinterpret_cast<uint32_t*>(mem + b.opw);
   r.mhdr = mhdr;
   r.mrow = mrow;
   r.nrow = nrow;
@@ -693,6 +699,7 @@ RowDesc row_desc(const sdim_circuit* c, uint8_t* mem, uint4* mhdr, uint8_t* mrow
   r.E = row_elems(c->n);
   r.EK = (p.nk + (c->d == 2 ? 0 : 1) + kRowLanes - 1) / kRowLanes;
   r.rowb = rowb;
+  row_memory(r, mem);
   return r;
 }
 
@@ -1025,13 +1032,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   if (!hr.empty()) {
     if ((rc = ensure(ctx, ctx->rows, std::max<size_t>(rmem, 256))) != SDIM_OK) return rc;
     const size_t base = reinterpret_cast<size_t>(ctx->rows.p);
-    for (RowDesc& r : hr) {
-      uint8_t** ptrs[] = {&r.raw, &r.xraw, &r.kpart, &r.ksign, &r.opf};
-      for (uint8_t** p : ptrs) *p += base;
-      r.opm = reinterpret_cast<int4*>(reinterpret_cast<uint8_t*>(r.opm) + base);
-      r.pop = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(r.pop) + base);
-      r.opw = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(r.opw) + base);
-    }
+    for (RowDesc& r : hr) row_memory(r, r.raw + base);
     for (RowGroup& g : rgroups) plan_row_group(ctx, g, hr.data(), rcirc);
   }
   // the row form's phase pass: odd d, and d = 2 without fires to apply, each row

@@ -91,6 +91,8 @@ struct RowDesc {
   uint8_t* xraw;   // nx rows: S[E] K[EK]
   uint8_t* kpart;  // d = 2: sign exponents per measurement and word, [nm][E]
   uint8_t* ksign;  // d = 2: sign exponents gathered from the updates, [nm]
+  uint8_t* nz;     // set by the updates: the row has an S entry, [nm]
+  uint8_t* vg;     // V for the other CTAs of a cluster, [2][E]
   uint8_t* opf;    // factor rows F of the random measurements, [..][2 E]
   int4* opm;       // their {pivot, exponent | commute parity << 8, ordinal, 1 + last op of the panel
                    // before it with its pivot (0: none) | no later one has it << 6}
@@ -107,7 +109,7 @@ struct RowDesc {
 };
 
 struct RowBytes {
-  size_t raw, xraw, kpart, ksign, opf, opm, pop, opw, total;  // offsets, and the total
+  size_t raw, xraw, kpart, ksign, nz, vg, opf, opm, pop, opw, total;  // offsets, and the total
 };
 
 inline RowBytes row_bytes(int n, int d, int nm, int nx, int nk) {
@@ -119,7 +121,9 @@ inline RowBytes row_bytes(int n, int d, int nm, int nx, int nk) {
   b.xraw = b.raw + up((size_t)nm * (2 * E + EK) * eb);
   b.kpart = b.xraw + up((size_t)nx * (E + EK) * eb);
   b.ksign = b.kpart + up(d == 2 ? (size_t)nm * E : 0);
-  b.opf = b.ksign + up(d == 2 ? (size_t)nm : 0);
+  b.nz = b.ksign + up(d == 2 ? (size_t)nm : 0);
+  b.vg = b.nz + up((size_t)nm);
+  b.opf = b.vg + up(2 * E * eb);
   b.opm = b.opf + up((size_t)nm * 2 * E * eb);
   b.pop = b.opm + up((size_t)nm * sizeof(int4));
   b.opw = b.pop + up(((size_t)nm / kRowPanel + 2) * sizeof(int));

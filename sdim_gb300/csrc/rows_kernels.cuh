@@ -111,6 +111,9 @@ struct El {
     return make_uint4((a.x & m) | ((uint32_t)(v & 1) << j), (a.y & m) | ((uint32_t)((v >> 1) & 1) << j),
                       (a.z & m) | ((uint32_t)(v >> 2) << j), 0u);
   }
+  static __device__ __forceinline__ T pick(uint32_t m, T a, T b) {  // m ? a : b
+    return make_uint4(mux(m, a.x, b.x), mux(m, a.y, b.y), mux(m, a.z, b.z), 0u);
+  }
   // lanes m set to v
   static __device__ __forceinline__ T put_at(T a, uint32_t m, int v) {
     return make_uint4(mux(m, lane_mask(v & 1), a.x), mux(m, lane_mask(v & 2), a.y), mux(m, lane_mask(v & 4), a.z), 0u);
@@ -159,6 +162,9 @@ struct El<3> {  // two planes (planes3.cuh)
   static __device__ __forceinline__ T addmul(T v, T f, int c) { return c == 1 ? add(v, f) : sub(v, f); }
   static __device__ __forceinline__ int get(T a, int j) { return p3_get(p(a), j); }
   static __device__ __forceinline__ T set(T a, int j, int v) { return t(p3_set(p(a), j, v)); }
+  static __device__ __forceinline__ T pick(uint32_t m, T a, T b) {
+    return make_uint2(mux(m, a.x, b.x), mux(m, a.y, b.y));
+  }
   static __device__ __forceinline__ T put_at(T a, uint32_t m, int v) {
     return make_uint2(mux(m, lane_mask(v == 1), a.x), mux(m, lane_mask(v == 2), a.y));
   }
@@ -190,6 +196,7 @@ struct El<2> {  // one plane
   static __device__ __forceinline__ T muladd(T v, T f, int c) { return v ^ (f & (0u - (uint32_t)c)); }
   static __device__ __forceinline__ int get(T a, int j) { return (int)((a >> j) & 1u); }
   static __device__ __forceinline__ T set(T a, int j, int v) { return (a & ~(1u << j)) | ((uint32_t)v << j); }
+  static __device__ __forceinline__ T pick(uint32_t m, T a, T b) { return mux(m, a, b); }
   static __device__ __forceinline__ T put_at(T a, uint32_t m, int v) { return mux(m, lane_mask(v), a); }
   static __device__ __forceinline__ int dot(T a, T b) { return __popc(a & b); }
   static __device__ __forceinline__ T shfl(T a, int l) { return __shfl_sync(0xffffffffu, a, l); }
@@ -233,12 +240,6 @@ struct Unit : El<D> {
     a.x &= m;
     a.y &= m;
     if constexpr (D != 3) a.z &= m;
-    return a;
-  }
-  static __device__ __forceinline__ T pick(uint32_t m, T a, T b) {  // m ? a : b
-    a.x = mux(m, a.x, b.x);
-    a.y = mux(m, a.y, b.y);
-    if constexpr (D != 3) a.z = mux(m, a.z, b.z);
     return a;
   }
   static __device__ __forceinline__ T bump(T a, int v) {  // the constant lane
@@ -741,6 +742,7 @@ struct PanelState {
   int kq[32];     // d = 2: parities that the updates add to it
   int tp[32];     // d = 2: parity of S . T of a random row
   int dsum[32];   // T . V of a deterministic row
+  uint32_t info[32];  // minfo
   uint8_t om[32][32];  // om[j][i]: raw entry of row i in row j's K column
   // what a warp offers for the next random row, by parity: the first
   // generator of the row in the warp's words (x: | residue << 16, -1 for none)
@@ -802,10 +804,9 @@ __device__ __forceinline__ void eliminate(const RowDesc& rd, int cnt, typename E
   };
   // this lane's entry at generator k (uniform) of the warp's words
   auto entry = [&](int k) {
-    T x = s[0];
+    T x = s[0];  // by masks: an index would put s into local memory
 #pragma unroll
-    for (int i = 1; i < CE; ++i)
-      if ((k >> 5) == i) x = s[i];
+    for (int i = 1; i < CE; ++i) x = E_::pick(lane_mask((k >> 5) == i), s[i], x);
     return E_::get(x, k & 31);
   };
   // d = 2: parity of S . T | parity of kacc << 1, of row r
@@ -992,7 +993,7 @@ __device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typ
     const int m = m0 + i;
     const T* row = P + (size_t)i * (2 * E + 1);
     uint8_t* out = rd.mrow + (size_t)m * 2 * rd.rowb;
-    const uint32_t info = __ldg(rd.minfo + m);
+    const uint32_t info = ps.info[i];
     const uint32_t nord = info & 0x7fffffffu, reset = info >> 31;
     if ((randm >> i) & 1u) {
       const int p = ps.pv[i] & 0xffff, e = inverse<D>(ps.pv[i] >> 16), pe = p / L, pl = p % L;
@@ -1026,24 +1027,95 @@ __device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typ
   __syncthreads();
 }
 
+// The first row from m on that may be random (its flag is set), nm for none.
+__device__ __forceinline__ int next_random(const RowDesc& rd, int m) {
+  const int lane = threadIdx.x & 31;
+  for (; m < rd.nm; m += 256) {
+    uint8_t f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int i = m + 32 * j + lane;
+      f[j] = i < rd.nm ? __ldcg(rd.nz + i) : (uint8_t)0;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t b = __ballot_sync(0xffffffffu, f[j] != 0);
+      if (b) return m + 32 * j + __ffs(b) - 1;
+    }
+  }
+  return rd.nm;
+}
+
+// Trace record of measurement m, an up-to-date row without S entries, by one
+// warp: the outcome is T . V and the row's own constant.
+template <int D, class GetV>
+__device__ __forceinline__ void det_row(const RowDesc& rd, int m, GetV phase) {
+  using E_ = El<D>;
+  using T = typename E_::T;
+  const int lane = threadIdx.x & 31, E = rd.E;
+  const T* src = reinterpret_cast<const T*>(rd.raw) + (size_t)m * (2 * E + rd.EK);
+  uint8_t* out = rd.mrow + (size_t)m * 2 * rd.rowb;
+  const uint32_t info = __ldg(rd.minfo + m);
+  T k0 = E_::zero();
+  int kk = 0, d = 0;
+  if constexpr (D == 2)
+    kk = lane == 31 ? (int)__ldcg(rd.ksign + m) : 0;
+  else
+    k0 = ldc(src + 2 * E);
+  for (int w = lane; w < E; w += 32) {
+    const T t = ldc(src + E + w);
+    if constexpr (D == 2) kk += (int)__ldcg(rd.kpart + (size_t)m * E + w);
+    d += E_::dot(t, phase(w));
+    reinterpret_cast<T*>(out)[w] = t;
+  }
+  d = __reduce_add_sync(0xffffffffu, d);
+  int det;
+  if constexpr (D == 2) {
+    kk = __reduce_add_sync(0xffffffffu, kk) & 3;
+    det = 2 * ((kk >> 1) + d & 1);
+  } else {
+    det = (d - E_::get(k0, 0) + D) % D;
+  }
+  if (lane == 0)
+    rd.mhdr[m] = make_uint4(2u * (info >> 31) | 1u, 0u, info & 0x7fffffffu, (uint32_t)det);
+  trace_pad<D>(out, E, rd.rowb, lane);
+}
+
 // One program per cluster of C CTAs.  rawt > 0: the raw pass first, 2^lg units
 // a CTA on rawt threads.  CTA 0 eliminates panel after panel (32
 // rows in shared memory); the panel's updates then go to the rows after it:
 // with C = 1 by this CTA itself, with more the next panel's rows by CTA 0 (it
 // eliminates them next) and the others' by the other CTAs meanwhile, so one
-// cluster barrier per panel is all they wait for.
+// cluster barrier per panel is all they wait for.  A panel that had no random
+// row leaves nothing to update; the rows after it up to the next one with S
+// entries are then deterministic and independent, a warp takes each, and their
+// panels cost no step (the rounds after the first of an error-correction
+// memory).
 template <int D, int CE, bool kSolo>
 __global__ void __launch_bounds__(32 * kRowWarps) k_rows_chain(const RowDesc* __restrict__ descs, int nd, int C, int rawt,
                                                                int lg) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ PanelOps po;
   __shared__ PanelState ps;
+  __shared__ RowDesc shared;
   using E_ = El<D>;
   using T = typename E_::T;
   const int r = C > 1 ? (int)cluster_rank() : 0;
   const int pi = (int)blockIdx.x / C;
   if (pi >= nd) return;  // the whole cluster
-  const RowDesc rd = descs[pi];
+  // odd d: in shared memory, its fields would take a third of the registers
+  // that the elements need (the elimination 28.4k cycles a panel at 256 qudits
+  // of d = 5, 23.8k with them there); d = 2 has the registers, and is 5% slower
+  // with it in shared memory
+  RowDesc own;
+  if constexpr (D == 2) {
+    own = descs[pi];
+  } else {
+    for (int i = threadIdx.x; i < (int)(sizeof(RowDesc) / 4); i += blockDim.x)
+      reinterpret_cast<uint32_t*>(&shared)[i] = reinterpret_cast<const uint32_t*>(descs + pi)[i];
+    __syncthreads();
+  }
+  const RowDesc& rd = D == 2 ? own : shared;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwp = (int)(blockDim.x >> 5);
   const int E = rd.E, RS = 2 * E + rd.EK;
   T* P = reinterpret_cast<T*>(smem);
@@ -1065,43 +1137,139 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_chain(const RowDesc* __
   // their constants (odd d) or sign exponents (d = 2)
   auto load_panel = [&](int k) {
     const int m0 = k * kRowPanel, cnt = min(kRowPanel, rd.nm - m0);
-    for (int i = warp; i < 32; i += nwp) {
-      int om = 0, kk = 0;
-      if (i < cnt) {
+    constexpr int R = D == 2 ? 2 : 1;  // rows at a time, all their loads first (two of odd d: too many registers)
+    for (int i0 = warp; i0 < 32; i0 += R * nwp) {
+      T kw[R], v[R][4], k0[R];
+      int kk[R];
+      uint32_t info[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int i = i0 + j * nwp;
+        const bool in = i < cnt;
         const T* src = raw + (size_t)(m0 + i) * RS;
-        const int v = m0 + lane + (D == 2 ? 0 : 1);
-        T kw = E_::zero();
-        if (m0 + lane < rd.nk && lane < i) kw = ldc(src + 2 * E + v / L);
+        const int q = m0 + lane + (D == 2 ? 0 : 1);
+        kw[j] = in && m0 + lane < rd.nk && lane < i ? ldc(src + 2 * E + q / L) : E_::zero();
+        info[j] = in ? __ldg(rd.minfo + m0 + i) : 0u;
+        kk[j] = 0;
+        k0[j] = E_::zero();
         if constexpr (D == 2) {
-          for (int w = lane; w < E; w += 32) kk += __ldcg(rd.kpart + (size_t)(m0 + i) * E + w);
-          kk = __reduce_add_sync(0xffffffffu, kk) + (int)__ldcg(rd.ksign + m0 + i);
+          const uint8_t* kp = rd.kpart + (size_t)(m0 + i) * E;
+          if (in && lane < E) kk[j] = (int)__ldcg(kp + lane);
+          if (in && lane + 32 < E) kk[j] += (int)__ldcg(kp + lane + 32);
+          if (in && lane == 31) kk[j] += (int)__ldcg(rd.ksign + m0 + i);
         } else {
-          kk = E_::get(ldc(src + 2 * E), 0);
+          if (in) k0[j] = ldc(src + 2 * E);
         }
-        copy_elems(src, 2 * E, lane, 32, [&](int e, T x) { P[(size_t)i * PS + e] = x; });
-        om = E_::get(kw, v % L);
+#pragma unroll
+        for (int h = 0; h < 4; ++h)  // 2 E <= 128 (n <= 2048)
+          if (in && lane + 32 * h < 2 * E) v[j][h] = ldc(src + lane + 32 * h);
       }
-      ps.om[lane][i] = (uint8_t)om;
-      if (lane == 0) {
-        ps.kk[i] = D == 2 ? kk & 3 : kk;
-        ps.kq[i] = ps.dsum[i] = 0;
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int i = i0 + j * nwp;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (i < cnt && lane + 32 * h < 2 * E) P[(size_t)i * PS + lane + 32 * h] = v[j][h];
+        ps.om[lane][i] = (uint8_t)E_::get(kw[j], (m0 + lane + (D == 2 ? 0 : 1)) % L);
+        const int k = D == 2 ? __reduce_add_sync(0xffffffffu, kk[j]) & 3 : E_::get(k0[j], 0);
+        if (lane == 0) {
+          ps.kk[i] = k;
+          ps.kq[i] = ps.dsum[i] = 0;
+          ps.info[i] = info[j];
+        }
       }
     }
     __syncthreads();
   };
-  if (r == 0) {
+  if (r == 0)
     for (int e = threadIdx.x; e < E; e += blockDim.x) V[e] = E_::zero();
-    load_panel(0);
-    factor_panel<D, CE, kSolo>(rd, 0, P, V, ps, nops);
-  }
-  for (int k = 0; k + 1 < panels; ++k) {
-    if (C > 1) cluster_sync_all(); else __syncthreads();
-    const int first = __ldcg(rd.pop + k), cnt = __ldcg(rd.pop + k + 1) - first;
-    const int b1 = (k + 1) * kRowPanel;
-    if (cnt > 0) stage_panel<D, true>(po, Fs, rd, k, first, cnt);
-    if (C > 1 && r == 0) {
-      load_panel(k + 1);
-      if (cnt > 0) {
+  bool flags = false;  // the flags rd.nz of the rows after the next panel are set
+  T* vg = reinterpret_cast<T*>(rd.vg);  // C > 1: V for the other CTAs, by parity of the step
+  for (int k = -1, step = 0; k + 1 < panels; ++step) {
+    int first = 0, cnt = 0, next = k + 1;
+    if (k >= 0) {
+      if (C > 1) cluster_sync_all(); else __syncthreads();
+      first = __ldcg(rd.pop + k);
+      cnt = __ldcg(rd.pop + k + 1) - first;
+    }
+    if (cnt == 0 && flags) {
+      // nothing left to update: on to the next panel with a row that may be
+      // random, the rows before it are all deterministic
+      const int m = (k + 1) * kRowPanel, e = next_random(rd, m);
+      next = e < rd.nm ? e / kRowPanel : panels;
+      const T* vp = vg + (step & 1) * E;
+      if (C == 1 || r > 0)
+        for (int i = m + (C > 1 ? (r - 1) * nwp + warp : warp); i < min(next * kRowPanel, rd.nm);
+             i += C > 1 ? (C - 1) * nwp : nwp)
+          det_row<D>(rd, i, [&](int w) { return C > 1 ? ldc(vp + w) : V[w]; });
+      if (r == 0 && threadIdx.x == 0)
+        for (int q = k + 2; q <= next; ++q) __stcg(rd.pop + q, first);
+      if (next == panels) break;
+    }
+    const int b1 = next * kRowPanel;
+    if (cnt > 0) {
+      stage_panel<D, true>(po, Fs, rd, k, first, cnt);
+      flags = true;
+    }
+    if (cnt > 0 && (C == 1 || r > 0)) {
+      // rows of the panels after the next (of all later ones with C = 1)
+      const int m0 = C > 1 ? b1 + kRowPanel : b1;
+      const int w0 = C > 1 ? (r - 1) * nwp + warp : warp, dw = C > 1 ? (C - 1) * nwp : nwp;
+      if constexpr (D == 2) {
+        for (int i0 = m0 + w0 * gpw; i0 < rd.nm; i0 += dw * gpw) {
+          const int i = i0 + lane / G;
+          const bool in = i < rd.nm;
+          uint32_t S[kRowGroupWords] = {}, Tt[kRowGroupWords] = {};
+          T* row = raw + (size_t)i * RS;
+#pragma unroll
+          for (int h = 0; h < kRowGroupWords; ++h) {
+            const int w = gl + h * G;
+            if (in && w < E) {
+              S[h] = ldc(row + w);
+              Tt[h] = ldc(row + E + w);
+            }
+          }
+          const uint32_t kw = in ? k_bits(row + 2 * E, rd.EK, k * kRowPanel) : 0u;
+          const int dk = update_row2<true>(po, Fs, S, Tt, kw, k * kRowPanel, E, 2 * E, INT_MAX, gl, G);
+#pragma unroll
+          for (int h = 0; h < kRowGroupWords; ++h) {
+            const int w = gl + h * G;
+            if (in && w < E) {
+              stc(row + w, S[h]);
+              stc(row + E + w, Tt[h]);
+            }
+          }
+          uint32_t any = 0u;
+#pragma unroll
+          for (int h = 0; h < kRowGroupWords; ++h) any |= S[h];
+          const uint32_t nz = __ballot_sync(0xffffffffu, any != 0u) >> (lane & ~(G - 1));
+          if (in && gl == 0) {
+            __stcg(rd.ksign + i, (uint8_t)((__ldcg(rd.ksign + i) + dk) & 3));
+            __stcg(rd.nz + i, (uint8_t)((nz << (32 - G)) != 0u));
+          }
+        }
+      } else {
+        T* buf = P + (size_t)warp * PS;
+        for (int i = m0 + w0; i < rd.nm; i += dw) {
+          T* row = raw + (size_t)i * RS;
+          copy_elems(row, 2 * E, lane, 32, [&](int e, T x) { buf[e] = x; });
+          __syncwarp();
+          update_row<D>(po, Fs, buf, row + 2 * E, E, rd.nk, ab);
+          uint32_t any = 0u;
+          for (int e = lane; e < 2 * E; e += 32) {
+            const T v = buf[e];
+            stc(row + e, v);
+            if (e < E) any |= E_::nzw(v);
+          }
+          any = __ballot_sync(0xffffffffu, any != 0u);
+          if (lane == 0) __stcg(rd.nz + i, (uint8_t)(any != 0u));
+        }
+      }
+    }
+    if (r == 0) {
+      if (C == 1) __syncthreads();
+      load_panel(next);
+      if (C > 1 && cnt > 0) {
         const int rows = min(kRowPanel, rd.nm - b1);
         if constexpr (D == 2) {
           for (int i0 = warp * gpw; i0 < rows; i0 += nwp * gpw) {
@@ -1135,56 +1303,12 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_chain(const RowDesc* __
         }
         __syncthreads();
       }
-      factor_panel<D, CE, kSolo>(rd, k + 1, P, V, ps, nops);
-    } else {
-      if (cnt > 0) {
-        // rows of the panels after the next (of all later ones with C = 1)
-        const int m0 = C > 1 ? b1 + kRowPanel : b1;
-        const int w0 = C > 1 ? (r - 1) * nwp + warp : warp, dw = C > 1 ? (C - 1) * nwp : nwp;
-        if constexpr (D == 2) {
-          for (int i0 = m0 + w0 * gpw; i0 < rd.nm; i0 += dw * gpw) {
-            const int i = i0 + lane / G;
-            const bool in = i < rd.nm;
-            uint32_t S[kRowGroupWords] = {}, Tt[kRowGroupWords] = {};
-            T* row = raw + (size_t)i * RS;
-#pragma unroll
-            for (int h = 0; h < kRowGroupWords; ++h) {
-              const int w = gl + h * G;
-              if (in && w < E) {
-                S[h] = ldc(row + w);
-                Tt[h] = ldc(row + E + w);
-              }
-            }
-            const uint32_t kw = in ? k_bits(row + 2 * E, rd.EK, k * kRowPanel) : 0u;
-            const int dk = update_row2<true>(po, Fs, S, Tt, kw, k * kRowPanel, E, 2 * E, INT_MAX, gl, G);
-#pragma unroll
-            for (int h = 0; h < kRowGroupWords; ++h) {
-              const int w = gl + h * G;
-              if (in && w < E) {
-                stc(row + w, S[h]);
-                stc(row + E + w, Tt[h]);
-              }
-            }
-            if (in && gl == 0) __stcg(rd.ksign + i, (uint8_t)((__ldcg(rd.ksign + i) + dk) & 3));
-          }
-        } else {
-          T* buf = P + (size_t)warp * PS;
-          for (int i = m0 + w0; i < rd.nm; i += dw) {
-            T* row = raw + (size_t)i * RS;
-            copy_elems(row, 2 * E, lane, 32, [&](int e, T x) { buf[e] = x; });
-            __syncwarp();
-            update_row<D>(po, Fs, buf, row + 2 * E, E, rd.nk, ab);
-            for (int e = lane; e < 2 * E; e += 32) stc(row + e, buf[e]);
-            __syncwarp();
-          }
-        }
-      }
-      if (C == 1) {
-        __syncthreads();
-        load_panel(k + 1);
-        factor_panel<D, CE, kSolo>(rd, k + 1, P, V, ps, nops);
-      }
+      const int before = nops;
+      factor_panel<D, CE, kSolo>(rd, next, P, V, ps, nops);
+      if (C > 1 && nops == before)  // what a skip may follow
+        for (int e = threadIdx.x; e < E; e += blockDim.x) stc(vg + (~step & 1) * E + e, V[e]);
     }
+    k = next;
   }
 }
 

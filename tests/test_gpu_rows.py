@@ -77,3 +77,33 @@ def test_mixed_batch_matches_oracle():
         br.add_spec(spec, 150 + 40 * k, 60 + k)
     for k, (spec, out) in enumerate(zip(specs, br.run())):
         assert np.array_equal(out, oracle_run([spec], 60 + k, 0, 150 + 40 * k)["records"]), k
+
+
+def _repeats(n, d, seed):
+    """Sweeps of M on all qudits with gates only before some: whole panels of
+    deterministic rows, after a random panel, at the end and up to a lone random row."""
+    rng = np.random.default_rng(seed)
+    meas = [("M", q, None, {}) for q in range(n)]
+    gates = workloads.all_gates_random(n, d, 3 * n, seed=rng, noise_probs=(0.3,)).ops[:-n]
+    more = workloads.all_gates_random(n, d, 2 * n, seed=rng).ops[:-n]
+    k = 1 + 124 // n
+    ops = gates + meas * k + [("H", int(rng.integers(n)), None, {})] + meas * k + more + meas * (k + 1)
+    return workloads.CircuitSpec(n, d, ops, "repeats")
+
+
+@pytest.mark.parametrize("d", [2, 3, 5, 7])
+@pytest.mark.parametrize("n", [9, 33, 130])
+def test_deterministic_panels_match_oracle(n, d):
+    _check(_repeats(n, d, 10 * n + d), 5, seed=n)
+
+
+@pytest.mark.parametrize("d", [2, 5])
+def test_deterministic_panels_in_a_batch(d):
+    """More programs than SMs: one CTA each."""
+    br = BatchRunner()
+    specs = [_repeats(4 + k % 7, d, k) for k in range(160)]
+    for k, spec in enumerate(specs):
+        br.add_spec(spec, 1 + k % 3, 90 + k)
+    for k, (spec, out) in enumerate(zip(specs, br.run(engine="trace"))):
+        if k % 8 == 0:
+            assert np.array_equal(out, oracle_run([spec], 90 + k, 0, 1 + k % 3)["records"]), k

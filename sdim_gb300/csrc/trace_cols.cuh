@@ -22,17 +22,20 @@
 //   deterministic k);  column 1 + nm + 2 j: A_j,  2 + nm + 2 j: B_j
 //   (j < nused, the N1 ordinals before the last measurement).
 #pragma once
+#include <type_traits>
+
 #include "trace_bits.cuh"
 
 namespace sdim {
 
-// First measurement that ordinal j's N1 update precedes (mhdr[k].z counts
-// the ordinals before measurement k, nondecreasing in k; j < mhdr[nm-1].z).
-__device__ __forceinline__ int fire_measurement(const uint4* __restrict__ mhdr, int nm, uint32_t j) {
+// First measurement that ordinal j's N1 update precedes (hdr[k].z counts the
+// ordinals before measurement k, nondecreasing in k; j < hdr[nm-1].z).  hdr is
+// the whole trace's headers, in shared memory where they fit.
+__device__ __forceinline__ int fire_measurement(const uint4* hdr, int nm, uint32_t j) {
   int lo = 0, hi = nm - 1;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (__ldg(&mhdr[mid].z) > j) hi = mid; else lo = mid + 1;
+    if (hdr[mid].z > j) hi = mid; else lo = mid + 1;
   }
   return lo;
 }
@@ -73,6 +76,13 @@ __host__ __device__ constexpr int column_window() {
 // each warp walks the measurements from the earliest input of its lanes on
 // (warp-uniform loop, broadcast shared-memory loads); a lane's delta is zero
 // until its input enters, so its bits before that stay zero.
+// Bound by the latency of a warp's walk (about one warp per SM in use), so all
+// that a measurement needs is loaded independently of the ones before it: the
+// fire inputs' rows before the walk, and in a deterministic run the RESET rows
+// in the same unrolled turn as the factors, gathered beside the delta instead
+// of XORed in by a second loop.  L = 7 memory, 385 measurements: 68 us with
+// the second loop and the searches in global memory, 35 us so; L = 5, 145
+// measurements: 28 and 17 us.
 template <int TW, int WARPS>
 __device__ __forceinline__ void column_block(const TraceDesc* __restrict__ tdp, long long g, uint4* shdr,
                                              uint32_t* srow, int* smin) {
@@ -84,63 +94,81 @@ __device__ __forceinline__ void column_block(const TraceDesc* __restrict__ tdp, 
   const int nm = tdp->nm, wn = tdp->wn, nw = tdp->nw;
   const long long ncols = column_count(nm, tdp->nused);
   const long long i = (g * WARPS + warp) * 32 + lane;
+  // measurements [wb, we) of the trace into shared memory
+  auto stage = [&](int wb, int we) {
+    const uint4* src = reinterpret_cast<const uint4*>(mrow + (size_t)wb * 2 * TW);
+    uint4* dst = reinterpret_cast<uint4*>(srow);
+    const int n4 = (we - wb) * 2 * TW / 4;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < n4; t += 32 * WARPS) dst[t] = __ldg(src + t);
+#pragma unroll 4
+    for (int t = threadIdx.x; t < we - wb; t += 32 * WARPS) shdr[t] = __ldg(mhdr + wb + t);
+    __syncthreads();
+  };
+  // the fire input's row (z_q for A_j, x_q for B_j); other columns: zero
+  const bool fire = i > nm && i < ncols;
+  uint32_t v[TW];
+#pragma unroll
+  for (int w = 0; w < TW; ++w) v[w] = 0u;
+  const uint32_t j = (uint32_t)((i - 1 - nm) >> 1);
+  if (fire) {
+    const uint32_t* inj = tdp->nrow + (size_t)j * 2 * TW + (((i - 1 - nm) & 1) ? 0 : TW);
+#pragma unroll
+    for (int w = 0; w < TW; ++w) v[w] = __ldg(inj + w);
+  }
+  const bool whole = nm <= WIN;  // one window holds the trace
+  if (whole) stage(0, nm);
+  const uint4* hdr = whole ? shdr : mhdr;
   // kind: 0 inactive, 1 the constant column, 2 an outcome, 3 a fire input
   int kind = 0, start = nm;
-  const uint32_t* inj = nullptr;  // the fire input's row (z_q for A_j, x_q for B_j)
   if (i == 0) {
     kind = 1;
     start = 0;
   } else if (i <= nm) {
     const int k = (int)(i - 1);
-    if (!(__ldg(&mhdr[k].x) & 1u)) {  // deterministic measurements have no outcome column
+    if (!(hdr[k].x & 1u)) {  // deterministic measurements have no outcome column
       kind = 2;
       start = k;
     }
-  } else if (i < ncols) {
-    const uint32_t j = (uint32_t)((i - 1 - nm) >> 1);
+  } else if (fire) {
     kind = 3;
-    start = fire_measurement(mhdr, nm, j);
-    inj = tdp->nrow + (size_t)j * 2 * TW + (((i - 1 - nm) & 1) ? 0 : TW);
+    start = fire_measurement(hdr, nm, j);
   }
   uint32_t* __restrict__ out = tdp->cols + (size_t)i * nw;
-  int k0 = start;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) k0 = min(k0, __shfl_xor_sync(0xffffffffu, k0, o));
-  if (threadIdx.x == 0) *smin = nm;
-  __syncthreads();
-  if (lane == 0) atomicMin(smin, k0);
-  __syncthreads();
-  const int kb0 = *smin;  // the block's first measurement
+  const int k0 = __reduce_min_sync(0xffffffffu, start);
+  int kb0 = 0;  // the block's first measurement
+  if (!whole) {
+    if (threadIdx.x == 0) *smin = nm;
+    __syncthreads();
+    if (lane == 0) atomicMin(smin, k0);
+    __syncthreads();
+    kb0 = *smin;
+  }
   if (kind)
     for (int w = 0; w < (k0 >> 5); ++w) out[w] = 0u;
   uint32_t d1[TW];
 #pragma unroll
   for (int w = 0; w < TW; ++w) d1[w] = 0u;
   uint32_t acc = 0u;
+  const uint32_t cst = kind == 1 ? 0xffffffffu : 0u;
   for (int wb = kb0; wb < nm; wb += WIN) {
     const int we = min(nm, wb + WIN);
-    __syncthreads();  // the previous window is done
-    for (int t = threadIdx.x; t < we - wb; t += 32 * WARPS) shdr[t] = __ldg(mhdr + wb + t);
-    {
-      const uint4* src = reinterpret_cast<const uint4*>(mrow + (size_t)wb * 2 * TW);
-      uint4* dst = reinterpret_cast<uint4*>(srow);
-      const int n4 = (we - wb) * 2 * TW / 4;
-      for (int t = threadIdx.x; t < n4; t += 32 * WARPS) dst[t] = __ldg(src + t);
+    if (!whole) {
+      __syncthreads();  // the previous window is done
+      stage(wb, we);
     }
-    __syncthreads();
     int k = max(wb, k0);
     while (k < we) {
       const uint4 h = shdr[k - wb];
       const uint32_t* row = srow + (size_t)(k - wb) * 2 * TW;
       if (kind == 3 && start == k) {
 #pragma unroll
-        for (int w = 0; w < TW; ++w) d1[w] ^= __ldg(inj + w);
+        for (int w = 0; w < TW; ++w) d1[w] ^= v[w];
       }
       if (!(h.x & 1u)) {
         // a random measurement: the rowsum and the pivot bits
         uint32_t r[TW];
-#pragma unroll
-        for (int w = 0; w < TW; ++w) r[w] = row[w];
+        srow_load<TW>(row, r);
         const int p = (int)h.y, wp = p >> 5, bp = p & 31;
         const uint32_t dp = (word_at<0, TW>(d1, wp) >> bp) & 1u;
         const uint32_t mk = 0u - dp;
@@ -165,59 +193,49 @@ __device__ __forceinline__ void column_block(const TraceDesc* __restrict__ tdp, 
       // parity from the delta at the run's start (independent, so they
       // overlap), each outcome corrected by the earlier RESETs of the run
       // that its factor sees (the header pass's coupling mask in y against
-      // the run's outcomes so far), then the run's RESET rows XORed in.  A
-      // fire input entering inside the run adds its own parities from its
-      // start on (its outcomes before that are zero).
-      int ke = k + 1;
-      while (ke < we && ke - k < 32 && (shdr[ke - wb].x & 1u)) ++ke;
-      const int len = ke - k;
+      // the run's outcomes so far), the run's RESET rows gathered in dz for
+      // its end.  A fire input entering inside the run adds its own parities
+      // from its start on (its outcomes before that are zero).
+      const int kl = k + lane;
+      const uint32_t stop = __ballot_sync(0xffffffffu, kl >= we || !(shdr[kl - wb].x & 1u));
+      const int len = stop ? __ffs(stop) - 1 : 32, ke = k + len;
       const bool late = kind == 3 && start > k && start < ke;
-      const uint32_t cst = kind == 1 ? 0xffffffffu : 0u;
-      uint32_t hist = 0u, bits = 0u;
-      if (__any_sync(0xffffffffu, late)) {
-        uint32_t v[TW];
+      uint32_t hist = 0u, dz[TW];
 #pragma unroll
-        for (int w = 0; w < TW; ++w) v[w] = late ? __ldg(inj + w) : 0u;
-        for (int i = 0; i < len; ++i) {
-          const uint4 hi = shdr[k + i - wb];
-          uint32_t f[FH];
-          srow_load<FH>(srow + (size_t)(k + i - wb) * 2 * TW, f);
-          uint32_t x = 0u, y = 0u;
+      for (int w = 0; w < TW; ++w) dz[w] = 0u;
+      auto turn = [&](int i, auto some_late) {
+        const uint4 hi = shdr[k + i - wb];
+        const uint32_t* fr = srow + (size_t)(k + i - wb) * 2 * TW;
+        uint32_t f[FH], z[TW];
+        srow_load<FH>(fr, f);
+        srow_load<TW>(fr + TW, z);
+        uint32_t x = 0u, y = 0u;
 #pragma unroll
-          for (int w = 0; w < FH; ++w) {
-            x ^= f[w] & d1[w];
-            y ^= f[w] & v[w];
-          }
-          uint32_t b = ((uint32_t)__popc(x) ^ (k + i >= start ? (uint32_t)__popc(y) : 0u)) & 1u;
-          b ^= (det_constant(hi.w) & cst) ^ ((uint32_t)__popc(hi.y & hist) & 1u);
-          hist = (hist << 1) | b;
+        for (int w = 0; w < FH; ++w) {
+          x ^= f[w] & d1[w];
+          if constexpr (some_late.value) y ^= f[w] & v[w];
         }
+        if constexpr (some_late.value) x = (uint32_t)__popc(x) ^ (late && k + i >= start ? (uint32_t)__popc(y) : 0u);
+        else x = (uint32_t)__popc(x);
+        const uint32_t b = (x ^ (det_constant(hi.w) & cst) ^ (uint32_t)__popc(hi.y & hist)) & 1u;
+        hist = (hist << 1) | b;
+        const uint32_t mk = (hi.x & 2u) ? 0u - b : 0u;
 #pragma unroll
-        for (int w = 0; w < TW; ++w) d1[w] ^= v[w];
+        for (int w = 0; w < TW; ++w) dz[w] ^= z[w] & mk;
+      };
+      if (__any_sync(0xffffffffu, late)) {
+        for (int i = 0; i < len; ++i) turn(i, std::true_type());
+#pragma unroll
+        for (int w = 0; w < TW; ++w) d1[w] ^= late ? v[w] : 0u;
       } else {
 #pragma unroll 4
-        for (int i = 0; i < len; ++i) {
-          const uint4 hi = shdr[k + i - wb];
-          uint32_t f[FH];
-          srow_load<FH>(srow + (size_t)(k + i - wb) * 2 * TW, f);
-          uint32_t x = 0u;
-#pragma unroll
-          for (int w = 0; w < FH; ++w) x ^= f[w] & d1[w];
-          const uint32_t b = ((uint32_t)__popc(x) ^ (det_constant(hi.w) & cst) ^ (uint32_t)__popc(hi.y & hist)) & 1u;
-          hist = (hist << 1) | b;
-        }
+        for (int i = 0; i < len; ++i) turn(i, std::false_type());
       }
+#pragma unroll
+      for (int w = 0; w < TW; ++w) d1[w] ^= dz[w];
       // hist holds the run's outcomes, the last in bit 0: bit i of bits =
       // measurement k + i
-      bits = __brev(hist) >> (32 - len);
-      for (int i = 0; i < len; ++i) {
-        if (!(shdr[k + i - wb].x & 2u)) continue;
-        uint32_t z[TW];
-        srow_load<TW>(srow + (size_t)(k + i - wb) * 2 * TW + TW, z);
-        const uint32_t mk = 0u - ((bits >> i) & 1u);
-#pragma unroll
-        for (int w = 0; w < TW; ++w) d1[w] ^= z[w] & mk;
-      }
+      const uint32_t bits = __brev(hist) >> (32 - len);
       // the run's outcomes into the record words: word k / 32 completes when
       // the run reaches its end
       const int sh = k & 31;

@@ -134,14 +134,15 @@ __global__ void __launch_bounds__(32 * kColumnWarps) k_column_pass(const TraceDe
 }
 
 // One single-warp block per 32-shot group of descs[0], from its record
-// columns: up to 16 column words, 32 blocks per SM at 64 registers.
+// columns: up to 16 column words, 24 blocks per SM at 80 registers (100,000
+// shots are 21).
 template <int NW>
-__global__ void __launch_bounds__(32, NW >= 32 ? 16 : 32)
+__global__ void __launch_bounds__(32, NW >= 32 ? 16 : 24)
     k_record_pass(const TraceDesc* __restrict__ descs, long long g0, long long groups, const int* status) {
-  __shared__ __align__(16) uint8_t rec[32 * kRecStride];
+  __shared__ RecordSmem<NW> sm;
   if (*(volatile const int*)status != DEV_OK) return;
   if ((long long)blockIdx.x >= groups) return;
-  record_group<NW>(descs, g0 + blockIdx.x, threadIdx.x, rec);
+  record_group<NW>(descs, g0 + blockIdx.x, threadIdx.x, sm);
 }
 
 // Blocks of the coin pass; descs with masks only, numbered through coin_begin.

@@ -64,6 +64,7 @@ struct sdim_ctx {
   DevBuf cdet;       // deterministic slice sums of the odd-d cluster x / z passes (TraceDescU8::dsum)
   DevBuf rows;          // row form of the x / z pass (rows.cuh): rows and updates
   DevBuf fdescs;        // the frame route's coin pass
+  DevBuf fwords;        // its record words, before the reference shot is added
   cudaStream_t aux = nullptr;                      // coin pass, concurrent with the x / z pass
   cudaStream_t fast = nullptr;                     // d = 2 row form beside a coin pass: the highest priority
   cudaEvent_t ev_fast = nullptr;
@@ -2224,7 +2225,8 @@ int sdim_ctx_destroy(sdim_ctx* ctx) {
   for (int i = 0; i < sdim_ctx::kXzStreams; ++i) cudaStreamSynchronize(ctx->xzs[i]);
   DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap, &ctx->arena,
                     &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->trace_u8, &ctx->xz_u8,
-                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rows, &ctx->fdescs};
+                    &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet, &ctx->rows, &ctx->fdescs,
+                    &ctx->fwords};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   if (ctx->staging) cudaFreeHost(ctx->staging);
@@ -2281,7 +2283,7 @@ int sdim_memory_info(sdim_ctx* ctx, int64_t info[3]) {
   const DevBuf* bufs[] = {&ctx->descs, &ctx->counters, &ctx->status, &ctx->gslots, &ctx->out, &ctx->snap,
                           &ctx->arena, &ctx->tdescs, &ctx->trace, &ctx->masks, &ctx->trace_u8,
                           &ctx->xz_u8, &ctx->xz_queue, &ctx->gslots_xz, &ctx->cols, &ctx->dsnap, &ctx->cdet,
-                          &ctx->rows, &ctx->fdescs};
+                          &ctx->rows, &ctx->fdescs, &ctx->fwords};
   int64_t held = 0;
   for (const DevBuf* b : bufs) held += (int64_t)b->cap;
   info[2] = held;
@@ -2523,19 +2525,14 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFuncSetAttribute");
       }
     ctx->rows_smem_set = true;
-    // the reference shot on the stream of highest priority, beside the coin
-    // pass of the first part of the shots; parts bound the masks' memory
+    // parts bound the memory of the masks and the record words
     const long long frames = nshots - 1;
-    const size_t per_shot = c->d == 2 ? coin_mask_bytes(rf.nchunk, 1024) / 1024 + coin_map_bytes(rf.nchunk, 1024) / 1024 : 0;
-    long long part = frames;
-    if (per_shot) part = std::min<long long>(part, std::max<long long>(32768, (long long)(kFrameMaskBudget / per_shot)));
-    CK(cudaEventRecord(ctx->ev_gf, s));
-    CK(cudaStreamWaitEvent(ctx->fast, ctx->ev_gf, 0));
-    std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
-    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE);
-    ctx->last_stream = s;
-    if (rc != SDIM_OK) return rc;
-    CK(cudaEventRecord(ctx->ev_fast, ctx->fast));
+    const size_t words = (size_t)c->nmeas * row_elem_bytes(c->d);  // per 32 shots
+    const size_t per_shot = words / 32 + 1 +
+                            (c->d == 2 ? coin_mask_bytes(rf.nchunk, 1024) / 1024 + coin_map_bytes(rf.nchunk, 1024) / 1024 : 0);
+    const long long part = std::min<long long>(frames, std::max<long long>(32768, (long long)(kFrameMaskBudget / per_shot)));
+    if ((rc = ensure(ctx, ctx->fwords, std::max<size_t>((size_t)((part + 31) / 32) * words, 256))) != SDIM_OK) return rc;
+    rf.words = static_cast<uint8_t*>(ctx->fwords.p);
     TraceDesc td;
     std::memset(&td, 0, sizeof(td));
     if (rf.nchunk) {
@@ -2550,7 +2547,7 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
       td.cmap = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ctx->masks.p) + coin_mask_bytes(rf.nchunk, part));
       rf.masks = static_cast<const uint2*>(ctx->masks.p);
     }
-    for (long long f0 = 0; f0 < frames; f0 += part) {
+    auto launch_part = [&](long long f0) {  // its coins and frames
       const long long fn = std::min(part, frames - f0);
       if (rf.nchunk) {
         td.c.shot0 = 1 + f0;
@@ -2562,7 +2559,6 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
         const cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) return cuda_fail(ctx, le, "coin pass launch");
       }
-      if (f0 == 0) CK(cudaStreamWaitEvent(s, ctx->ev_fast, 0));
       rf.out = dst + (size_t)(1 + f0) * c->nmeas;
       rf.shot0 = 1 + f0;
       rf.nshots = (int)fn;
@@ -2570,7 +2566,23 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
       rf.mrel = 0;
       row_ops(c->d).frame((int)((fn + 32 * warps - 1) / (32 * warps)), warps, fsmem, s, rf);
       const cudaError_t le = cudaGetLastError();
-      if (le != cudaSuccess) return cuda_fail(ctx, le, "frame pass launch");
+      return le == cudaSuccess ? SDIM_OK : cuda_fail(ctx, le, "frame pass launch");
+    };
+    // the reference shot beside the first part's coins and frames, on the
+    // stream of highest priority; only the output pass needs it
+    CK(cudaEventRecord(ctx->ev_gf, s));
+    CK(cudaStreamWaitEvent(ctx->fast, ctx->ev_gf, 0));
+    std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
+    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE);
+    ctx->last_stream = s;
+    if (rc != SDIM_OK) return rc;
+    CK(cudaEventRecord(ctx->ev_fast, ctx->fast));
+    for (long long f0 = 0; f0 < frames; f0 += part) {
+      if ((rc = launch_part(f0)) != SDIM_OK) return rc;
+      if (f0 == 0) CK(cudaStreamWaitEvent(s, ctx->ev_fast, 0));
+      row_ops(c->d).frame_out(s, rf);
+      const cudaError_t le = cudaGetLastError();
+      if (le != cudaSuccess) return cuda_fail(ctx, le, "frame output pass launch");
     }
   } else {
     // shot 0: the noiseless tableau shot, into row 0, on the trace engines

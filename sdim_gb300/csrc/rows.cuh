@@ -175,6 +175,7 @@ struct RowFrameDesc {
   const uint2* nhdr;     // odd d: N1 (coin threshold, opcode)
   const uint8_t* ref;    // records of the reference shot
   uint8_t* out;          // nshots x nm records
+  uint8_t* words;        // frame words of the records: nm elements per 32 shots
   const uint2* masks;    // d = 2: the coin pass's fire masks, mshots shots a chunk, from shot mrel on
   unsigned long long seed;
   long long shot0;       // stream index of the first shot, below 2^32
@@ -205,6 +206,8 @@ struct RowOps {
   // frame pass: `blocks` CTAs of `warps` (1 to 4) warps, 32 shots each
   size_t (*frame_smem)(const RowFrameDesc& f, int warps);
   void (*frame)(int blocks, int warps, size_t smem, cudaStream_t s, const RowFrameDesc& f);
+  // the records from the frame pass's words and the reference shot's records
+  void (*frame_out)(cudaStream_t s, const RowFrameDesc& f);
 };
 const RowOps& row_ops_2();
 const RowOps& row_ops_3();

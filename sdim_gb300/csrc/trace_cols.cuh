@@ -24,6 +24,7 @@
 #pragma once
 #include <type_traits>
 
+#include "record_out.cuh"
 #include "trace_bits.cuh"
 
 namespace sdim {
@@ -255,12 +256,6 @@ __device__ __forceinline__ void column_block(const TraceDesc* __restrict__ tdp, 
     for (int w = ((nm - 1) >> 5) + 1; w < nw; ++w) out[w] = 0u;
 }
 
-// Four record bytes from four record bits and four deterministic flags
-// (nibbles): byte b = bit b | flag b << 7.
-__device__ __forceinline__ uint32_t record_bytes(uint32_t bits4, uint32_t det4) {
-  return ((bits4 * 0x00204081u) & 0x01010101u) | (((det4 * 0x00204081u) & 0x01010101u) << 7);
-}
-
 // Shared memory of a record-pass warp: its shots' record bits, the
 // deterministic measurements (a word to spare each, so that 16 bits can be cut
 // out at any place, and rows an odd number of words apart), and the shared
@@ -274,9 +269,7 @@ struct RecordSmem {
 
 // One 32-shot group (lane = shot) from the column table: NW words of record
 // bits per lane.  Fires come from the coin pass's masks; the outcome draws
-// are the replay's (measurement k, shot, domain 0).  The group's records are
-// one contiguous piece of the output: each lane cuts 16 of its bytes at a time
-// out of the bits, whatever rows they belong to, and stores them at once.
+// are the replay's (measurement k, shot, domain 0).
 // Bound by latency, about five warps a scheduler: a fire's columns are on
 // their way while the next one's mask is fetched, two outcomes are drawn side
 // by side.  100,000 shots of 385 measurements: 58 us with byte stores staged 64
@@ -364,36 +357,7 @@ __device__ __forceinline__ void record_group(const TraceDesc* __restrict__ tdp, 
 #pragma unroll
   for (int w = 0; w < NW; ++w) sm.bits[lane][w] = b[w];
   __syncwarp();
-  // bytes [0, total) of the group: up to 15 in front of the first 16-byte boundary, whole ones, the rest
-  uint8_t* __restrict__ gout = tdp->c.out + first * (long long)nmeas;
-  const int total = rows * nmeas;
-  const int head = min(total, (int)((0u - (uint32_t)reinterpret_cast<size_t>(gout)) & 15u));
-  const int body = (total - head) & ~15, tail = total - head - body;
-  if (lane < head + tail) {
-    const int o = lane < head ? lane : body + lane, r = o / nmeas, k = o - r * nmeas;
-    const uint32_t v = (sm.bits[r][k >> 5] >> (k & 31)) & 1u, d = (sm.det[k >> 5] >> (k & 31)) & 1u;
-    gout[o] = (uint8_t)(v | (d << 7));
-  }
-  int r = (head + 16 * lane) / nmeas, k = head + 16 * lane - r * nmeas;
-  const int dr = 512 / nmeas, dk = 512 - dr * nmeas;
-  for (int o = 16 * lane; o < body; o += 512) {
-    uint32_t v = __funnelshift_r(sm.bits[r][k >> 5], sm.bits[r][(k >> 5) + 1], k & 31);
-    uint32_t d = __funnelshift_r(sm.det[k >> 5], sm.det[(k >> 5) + 1], k & 31);
-    for (int at = nmeas - k, rr = r + 1; at < 16; at += nmeas, ++rr) {  // the next rows' first bits
-      const uint32_t m = (1u << at) - 1u;
-      v = (v & m) | (sm.bits[rr][0] << at);
-      d = (d & m) | (sm.det[0] << at);
-    }
-    *reinterpret_cast<uint4*>(gout + head + o) =
-        make_uint4(record_bytes(v & 15u, d & 15u), record_bytes((v >> 4) & 15u, (d >> 4) & 15u),
-                   record_bytes((v >> 8) & 15u, (d >> 8) & 15u), record_bytes((v >> 12) & 15u, (d >> 12) & 15u));
-    r += dr;
-    k += dk;
-    if (k >= nmeas) {
-      k -= nmeas;
-      ++r;
-    }
-  }
+  store_records<1>(tdp->c.out + first * (long long)nmeas, rows, nmeas, lane, &sm.bits[0][0], NW + 1, sm.det);
 }
 
 }  // namespace sdim

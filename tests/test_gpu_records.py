@@ -45,3 +45,23 @@ def test_record_bytes_at_any_width_and_address(nm, off, shot0):
     got = out.cpu().numpy()
     assert np.array_equal(got[off : off + shots * nm].reshape(shots, nm), _replay(prog, shots, 7, shot0))
     assert (got[:off] == 99).all() and (got[off + shots * nm :] == 99).all()
+
+
+@pytest.mark.parametrize("d,nms", [(2, (1, 15, 16, 17, 33, 385, 3100)), (3, (1, 16, 31, 65, 1600)),
+                                   (5, (1, 17, 64, 1100)), (7, (1, 16, 33, 1100))])
+def test_frame_records_at_any_width(d, nms):
+    """The frame route's output pass: whole rows in shared memory and, past
+    its limit, a byte at a time; a partial last group; against the frame oracle."""
+    import oracle
+    from oracle import frame
+    rng = np.random.default_rng(d)
+    for nm in nms:
+        ops = [("H", 0, None, {}), ("CNOT", 0, 1, {}), ("H", 2, None, {}), ("N1", 1, None, {"prob": 0.3, "noise_channel": "d"})]
+        for k in range(nm):
+            ops.append((("M", "RESET")[int(rng.integers(8) == 0)], int(rng.integers(4)), None, {}))
+            if k % 5 == 0:
+                ops += [("H", int(rng.integers(4)), None, {}), ("N1", 2, None, {"prob": 0.1, "noise_channel": "f"})]
+        spec = CircuitSpec(4, d, ops, "widths")
+        rec = Program(spec.build()).sample_frames(70, seed=nm)
+        want = frame.simulate(oracle.OracleProgram([spec], 4, d), nm, 70)
+        assert np.array_equal(rec, want), nm

@@ -1568,15 +1568,16 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
 template <int D>
 struct FrameSmem {
   using T = typename El<D>::T;
-  int fb, cb;              // Philox blocks of the frame draws, of the coins (odd d)
-  size_t ordf, ordc, warp0, x, z, rec, fire, warp;
+  int fb, cb;  // Philox blocks of the frame draws, of the coins (odd d, whole 32 ordinals)
+  size_t ordf, ordc, thr, warp0, x, z, rec, fire, warp;
   __host__ __device__ FrameSmem(int n, int nm, int nused, int nchunk, int cap) {
     auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
     fb = (n + nm + 3) / 4;
-    cb = D == 2 ? 0 : (nused + 3) / 4;
+    cb = D == 2 ? 0 : (nused + 31) / 32 * 8;
     ordf = kRawOps * 16 + up(4 * (kRawLayers + 1));
     ordc = ordf + (size_t)fb * sizeof(CoinOrdinal);
-    warp0 = ordc + (size_t)cb * sizeof(CoinOrdinal);
+    thr = ordc + (size_t)cb * sizeof(CoinOrdinal);
+    warp0 = thr + (size_t)cb * 16;
     x = 0;
     z = x + up((size_t)n * sizeof(T));
     rec = z + up((size_t)n * sizeof(T));
@@ -1597,6 +1598,7 @@ __global__ void __launch_bounds__(128) k_rows_frame(const RowFrameDesc fd) {
   uint32_t* wlay = reinterpret_cast<uint32_t*>(smem + kRawOps * 16);
   CoinOrdinal* ordf = reinterpret_cast<CoinOrdinal*>(smem + L_.ordf);
   CoinOrdinal* ordc = reinterpret_cast<CoinOrdinal*>(smem + L_.ordc);
+  uint32_t* thr = reinterpret_cast<uint32_t*>(smem + L_.thr);
   uint8_t* mem = smem + L_.warp0 + warp * L_.warp;
   T* X = reinterpret_cast<T*>(mem + L_.x);
   T* Z = reinterpret_cast<T*>(mem + L_.z);
@@ -1607,13 +1609,16 @@ __global__ void __launch_bounds__(128) k_rows_frame(const RowFrameDesc fd) {
   const PhiloxKeys K(fd.seed);
   for (int i = t; i < L_.fb; i += nt) ordf[i] = coin_ordinal(K, (uint32_t)i, 0u, 3u);
   for (int i = t; i < L_.cb; i += nt) ordc[i] = coin_ordinal(K, (uint32_t)i, 0u, 1u);
+  for (int i = t; i < 4 * L_.cb; i += nt) thr[i] = i < fd.nused ? __ldg(&fd.nhdr[i].x) : 0xffffffffu;
   __syncthreads();
   const long long first = ((long long)blockIdx.x * (nt >> 5) + warp) * 32;  // of the launch's shots
   const long long rel = first + lane;
   const bool live = rel < fd.nshots;
   const uint32_t shot = (uint32_t)(fd.shot0 + rel);  // shots are below 2^32: shot_hi 0
   const uint2 sh = coin_shot(K, shot, 0u);
-  // frame draws: z of qudit e at the start (e < n), after measurement e - n
+  // frame draws: z of qudit e at the start (e < n), after measurement e - n;
+  // four blocks' chains side by side
+#pragma unroll 4
   for (int b = 0; b < L_.fb; ++b) {
     const uint4 w = coin_block(K, ordf[b], sh);
     const uint32_t v[4] = {w.x, w.y, w.z, w.w};
@@ -1667,22 +1672,21 @@ __global__ void __launch_bounds__(128) k_rows_frame(const RowFrameDesc fd) {
   } else {
     for (int i = lane; i < 2 * fd.nused; i += 32) fire[i] = E_::zero();
     __syncwarp();
-    for (int b = 0; b < L_.cb; ++b) {
-      const uint4 w = coin_block(K, ordc[b], sh);
-      const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+    for (int b0 = 0; b0 < L_.cb; b0 += 8) {  // 32 ordinals' coins, then their few fires
       uint32_t f = 0u;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = 4 * b + q;
-        if (j < fd.nused) {
-          const uint2 nh = __ldg(fd.nhdr + j);
-          if (v[q] >= nh.x && nh.y != OP_N1OFF) f |= 1u << q;
-        }
+      for (int b = 0; b < 8; ++b) {
+        const uint4 w = coin_block(K, ordc[b0 + b], sh), th = reinterpret_cast<const uint4*>(thr)[b0 + b];
+        f |= ((uint32_t)(w.x >= th.x) | ((uint32_t)(w.y >= th.y) << 1) | ((uint32_t)(w.z >= th.z) << 2) |
+              ((uint32_t)(w.w >= th.w) << 3)) << (4 * b);
       }
       while (live && f) {
-        const int j = 4 * b + __ffs(f) - 1;
+        const int j = 4 * b0 + __ffs(f) - 1;
         f &= f - 1u;
-        const int2 ab = noise_choice(__ldg(&fd.nhdr[j].y), D, fd.seed, (long long)shot, (uint32_t)j);
+        // a coin of 0xffffffff meets the threshold of an ordinal that never fires
+        const uint32_t op = j < fd.nused ? __ldg(&fd.nhdr[j].y) : (uint32_t)OP_N1OFF;
+        if (op == OP_N1OFF) continue;
+        const int2 ab = noise_choice(op, D, fd.seed, (long long)shot, (uint32_t)j);
         E_::put(fire + 2 * j, lane, ab.x);
         E_::put(fire + 2 * j + 1, lane, ab.y);
       }

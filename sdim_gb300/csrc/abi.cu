@@ -2569,16 +2569,18 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
       return le == cudaSuccess ? SDIM_OK : cuda_fail(ctx, le, "frame pass launch");
     };
     // the reference shot beside the first part's coins and frames, on the
-    // stream of highest priority; only the output pass needs it
+    // stream of highest priority; only the output pass needs it, so it is
+    // launched behind them (L = 7, 100,000 frames: 338 us in front, 328 so)
     CK(cudaEventRecord(ctx->ev_gf, s));
     CK(cudaStreamWaitEvent(ctx->fast, ctx->ev_gf, 0));
+    if ((rc = launch_part(0)) != SDIM_OK) return rc;
     std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
     rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE);
     ctx->last_stream = s;
     if (rc != SDIM_OK) return rc;
     CK(cudaEventRecord(ctx->ev_fast, ctx->fast));
     for (long long f0 = 0; f0 < frames; f0 += part) {
-      if ((rc = launch_part(f0)) != SDIM_OK) return rc;
+      if (f0 > 0 && (rc = launch_part(f0)) != SDIM_OK) return rc;
       if (f0 == 0) CK(cudaStreamWaitEvent(s, ctx->ev_fast, 0));
       row_ops(c->d).frame_out(s, rf);
       const cudaError_t le = cudaGetLastError();

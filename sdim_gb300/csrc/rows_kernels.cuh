@@ -21,6 +21,13 @@ constexpr int L = kRowLanes;
 
 __device__ __forceinline__ uint32_t mux(uint32_t m, uint32_t a, uint32_t b) { return (m & a) | (~m & b); }
 __device__ __forceinline__ uint32_t maj(uint32_t a, uint32_t b, uint32_t c) { return (a & b) | (a & c) | (b & c); }
+// Bitwise function of three words by its truth table (bit 4 a + 2 b + c of F).
+template <int F>
+__device__ __forceinline__ uint32_t logic3(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(r) : "r"(a), "r"(b), "r"(c), "n"(F));
+  return r;
+}
 __device__ __forceinline__ uint32_t lane_mask(bool b) { return b ? 0xffffffffu : 0u; }
 
 // Three planes (d = 5, 7): bit 0 in x, bit 1 in y, bit 2 in z; w unused.
@@ -83,26 +90,60 @@ struct El {
       return add(v, make_uint4(mux(mn, u.x, t.x), t.y, mux(mn, u.z, t.z), 0u));
     }
   }
-  // v + c f, c uniform and not 0
-  static __device__ __forceinline__ T addmul(T v, T f, int c) {
-    if constexpr (D == 7) {
-      switch (c) {
-        case 1: return add(v, f);
-        case 2: return add(v, dbl(f));
-        case 3: return sub(v, dbl(dbl(f)));
-        case 4: return add(v, dbl(dbl(f)));
-        case 5: return sub(v, dbl(f));
-        default: return sub(v, f);
-      }
-    } else {
-      switch (c) {
-        case 1: return add(v, f);
-        case 2: return add(v, dbl(f));
-        case 3: return sub(v, dbl(f));
-        default: return sub(v, f);
-      }
+  // A sum under way, carries saved: the planes s and c (of the same weights)
+  // count together.  d = 7 counts mod 7, d = 5 mod 15 in four planes, so that a
+  // carry out of the last plane is one into the first, a negative is the
+  // complement and twice a value its rotation: a term costs a full adder, two
+  // instructions, per plane, where a whole addition mod d takes half as many
+  // again (d = 7) to twice as many.
+  struct Sum {
+    static constexpr int P = D == 7 ? 3 : 4;
+    uint32_t s[P], c[P];
+    __device__ __forceinline__ explicit Sum(T v) {
+      s[0] = v.x;
+      s[1] = v.y;
+      s[2] = v.z;
+      if constexpr (P == 4) s[3] = 0u;
+#pragma unroll
+      for (int i = 0; i < P; ++i) c[i] = 0u;
     }
-  }
+    // + C f, f = 0 for none
+    template <int C>
+    __device__ __forceinline__ void add(T f) {
+      constexpr bool kNeg = C > D / 2;
+      constexpr int A = kNeg ? D - C : C, R = D == 7 && A == 3 ? 2 : A - 1;  // 3 = -4 mod 7
+      constexpr bool kInv = D == 7 && A == 3 ? !kNeg : kNeg;
+      const uint32_t g[4] = {f.x, f.y, f.z, 0u};
+      uint32_t m[P];
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        const uint32_t a = kInv ? ~g[(i + P - R) % P] : g[(i + P - R) % P];
+        m[i] = maj(s[i], c[i], a);
+        s[i] ^= c[i] ^ a;
+      }
+#pragma unroll
+      for (int i = 0; i < P; ++i) c[(i + 1) % P] = m[i];
+    }
+    __device__ __forceinline__ T value() const {
+      if constexpr (D == 7) return El::add(make_uint4(s[0], s[1], s[2], 0u), make_uint4(c[0], c[1], c[2], 0u));
+      uint32_t r[4], k = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        r[i] = s[i] ^ c[i % P] ^ k;
+        k = maj(s[i], c[i % P], k);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // the carry back in
+        const uint32_t t = r[i] & k;
+        r[i] ^= k;
+        k = t;
+      }
+      // 0 .. 15 mod 5: by the low three planes for either value of the high one
+      return make_uint4(mux(r[3], logic3<0x29>(r[2], r[1], r[0]), logic3<0x4a>(r[2], r[1], r[0])),
+                        mux(r[3], logic3<0x31>(r[2], r[1], r[0]), logic3<0x8c>(r[2], r[1], r[0])),
+                        mux(r[3], logic3<0x42>(r[2], r[1], r[0]), logic3<0x10>(r[2], r[1], r[0])), 0u);
+    }
+  };
   static __device__ __forceinline__ int get(T a, int j) {
     const int v = (int)((a.x >> j) & 1u) | (int)(((a.y >> j) & 1u) << 1) | (int)(((a.z >> j) & 1u) << 2);
     return D == 7 && v == 7 ? 0 : v;
@@ -160,7 +201,24 @@ struct El<3> {  // two planes (planes3.cuh)
     const uint32_t m1 = lane_mask(c == 1), m2 = lane_mask(c == 2);
     return add(v, make_uint2((f.x & m1) | (f.y & m2), (f.y & m1) | (f.x & m2)));
   }
-  static __device__ __forceinline__ T addmul(T v, T f, int c) { return c == 1 ? add(v, f) : sub(v, f); }
+  struct Sum {  // mod 3 in two planes, as El<D>::Sum
+    uint32_t s[2], c[2];
+    __device__ __forceinline__ explicit Sum(T v) : s{v.x, v.y}, c{0u, 0u} {}
+    template <int C>
+    __device__ __forceinline__ void add(T f) {
+      const uint32_t a = C == 1 ? f.x : f.y, b = C == 1 ? f.y : f.x;
+      const uint32_t m = maj(s[0], c[0], a), n = maj(s[1], c[1], b);
+      s[0] ^= c[0] ^ a;
+      s[1] ^= c[1] ^ b;
+      c[0] = n;
+      c[1] = m;
+    }
+    __device__ __forceinline__ T value() const {
+      const uint32_t a = s[0] ^ c[0], k = s[0] & c[0], b = s[1] ^ c[1] ^ k, m = maj(s[1], c[1], k);
+      const uint32_t x = a ^ m, y = b ^ (a & m);
+      return make_uint2(x & ~y, y & ~x);  // 3 is 0
+    }
+  };
   static __device__ __forceinline__ int get(T a, int j) { return p3_get(p(a), j); }
   static __device__ __forceinline__ T set(T a, int j, int v) { return t(p3_set(p(a), j, v)); }
   static __device__ __forceinline__ T pick(uint32_t m, T a, T b) {
@@ -527,49 +585,57 @@ __device__ void stage_panel(PanelOps& po, typename El<D>::T* Fs, const RowDesc& 
   __syncthreads();
 }
 
-// Odd d: the elements [e0, cnt) of a row, buf, += sum of the panel's factor
-// rows times ab[0, nops), 32 elements a turn, up to the last whole turn or one
-// that is more than half full; returns the elements done.  The multiples are
-// uniform over the warp, so each takes its cheapest form.
-template <int D>
-__device__ __forceinline__ int combine_row(const PanelOps& po, const typename El<D>::T* Fs, typename El<D>::T* buf,
-                                           int cnt, const int* ab) {
-  using E_ = El<D>;
-  using T = typename E_::T;
-  const int lane = threadIdx.x & 31, nops = po.nops;
-  int e0 = 0;
-  for (; cnt - e0 > 16; e0 += 32) {
-    const int e = e0 + lane;
-    const bool in = e < cnt;
-    const T* f = Fs + (in ? e : 0);
-    T v = in ? buf[e] : E_::zero();
-#pragma unroll 2
-    for (int h = 0; h < nops; ++h) {
-      const int a = ab[h];
-      if (a != 0) v = E_::addmul(v, f[h * cnt], a);
-    }
-    if (in) buf[e] = v;
+// fn(integral_constant<int, c>) for c = 1 .. D - 1.
+template <int D, int C = 1, class Fn>
+__device__ __forceinline__ void each_multiple(Fn fn) {
+  if constexpr (C < D) {
+    fn(std::integral_constant<int, C>());
+    each_multiple<D, C + 1>(fn);
   }
-  return min(e0, cnt);
 }
 
-// The rest of a row, at most 16 elements from e0 on: lanes to spare take their
-// share of the ops, and the partial sums meet by shuffles.
+// Odd d: buf[0, cnt) += sum of the panel's factor rows times av (lane h: op h),
+// a lane to an element; where a turn's elements leave lanes over, K of them
+// share one, each with every K-th op, and the partial sums meet by shuffles.
+// The ops are taken multiple by multiple (ord: 32 bytes for their order), so
+// that a term is a carry-saving add of fixed form without a branch.
+// Bound by its logic instructions.  A panel of 31 rows: 256 qudits of d = 5 11.7k
+// cycles with additions mod d behind a branch per term, 6.6k so; 517 of d = 7
+// 12.8k and 9k; the step of 384 uneven programs 3534 us and 3423.
 template <int D>
-__device__ __forceinline__ void combine_tail(const PanelOps& po, const typename El<D>::T* Fs, typename El<D>::T* buf,
-                                             int e0, int cnt, const int* ab) {
+__device__ __forceinline__ void combine_row(const typename El<D>::T* Fs, typename El<D>::T* buf, int cnt, int av,
+                                            uint8_t* ord) {
   using E_ = El<D>;
   using T = typename E_::T;
-  const int lane = threadIdx.x & 31, nops = po.nops;
-  if (e0 < cnt) {
-    int G = 16;
+  const int lane = threadIdx.x & 31;
+  int n[D] = {}, first = 0;
+  each_multiple<D>([&](auto c) {
+    constexpr int C = c.value;
+    const uint32_t m = __ballot_sync(0xffffffffu, av == C);
+    n[C] = __popc(m);
+    if (av == C) ord[first + __popc(m & ((1u << lane) - 1u))] = (uint8_t)lane;
+    first += n[C];
+  });
+  __syncwarp();
+  for (int e0 = 0; e0 < cnt; e0 += 32) {
+    int G = 32;
     while (G > 1 && (G >> 1) >= cnt - e0) G >>= 1;
     const int K = 32 / G, part = lane / G, e = e0 + (lane & (G - 1));
     const bool in = e < cnt;
-    const T* f = Fs + (in ? e : 0);
-    T v = in && part == 0 ? buf[e] : E_::zero();
-    for (int h = part; h < nops; h += K) v = E_::muladd(v, f[h * cnt], ab[h]);
-    for (int o = G; o < 32; o <<= 1) v = E_::add(v, E_::shfl_xor(v, o));
+    typename E_::Sum sum(in && part == 0 ? buf[e] : E_::zero());
+    const uint8_t* o = ord + part;
+    each_multiple<D>([&](auto c) {
+      constexpr int C = c.value;
+#pragma unroll 2
+      for (int i = 0; i < n[C]; i += K) {
+        T f = E_::zero();
+        if (in && i + part < n[C]) f = Fs[o[i] * cnt + e];
+        sum.template add<C>(f);
+      }
+      o += n[C];
+    });
+    T v = sum.value();
+    for (int p = G; p < 32; p <<= 1) v = E_::add(v, E_::shfl_xor(v, p));
     if (in && part == 0) buf[e] = v;
   }
   __syncwarp();
@@ -619,9 +685,8 @@ __device__ __forceinline__ void update_row(const PanelOps& po, const typename El
       E_::put(buf + E + pe, pl, small_mod<D>(po.e[lane] * av));
     }
   }
-  ab[lane] = av;
   __syncwarp();
-  combine_tail<D>(po, Fs, buf, combine_row<D>(po, Fs, buf, 2 * E, ab), 2 * E, ab);
+  combine_row<D>(Fs, buf, 2 * E, av, a0b);
 }
 
 // The same for the stabilizer half alone, through the panel's ops with
@@ -649,7 +714,6 @@ __device__ __forceinline__ void update_half_row(const PanelOps& po, const typena
     const int a = small_mod<D>(__shfl_sync(0xffffffffu, av, h));
     av = lane == h ? a : av + a * po.G[h][lane];
   }
-  ab[lane] = lane < non ? av : 0;
   // S[p] from measurement h's K column.  An op past `after` replaces nothing,
   // but its pivot's entry is missing in the combination below (cleared): it is
   // the value gathered above.
@@ -659,7 +723,7 @@ __device__ __forceinline__ void update_half_row(const PanelOps& po, const typena
     E_::put(buf + pe, pl, lane < non ? om : small_mod<D>(av));
   }
   __syncwarp();
-  combine_tail<D>(po, Fs, buf, combine_row<D>(po, Fs, buf, E, ab), E, ab);
+  combine_row<D>(Fs, buf, E, lane < non ? av : 0, reinterpret_cast<uint8_t*>(ab));
 }
 
 // d = 2: lanes of a row's group (a power of two of at least E words, at most

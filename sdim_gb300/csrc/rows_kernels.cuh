@@ -1067,14 +1067,15 @@ __device__ void factor_panel(const RowDesc& rd, int k, typename El<D>::T* P, typ
       for (int w = lane; w < 2 * E; w += 32) {
         T v = row[w];
         if (w == pe || w == E + pe) v = E_::set(v, pl, 0);
-        stc(f + w, E_::mulc(v, D == 2 ? 1 : D - e));
-        if (w < E) reinterpret_cast<T*>(out)[w] = E_::neg(v);
+        v = E_::mulc(v, D == 2 ? 1 : D - e);
+        stc(f + w, v);
+        if (w < E) reinterpret_cast<T*>(out)[w] = v;
       }
       if (lane == 0) {
         const int o = h - nopsum;
         __stcg(rd.opm + h, make_int4(p, D == 2 ? 1 | (ps.tp[i] << 8) : e, m,
                                          D == 2 ? 0 : (ps.dup[o] + 1) | (ps.last[o] << 6)));
-        rd.mhdr[m] = make_uint4(2u * reset | (D == 2 ? 0u : (uint32_t)e << 8), (uint32_t)p, nord, 0u);
+        rd.mhdr[m] = make_uint4(2u * reset, (uint32_t)p, nord, 0u);
       }
     } else {
       for (int w = lane; w < E; w += 32) reinterpret_cast<T*>(out)[w] = row[E + w];
@@ -1493,6 +1494,7 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
   const unsigned long long seed = td.c.seed;
   constexpr int WIN = 32;
   const int pitch = td.pitch;  // staged bytes of a measurement, a multiple of 16
+  const bool resets = pitch > td.rowb;  // with the z_q rows of RESETs
   uint4* hdr = reinterpret_cast<uint4*>(smem);  // [2][WIN]
   uint8_t* rows = smem + 2 * WIN * 16;          // [2][WIN][pitch]
   uint8_t* mo = rows + 2 * (size_t)WIN * pitch + warp * (2 * 32 * 36) + sl * 36;  // this shot's outcomes
@@ -1529,9 +1531,33 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
     for (int k = gl; k < cnt; k += LG)
       if ((rnd >> k) & 1u) mo[k] = (uint8_t)mulshift(stream_block(seed, shot, (uint32_t)(wb + k), 0u).x, D);
     __syncwarp();
-    for (int k = 0; k < cnt; ++k) {
-      const uint4 h = hw[k];
+    // what a measurement reads, one ahead of its use
+    uint4 hn = make_uint4(0u, 0u, 0u, 0u);
+    T rn[WPL], zn[WPL];
+    int mn = 0;
+    auto fetch = [&](int k) {
       const T* row = reinterpret_cast<const T*>(rw + (size_t)k * pitch);
+      hn = hw[k];
+      mn = mo[k];
+#pragma unroll
+      for (int i = 0; i < WPL; ++i) {
+        const int e = gl + i * LG;
+        rn[i] = e < E ? row[e] : E_::zero();
+        zn[i] = e < E && resets ? reinterpret_cast<const T*>(reinterpret_cast<const uint8_t*>(row) + td.rowb)[e]
+                                : E_::zero();
+      }
+    };
+    fetch(0);
+    for (int k = 0; k < cnt; ++k) {
+      const uint4 h = hn;
+      T r[WPL], zr[WPL];
+#pragma unroll
+      for (int i = 0; i < WPL; ++i) {
+        r[i] = rn[i];
+        zr[i] = zn[i];
+      }
+      int m = mn;
+      if (k + 1 < cnt) fetch(k + 1);
       if constexpr (D != 2) {
         // N1 before the measurement: four coins a lane at a time; a group
         // applies one fire a turn
@@ -1573,39 +1599,26 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
           }
         }
       }
-      int m;
       if (!(h.x & 1u)) {
         const int p = (int)h.y, pe = p / L, pl = p % L;
         T x = d[0];
 #pragma unroll
-        for (int i = 1; i < WPL; ++i)
-          if ((pe >> lg) == i) x = d[i];
-        int dp = __shfl_sync(0xffffffffu, E_::get(x, pl), pe & (LG - 1), LG);
-        if constexpr (D != 2) dp = small_mod<D>(dp * (int)(h.x >> 8));
-        m = mo[k];
+        for (int i = 1; i < WPL; ++i) x = E_::pick(lane_mask((pe >> lg) == i), d[i], x);
+        const int dp = __shfl_sync(0xffffffffu, E_::get(x, pl), pe & (LG - 1), LG);
         const int nv = D == 2 ? m : m ? D - m : 0;
 #pragma unroll
-        for (int i = 0; i < WPL; ++i) {
-          const int e = gl + i * LG;
-          if (e < E) d[i] = E_::put_at(E_::muladd(d[i], row[e], dp), e == pe ? 1u << pl : 0u, nv);
-        }
+        for (int i = 0; i < WPL; ++i)
+          d[i] = E_::put_at(E_::muladd(d[i], r[i], dp), gl + i * LG == pe ? 1u << pl : 0u, nv);
       } else {
         int s = 0;
 #pragma unroll
-        for (int i = 0; i < WPL; ++i) {
-          const int e = gl + i * LG;
-          if (e < E) s += E_::dot(row[e], d[i]);
-        }
+        for (int i = 0; i < WPL; ++i) s += E_::dot(r[i], d[i]);
         for (int o = LG >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         m = D == 2 ? (((((int)h.w + 2 * s) & 3) + 1) >> 1) & 1 : (D - ((int)h.w + s) % D) % D;
       }
       if (h.x & 2u) {
-        const T* zr = reinterpret_cast<const T*>(rw + (size_t)k * pitch + td.rowb);
 #pragma unroll
-        for (int i = 0; i < WPL; ++i) {
-          const int e = gl + i * LG;
-          if (e < E) d[i] = E_::muladd(d[i], zr[e], m);
-        }
+        for (int i = 0; i < WPL; ++i) d[i] = E_::muladd(d[i], zr[i], m);
       }
       if (gl == 0) rec0[sl * 36 + k] = (uint8_t)(m | (int)((h.x & 1u) << 7));
     }

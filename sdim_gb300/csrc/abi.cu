@@ -693,6 +693,7 @@ RowDesc row_desc(const sdim_circuit* c, uint8_t* mem, uint4* mhdr, uint8_t* mrow
   r.nrow = nrow;
   r.n = c->n;
   r.d = c->d;
+  r.nops = p.nops;
   r.nlayers = p.nlayers;
   r.nm = c->nmeas;
   r.nx = p.nx;

@@ -101,7 +101,7 @@ struct RowDesc {
   uint4* mhdr;     // the trace
   uint8_t* mrow;   // rows of rowb bytes, two per measurement
   uint8_t* nrow;   // rows of rowb bytes, two per N1 ordinal
-  int n, d, nlayers, nm, nx, nk;
+  int n, d, nops, nlayers, nm, nx, nk;
   int E, EK;
   int rowb;         // bytes of a trace row
   int tile_begin;   // first raw-pass CTA of this program

@@ -411,13 +411,15 @@ __device__ __forceinline__ void raw_op(const RowDesc& rd, const uint4* o, int u,
 // Gates move no data between column words, so a CTA walks the layers on its
 // 2^lg units (u0 on) of every qudit alone; a layer's ops are on disjoint
 // qudits, so its (op, unit) tasks run in any order and one barrier ends it.
-// Bound by the chain of layers (two shared-memory reads, a gate and a barrier
-// each).  Threads 0 .. nt - 1 of the block; mem: raw_bytes(n, lg).
+// Bound by the chain of layers (a shared-memory read, a gate, its dumps and a
+// barrier each), 600 to 1,000 cycles a layer, so the ops come from global memory
+// a window ahead and, for d = 2, from shared memory a layer ahead.
+// Threads 0 .. nt - 1 of the block; mem: raw_bytes(n, lg).
 constexpr int kRawOps = 768, kRawLayers = 255;
 
 template <int D>
 __host__ __device__ inline size_t raw_bytes(int n, int lg) {
-  return 2 * ((size_t)n << lg) * sizeof(typename Unit<D>::T) + kRawOps * sizeof(uint4) + 4 * (kRawLayers + 1);
+  return 2 * ((size_t)n << lg) * sizeof(typename Unit<D>::T) + 2 * kRawOps * sizeof(uint4) + 4 * (kRawLayers + 2);
 }
 
 template <int D>
@@ -428,7 +430,7 @@ __device__ void raw_program(const RowDesc& rd, int u0, int lg, int nt, uint8_t* 
   const int n = rd.n, E = rd.E, cw = 1 << lg;
   const int units = (D == 2 ? E : 2 * E) + rd.EK;
   uint4* wops = reinterpret_cast<uint4*>(mem);
-  UT* x = reinterpret_cast<UT*>(wops + kRawOps);
+  UT* x = reinterpret_cast<UT*>(wops + 2 * kRawOps);
   UT* z = x + ((size_t)n << lg);
   uint32_t* wlay = reinterpret_cast<uint32_t*>(z + ((size_t)n << lg));
   auto sync = [&]() { asm volatile("bar.sync 2, %0;" ::"r"(nt) : "memory"); };
@@ -448,40 +450,74 @@ __device__ void raw_program(const RowDesc& rd, int u0, int lg, int nt, uint8_t* 
   const int c = t & (cw - 1), u = u0 + c, k0 = t >> lg, dk = nt >> lg;
   const bool mine = u < units, konst = u == (D == 2 ? 0 : 2 * E);
   // the ops of the layers that fit the window, in shared memory (a layer that
-  // does not fit by itself is read in place)
-  int l = 0;
-  while (l < rd.nlayers) {
+  // does not fit by itself is read in place), the next window's on their way
+  const uint32_t all = (uint32_t)rd.nops;
+  auto stage = [&](uint32_t w, int b) {
+    const uint32_t cnt = min(all - w, (uint32_t)kRawOps);
+    for (uint32_t i = t; i < cnt; i += nt) {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(wops + b * kRawOps + i);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rd.ops + w + i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int buf = 0;
+  stage(0u, 0);
+  for (int l = 0; l < rd.nlayers; l += kRawLayers) {
     const int nl = min(kRawLayers, rd.nlayers - l);
     for (int i = t; i <= nl; i += nt) wlay[i] = __ldg(rd.lay + l + i);
     sync();
-    const uint32_t w0 = wlay[0], wend = min(wlay[nl], w0 + (uint32_t)kRawOps);
-    for (uint32_t i0 = w0 + t; i0 < wend; i0 += 4 * nt) {
-      uint4 v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (i0 + j * nt < wend) v[j] = __ldg(rd.ops + i0 + j * nt);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (i0 + j * nt < wend) wops[i0 + j * nt - w0] = v[j];
-    }
-    sync();
-    int i = 0;
-    uint32_t b = w0;
-    for (; i < nl; ++i) {
-      const uint32_t e = wlay[i + 1];
-      if (e > wend) {
-        if (i > 0) break;
+    for (int i = 0; i < nl;) {
+      const uint32_t w0 = wlay[i];
+      int ie = i;  // layers [i, ie) fit
+      for (bool more = true; more;) {
+        const int q = ie + 1 + (t & 31);
+        const uint32_t fit = __ballot_sync(0xffffffffu, q <= nl && wlay[q] <= w0 + kRawOps);
+        ie += __popc(fit);
+        more = fit == 0xffffffffu;
+      }
+      const bool whole = ie > i;
+      if (!whole) ie = i + 1;
+      stage(wlay[ie], buf ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      sync();
+      const uint4* win = wops + buf * kRawOps - w0;
+      uint32_t b = w0;
+      if (!whole) {
+        const uint32_t e = wlay[ie];
         if (mine)
           for (uint32_t k = b + k0; k < e; k += dk) raw_op<D>(rd, rd.ops + k, u, c, lg, x, z, konst);
-      } else if (mine) {
-        for (uint32_t k = b + k0; k < e; k += dk) raw_op<D>(rd, wops + (k - w0), u, c, lg, x, z, konst);
+        i = ie;
+        sync();
       }
-      b = e;
-      sync();
+      if constexpr (D == 2) {  // (odd d: more registers, 100 cycles a layer slower so)
+        uint32_t e = wlay[i + 1];
+        uint4 ahead = make_uint4(0u, 0u, 0u, 0u);
+        if (i < ie && b + k0 < e) ahead = win[b + k0];
+        for (; i < ie; ++i) {
+          uint4 o = ahead;
+          const uint32_t e2 = i + 1 < ie ? wlay[i + 2] : e;
+          if (e + k0 < e2) ahead = win[e + k0];
+          if (mine)
+            for (uint32_t k = b + k0; k < e;) {
+              raw_op<D>(rd, &o, u, c, lg, x, z, konst);
+              if ((k += dk) < e) o = win[k];
+            }
+          b = e;
+          e = e2;
+          sync();
+        }
+      }
+      for (; i < ie; ++i) {
+        const uint32_t e = wlay[i + 1];
+        if (mine)
+          for (uint32_t k = b + k0; k < e; k += dk) raw_op<D>(rd, win + k, u, c, lg, x, z, konst);
+        b = e;
+        sync();
+      }
+      buf ^= 1;
     }
-    l += i;
-    sync();
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 template <int D>
@@ -1642,6 +1678,8 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
 // record words stay in shared memory to the end; the output pass
 // (k_rows_frame_out) adds the reference shot.
 // Bound by the Philox blocks of the draws.
+constexpr int kFrameOps = 768;  // ops of a window
+
 template <int D>
 struct FrameSmem {
   using T = typename El<D>::T;
@@ -1651,7 +1689,7 @@ struct FrameSmem {
     auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
     fb = (n + nm + 3) / 4;
     cb = D == 2 ? 0 : (nused + 31) / 32 * 8;
-    ordf = kRawOps * 16 + up(4 * (kRawLayers + 1));
+    ordf = kFrameOps * 16 + up(4 * (kRawLayers + 1));  // a window of ops, one of layers
     ordc = ordf + (size_t)fb * sizeof(CoinOrdinal);
     thr = ordc + (size_t)cb * sizeof(CoinOrdinal);
     warp0 = thr + (size_t)cb * 16;
@@ -1672,7 +1710,7 @@ __global__ void __launch_bounds__(128) k_rows_frame(const RowFrameDesc fd) {
   const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5;
   const int n = fd.n, nm = fd.nm;
   uint4* wops = reinterpret_cast<uint4*>(smem);
-  uint32_t* wlay = reinterpret_cast<uint32_t*>(smem + kRawOps * 16);
+  uint32_t* wlay = reinterpret_cast<uint32_t*>(smem + kFrameOps * 16);
   CoinOrdinal* ordf = reinterpret_cast<CoinOrdinal*>(smem + L_.ordf);
   CoinOrdinal* ordc = reinterpret_cast<CoinOrdinal*>(smem + L_.ordc);
   uint32_t* thr = reinterpret_cast<uint32_t*>(smem + L_.thr);
@@ -1857,7 +1895,7 @@ __global__ void __launch_bounds__(128) k_rows_frame(const RowFrameDesc fd) {
     const int nl = min(kRawLayers, fd.nlayers - l);
     for (int i = t; i <= nl; i += nt) wlay[i] = __ldg(fd.lay + l + i);
     __syncthreads();
-    const uint32_t w0 = wlay[0], wend = min(wlay[nl], w0 + (uint32_t)kRawOps);
+    const uint32_t w0 = wlay[0], wend = min(wlay[nl], w0 + (uint32_t)kFrameOps);
     for (uint32_t i = w0 + t; i < wend; i += nt) wops[i - w0] = staged(i);
     __syncthreads();
     int i = 0;

@@ -718,9 +718,9 @@ int launch_row_chain(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaSt
   return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row chain pass launch");
 }
 
-int launch_row_extra(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s) {
+int launch_row_extra(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaStream_t s, bool close) {
   if (g.xctas == 0) return SDIM_OK;
-  row_ops(g.d).extra(g.xctas, g.extra_smem, s, rd + g.b, g.e - g.b);
+  row_ops(g.d).extra(close, g.xctas, g.extra_smem, s, rd + g.b, g.e - g.b);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row extra pass launch");
 }
@@ -1037,6 +1037,11 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     for (RowDesc& r : hr) row_memory(r, r.raw + base);
     for (RowGroup& g : rgroups) plan_row_group(ctx, g, hr.data(), rcirc);
   }
+  // the row form's later passes take their places on the SMs early (follow.cuh)
+  // unless the chains of all groups fill them about twice over
+  long long chain_ctas = 0;
+  for (const RowGroup& g : rgroups) chain_ctas += (long long)g.ctas * (g.e - g.b);
+  const bool close = chain_ctas <= 2LL * ctx->num_sms;
   // the row form's phase pass: odd d, and d = 2 without fires to apply, each row
   // group's programs in a launch (those of a kept trace last, in one of their
   // own).  One element a lane up to kRowPhaseWarps warps in a launch, else two
@@ -1127,7 +1132,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       size_t smem = 0;
       for (int i = b; i < e; ++i) smem = std::max(smem, row_phase_smem(phr[i].pitch));
       const RowPhaseDesc& last = phr[e - 1];
-      row_ops(last.c.d).phase(r.wpl, last.block_begin + row_phase_blocks(last), smem, st,
+      row_ops(last.c.d).phase(close, r.wpl, last.block_begin + row_phase_blocks(last), smem, st,
                               dp + b, e - b);
       const cudaError_t le = cudaGetLastError();
       if (le != cudaSuccess) return cuda_fail(ctx, le, "row phase pass launch");
@@ -1240,7 +1245,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       if ((rc = launch_coins()) != SDIM_OK) return rc;
       coins_out = true;
     }
-    if ((rc = launch_row_extra(ctx, g, dr, st)) != SDIM_OK) return rc;
+    if ((rc = launch_row_extra(ctx, g, dr, st, close)) != SDIM_OK) return rc;
     if (fan && (rc = launch_row_phase(g.pb, g.pe, st)) != SDIM_OK) return rc;
   }
   if (d2_tab) {

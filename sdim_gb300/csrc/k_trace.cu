@@ -1,6 +1,7 @@
 // Trace engine kernels (d = 2): the x / z pass, one CTA per program over its
 // layered schedule, the phase pass, one lane per shot, and the column and
 // record passes that replace the phase pass for a single program.
+#include "follow.cuh"
 #include "trace_bits.cuh"
 #include "trace_cols.cuh"
 #include "variants.cuh"
@@ -38,6 +39,8 @@ __global__ void __launch_bounds__(THREADS) k_trace_pass(const TraceDesc* __restr
 //    pass evaluates such runs of deterministic measurements at once and
 //    corrects each outcome by the earlier RESETs it sees; lane = t).
 __global__ void __launch_bounds__(128) k_header_pass(const TraceDesc* __restrict__ descs, const int* status) {
+  follow_wait();
+  follow_ready();
   if (*(volatile const int*)status != DEV_OK) return;
   const TraceDesc* tdp = descs;
   const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(32 * kColumnWarps) k_column_pass(const TraceDe
   __shared__ uint4 shdr[column_window<TW>()];
   __shared__ __align__(16) uint32_t srow[column_window<TW>() * 2 * TW];
   __shared__ int smin;
+  follow_wait();
   if (*(volatile const int*)status != DEV_OK) return;  // the trace is incomplete (uniform over the block)
   column_block<TW, kColumnWarps>(descs, blockIdx.x, shdr, srow, &smin);
 }
@@ -184,7 +188,7 @@ void launch_philox_probe(int grid, cudaStream_t s, const unsigned long long* see
 }
 
 void launch_header_pass(int grid, cudaStream_t s, const TraceDesc* descs, const int* status) {
-  k_header_pass<<<grid, 128, 0, s>>>(descs, status);
+  launch_following(true, k_header_pass, grid, 128, 0, s, descs, status);
 }
 
 void launch_coin_pass(int grid, cudaStream_t s, const TraceDesc* descs, int ndesc) {
@@ -230,11 +234,11 @@ bool launch_phase_spl(int tw, int grid, int block, cudaStream_t s, const TraceDe
 
 bool launch_column_pass(int tw, int grid, cudaStream_t s, const TraceDesc* descs, const int* status) {
   switch (tw) {
-    case 2: k_column_pass<2><<<grid, 32 * kColumnWarps, 0, s>>>(descs, status); return true;
-    case 4: k_column_pass<4><<<grid, 32 * kColumnWarps, 0, s>>>(descs, status); return true;
-    case 8: k_column_pass<8><<<grid, 32 * kColumnWarps, 0, s>>>(descs, status); return true;
-    case 16: k_column_pass<16><<<grid, 32 * kColumnWarps, 0, s>>>(descs, status); return true;
-    case 32: k_column_pass<32><<<grid, 32 * kColumnWarps, 0, s>>>(descs, status); return true;
+    case 2: launch_following(true, k_column_pass<2>, grid, 32 * kColumnWarps, 0, s, descs, status); return true;
+    case 4: launch_following(true, k_column_pass<4>, grid, 32 * kColumnWarps, 0, s, descs, status); return true;
+    case 8: launch_following(true, k_column_pass<8>, grid, 32 * kColumnWarps, 0, s, descs, status); return true;
+    case 16: launch_following(true, k_column_pass<16>, grid, 32 * kColumnWarps, 0, s, descs, status); return true;
+    case 32: launch_following(true, k_column_pass<32>, grid, 32 * kColumnWarps, 0, s, descs, status); return true;
     default: return false;
   }
 }

@@ -199,10 +199,10 @@ struct RowOps {
   // 8) of `block` threads per program; rawt > 0: with the raw pass in front,
   // 2^lg units a CTA on rawt threads (smem at least raw_smem)
   cudaError_t (*chain)(int slice, int ctas, int block, int rawt, int lg, size_t smem, cudaStream_t s, const RowDesc* descs, int nd);
-  // extra pass: `ctas` CTAs, extra_per_cta rows each
-  void (*extra)(int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd);
+  // extra pass: `ctas` CTAs, extra_per_cta rows each (close: follow.cuh)
+  void (*extra)(bool close, int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd);
   // phase pass: `blocks` CTAs of 128 threads, wpl (1, 2 or 4) elements a lane
-  void (*phase)(int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd);
+  void (*phase)(bool close, int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd);
   // frame pass: `blocks` CTAs of `warps` (1 to 4) warps, 32 shots each
   size_t (*frame_smem)(const RowFrameDesc& f, int warps);
   void (*frame)(int blocks, int warps, size_t smem, cudaStream_t s, const RowFrameDesc& f);

@@ -1,6 +1,7 @@
 // Row form of the x / z pass (rows.cuh), device side: the raw, chain and extra
 // passes.  Instantiated for d = 2, 3, 5 and 7 in k_rows_<d>.cu.
 #pragma once
+#include "follow.cuh"
 #include "philox.cuh"
 #include "planes3.cuh"
 #include "record_out.cuh"
@@ -1308,6 +1309,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_chain(const RowDesc* __
         for (int q = k + 2; q <= next; ++q) __stcg(rd.pop + q, first);
       if (next == panels) break;
     }
+    if (next + 1 == panels) follow_ready();  // one panel to go
     const int b1 = next * kRowPanel;
     if (cnt > 0) {
       stage_panel<D, true>(po, Fs, rd, k, first, cnt);
@@ -1445,6 +1447,8 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_extra(const RowDesc* __
   __shared__ PanelOps po;
   using E_ = El<D>;
   using T = typename E_::T;
+  follow_wait();
+  follow_ready();
   const RowDesc rd = descs[find_tile(descs, nd, (int)blockIdx.x, true)];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int E = rd.E, XS = E + rd.EK;
@@ -1511,6 +1515,7 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
   extern __shared__ __align__(16) uint8_t smem[];
   using E_ = El<D>;
   using T = typename E_::T;
+  follow_wait();
   int di = 0;
   {
     int hi = nd - 1;
@@ -2064,13 +2069,12 @@ RowOps row_ops() {
     k_rows_raw<D><<<tiles, block, smem, s>>>(descs, nd, lg);
   };
   o.chain = chain<D>;
-  o.extra = [](int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd) {
-    k_rows_extra<D><<<ctas, 32 * kRowWarps, smem, s>>>(descs, nd);
+  o.extra = [](bool close, int ctas, size_t smem, cudaStream_t s, const RowDesc* descs, int nd) {
+    launch_following(close, k_rows_extra<D>, ctas, 32 * kRowWarps, smem, s, descs, nd);
   };
-  o.phase = [](int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd) {
-    if (wpl == 1) k_rows_phase<D, 1><<<blocks, 128, smem, s>>>(descs, nd);
-    else if (wpl == 2) k_rows_phase<D, 2><<<blocks, 128, smem, s>>>(descs, nd);
-    else k_rows_phase<D, 4><<<blocks, 128, smem, s>>>(descs, nd);
+  o.phase = [](bool close, int wpl, int blocks, size_t smem, cudaStream_t s, const RowPhaseDesc* descs, int nd) {
+    launch_following(close, wpl == 1 ? k_rows_phase<D, 1> : wpl == 2 ? k_rows_phase<D, 2> : k_rows_phase<D, 4>, blocks,
+                     128, smem, s, descs, nd);
   };
   o.frame_smem = [](const RowFrameDesc& f, int warps) {
     const FrameSmem<D> l(f.n, f.nm, f.nused, f.nchunk, f.cap);

@@ -606,9 +606,14 @@ struct RowGroup {
 //     leave SMs idle and the program has more than two panels; else one CTA.
 //     With more programs than SMs, CTAs no larger than the elimination needs,
 //     so that several share an SM.
+//     (517 qudits of d = 7: one CTA 1505 us, eight 874; 256 of d = 5: 470 and
+//     356; 97 qubits: 111 and 108; programs of two panels: equal.)
 //   raw pass: in front of the chain pass in the same launch while the clusters
-//     do not fill the SMs and its state fits their shared memory (one launch
-//     less, and a coin pass beside it finds those SMs taken); else its own
+//     do not fill the SMs, its state fits their shared memory and, of a single
+//     program, a layer's tasks their threads (one launch less, and a coin pass beside it finds
+//     those SMs taken; 256 qudits of d = 5, 300 tasks a layer: 356 us, 360 in a
+//     launch of its own; 517 of d = 7, 1,200 tasks: 874 and 856;
+//     384 uneven programs with that rule for all groups: 3371 and 3462); else its own
 //     launch, a unit (column word) per CTA while that leaves the SMs room, 2
 //     or 4 once there are several CTAs per SM, which read the layers' ops once
 //     for all of them.
@@ -628,14 +633,14 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
     for (int k = 8; k > 1 && g.ctas == 1; k >>= 1)
       if ((long long)k * (g.e - g.b) <= ctx->num_sms) g.ctas = k;
   const bool batch = (long long)g.ctas * (g.e - g.b) > ctx->num_sms;
-  g.cblock = !batch ? 32 * kRowWarps : g.slice < 16 ? 128 : g.slice == 17 ? 256 : 32 * kRowWarps;
+  g.cblock = !batch ? 32 * kRowWarps : g.slice < 16 || g.slice == kRowSliceSmall ? 128 : g.slice == 17 ? 256 : 32 * kRowWarps;
   g.chain_smem = row_ops(g.d).chain_smem(nmax, g.cblock);
   g.extra_smem = row_ops(g.d).extra_smem(nmax);
   // the raw pass in front of the chain pass, on its CTAs
   g.rawt = 0;
   for (g.lg = 0; (g.ctas << g.lg) < umax; ++g.lg) {}
   const size_t fused = row_ops(g.d).raw_smem(nmax, g.lg);
-  if (!batch && fused <= optin) {
+  if (!batch && fused <= optin && (g.e - g.b > 1 || (tasks << g.lg) <= g.cblock)) {
     g.rawt = 32;
     while (g.rawt < g.cblock && g.rawt < (tasks << g.lg)) g.rawt <<= 1;
     g.chain_smem = std::max(g.chain_smem, fused);
@@ -657,7 +662,8 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
 }
 
 // Warps in one phase-pass launch up to which a lane holds one element: about
-// six per scheduler.
+// six per scheduler (256 qudits of d = 5, eight elements: 10,000 shots, 2,500
+// warps, 428 us with one and 433 with two; 20,000 shots 518 and 478).
 constexpr long long kRowPhaseWarps = 152LL * 4 * 6;
 
 int row_phase_blocks(const RowPhaseDesc& p) {
@@ -784,7 +790,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
                           static_cast<uint8_t*>(nrow), rowb));
     rcirc.push_back(c);
     rmem += row_bytes(c->n, c->d, c->nmeas, c->rows.nx, c->rows.nk).total;
-    const int sl = row_slice(row_elems(c->n));
+    const int sl = row_slice(row_elems(c->n), c->d);
     if (rgroups.empty() || rgroups.back().d != c->d || rgroups.back().slice != sl)
       rgroups.push_back(RowGroup{c->d, sl, (int)hr.size() - 1, 0});
     rgroups.back().e = (int)hr.size();

@@ -139,9 +139,17 @@ inline int row_units(int n, int d, int nk) {
 }
 
 // How the chain pass spreads a row of E elements: its S (and T) elements per
-// lane, 16 added when several warps share a row.  Up to four elements one warp
-// holds whole rows, and a step needs no barrier.
-inline int row_slice(int E) { return E <= 1 ? 1 : E <= 2 ? 2 : E <= 4 ? 4 : 16 + (E <= 8 ? 1 : E <= 24 ? 2 : 4); }
+// lane, 16 added when several warps share a row.  One warp with whole rows
+// needs no barrier a step, but walks all its elements in each: up to four for
+// d = 2 (128 qubits: 122 us, with a warp per element 135), two for odd d (128
+// qudits of d = 5: 197 us with four a lane, 184 with a warp per element; 100
+// qutrits 145 and 135).  Programs of one slice are one launch: kRowSliceSmall,
+// a warp per element of up to four, is apart from wider rows, since a larger
+// group gets smaller clusters.
+constexpr int kRowSliceSmall = 16 + 32 + 1;
+inline int row_slice(int E, int d) {
+  return E <= 1 ? 1 : E <= 2 ? 2 : E <= 4 ? (d == 2 ? 4 : kRowSliceSmall) : 16 + (E <= 8 ? 1 : E <= 24 ? 2 : 4);
+}
 
 // A program in the row form's phase pass.
 struct RowPhaseDesc {

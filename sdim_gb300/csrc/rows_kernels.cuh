@@ -2007,14 +2007,16 @@ size_t raw_smem(int n, int lg) {
   return round16(raw_bytes<D>(n, lg));
 }
 
-// Chain-pass instances, by row_slice.
-template <class Fn>
+// Chain-pass instances, by row_slice (4 for d = 2 alone).
+template <int D, class Fn>
 cudaError_t for_slice(int slice, Fn fn) {
   using std::integral_constant;
+  if constexpr (D == 2)
+    if (slice == 4) return fn(integral_constant<int, 4>(), std::true_type());
   switch (slice) {
     case 1: return fn(integral_constant<int, 1>(), std::true_type());
     case 2: return fn(integral_constant<int, 2>(), std::true_type());
-    case 4: return fn(integral_constant<int, 4>(), std::true_type());
+    case kRowSliceSmall:
     case 17: return fn(integral_constant<int, 1>(), std::false_type());
     case 18: return fn(integral_constant<int, 2>(), std::false_type());
     default: return fn(integral_constant<int, 4>(), std::false_type());
@@ -2027,7 +2029,7 @@ cudaError_t set_smem(int optin) {
   cudaError_t e = set_dynamic_smem(k_rows_raw<D>, optin);
   for (int sl : kSlices)
     if (e == cudaSuccess)
-      e = for_slice(sl, [&](auto c, auto solo) { return set_dynamic_smem(k_rows_chain<D, c.value, solo.value>, optin); });
+      e = for_slice<D>(sl, [&](auto c, auto solo) { return set_dynamic_smem(k_rows_chain<D, c.value, solo.value>, optin); });
   if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 1>, optin);
   if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 2>, optin);
   if (e == cudaSuccess) e = set_dynamic_smem(k_rows_phase<D, 4>, optin);
@@ -2049,7 +2051,7 @@ cudaError_t chain(int slice, int C, int block, int rawt, int lg, size_t smem, cu
   a.val.clusterDim.y = a.val.clusterDim.z = 1;
   cfg.attrs = &a;
   cfg.numAttrs = C > 1 ? 1 : 0;
-  return for_slice(slice, [&](auto c, auto solo) {
+  return for_slice<D>(slice, [&](auto c, auto solo) {
     return cudaLaunchKernelEx(&cfg, k_rows_chain<D, c.value, solo.value>, descs, nd, C, rawt, lg);
   });
 }

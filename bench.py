@@ -899,7 +899,8 @@ def run_single(args, torch, dist, ws, rank, local):
         roofline = {"bound": "int-multiply (Philox4x32-10 blocks)", "achieved": ach / 1e9, "peak": prate / 1e9,
                     "unit": "Gblock/s", "frac": ach / prate,
                     "traffic": read_traffic("trace_engine_surface_L7.md") if args.workload == "surface" else None,
-                    "kernel": "trace engine step: k_trace_pass (x/z, 1 CTA) alongside k_coin_pass, then " +
+                    "kernel": "trace engine step: k_rows_chain and k_rows_extra (x/z, a cluster of 8 CTAs) alongside "
+                              "k_coin_pass, then " +
                               (f"k_column_pass<{trace_words(n)}> and k_record_pass<{nw}>" if columns else
                                f"k_phase_pass<{trace_words(n)}>"),
                     "peak_source": "Philox throughput measured live by sdim_probe_philox_rate",
@@ -925,9 +926,9 @@ def run_single(args, torch, dist, ws, rank, local):
                         "xz_pass": {
                             "ms": passes[0], "measurements": n_meas,
                             "us_per_measurement": 1e3 * passes[0] / max(n_meas, 1),
-                            "bound": "latency: one CTA walks the layered schedule; barriers and dependent "
-                                     "shared-memory chains per measurement block",
-                            "timed": "CUDA events from the step's first kernel to the end of k_trace_pass"},
+                            "bound": "latency: the layers of gates, then a dependent chain per random measurement "
+                                     "of a panel",
+                            "timed": "CUDA events from the step's first kernel to the end of k_rows_extra"},
                         "column_pass": {
                             "ms": passes[2] if columns else None, "columns": ncols, "column_words": nw,
                             "us_per_measurement": 1e3 * passes[2] / max(n_meas, 1) if columns else None,
@@ -956,19 +957,25 @@ def run_single(args, torch, dist, ws, rank, local):
             # SMs it runs on
             xz_ms = stages[0]
             sms, _ = u8_xz_layout(n, 1, ctx.smem_optin, ctx.num_sms, d)
+            rows = args.xz == "auto" and d in (3, 5, 7) and n <= 2048  # the row form: a cluster of 8 CTAs, or one
+            if rows:
+                sms = 8 if spec.num_measurements() > 62 else 1
             share = peak * sms / ctx.num_sms
             xz_ach = per_shot_bytes / (xz_ms / 1e3) / 1e9
-            xz_kernel = xz_kernel_name(ctx.lib.sdim_trace_xz_mode(n, d, 1, 0, ctx.smem_optin, ctx.num_sms))
+            xz_kernel = "k_rows_chain" if rows else \
+                xz_kernel_name(ctx.lib.sdim_trace_xz_mode(n, d, 1, 0, ctx.smem_optin, ctx.num_sms))
             roofline = {"bound": f"smem (x/z pass, latency-bound on {sms} CTA{'s' if sms > 1 else ''})",
                         "achieved": xz_ach, "peak": share, "unit": "GB/s", "frac": xz_ach / share,
                         "traffic": read_traffic(f"trace_engine_{args.workload}.md"),
                         "traffic_source": "DRAM bytes of one step under ncu, read from profiles/ (not measured "
                                           "in this run)",
-                        "kernel": f"{xz_kernel}<{d}> (x/z pass{', with k_cluster_det_headers after it' if sms == 8 else ''}), "
-                                  f"then k_phase_pass_u8<{d}>",
+                        "kernel": f"{xz_kernel}<{d}> (x/z pass{', with k_cluster_det_headers after it' if sms == 8 and not rows else ''}), "
+                                  f"then {'k_rows_phase' if rows else 'k_phase_pass_u8'}<{d}>",
                         "xz_latency": {"ms": xz_ms, "measurements": spec.num_measurements(),
                                        "us_per_measurement": 1e3 * xz_ms / max(spec.num_measurements(), 1),
-                                       "bound": "latency: the measurements run one after another, each with its "
+                                       "bound": "latency: a dependent chain per random measurement, after the "
+                                                "layers of gates" if rows else
+                                                "latency: the measurements run one after another, each with its "
                                                 "pivot search, barriers and rank-1 update or slice sums; the "
                                                 "gates between them are walked in order"},
                         "peak_source": f"sdim_probe_smem_bandwidth x {sms}/{ctx.num_sms} SMs",

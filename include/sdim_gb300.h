@@ -47,20 +47,24 @@ extern "C" {
 #define SDIM_FLAG_TEAM_WARP 64u  /* shot groups on one warp each, whatever n */
 #define SDIM_FLAG_TEAM_CTA 128u  /* shot groups on one CTA each, whatever n */
 #define SDIM_FLAG_TRACE 256u     /* trace engines (one x / z pass per program, then a per-shot phase
-                                    replay) whatever the shot count; by default they run from 128
-                                    shots or 160 qudits (n up to 2048) */
+                                    replay) whatever the shot count; by default they run every
+                                    program whose x / z pass has a row form (d = 2, 3, 5, 7, n up to
+                                    2048, no two-qudit gate on one qudit twice), others from 128 shots
+                                    or 160 qudits (n up to 2048).  The row form gives way to a tableau
+                                    pass with SDIM_FLAG_FORCE_GMEM, SPLIT_XZ, CLUSTER_XZ, U8_XZ,
+                                    PACKED_XZ or UNLAYERED */
 #define SDIM_FLAG_NO_TRACE 512u  /* no trace engine: shot-group engines only */
 #define SDIM_FLAG_NO_COIN_PASS 1024u /* trace engine: draw N1 coins inside the phase pass, no coin pass */
 #define SDIM_FLAG_SPLIT_XZ 2048u /* odd-d trace engine: x / z pass on a CTA pair whenever it fits */
 #define SDIM_FLAG_CLUSTER_XZ 4096u /* odd-d trace engine: x / z pass on a cluster of 8 CTAs whatever n,
                                       columns in shared memory where they fit (global memory with
-                                      SDIM_FLAG_FORCE_GMEM); by default the cluster takes the programs
-                                      that do not fit one CTA in batches of fewer than 76 odd-d trace
+                                      SDIM_FLAG_FORCE_GMEM); of the programs without a row form the
+                                      cluster takes those that do not fit one CTA in batches of fewer than 76 odd-d trace
                                       programs (larger batches use CTA pairs, then single CTAs streaming
                                       from global memory) */
 #define SDIM_FLAG_U8_XZ 16384u /* odd-d trace engine: x / z pass on residue bytes (the forms of d >= 11)
                                  instead of the two-bit-plane tableau (d = 3) or 4-bit lanes (d = 5, 7),
-                                 which batches of 76+ odd-d trace programs use by default */
+                                 which batches of 76+ odd-d trace programs without a row form use */
 #define SDIM_FLAG_PACKED_XZ 131072u /* odd-d trace engine, d = 3, 5, 7: the packed x / z pass (bit planes,
                                        4-bit lanes) also for runs of fewer than 76 odd-d trace programs */
 #define SDIM_FLAG_LANE_SHOTS_1 65536u /* d = 2 trace engine: one shot per phase-pass lane (by default two
@@ -215,7 +219,8 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
                     const double* noise_prob, const int32_t* n, const int32_t* d, const uint64_t* seeds,
                     const int64_t* shot0, const int64_t* nshots, uint8_t* const* outs, void* stream,
                     unsigned flags);
-/* The form the odd-d trace engine's x / z pass takes for a program of n
+/* The tableau form that the odd-d trace engine's x / z pass takes, where it
+ * does not run in row form (SDIM_FLAG_TRACE above), for a program of n
  * qudits and odd prime dimension d in a run with odd_trace_programs odd-d
  * trace programs, on a device with smem_optin bytes of opt-in shared memory
  * per block and num_sms SMs: 0 one CTA, byte tableau in shared memory; 1 a

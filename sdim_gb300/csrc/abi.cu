@@ -1224,7 +1224,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   // it: on the stream of highest priority, up to its column pass, since the
   // coin pass's blocks take every SM that the short chain leaves and the passes
   // after it would wait for them to drain (the L = 7 step: 381 us with them on
-  // the caller's stream)
+  // the caller's stream, 322 so)
   const bool d2_fast = k == 1 && coins && d2_xz && hd[0].rows;
   cudaStream_t xs = s;
   if (d2_fast) {

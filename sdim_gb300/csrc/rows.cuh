@@ -97,7 +97,7 @@ struct RowDesc {
   int4* opm;       // their {pivot, exponent | commute parity << 8, ordinal, 1 + last op of the panel
                    // before it with its pivot (0: none) | no later one has it << 6}
   int* pop;        // first op of each panel, [panels + 1]
-  uint32_t* opw;   // odd d: each panel's matrix W, [panels][32][8] words (k_rows.cu: PanelOps::Wt)
+  uint32_t* opw;   // odd d: each panel's matrix W, [panels][32][8] words (rows_kernels.cuh: PanelOps::Wt)
   uint4* mhdr;     // the trace
   uint8_t* mrow;   // rows of rowb bytes, two per measurement
   uint8_t* nrow;   // rows of rowb bytes, two per N1 ordinal

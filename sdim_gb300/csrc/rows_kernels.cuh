@@ -869,7 +869,10 @@ __device__ __forceinline__ void bar_threads(int n) { asm volatile("bar.sync 1, %
 // offers that one.  Deterministic rows cost a dot product and no step.
 // kSolo: one warp holds whole rows (E <= CE) and needs neither offers nor
 // barriers.
-// Bound by the step's chain of dependent instructions, not by their number.
+// Bound by the step's chain of dependent instructions, then by their number
+// (integer logic issues at half rate).  Panels of 31 rows: 17k to 27k cycles at
+// 256 qudits of d = 5, 52k at 517 of d = 7, 27k at 451 qubits.  A pivot's warp
+// running on alone with the others behind it took twice that.
 template <int D, int CE, bool kSolo>
 __device__ __forceinline__ void eliminate(const RowDesc& rd, int cnt, typename El<D>::T* P, typename El<D>::T* V,
                                           PanelState& ps) {
@@ -1185,8 +1188,8 @@ __device__ __forceinline__ void det_row(const RowDesc& rd, int m, GetV phase) {
 }
 
 // One program per cluster of C CTAs.  rawt > 0: the raw pass first, 2^lg units
-// a CTA on rawt threads.  CTA 0 eliminates panel after panel (32
-// rows in shared memory); the panel's updates then go to the rows after it:
+// a CTA on rawt threads.  CTA 0 eliminates panel after panel (31
+// rows and V in shared memory); the panel's updates then go to the rows after it:
 // with C = 1 by this CTA itself, with more the next panel's rows by CTA 0 (it
 // eliminates them next) and the others' by the other CTAs meanwhile, so one
 // cluster barrier per panel is all they wait for.  A panel that had no random
@@ -1194,6 +1197,11 @@ __device__ __forceinline__ void det_row(const RowDesc& rd, int m, GetV phase) {
 // entries are then deterministic and independent, a warp takes each, and their
 // panels cost no step (the rounds after the first of an error-correction
 // memory).
+// Bound by CTA 0's elimination, about 550 cycles a random row in one warp and
+// 1,000 to 1,900 across warps, and by the layers in front.  As tableau passes,
+// every random measurement updating all generators: 256 qudits of d = 5, 516
+// measurements, 2,170 us, 390 so; the L = 7 memory 157 and 65 (102 with every
+// deterministic panel a step).
 template <int D, int CE, bool kSolo>
 __global__ void __launch_bounds__(32 * kRowWarps) k_rows_chain(const RowDesc* __restrict__ descs, int nd, int C, int rawt,
                                                                int lg) {
@@ -1440,7 +1448,9 @@ __device__ __forceinline__ uint8_t* extra_row(const RowDesc& rd, uint32_t who) {
 }
 
 // Stabilizer halves of the rows that only the phase pass reads, through every
-// update that precedes them.
+// update that precedes them.  Apart from the chain, since nothing in it waits
+// for them: bound by their own updates, 38 us for the 256 RESETs of 256 qudits
+// of d = 5, 9 us for the L = 7 memory's rows.
 template <int D>
 __global__ void __launch_bounds__(32 * kRowWarps) k_rows_extra(const RowDesc* __restrict__ descs, int nd) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1508,8 +1518,11 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_rows_extra(const RowDesc* __
 // while the 32 before them run, and a window's outcomes are drawn at its start
 // with every lane on another draw.  A measurement then needs no barrier: a
 // shuffle for the pivot's delta or log LG for a factor sum.
-// Bound by a measurement's chain of about 60 instructions where the warps are
-// few, by their issue where they are many (then WPL elements a lane).
+// Bound by a measurement's chain of dependent instructions where the warps are
+// few, by their issue (172 a measurement and warp at d = 5) where they are many
+// (then WPL elements a lane).  As residue bytes, 32 shots a CTA with barriers a
+// measurement, 256 qudits of d = 5 and 4,096 shots took 760 us; 185 us with
+// packed rows, 175 with a measurement's reads one ahead.
 template <int D, int WPL>
 __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restrict__ descs, int nd) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1682,7 +1695,10 @@ __global__ void __launch_bounds__(128) k_rows_phase(const RowPhaseDesc* __restri
 // shots fires, behind a bitmap), else by atomics into a word per ordinal.  The
 // record words stay in shared memory to the end; the output pass
 // (k_rows_frame_out) adds the reference shot.
-// Bound by the Philox blocks of the draws.
+// Bound by its instructions, 22k a warp for the L = 7 memory: the draws' Philox
+// blocks and the ops about equally.  A byte per shot and qudit, a lane per shot:
+// 100,000 shots 1,500 us; on bit planes 130, 115 with four blocks of draws side
+// by side.  10,000 shots of 48 qutrits: 78 and 46 us.
 constexpr int kFrameOps = 768;  // ops of a window
 
 template <int D>

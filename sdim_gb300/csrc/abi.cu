@@ -633,7 +633,7 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
     for (int k = 8; k > 1 && g.ctas == 1; k >>= 1)
       if ((long long)k * (g.e - g.b) <= ctx->num_sms) g.ctas = k;
   const bool batch = (long long)g.ctas * (g.e - g.b) > ctx->num_sms;
-  g.cblock = !batch ? 32 * kRowWarps : g.slice < 16 || g.slice == kRowSliceSmall ? 128 : g.slice == 17 ? 256 : 32 * kRowWarps;
+  g.cblock = !batch ? 32 * kRowWarps : g.slice < 16 || g.slice == kRowSliceSmall ? 128 : g.slice == kRowSliceMid ? 256 : 32 * kRowWarps;
   g.chain_smem = row_ops(g.d).chain_smem(nmax, g.cblock);
   g.extra_smem = row_ops(g.d).extra_smem(nmax);
   // the raw pass in front of the chain pass, on its CTAs

@@ -143,12 +143,14 @@ inline int row_units(int n, int d, int nk) {
 // needs no barrier a step, but walks all its elements in each: up to four for
 // d = 2 (128 qubits: 122 us, with a warp per element 135), two for odd d (128
 // qudits of d = 5: 197 us with four a lane, 184 with a warp per element; 100
-// qutrits 145 and 135).  Programs of one slice are one launch: kRowSliceSmall,
-// a warp per element of up to four, is apart from wider rows, since a larger
-// group gets smaller clusters.
-constexpr int kRowSliceSmall = 16 + 32 + 1;
+// qutrits 145 and 135).  Then two a lane (256 qudits of d = 5: 359 us, one 368;
+// 500: 706, one 744) and four past 24 (1,000 of d = 7: 1677 us, two 1767).
+// Programs of one slice are one launch: kRowSliceSmall, a warp per element of up
+// to four, and kRowSliceMid, two a lane of up to eight, are apart from wider
+// rows, since a larger group gets smaller clusters.
+constexpr int kRowSliceSmall = 16 + 32 + 1, kRowSliceMid = 16 + 32 + 2;
 inline int row_slice(int E, int d) {
-  return E <= 1 ? 1 : E <= 2 ? 2 : E <= 4 ? (d == 2 ? 4 : kRowSliceSmall) : 16 + (E <= 8 ? 1 : E <= 24 ? 2 : 4);
+  return E <= 1 ? 1 : E <= 2 ? 2 : E <= 4 ? (d == 2 ? 4 : kRowSliceSmall) : E <= 8 ? kRowSliceMid : E <= 24 ? 18 : 20;
 }
 
 // A program in the row form's phase pass.

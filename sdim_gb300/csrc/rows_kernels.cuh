@@ -2023,22 +2023,24 @@ size_t raw_smem(int n, int lg) {
   return round16(raw_bytes<D>(n, lg));
 }
 
-// Chain-pass instances, by row_slice (4 for d = 2 alone).
+// Chain-pass instances, by row_slice (4 for d = 2 alone, kRowSliceSmall for odd d).
 template <int D, class Fn>
 cudaError_t for_slice(int slice, Fn fn) {
   using std::integral_constant;
-  if constexpr (D == 2)
+  if constexpr (D == 2) {
     if (slice == 4) return fn(integral_constant<int, 4>(), std::true_type());
+  } else {
+    if (slice == kRowSliceSmall) return fn(integral_constant<int, 1>(), std::false_type());
+  }
   switch (slice) {
     case 1: return fn(integral_constant<int, 1>(), std::true_type());
     case 2: return fn(integral_constant<int, 2>(), std::true_type());
-    case kRowSliceSmall:
-    case 17: return fn(integral_constant<int, 1>(), std::false_type());
-    case 18: return fn(integral_constant<int, 2>(), std::false_type());
+    case kRowSliceMid:
+    case 16 + 2: return fn(integral_constant<int, 2>(), std::false_type());
     default: return fn(integral_constant<int, 4>(), std::false_type());
   }
 }
-constexpr int kSlices[] = {1, 2, 4, 17, 18, 20};
+constexpr int kSlices[] = {1, 2, 4, kRowSliceSmall, kRowSliceMid, 20};
 
 template <int D>
 cudaError_t set_smem(int optin) {

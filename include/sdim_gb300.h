@@ -249,6 +249,29 @@ int sdim_trace_xz_mode(int32_t n, int32_t d, int64_t odd_trace_programs, unsigne
  * counterpart in the reference. */
 int sdim_program_words(const int32_t* ops, int64_t nops, const double* noise_prob, int32_t n, int32_t d,
                        int32_t layered, uint32_t* out, int64_t cap, int64_t* count);
+/* The row form of a program's x / z pass (rows as in sdim_encode_circuit; see
+ * SDIM_FLAG_TRACE): out[0] its ops, 0 when the program has none and takes the
+ * tableau passes, [1] layers, [2] measurements, [3] rows that only the phase
+ * pass reads (two per N1, one per RESET), [4] measurements whose Z_q a later
+ * row may hold, [5] bytes of its rows and updates.  Host-only (no device is
+ * touched), for inspection and tests.  The codes of sdim_encode_circuit.  No
+ * counterpart in the reference. */
+int sdim_row_program(const int32_t* ops, int64_t nops, const double* noise_prob, int32_t n, int32_t d,
+                     int64_t out[6]);
+/* The launch shape of the row form's passes for `count` programs of one d that
+ * share a launch, on a device with smem_optin bytes of opt-in shared memory per
+ * block and num_sms SMs; programs holds count x 6 values as sdim_row_program
+ * gives them.  out[0] CTAs per program of the chain pass, [1] their threads,
+ * [2] threads of a CTA that run the raw pass in front of it (0: a launch of
+ * its own), [3] log2 of the column words of a raw-pass CTA, [4] threads of a
+ * raw-pass CTA (0 when in front of the chain pass), [5] raw-pass CTAs of all
+ * programs at that many words each, [6] column words of the widest program,
+ * [7] CTAs of the extra pass.  Host-only (no device is touched), for
+ * inspection and tests.  SDIM_EINVAL for programs that do not share a launch
+ * (different spread of a row over lanes and warps) or without a row form.  No
+ * counterpart in the reference. */
+int sdim_row_plan(int32_t d, int32_t count, const int32_t* n, const int64_t* programs, int32_t smem_optin,
+                  int32_t num_sms, int32_t out[8]);
 /* Measured shared-memory read bandwidth of the device in GB/s (all SMs):
  * the roofline denominator for tableaux resident in shared memory.  No
  * counterpart in the reference (which has no device code). */

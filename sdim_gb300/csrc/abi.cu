@@ -609,15 +609,16 @@ struct RowGroup {
 //     (517 qudits of d = 7: one CTA 1505 us, eight 874; 256 of d = 5: 470 and
 //     356; 97 qubits: 111 and 108; programs of two panels: equal.)
 //   raw pass: in front of the chain pass in the same launch while the clusters
-//     do not fill the SMs, its state fits their shared memory and, of a single
-//     program, a layer's tasks their threads (one launch less, and a coin pass beside it finds
+//     do not fill the SMs, its state fits their shared memory, a CTA has a thread for
+//     each of its units (a thread serves one, raw_program) and, of a single
+//     program, for each of a layer's tasks (one launch less, and a coin pass beside it finds
 //     those SMs taken; 256 qudits of d = 5, 300 tasks a layer: 356 us, 360 in a
 //     launch of its own; 517 of d = 7, 1,200 tasks: 874 and 856;
 //     384 uneven programs with that rule for all groups: 3371 and 3462); else its own
 //     launch, a unit (column word) per CTA while that leaves the SMs room, 2
 //     or 4 once there are several CTAs per SM, which read the layers' ops once
 //     for all of them.
-void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vector<const sdim_circuit*>& c) {
+int plan_row_group(sdim_ctx* ctx, RowGroup& g, RowDesc* h) {
   long long units = 0, tasks = 1;
   int nmax = 1, nmmax = 0, umax = 1;
   for (int i = g.b; i < g.e; ++i) {
@@ -625,7 +626,7 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
     umax = std::max(umax, row_units(h[i].n, g.d, h[i].nk));
     nmax = std::max(nmax, h[i].n);
     nmmax = std::max(nmmax, h[i].nm);
-    tasks = std::max<long long>(tasks, c[i]->rows.nops / std::max(1, h[i].nlayers));
+    tasks = std::max<long long>(tasks, h[i].nops / std::max(1, h[i].nlayers));
   }
   const size_t optin = (size_t)ctx->smem_optin - 12288;  // less the kernels' static arrays
   g.ctas = 1;
@@ -640,7 +641,7 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
   g.rawt = 0;
   for (g.lg = 0; (g.ctas << g.lg) < umax; ++g.lg) {}
   const size_t fused = row_ops(g.d).raw_smem(nmax, g.lg);
-  if (!batch && fused <= optin && (g.e - g.b > 1 || (tasks << g.lg) <= g.cblock)) {
+  if (!batch && fused <= optin && (1 << g.lg) <= g.cblock && (g.e - g.b > 1 || (tasks << g.lg) <= g.cblock)) {
     g.rawt = 32;
     while (g.rawt < g.cblock && g.rawt < (tasks << g.lg)) g.rawt <<= 1;
     g.chain_smem = std::max(g.chain_smem, fused);
@@ -659,6 +660,11 @@ void plan_row_group(const sdim_ctx* ctx, RowGroup& g, RowDesc* h, const std::vec
     const int per = row_ops(g.d).extra_per_cta(h[i].n);
     g.xctas += (h[i].nx + per - 1) / per;
   }
+  // what the raw pass's loops rest on: whole strides of units, a thread at least for each
+  const int threads = g.rawt ? g.rawt : g.block;
+  if ((1 << g.lg) > threads || threads % (1 << g.lg) || (g.rawt && (g.ctas << g.lg) < umax))
+    return fail(ctx, SDIM_ECUDA, "row raw pass: more column words than threads");
+  return SDIM_OK;
 }
 
 // Warps in one phase-pass launch up to which a lane holds one element: about
@@ -779,7 +785,6 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     }
   // row-form programs: their descriptors, d = 2 first
   std::vector<RowDesc> hr;
-  std::vector<const sdim_circuit*> rcirc;
   std::vector<RowGroup> rgroups;
   size_t rmem = 0;
   std::vector<int> rjob;  // their indices in jobs (d = 2) or ujobs
@@ -788,7 +793,6 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     // memory offsets first, the base pointer once the buffer's size is known
     hr.push_back(row_desc(c, reinterpret_cast<uint8_t*>(rmem), mhdr, static_cast<uint8_t*>(mrow),
                           static_cast<uint8_t*>(nrow), rowb));
-    rcirc.push_back(c);
     rmem += row_bytes(c->n, c->d, c->nmeas, c->rows.nx, c->rows.nk).total;
     const int sl = row_slice(row_elems(c->n), c->d);
     if (rgroups.empty() || rgroups.back().d != c->d || rgroups.back().slice != sl)
@@ -1041,7 +1045,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     if ((rc = ensure(ctx, ctx->rows, std::max<size_t>(rmem, 256))) != SDIM_OK) return rc;
     const size_t base = reinterpret_cast<size_t>(ctx->rows.p);
     for (RowDesc& r : hr) row_memory(r, r.raw + base);
-    for (RowGroup& g : rgroups) plan_row_group(ctx, g, hr.data(), rcirc);
+    for (RowGroup& g : rgroups)
+      if ((rc = plan_row_group(ctx, g, hr.data())) != SDIM_OK) return rc;
   }
   // the row form's later passes take their places on the SMs early (follow.cuh)
   // unless the chains of all groups fill them about twice over
@@ -2090,6 +2095,58 @@ int sdim_trace_xz_mode(int32_t n, int32_t d, int64_t odd_trace_programs, unsigne
       num_sms <= 0)
     return SDIM_EINVAL;
   return odd_xz_mode(n, d, (long long)odd_trace_programs, flags, (size_t)smem_optin, num_sms);
+}
+
+int sdim_row_program(const int32_t* ops, int64_t nops, const double* noise_prob, int32_t n, int32_t d, int64_t out[6]) {
+  if (!out || (nops > 0 && !ops) || nops < 0) return SDIM_EINVAL;
+  std::vector<uint2> dev;
+  int nmeas = 0, nn1 = 0;
+  const int rc = encode_rows(nullptr, ops, nops, noise_prob, n, d, dev, nmeas, nn1);
+  if (rc != SDIM_OK) return rc;
+  RowProgram r;
+  append_rows(dev, 0, dev.size(), n, d, nmeas, r);
+  out[0] = r.nops;
+  out[1] = r.nlayers;
+  out[2] = nmeas;
+  out[3] = r.nx;
+  out[4] = r.nk;
+  out[5] = r.nops ? (int64_t)row_bytes(n, d, nmeas, r.nx, r.nk).total : 0;
+  return SDIM_OK;
+}
+
+int sdim_row_plan(int32_t d, int32_t count, const int32_t* n, const int64_t* programs, int32_t smem_optin,
+                  int32_t num_sms, int32_t out[8]) {
+  if (!row_dim(d) || count < 1 || !n || !programs || !out || smem_optin <= 0 || num_sms <= 0) return SDIM_EINVAL;
+  sdim_ctx ctx;  // the planner reads the two limits alone
+  ctx.smem_optin = smem_optin;
+  ctx.num_sms = num_sms;
+  std::vector<RowDesc> h(count);
+  int units = 0;
+  for (int i = 0; i < count; ++i) {
+    const int64_t* p = programs + 6 * i;
+    if (n[i] < 1 || n[i] > 2048 || p[0] < 1 || row_slice(row_elems(n[i]), d) != row_slice(row_elems(n[0]), d))
+      return SDIM_EINVAL;
+    std::memset(&h[i], 0, sizeof(RowDesc));
+    h[i].n = n[i];
+    h[i].d = d;
+    h[i].nops = (int)p[0];
+    h[i].nlayers = (int)p[1];
+    h[i].nm = (int)p[2];
+    h[i].nx = (int)p[3];
+    h[i].nk = (int)p[4];
+    units = std::max(units, row_units(n[i], d, h[i].nk));
+  }
+  RowGroup g{d, row_slice(row_elems(n[0]), d), 0, count};
+  const int rc = plan_row_group(&ctx, g, h.data());
+  out[0] = g.ctas;
+  out[1] = g.cblock;
+  out[2] = g.rawt;
+  out[3] = g.lg;
+  out[4] = g.rawt ? 0 : g.block;
+  out[5] = g.tiles;
+  out[6] = units;
+  out[7] = g.xctas;
+  return rc;
 }
 
 int sdim_probe_smem_bandwidth(sdim_ctx* ctx, double* gbs) {

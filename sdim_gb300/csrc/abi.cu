@@ -2643,8 +2643,10 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
     CK(cudaEventRecord(ctx->ev_gf, s));
     CK(cudaStreamWaitEvent(ctx->fast, ctx->ev_gf, 0));
     if ((rc = launch_part(0)) != SDIM_OK) return rc;
+    // (its own fires, if it holds any N1, are drawn in its phase pass: the fire
+    // masks in ctx->masks are the frames' while both run)
     std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
-    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE);
+    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE | SDIM_FLAG_NO_COIN_PASS);
     ctx->last_stream = s;
     if (rc != SDIM_OK) return rc;
     CK(cudaEventRecord(ctx->ev_fast, ctx->fast));

@@ -559,6 +559,7 @@ class Timer:
             step_fn()
             e1.record(self.stream)
             self.ctx.sync()
+            e1.synchronize()  # ctx.sync waits for the library's own stream alone
             step_ms.append(e0.elapsed_time(e1))
             kern_ms.append(self.ctx.last_kernel_ms())
             self.stage_ms.append(self.ctx.last_stage_ms())
@@ -604,6 +605,7 @@ def graph_replay(args, torch, ctx, timer, stream, entries, units_per_step, expec
             run.launch(shot0=moved(args.warmup + 1 + k), stream=stream.cuda_stream)
             e1.record(stream)
             run.sync()
+            e1.synchronize()  # run.sync waits for the replay, which ends before e1
             ms.append(e0.elapsed_time(e1))
         run.launch(shot0=moved(0), stream=stream.cuda_stream)
         run.sync()

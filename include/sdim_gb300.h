@@ -47,12 +47,15 @@ extern "C" {
 #define SDIM_FLAG_TEAM_WARP 64u  /* shot groups on one warp each, whatever n */
 #define SDIM_FLAG_TEAM_CTA 128u  /* shot groups on one CTA each, whatever n */
 #define SDIM_FLAG_TRACE 256u     /* trace engines (one x / z pass per program, then a per-shot phase
-                                    replay) whatever the shot count; by default they run every
-                                    program whose x / z pass has a row form (d = 2, 3, 5, 7, n up to
-                                    2048, no two-qudit gate on one qudit twice), others from 128 shots
-                                    or 160 qudits (n up to 2048).  The row form gives way to a tableau
-                                    pass with SDIM_FLAG_FORCE_GMEM, SPLIT_XZ, CLUSTER_XZ, U8_XZ,
-                                    PACKED_XZ or UNLAYERED */
+                                    replay) whatever the shot count; by default they run programs
+                                    from 128 shots or 160 qudits (n up to 2048), and any program whose
+                                    x / z pass takes the row form.  A program has one for d = 2, 3, 5,
+                                    7, n up to 2048 and no two-qudit gate on one qudit twice; it takes
+                                    it where the run's estimated time is the shorter for it (a program
+                                    or some dozens nearly always; of hundreds of small ones, or with
+                                    thousands of measurements on a few qudits, often not), with
+                                    SDIM_FLAG_ROWS always, and not with SDIM_FLAG_NO_ROWS, FORCE_GMEM,
+                                    SPLIT_XZ, CLUSTER_XZ, U8_XZ, PACKED_XZ or UNLAYERED */
 #define SDIM_FLAG_NO_TRACE 512u  /* no trace engine: shot-group engines only */
 #define SDIM_FLAG_NO_COIN_PASS 1024u /* trace engine: draw N1 coins inside the phase pass, no coin pass */
 #define SDIM_FLAG_SPLIT_XZ 2048u /* odd-d trace engine: x / z pass on a CTA pair whenever it fits */
@@ -92,6 +95,10 @@ extern "C" {
 #define SDIM_FLAG_DIRECT_HOST 8192u /* host outputs in page-locked memory: the kernels store the records
                                        into the host buffer directly, with no device buffer and no copy
                                        (by default records go to device memory, then one copy down) */
+
+#define SDIM_FLAG_ROWS 32768u /* trace engine and row form for every program that has one, whatever the
+                                 run's estimate (SDIM_FLAG_TRACE) */
+#define SDIM_FLAG_NO_ROWS 4194304u /* no row form: the shot-group engines and the trace engines' tableau passes */
 
 /* snapshot modes for sdim_snapshot */
 #define SDIM_SNAP_EVERY_INSTRUCTION 1
@@ -258,6 +265,13 @@ int sdim_program_words(const int32_t* ops, int64_t nops, const double* noise_pro
  * counterpart in the reference. */
 int sdim_row_program(const int32_t* ops, int64_t nops, const double* noise_prob, int32_t n, int32_t d,
                      int64_t out[6]);
+/* Which programs of a run (op tables as in sdim_run_tables, nshots[i] shots
+ * each) take the row form by default or with `flags`, on a device with num_sms
+ * SMs: out[i] 1 or 0.  Host-only (no device is touched), for inspection and
+ * tests.  The codes of sdim_encode_circuit.  No counterpart in the reference. */
+int sdim_row_choice(int32_t ncirc, const int32_t* rows, const int64_t* row_begin, const double* noise_prob,
+                    const int32_t* n, const int32_t* d, const int64_t* nshots, unsigned flags, int32_t num_sms,
+                    uint8_t* out);
 /* The launch shape of the row form's passes for `count` programs of one d that
  * share a launch, on a device with smem_optin bytes of opt-in shared memory per
  * block and num_sms SMs; programs holds count x 6 values as sdim_row_program

@@ -39,13 +39,16 @@ FLAG_REUSE_XZ = 262144
 FLAG_COLUMNS = 524288
 FLAG_PHASE_REPLAY = 1048576
 FLAG_UNLAYERED = 2097152
+FLAG_ROWS = 32768
+FLAG_NO_ROWS = 4194304
 
 
 def engine_flags(engine) -> int:
     """Run flags that select a batched engine by name (None: the library's
-    choice by shot count and dimension)."""
+    choice by its estimate of the run).  "trace" takes the trace engines,
+    "rows" and "tableau" one form of their x / z pass."""
     table = {None: 0, "auto": 0, "trace": FLAG_TRACE, "group": FLAG_NO_TRACE, "per_shot": FLAG_PER_SHOT,
-             "group_warp": FLAG_TEAM_WARP, "group_cta": FLAG_TEAM_CTA}
+             "rows": FLAG_TRACE | FLAG_ROWS, "tableau": FLAG_TRACE | FLAG_NO_ROWS, "group_warp": FLAG_TEAM_WARP, "group_cta": FLAG_TEAM_CTA}
     if engine not in table:
         raise ValueError(f"unknown engine {engine!r}; expected one of {sorted(k for k in table if k)}")
     return table[engine]
@@ -88,6 +91,7 @@ SIGNATURES = {
     "sdim_trace_xz_mode": (C.c_int, [C.c_int32, C.c_int32, C.c_int64, C.c_uint, C.c_int32, C.c_int32]),
     "sdim_program_words": (C.c_int, [_P, C.c_int64, _P, C.c_int32, C.c_int32, C.c_int32, _P, C.c_int64, _P]),
     "sdim_row_program": (C.c_int, [_P, C.c_int64, _P, C.c_int32, C.c_int32, _P]),
+    "sdim_row_choice": (C.c_int, [C.c_int32, _P, _P, _P, _P, _P, _P, C.c_uint, C.c_int32, _P]),
     "sdim_row_plan": (C.c_int, [C.c_int32, C.c_int32, _P, _P, C.c_int32, C.c_int32, _P]),
     "sdim_probe_philox_rate": (C.c_int, [_P, C.POINTER(C.c_double)]),
     "sdim_graph_create": (C.c_int, [_P, C.c_int, _P, _P, _P, _P, _P, C.c_uint, C.POINTER(_P)]),

@@ -16,6 +16,7 @@
 #include "../../include/sdim_gb300.h"
 #include "frame.cuh"
 #include "kernels.cuh"
+#include "route_cost.cuh"
 #include "rows.cuh"
 #include "trace.cuh"
 #include "variants.cuh"
@@ -412,7 +413,7 @@ struct Job {
   int64_t shot0, nshots;
   uint8_t* out_dev;
   int index = -1;  // position in the caller's batch (graph capture: whose seed a descriptor holds)
-  bool rows = false;  // trace engine: its x / z pass runs in the row form
+  bool rows = false;  // trace engine, its x / z pass in the row form (choose_rows)
 };
 
 // Host -> device copy of `count` descriptors of `each` bytes, each holding a
@@ -490,17 +491,18 @@ int job_variant(const sdim_circuit* c, unsigned flags) {
   return c->gvariant;
 }
 
-// Whether a trace-engine job's x / z pass runs in the row form (rows.cuh):
-// wherever the encoder built one, unless a flag names a tableau pass.
+// Whether a program may take the row form (rows.cuh): the encoder built one,
+// and no flag names another engine or a tableau pass.
 bool row_form(const sdim_circuit* c, unsigned flags) {
-  return c->rows.nops > 0 && !(flags & (SDIM_FLAG_FORCE_GMEM | SDIM_FLAG_SPLIT_XZ | SDIM_FLAG_CLUSTER_XZ |
-                                        SDIM_FLAG_U8_XZ | SDIM_FLAG_PACKED_XZ | SDIM_FLAG_UNLAYERED));
+  return c->rows.nops > 0 &&
+         !(flags & (SDIM_FLAG_FORCE_GMEM | SDIM_FLAG_SPLIT_XZ | SDIM_FLAG_CLUSTER_XZ | SDIM_FLAG_U8_XZ |
+                    SDIM_FLAG_PACKED_XZ | SDIM_FLAG_UNLAYERED | SDIM_FLAG_NO_ROWS));
 }
 
-// Below this many shots a program without a row form runs on the shot-group engine: one x / z
-// pass per program plus a phase pass only pays once there are several 32-shot
-// groups to share it, and in a batch of small programs the group engine's
-// single persistent launch keeps every SM busy.
+// Below this many shots a program that does not take the row form runs on the
+// shot-group engine: one x / z pass per program plus a phase pass only pays once
+// there are several 32-shot groups to share it, and in a batch of small programs
+// the group engine's single persistent launch keeps every SM busy.
 constexpr int64_t kTraceMinShots = 128;
 
 // From this many qudits the trace engines take a program at any shot count:
@@ -516,8 +518,8 @@ bool use_trace(const Job& j, unsigned flags) {
   if (flags & (SDIM_FLAG_PLAIN | SDIM_FLAG_PER_SHOT | SDIM_FLAG_TEAM_WARP | SDIM_FLAG_TEAM_CTA |
                SDIM_FLAG_NO_TRACE))
     return false;
-  if (j.c->d != 2 || trace_words(j.c->n) == 0 || j.nshots <= 0 || !(j.c->d_steps || row_form(j.c, flags))) return false;
-  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || row_form(j.c, flags);
+  if (j.c->d != 2 || trace_words(j.c->n) == 0 || j.nshots <= 0 || !(j.c->d_steps || j.rows)) return false;
+  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || j.rows;
 }
 
 // Device memory of the fire masks of one part of the frame route's shots.
@@ -589,7 +591,37 @@ bool use_trace_u8(const Job& j, unsigned flags) {
                SDIM_FLAG_NO_TRACE))
     return false;
   if (j.c->d == 2 || j.c->n > kTraceU8MaxQudits || j.nshots <= 0) return false;
-  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || row_form(j.c, flags);
+  return (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || j.c->n >= kTraceMinQudits || j.rows;
+}
+
+// Sets Job::rows: of the programs that have a row form, those that the run's
+// estimate gives to it (route_cost.cuh); all of them with SDIM_FLAG_ROWS, or
+// where a single program's trace is kept (every later call then replays it).
+void choose_rows(std::vector<Job>& jobs, unsigned flags, int num_sms) {
+  for (Job& j : jobs) j.rows = false;
+  if (flags & (SDIM_FLAG_PLAIN | SDIM_FLAG_PER_SHOT | SDIM_FLAG_TEAM_WARP | SDIM_FLAG_TEAM_CTA | SDIM_FLAG_NO_TRACE))
+    return;
+  std::vector<size_t> at;
+  for (size_t i = 0; i < jobs.size(); ++i)
+    if (jobs[i].nshots > 0 && row_form(jobs[i].c, flags)) at.push_back(i);
+  if ((flags & SDIM_FLAG_ROWS) || ((flags & SDIM_FLAG_REUSE_XZ) && jobs.size() == 1)) {
+    for (size_t i : at) jobs[i].rows = true;
+    return;
+  }
+  auto launch = [&](const sdim_circuit* c) { return 64 * c->d + row_slice(row_elems(c->n), c->d); };
+  long long share[64 * 8] = {};
+  for (size_t i : at) ++share[launch(jobs[i].c)];
+  std::vector<RouteShape> shapes;
+  std::vector<long long> programs;
+  for (size_t i : at) {
+    const sdim_circuit* c = jobs[i].c;
+    const bool trace = (flags & SDIM_FLAG_TRACE) || jobs[i].nshots >= kTraceMinShots || c->n >= kTraceMinQudits;
+    shapes.push_back(RouteShape{c->n, c->d, c->nmeas, c->nn1, c->nops - c->nn1 - c->nmeas, c->rows.nlayers, c->rows.nx,
+                                jobs[i].nshots, trace});
+    programs.push_back(share[launch(c)]);
+  }
+  const std::vector<char> take = choose_row_form(shapes, programs, num_sms);
+  for (size_t i = 0; i < at.size(); ++i) jobs[at[i]].rows = take[i];
 }
 
 // The row-form programs of one d and chain-pass slice in a run: descriptors
@@ -771,17 +803,16 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     }
     ctx->rows_smem_set = true;
   }
-  // which programs take the row form: those that have one, within the budget
-  // of the slots that the tableau passes would use
+  // the row form's programs stay within the budget of the slots that the
+  // tableau passes would use
   size_t row_total = 0;
   for (std::vector<Job>* list : {&jobs, &ujobs})
     for (Job& j : *list) {
-      if (!row_form(j.c, flags)) continue;
+      if (!j.rows) continue;
       const size_t b = row_bytes(j.c->n, j.c->d, j.c->nmeas, j.c->rows.nx, j.c->rows.nk).total;
       const bool other = j.c->d != 2 || j.c->d_steps;  // sdim_run_tables builds schedules when the rows exceed the budget
-      if (other && row_total + b > ctx->gmem_slot_budget) continue;
-      row_total += b;
-      j.rows = true;
+      if (other && row_total + b > ctx->gmem_slot_budget) j.rows = false;
+      else row_total += b;
     }
   // row-form programs: their descriptors, d = 2 first
   std::vector<RowDesc> hr;
@@ -1458,6 +1489,7 @@ int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsig
   ctx->last_stream = s;
   ctx->xz_pending = nullptr;
   ctx->pend_trace = ctx->pend_cols = false;
+  choose_rows(all_jobs, flags, ctx->num_sms);
   std::vector<Job> jobs, tjobs, ujobs;
   for (const Job& j : all_jobs) (use_trace(j, flags) ? tjobs : use_trace_u8(j, flags) ? ujobs : jobs).push_back(j);
   int rc;
@@ -1894,9 +1926,9 @@ void append_schedule(std::vector<uint2>& dev, size_t op_begin, size_t nops, int 
 // the program order between qudits, so a measurement holds no other qudit's
 // gates up.  None (out.nops = 0) for a program without measurements, with a
 // two-qudit gate on one qudit twice (not a symplectic map), or whose rows
-// would take more than kRowBytesMost or kRowWorkMost: there the cost of
-// carrying every row through every earlier update (quadratic in the
-// measurements) passes that of the tableau passes.
+// would take more than kRowBytesMost or kRowWorkMost (element updates), which
+// bound a program's memory and the longest chain (about 0.2 s); within them the
+// run's estimate decides (route_cost.cuh).
 constexpr size_t kRowBytesMost = (size_t)256 << 20;
 constexpr double kRowWorkMost = 4e9;
 
@@ -2111,6 +2143,31 @@ int sdim_row_program(const int32_t* ops, int64_t nops, const double* noise_prob,
   out[3] = r.nx;
   out[4] = r.nk;
   out[5] = r.nops ? (int64_t)row_bytes(n, d, nmeas, r.nx, r.nk).total : 0;
+  return SDIM_OK;
+}
+
+int sdim_row_choice(int32_t ncirc, const int32_t* rows, const int64_t* row_begin, const double* noise_prob,
+                    const int32_t* n, const int32_t* d, const int64_t* nshots, unsigned flags, int32_t num_sms,
+                    uint8_t* out) {
+  if (ncirc < 0 || num_sms <= 0 || (ncirc > 0 && (!rows || !row_begin || !n || !d || !nshots || !out)))
+    return SDIM_EINVAL;
+  std::vector<sdim_circuit> circs(ncirc);
+  std::vector<Job> jobs;
+  for (int i = 0; i < ncirc; ++i) {
+    std::vector<uint2> dev;
+    sdim_circuit& c = circs[i];
+    const int64_t r0 = row_begin[i], r1 = row_begin[i + 1];
+    const int rc = encode_rows(nullptr, rows + 4 * r0, r1 - r0, noise_prob ? noise_prob + r0 : nullptr, n[i], d[i], dev,
+                               c.nmeas, c.nn1);
+    if (rc != SDIM_OK) return rc;
+    c.n = n[i];
+    c.d = d[i];
+    c.nops = (int)dev.size();
+    append_rows(dev, 0, dev.size(), n[i], d[i], c.nmeas, c.rows);
+    jobs.push_back(Job{&c, 0, 0, nshots[i], nullptr});
+  }
+  choose_rows(jobs, flags, num_sms);
+  for (int i = 0; i < ncirc; ++i) out[i] = jobs[i].rows;
   return SDIM_OK;
 }
 
@@ -2928,7 +2985,6 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
     c.nops_user = r1 - r0;
     c.nops = (int)(dev.size() - op_off[i]);
     append_rows(dev, op_off[i], (size_t)c.nops, n[i], d[i], nmeas, c.rows);
-    if (row_form(&c, flags)) row_total += row_bytes(n[i], d[i], nmeas, c.rows.nx, c.rows.nk).total;
     c.variant = variant_for(d[i]);
     c.gvariant = group_variant_for(d[i], n[i], 0);
     c.gblock = variant_ops(c.gvariant).cta ? cta_block_for(n[i]) : 32;
@@ -2938,9 +2994,16 @@ int sdim_run_tables(sdim_ctx* ctx, int ncirc, const int32_t* rows, const int64_t
   // a batch takes only with fewer than num_sms / 2 odd-d programs
   // (odd_xz_mode; SDIM_FLAG_CLUSTER_XZ in a larger batch walks the instructions
   // as written)
+  // (launch_jobs makes the same choice again)
+  std::vector<Job> plan;
+  for (int i = 0; i < ncirc; ++i) plan.push_back(Job{&circs[i], 0, 0, nshots[i], nullptr});
+  choose_rows(plan, flags, ctx->num_sms);
+  for (int i = 0; i < ncirc; ++i)
+    if (plan[i].rows)
+      row_total += row_bytes(n[i], d[i], circs[i].nmeas, circs[i].rows.nx, circs[i].rows.nk).total;
   int odd = 0;
   const bool rows_fit = row_total <= ctx->gmem_slot_budget;
-  auto by_rows = [&](int i) { return rows_fit && row_form(&circs[i], flags); };
+  auto by_rows = [&](int i) { return rows_fit && plan[i].rows; };
   for (int i = 0; i < ncirc; ++i) odd += d[i] != 2 && !by_rows(i) ? 1 : 0;
   for (int i = 0; i < ncirc; ++i) {
     const size_t ops = (size_t)circs[i].nops;

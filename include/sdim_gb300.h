@@ -316,7 +316,12 @@ int sdim_host_free(void* p);
 double sdim_last_kernel_ms(const sdim_ctx* ctx);
 /* The same span split by stage: out[0] the trace engine's x / z passes
  * (with the odd-d cluster's deterministic-header pass after them), out[1]
- * its phase passes, out[2] every other engine's kernels.  In a batch
+ * its phase passes, out[2] every other engine's kernels.  Row-form programs
+ * of several launches (different d or widths) run side by side, each launch's
+ * phase pass behind its x / z pass: out[0] then holds their phase passes too.
+ * Of sdim_frame_run out[0] spans the reference shot's x / z pass, with the
+ * coins and frames of the first part beside it, out[2] the frames and records
+ * after it.  In a batch
  * that has both, the shot-group engines run on their own stream beside the
  * trace engines: out[2] is then their own span, which overlaps out[0] and
  * out[1].  No counterpart in the reference (its shot loop is not staged). */

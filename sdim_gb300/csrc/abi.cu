@@ -1483,7 +1483,8 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
 // items are shots for per-shot engines and 32-shot groups for group engines;
 // inside a variant the most expensive programs are queued first.  d = 2 jobs
 // with enough shots go to the trace engine first (use_trace).
-int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsigned flags) {
+// started: the caller has recorded the start of the timed span (ev0) itself.
+int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsigned flags, bool started = false) {
   const bool plain = flags & SDIM_FLAG_PLAIN;
   const bool force_gmem = flags & SDIM_FLAG_FORCE_GMEM;
   ctx->last_stream = s;
@@ -1540,7 +1541,7 @@ int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsig
     return rc;
   CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(int), s));
   if (!jobs.empty()) CK(cudaMemsetAsync(ctx->counters.p, 0, sizeof(unsigned long long) * V_COUNT, s));
-  if (flags & SDIM_FLAG_TIME) CK(cudaEventRecord(ctx->ev0, s));
+  if ((flags & SDIM_FLAG_TIME) && !started) CK(cudaEventRecord(ctx->ev0, s));
   int* status = static_cast<int*>(ctx->status.p);
   // with trace programs in the batch the shot-group engines run on a stream
   // of their own, beside the trace engines (the uneven batch: their 23 ms
@@ -2699,11 +2700,13 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
     // launched behind them (L = 7, 100,000 frames: 338 us in front, 328 so)
     CK(cudaEventRecord(ctx->ev_gf, s));
     CK(cudaStreamWaitEvent(ctx->fast, ctx->ev_gf, 0));
+    if (flags & SDIM_FLAG_TIME) CK(cudaEventRecord(ctx->ev0, s));  // the span begins with the coins and frames
     if ((rc = launch_part(0)) != SDIM_OK) return rc;
     // (its own fires, if it holds any N1, are drawn in its phase pass: the fire
     // masks in ctx->masks are the frames' while both run)
     std::vector<Job> jobs{Job{ref, seed, 0, 1, dst}};
-    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE | SDIM_FLAG_NO_COIN_PASS);
+    rc = launch_jobs(ctx, jobs, ctx->fast, (flags & ~SDIM_FLAG_ASYNC) | SDIM_FLAG_TRACE | SDIM_FLAG_NO_COIN_PASS,
+                     true);
     ctx->last_stream = s;
     if (rc != SDIM_OK) return rc;
     CK(cudaEventRecord(ctx->ev_fast, ctx->fast));

@@ -120,9 +120,11 @@ int sdim_device_info(sdim_ctx* ctx, int64_t info[4]);
 /* info[0] = free device bytes, [1] = total device bytes, [2] = bytes this
  * context holds in its buffers.  Used by the serving loop's admission. */
 int sdim_memory_info(sdim_ctx* ctx, int64_t info[3]);
-/* Device bytes a run of nshots shots of circ needs: out[0] records,
- * out[1] one shot-group slot (shared-memory part plus x / z part) plus,
- * for d = 2, the trace the trace engine writes. */
+/* Device bytes a run of nshots shots of circ needs at most on any route, but
+ * for the fire masks: out[0] records, out[1] one shot-group slot
+ * (shared-memory part plus x / z part), the trace that the trace engine writes
+ * where it may take the program, and the row form's rows and updates where the
+ * program has one. */
 int sdim_program_bytes(const sdim_circuit* circ, int64_t nshots, int64_t out[2]);
 
 /* Encodes one program.  ops is nops rows of 4 int32:

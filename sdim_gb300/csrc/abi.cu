@@ -2423,7 +2423,14 @@ int sdim_program_bytes(const sdim_circuit* c, int64_t nshots, int64_t out[2]) {
   out[0] = (int64_t)nshots * c->nmeas;                   // records
   out[1] = (int64_t)(g.hot_bytes(c->n) + g.big_bytes(c->n));  // one group slot
   const int tw = c->d == 2 ? trace_words(c->n) : 0;
+  const bool rows = c->rows.nops > 0;
   if (tw) out[1] += (int64_t)trace_bytes(c->nmeas, c->nn1, tw);
+  if (c->d != 2 && c->n <= kTraceU8MaxQudits && (rows || nshots >= kTraceMinShots || c->n >= kTraceMinQudits)) {
+    size_t o[5];
+    trace_offsets_u8(c->nmeas, c->nn1, trace_row_bytes_u8(c->n), o);  // the tableau pass's rows, the wider ones
+    out[1] += (int64_t)o[4];
+  }
+  if (rows) out[1] += (int64_t)row_bytes(c->n, c->d, c->nmeas, c->rows.nx, c->rows.nk).total;
   return SDIM_OK;
 }
 

@@ -704,9 +704,9 @@ int plan_row_group(sdim_ctx* ctx, RowGroup& g, RowDesc* h) {
 // warps, 428 us with one and 433 with two; 20,000 shots 518 and 478).
 constexpr long long kRowPhaseWarps = 152LL * 4 * 6;
 
-int row_phase_blocks(const RowPhaseDesc& p) {
+long long row_phase_blocks(const RowPhaseDesc& p) {
   const int per = 4 * (32 >> p.lg);  // shots of a CTA
-  return (p.c.nshots + per - 1) / per;
+  return ((long long)p.c.nshots + per - 1) / per;
 }
 
 // Every pointer into the passes' memory, which begins at mem (and at r.raw).
@@ -1109,9 +1109,9 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
     phr.push_back(p);
     phjob.push_back(job);
   };
-  auto end_phase_run = [&](int b) {
+  auto end_phase_run = [&](int b) -> int {
     const int e = (int)phr.size();
-    if (b == e) return;
+    if (b == e) return SDIM_OK;
     int wpl = 1;
     for (; wpl < 4; wpl <<= 1) {
       long long warps = 0;
@@ -1123,13 +1123,15 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       }
       if (fits && warps <= kRowPhaseWarps) break;
     }
-    int blocks = 0;
+    long long blocks = 0;
     for (int i = b; i < e; ++i) {
       phr[i].lg = row_phase_lg(phr[i].E, wpl);
-      phr[i].block_begin = blocks;
+      phr[i].block_begin = (int)blocks;
       blocks += row_phase_blocks(phr[i]);
+      if (blocks > 0x7fffffffLL) return fail(ctx, SDIM_EINVAL, "too many shots in one phase pass");
     }
     pruns.push_back(PhaseRun{b, e, wpl});
+    return SDIM_OK;
   };
   for (RowGroup& g : rgroups) {
     g.pb = (int)phr.size();
@@ -1143,14 +1145,14 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
                   jobs[j].c->rows.nx > 0, jobs[j].index);
     }
     g.pe = (int)phr.size();
-    end_phase_run(g.pb);
+    if ((rc = end_phase_run(g.pb)) != SDIM_OK) return rc;
   }
   const bool kept_phase = skip_xz && !colform && d2_packed(0);
   if (kept_phase) {
     const int b = (int)phr.size();
     add_phase(hd[0].c, hd[0].mhdr, hd[0].mrow, nullptr, nullptr, hd[0].nm, 0, 4 * hd[0].tw, jobs[0].c->rows.nx > 0,
               jobs[0].index);
-    end_phase_run(b);
+    if ((rc = end_phase_run(b)) != SDIM_OK) return rc;
   }
   // ---- every descriptor array in one upload
   const RowPhaseDesc* dp = nullptr;
@@ -1174,7 +1176,7 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
       size_t smem = 0;
       for (int i = b; i < e; ++i) smem = std::max(smem, row_phase_smem(phr[i].pitch));
       const RowPhaseDesc& last = phr[e - 1];
-      row_ops(last.c.d).phase(close, r.wpl, last.block_begin + row_phase_blocks(last), smem, st,
+      row_ops(last.c.d).phase(close, r.wpl, (int)(last.block_begin + row_phase_blocks(last)), smem, st,
                               dp + b, e - b);
       const cudaError_t le = cudaGetLastError();
       if (le != cudaSuccess) return cuda_fail(ctx, le, "row phase pass launch");

@@ -274,6 +274,16 @@ int sdim_row_program(const int32_t* ops, int64_t nops, const double* noise_prob,
 int sdim_row_choice(int32_t ncirc, const int32_t* rows, const int64_t* row_begin, const double* noise_prob,
                     const int32_t* n, const int32_t* d, const int64_t* nshots, unsigned flags, int32_t num_sms,
                     uint8_t* out);
+/* Whether shots 1 .. nshots - 1 of a frame run (sdim_frame_run; rows as in
+ * sdim_encode_circuit) run on bit planes, 32 shots a word (1), or as a byte per
+ * qudit and shot (0), on a device with these limits (smem_reserved: the bytes
+ * the driver takes of each block).  Planes need a row form and shared memory for
+ * every N1 sample of a warp, and are taken where they are estimated the shorter
+ * run; SDIM_FLAG_ROWS takes them where they fit, SDIM_FLAG_NO_ROWS and
+ * FORCE_GMEM never.  Host-only (no device is touched), for inspection and tests.
+ * The codes of sdim_encode_circuit.  No counterpart in the reference. */
+int sdim_frame_route(const int32_t* ops, int64_t nops, const double* noise_prob, int32_t n, int32_t d, int64_t nshots,
+                     unsigned flags, int32_t smem_optin, int32_t smem_per_sm, int32_t smem_reserved, int32_t num_sms);
 /* The launch shape of the row form's passes for `count` programs of one d that
  * share a launch, on a device with smem_optin bytes of opt-in shared memory per
  * block and num_sms SMs; programs holds count x 6 values as sdim_row_program

@@ -92,6 +92,8 @@ SIGNATURES = {
     "sdim_program_words": (C.c_int, [_P, C.c_int64, _P, C.c_int32, C.c_int32, C.c_int32, _P, C.c_int64, _P]),
     "sdim_row_program": (C.c_int, [_P, C.c_int64, _P, C.c_int32, C.c_int32, _P]),
     "sdim_row_choice": (C.c_int, [C.c_int32, _P, _P, _P, _P, _P, _P, C.c_uint, C.c_int32, _P]),
+    "sdim_frame_route": (C.c_int, [_P, C.c_int64, _P, C.c_int32, C.c_int32, C.c_int64, C.c_uint, C.c_int32, C.c_int32,
+                                   C.c_int32, C.c_int32]),
     "sdim_row_plan": (C.c_int, [C.c_int32, C.c_int32, _P, _P, C.c_int32, C.c_int32, _P]),
     "sdim_probe_philox_rate": (C.c_int, [_P, C.POINTER(C.c_double)]),
     "sdim_graph_create": (C.c_int, [_P, C.c_int, _P, _P, _P, _P, _P, C.c_uint, C.POINTER(_P)]),

@@ -769,6 +769,36 @@ int launch_row_extra(sdim_ctx* ctx, const RowGroup& g, const RowDesc* rd, cudaSt
   return e == cudaSuccess ? SDIM_OK : cuda_fail(ctx, e, "row extra pass launch");
 }
 
+// Warps of a CTA of the frame pass on bit planes, whose description and shared
+// memory are set, or 0 where a frame run of nshots shots takes the byte-per-shot
+// kernel: the program has no row form, does not fit, or is estimated longer on
+// planes (route_cost.cuh).
+int frame_warps(const sdim_circuit* c, int64_t nshots, unsigned flags, size_t smem_optin, size_t smem_per_sm,
+                size_t smem_reserved, int num_sms, RowFrameDesc& rf, size_t& smem) {
+  std::memset(&rf, 0, sizeof(rf));
+  if (nshots < 2 || c->rows.nops == 0 || (flags & (SDIM_FLAG_FORCE_GMEM | SDIM_FLAG_NO_ROWS))) return 0;
+  rf.ops = reinterpret_cast<const uint4*>(c->d_blob + c->rows.ops_off);
+  rf.lay = reinterpret_cast<const uint32_t*>(c->d_blob + c->rows.lay_off);
+  rf.xinfo = c->d_blob + c->rows.xinfo_off;
+  rf.nhdr = c->d_blob + c->rows.nhdr_off;
+  rf.nlayers = c->rows.nlayers;
+  rf.n = c->n;
+  rf.nm = c->nmeas;
+  rf.nused = c->rows.nn1;
+  rf.nchunk = c->d == 2 ? (rf.nused + kCoinChunk - 1) / kCoinChunk : 0;
+  // fired ordinals of a warp: the mean and six deviations; past that the pass
+  // gathers a word from the masks
+  rf.cap = (int)std::min<double>(rf.nused, c->rows.fires + 6.0 * std::sqrt(c->rows.fires) + 32.0);
+  int warps = 4;
+  for (; warps > 0; warps >>= 1)
+    if ((smem = row_ops(c->d).frame_smem(rf, warps)) + 1024 <= smem_optin) break;
+  if (!warps || (flags & SDIM_FLAG_ROWS)) return warps;
+  const FrameShape f{c->n, c->d, c->nmeas, rf.nused, rf.nlayers, c->nfops, c->rows.fires, nshots - 1};
+  const int planes = std::max(1, (int)(smem_per_sm / (smem + smem_reserved))) * warps;
+  const int bytes = std::max(1, (int)(smem_per_sm / (frame_smem_bytes(c->n) + smem_reserved)));
+  return frame_bytes_us(f, bytes, num_sms) < 0.85 * frame_planes_us(f, planes, num_sms) ? 0 : warps;
+}
+
 // Trace-engine launches: the x / z pass of every program (d = 2 jobs, then
 // odd-d jobs per variant of d), the coin pass of the d = 2 jobs alongside on
 // the second stream, then the phase passes (d = 2 per trace-row width, odd
@@ -2174,6 +2204,24 @@ int sdim_row_choice(int32_t ncirc, const int32_t* rows, const int64_t* row_begin
   return SDIM_OK;
 }
 
+int sdim_frame_route(const int32_t* ops, int64_t nops, const double* noise_prob, int32_t n, int32_t d, int64_t nshots,
+                     unsigned flags, int32_t smem_optin, int32_t smem_per_sm, int32_t smem_reserved, int32_t num_sms) {
+  if ((nops > 0 && !ops) || nops < 0 || smem_optin <= 0 || smem_per_sm <= 0 || smem_reserved < 0 || num_sms <= 0)
+    return SDIM_EINVAL;
+  std::vector<uint2> dev;
+  sdim_circuit c;
+  const int rc = encode_rows(nullptr, ops, nops, noise_prob, n, d, dev, c.nmeas, c.nn1);
+  if (rc != SDIM_OK) return rc;
+  c.n = n;
+  c.d = d;
+  append_rows(dev, 0, dev.size(), n, d, c.nmeas, c.rows);
+  append_frame_ops(ops, nops, noise_prob, dev, c.fops_off, c.nfops);
+  RowFrameDesc rf;
+  size_t smem = 0;
+  return frame_warps(&c, nshots, flags, (size_t)smem_optin, (size_t)smem_per_sm, (size_t)smem_reserved, num_sms, rf,
+                     smem) > 0;
+}
+
 int sdim_row_plan(int32_t d, int32_t count, const int32_t* n, const int64_t* programs, int32_t smem_optin,
                   int32_t num_sms, int32_t out[8]) {
   if (!row_dim(d) || count < 1 || !n || !programs || !out || smem_optin <= 0 || num_sms <= 0) return SDIM_EINVAL;
@@ -2630,30 +2678,13 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
                        ctx->stream));
   }
   cudaStream_t s = ctx->stream;
-  // shots 1 .. nshots - 1 on bit planes where the program has a row form that
-  // fits: frames against row 0
+  // shots 1 .. nshots - 1: frames against row 0
   RowFrameDesc rf;
-  std::memset(&rf, 0, sizeof(rf));
-  int warps = 0;  // of a frame-pass CTA; 0: the byte-per-shot kernel
   size_t fsmem = 0;
-  if (nshots > 1 && c->rows.nops > 0 && !(flags & SDIM_FLAG_FORCE_GMEM)) {
-    rf.ops = reinterpret_cast<const uint4*>(c->d_blob + c->rows.ops_off);
-    rf.lay = reinterpret_cast<const uint32_t*>(c->d_blob + c->rows.lay_off);
-    rf.xinfo = c->d_blob + c->rows.xinfo_off;
-    rf.nhdr = c->d_blob + c->rows.nhdr_off;
-    rf.ref = dst;
-    rf.seed = seed;
-    rf.nlayers = c->rows.nlayers;
-    rf.n = c->n;
-    rf.nm = c->nmeas;
-    rf.nused = c->rows.nn1;
-    rf.nchunk = c->d == 2 ? (rf.nused + kCoinChunk - 1) / kCoinChunk : 0;
-    // fired ordinals of a warp: the mean and six deviations; past that the pass
-    // gathers a word from the masks
-    rf.cap = (int)std::min<double>(rf.nused, c->rows.fires + 6.0 * std::sqrt(c->rows.fires) + 32.0);
-    for (warps = 4; warps > 0; warps >>= 1)
-      if ((fsmem = row_ops(c->d).frame_smem(rf, warps)) + 1024 <= (size_t)ctx->smem_optin) break;
-  }
+  int warps = frame_warps(c, nshots, flags, (size_t)ctx->smem_optin, (size_t)ctx->smem_per_sm,
+                          (size_t)ctx->smem_reserved, ctx->num_sms, rf, fsmem);
+  rf.ref = dst;
+  rf.seed = seed;
   if (warps) {
     for (int d : {2, 3, 5, 7})
       if (!ctx->rows_smem_set) {

@@ -147,4 +147,43 @@ inline std::vector<char> choose_row_form(const std::vector<RouteShape>& p, const
   return best;
 }
 
+// The frame route: whether shots 1 .. nshots - 1 run on bit planes (k_rows_frame)
+// or a byte per qudit and shot (k_frame_pass).  The planes' warps walk the layers
+// two to twenty times sooner, but each holds all its N1 samples in shared memory:
+// with thousands of ordinals a few warps an SM are left, and many shots take turn
+// after turn.  Measured on GB300, planes and bytes (ms):
+//   7 qudits of d = 7, 2,500 ordinals, 20,000 shots      1.54   2.25
+//                                     100,000 shots      5.57   2.56
+//   7 qubits, 60,000 ordinals of probability 0.001, 20,000 shots   16.5   41.2
+//                                                  300,000 shots  144.9   95.4
+//   7 qubits, 10,000 ordinals, 300,000 shots             7.95  15.73
+//   100 qubits, 60,000 ordinals, 300,000 shots          39.3   95.3
+// On 112 such pairs (d = 2, 3, 7, 7 and 100 qudits, 1,000 to 400,000 ordinals,
+// 2,000 to 300,000 shots) the estimates below take the faster kernel every time.
+struct FrameShape {
+  int n, d, nmeas, used, layers;  // used: N1 ordinals before the last measurement
+  long long ops;
+  double fires;  // expected number of them that any of 32 shots fires
+  long long shots;
+};
+
+inline double frame_turns(long long shots, int warps_per_sm, int num_sms) {
+  return (double)shots / (32.0 * num_sms * warps_per_sm);
+}
+
+// Microseconds with that many warps resident on an SM.
+inline double frame_planes_us(const FrameShape& f, int warps_per_sm, int num_sms) {
+  const int held = std::min(warps_per_sm, 40);
+  const double turns = frame_turns(f.shots, held, num_sms);
+  const double a_turn = 20 + f.layers * (f.d == 2 ? 0.235 : f.d == 3 ? 0.28 : 0.37) + f.used * (f.d == 2 ? 0.02 : 0.027) +
+                        (f.d == 2 ? 0.3 * f.fires : 0.0);
+  return a_turn * std::max(1.0, turns) * (1 + 0.05 * held * std::min(1.0, turns));
+}
+inline double frame_bytes_us(const FrameShape& f, int warps_per_sm, int num_sms) {
+  const int held = std::min(warps_per_sm, 32);
+  const double turns = frame_turns(f.shots, held, num_sms);
+  const double a_turn = f.ops * (f.d == 2 ? 0.28 : 0.46) + (f.d == 2 ? 1.5 : 3.4) * (f.n + f.nmeas);
+  return a_turn * std::max(1.0, turns) * (1 + 0.004 * held * std::min(1.0, turns));
+}
+
 }  // namespace sdim

@@ -82,3 +82,24 @@ def test_frames_in_two_parts():
     quiet = DeviceProgram(ctx, encode_program([spec.build()], 6, 2, noise=False))
     shots = 115000
     assert np.array_equal(_frames(ctx, noisy, quiet, 9, shots), _frames(ctx, noisy, quiet, 9, shots, _lib.FLAG_FORCE_GMEM))
+
+
+@pytest.mark.parametrize("d", [2, 3, 5, 7])
+def test_both_kernels_give_the_records(d):
+    """On bit planes, as bytes, and as the run's estimate has it, for a program of
+    so many ordinals that it takes both by the number of its shots."""
+    rng = np.random.default_rng(d)
+    ops = []
+    for k in range(60000 if d == 2 else 2400):
+        a, b = (int(x) for x in rng.permutation(7)[:2])
+        ops += [("CNOT", a, b, {}), ("N1", a, None, {"prob": 0.001, "noise_channel": "dfp"[k % 3]})]
+        if k % 400 == 0:
+            ops.append((("M", "RESET")[k // 400 % 2], b, None, {}))
+    spec = CircuitSpec(7, d, ops + [("M", q, None, {}) for q in range(7)], "many")
+    ctx = _lib.Context.default(0)
+    noisy = DeviceProgram(ctx, encode_program([spec.build()], 7, d))
+    quiet = DeviceProgram(ctx, encode_program([spec.build()], 7, d, noise=False))
+    for shots in (50, 130000):
+        want = _frames(ctx, noisy, quiet, 3, shots, _lib.FLAG_NO_ROWS)
+        for flags in (0, _lib.FLAG_ROWS, _lib.FLAG_FORCE_GMEM):
+            assert np.array_equal(_frames(ctx, noisy, quiet, 3, shots, flags), want), (shots, flags)

@@ -2685,6 +2685,18 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
                           (size_t)ctx->smem_reserved, ctx->num_sms, rf, fsmem);
   rf.ref = dst;
   rf.seed = seed;
+  // parts bound the memory of the masks and the record words; without room for a
+  // part the byte kernel, which needs none, takes the run
+  const long long frames = nshots - 1;
+  const size_t words = (size_t)c->nmeas * row_elem_bytes(c->d);  // per 32 shots
+  const size_t per_shot = words / 32 + 1 +
+                          (c->d == 2 ? coin_mask_bytes(rf.nchunk, 1024) / 1024 + coin_map_bytes(rf.nchunk, 1024) / 1024 : 0);
+  const long long part = std::min<long long>(frames, std::max<long long>(32768, (long long)(kFrameMaskBudget / per_shot)));
+  if (warps && (ensure(ctx, ctx->fwords, std::max<size_t>((size_t)((part + 31) / 32) * words, 256)) != SDIM_OK ||
+                (rf.nchunk && (ensure(ctx, ctx->masks, coin_mask_bytes(rf.nchunk, part) +
+                                                           coin_map_bytes(rf.nchunk, part)) != SDIM_OK ||
+                               ensure(ctx, ctx->fdescs, sizeof(TraceDesc)) != SDIM_OK))))
+    warps = 0;
   if (warps) {
     for (int d : {2, 3, 5, 7})
       if (!ctx->rows_smem_set) {
@@ -2692,20 +2704,10 @@ int sdim_frame_run(sdim_ctx* ctx, const sdim_circuit* c, const sdim_circuit* ref
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaFuncSetAttribute");
       }
     ctx->rows_smem_set = true;
-    // parts bound the memory of the masks and the record words
-    const long long frames = nshots - 1;
-    const size_t words = (size_t)c->nmeas * row_elem_bytes(c->d);  // per 32 shots
-    const size_t per_shot = words / 32 + 1 +
-                            (c->d == 2 ? coin_mask_bytes(rf.nchunk, 1024) / 1024 + coin_map_bytes(rf.nchunk, 1024) / 1024 : 0);
-    const long long part = std::min<long long>(frames, std::max<long long>(32768, (long long)(kFrameMaskBudget / per_shot)));
-    if ((rc = ensure(ctx, ctx->fwords, std::max<size_t>((size_t)((part + 31) / 32) * words, 256))) != SDIM_OK) return rc;
     rf.words = static_cast<uint8_t*>(ctx->fwords.p);
     TraceDesc td;
     std::memset(&td, 0, sizeof(td));
     if (rf.nchunk) {
-      if ((rc = ensure(ctx, ctx->masks, coin_mask_bytes(rf.nchunk, part) + coin_map_bytes(rf.nchunk, part))) != SDIM_OK)
-        return rc;
-      if ((rc = ensure(ctx, ctx->fdescs, sizeof(TraceDesc))) != SDIM_OK) return rc;
       td.c.seed = seed;
       td.nthr = c->d_nthr;
       td.nhdr = c->d_nhdr;

@@ -103,3 +103,29 @@ def test_both_kernels_give_the_records(d):
         want = _frames(ctx, noisy, quiet, 3, shots, _lib.FLAG_NO_ROWS)
         for flags in (0, _lib.FLAG_ROWS, _lib.FLAG_FORCE_GMEM):
             assert np.array_equal(_frames(ctx, noisy, quiet, 3, shots, flags), want), (shots, flags)
+
+
+def test_frames_without_room_for_the_masks():
+    """A device whose memory is taken: the masks of a part (about 350 MB) do not
+    fit, and the byte kernel takes the run."""
+    import torch
+    rng = np.random.default_rng(3)
+    ops = []
+    for k in range(40000):
+        a, b = (int(x) for x in rng.permutation(6)[:2])
+        ops += [("CNOT", a, b, {})] * (k % 3 == 0) + [("N1", a, None, {"prob": 0.0005, "noise_channel": "d"})]
+    spec = CircuitSpec(6, 2, ops + [("M", q, None, {}) for q in range(6)], "room")
+    ctx = _lib.Context(0)
+    noisy = DeviceProgram(ctx, encode_program([spec.build()], 6, 2))
+    quiet = DeviceProgram(ctx, encode_program([spec.build()], 6, 2, noise=False))
+    shots = 34000
+    want = _frames(ctx, noisy, quiet, 5, shots, _lib.FLAG_NO_ROWS)
+    torch.cuda.synchronize()
+    taken = torch.empty(torch.cuda.mem_get_info()[0] - (160 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = _frames(ctx, noisy, quiet, 5, shots, _lib.FLAG_ROWS)
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+    assert np.array_equal(got, want)
+    ctx.close()

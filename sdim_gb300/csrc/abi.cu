@@ -105,6 +105,7 @@ struct sdim_ctx {
   int smem_attr_set[V_COUNT] = {};
   bool trace_smem_set = false;
   bool rows_smem_set = false;
+  bool rows_short = false;  // no device memory for the row form's rows (in a capture: for all of it)
   bool frame_smem_set = false;
   int trace_threads = kTracePassThreads;  // x / z pass CTA size (SDIM_TRACE_PASS_THREADS: 256 or 512)
   GraphCapture* capture = nullptr;  // set while sdim_graph_create runs on its private context
@@ -1103,7 +1104,10 @@ int launch_trace_jobs(sdim_ctx* ctx, std::vector<Job> jobs, std::vector<Job> ujo
   }
   RowDesc* dr = nullptr;
   if (!hr.empty()) {
-    if ((rc = ensure(ctx, ctx->rows, std::max<size_t>(rmem, 256))) != SDIM_OK) return rc;
+    if ((rc = ensure(ctx, ctx->rows, std::max<size_t>(rmem, 256))) != SDIM_OK) {
+      ctx->rows_short = true;  // nothing is launched yet: launch_jobs starts over without them
+      return rc;
+    }
     const size_t base = reinterpret_cast<size_t>(ctx->rows.p);
     for (RowDesc& r : hr) row_memory(r, r.raw + base);
     for (RowGroup& g : rgroups)
@@ -1522,7 +1526,8 @@ int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsig
   ctx->last_stream = s;
   ctx->xz_pending = nullptr;
   ctx->pend_trace = ctx->pend_cols = false;
-  choose_rows(all_jobs, flags, ctx->num_sms);
+  if (!ctx->capture) ctx->rows_short = false;
+  choose_rows(all_jobs, ctx->rows_short ? flags | SDIM_FLAG_NO_ROWS : flags, ctx->num_sms);
   std::vector<Job> jobs, tjobs, ujobs;
   for (const Job& j : all_jobs) (use_trace(j, flags) ? tjobs : use_trace_u8(j, flags) ? ujobs : jobs).push_back(j);
   int rc;
@@ -1587,7 +1592,10 @@ int launch_jobs(sdim_ctx* ctx, std::vector<Job>& all_jobs, cudaStream_t s, unsig
     CK(cudaStreamWaitEvent(ctx->grp, ctx->ev_gf, 0));
     gs = ctx->grp;
   }
-  if ((rc = launch_trace_jobs(ctx, tjobs, ujobs, s, flags, status)) != SDIM_OK) return rc;
+  rc = launch_trace_jobs(ctx, tjobs, ujobs, s, flags, status);
+  if (rc == SDIM_ENOMEM && ctx->rows_short && !(flags & SDIM_FLAG_NO_ROWS))  // the routes that need none of it
+    return launch_jobs(ctx, all_jobs, s, flags | SDIM_FLAG_NO_ROWS, started);
+  if (rc != SDIM_OK) return rc;
   if (side && (flags & SDIM_FLAG_TIME)) CK(cudaEventRecord(ctx->ev_g0, gs));
   for (size_t gi = 0; gi < groups.size(); ++gi) {
     const Group& g = groups[gi];

@@ -97,3 +97,34 @@ def test_a_run_of_different_routes(engine):
     for k, (spec, out) in enumerate(zip(specs, br.run(engine=engine))):
         if k % 60 in (0, 7) or spec.num_qudits > 100 or len(spec.ops) > 1000:
             assert np.array_equal(out, oracle_run([spec], 300 + k, 0, shots[k])["records"]), k
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_without_room_for_the_rows(captured):
+    """A device whose memory is taken: 40 programs of 33 MB of rows each, with
+    160 MB left, take the routes that need none."""
+    import torch
+    from sdim_gb300 import _lib
+    spec = _long(4, 2, 16500, seed=2)
+    br = BatchRunner(_lib.Context(0))
+    dp = _program(br, spec)
+    for k in range(40):
+        br.add_program(dp, 2, 60 + k)
+    out = torch.zeros(40 * 2 * dp.num_records, dtype=torch.uint8, device="cuda")
+    ptrs = [out.data_ptr() + 2 * k * dp.num_records for k in range(40)]
+    torch.cuda.synchronize()
+    taken = torch.empty(torch.cuda.mem_get_info()[0] - (160 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        if captured:
+            run = br.capture(ptrs, engine="rows")
+            run.launch()
+            run.sync()
+            run.close()
+        else:
+            br.run_device(ptrs, engine="rows")
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+    got = out.cpu().numpy().reshape(40, 2, dp.num_records)
+    for k in (0, 39):
+        assert np.array_equal(got[k], oracle_run([spec], 60 + k, 0, 2)["records"]), k

@@ -17,8 +17,9 @@ Workloads (--workload):
                      {2,3,5,7}, 4n gates {H,P,CNOT} + MEASURE all, shots uniform in
                      [1,64]; one persistent launch per engine variant.
 
-Arms: the default is the GB300 engine (the library's choice: the trace
-engines from 128 shots or 160 qudits, shot-group persistent kernels below): `value` from
+Arms: the default is the GB300 engine (the library's choice: the row form where
+its estimate of the run has it, else the trace engines' tableau passes from 128
+shots or 160 qudits, shot-group persistent kernels below): `value` from
 CUDA events on the launching stream with records in device memory, `e2e`
 through the C ABI with pinned host records and the copies inside the timed
 region; the other engines, the per-shot engine and the plain form (one
@@ -359,11 +360,54 @@ def philox_peak(ctx):
     return v.value
 
 
-def trace_routed(n, d, shots):
-    """Whether the library runs a program on a trace engine (batched form)."""
-    if d == 2:
-        return trace_words(n) > 0 and (shots >= TRACE_MIN_SHOTS or n >= TRACE_MIN_QUDITS)
-    return n <= TRACE_U8_MAX_QUDITS and (shots >= TRACE_MIN_SHOTS or n >= TRACE_MIN_QUDITS)
+def row_form_of(ctx, encs, shots, flags=0):
+    """Which programs of a run take the row form (sdim_row_choice)."""
+    from sdim_gb300 import _lib
+    k = len(encs)
+    begin = np.concatenate([[0], np.cumsum([e.ops.shape[0] for e in encs])]).astype(np.int64)
+    ops = np.ascontiguousarray(np.concatenate([e.ops for e in encs]), dtype=np.int32)
+    probs = np.ascontiguousarray(np.concatenate([e.probs for e in encs]), dtype=np.float64)
+    n, d = (np.array([getattr(e, f) for e in encs], np.int32) for f in "nd")
+    ns, out = np.asarray(shots, np.int64), np.zeros(k, np.uint8)
+    _lib.check(ctx.lib.sdim_row_choice(k, ops.ctypes.data, begin.ctypes.data, probs.ctypes.data, n.ctypes.data,
+                                       d.ctypes.data, ns.ctypes.data, flags, ctx.num_sms, out.ctypes.data), ctx.ptr, "route")
+    return out.astype(bool)
+
+
+def row_program_of(ctx, enc):
+    """sdim_row_program's six values of a program, all 0 without a row form."""
+    import ctypes
+    from sdim_gb300 import _lib
+    out = (ctypes.c_int64 * 6)()
+    ops, probs = np.ascontiguousarray(enc.ops), np.ascontiguousarray(enc.probs)
+    _lib.check(ctx.lib.sdim_row_program(ops.ctypes.data, int(ops.shape[0]), probs.ctypes.data, enc.n, enc.d, out),
+               ctx.ptr, "row program")
+    return list(out)
+
+
+def row_launches(ctx, d, n, infos):
+    """Kernels of the row form's x / z passes for programs that share a launch:
+    raw pass (unless in front of the chain), chain and extra pass."""
+    import ctypes
+    ns, p = np.asarray(n, np.int32), np.ascontiguousarray(infos, dtype=np.int64)
+    out = (ctypes.c_int32 * 8)()
+    if ctx.lib.sdim_row_plan(d, len(ns), ns.ctypes.data, p.ctypes.data, ctx.smem_optin, ctx.num_sms, out) != 0:
+        return 3
+    return 1 + (out[2] == 0) + (out[7] > 0)
+
+
+def frame_planes(ctx, enc, shots):
+    """Whether the frame route runs a program on bit planes (sdim_frame_route)."""
+    ops, probs = np.ascontiguousarray(enc.ops), np.ascontiguousarray(enc.probs)
+    return ctx.lib.sdim_frame_route(ops.ctypes.data, int(ops.shape[0]), probs.ctypes.data, enc.n, enc.d, shots, 0,
+                                    ctx.smem_optin, ctx.smem_optin + 1024, 1024, ctx.num_sms) == 1
+
+
+def trace_routed(n, d, shots, rows=False):
+    """Whether the library runs a program on a trace engine (batched form);
+    rows: it takes the row form."""
+    wide = trace_words(n) > 0 if d == 2 else n <= TRACE_U8_MAX_QUDITS
+    return wide and (rows or shots >= TRACE_MIN_SHOTS or n >= TRACE_MIN_QUDITS)
 
 
 def u8_single_cta(n, smem_optin):
@@ -620,6 +664,14 @@ def graph_replay(args, torch, ctx, timer, stream, entries, units_per_step, expec
             "graph_nodes": info["nodes"], "kernel_nodes": info["kernel_nodes"]}
 
 
+def frame_launches(ctx, enc, ref_enc, planes):
+    """Kernels of a frame run: the reference shot's x / z passes and replay, then
+    coins (d = 2 with N1), frames and records on planes, or the byte kernel."""
+    info = row_program_of(ctx, ref_enc)
+    shot0 = 1 + (row_launches(ctx, enc.d, [enc.n], [info]) if info[0] else 1)
+    return shot0 + (2 + (enc.d == 2 and bool((enc.ops[:, 0] == 17).any())) if planes else 1)
+
+
 def frame_route(args, torch, ctx, prog, dp, spec, shots, timer):
     """The reference's multi-shot route (Program.simulate(shots) without
     force_tableau): noiseless tableau shot 0, Pauli frames for the rest, on
@@ -651,11 +703,14 @@ def frame_route(args, torch, ctx, prog, dp, spec, shots, timer):
     if not np.array_equal(host[:, :nrec].numpy(), dev):
         raise AssertionError("frame route: end-to-end records differ from the device-timed run")
     units = len(spec.ops) * shots
+    planes = frame_planes(ctx, dp.enc, shots)
     out = {"value": units / (kms / 1e3), "unit": UNIT, "kernel_ms": kms,
-           "form": "noiseless tableau shot 0, then one lane per shot carrying x / z frames (k_frame_pass)",
+           "form": "noiseless tableau shot 0 beside the frames of the rest, 32 shots a word on bit planes "
+                   "(k_rows_frame), then the records of both (k_rows_frame_out)" if planes else
+                   "noiseless tableau shot 0, then one lane per shot carrying x / z frames (k_frame_pass)",
            "e2e": {"value": units * args.steps / (sum(e2e_ms) / 1e3), "unit": UNIT,
                    "ms_per_step": statistics.mean(e2e_ms), "d2h_bytes_per_step": int(shots * nrec)},
-           "gpu_launches_per_step": 2}
+           "gpu_launches_per_step": frame_launches(ctx, dp.enc, ref.enc, planes)}
     if not args.no_cpu:
         import oracle
         from oracle import frame
@@ -676,6 +731,15 @@ def frame_route(args, torch, ctx, prog, dp, spec, shots, timer):
     return out
 
 
+def step_launches(ctx, enc, rows, on_trace, passes):
+    """Kernels of one step of a single program: x / z passes, coin pass, then
+    header, column and record pass (with record columns) or the replay."""
+    if not on_trace:
+        return 1
+    xz = row_launches(ctx, enc.d, [enc.n], [row_program_of(ctx, enc)]) if rows else 1
+    return xz + (passes[1] > 0.0) + (3 if passes[2] > 0.0 else 1)
+
+
 def run_single(args, torch, dist, ws, rank, local):
     from sdim_gb300 import Program, _lib
 
@@ -694,10 +758,10 @@ def run_single(args, torch, dist, ws, rank, local):
 
     engine_flags = _lib.engine_flags(None if args.engine == "auto" else args.engine)
     engine_flags |= {"auto": 0, "packed": _lib.FLAG_PACKED_XZ, "bytes": _lib.FLAG_U8_XZ}[args.xz]
-    trace_used = (d == 2 and trace_words(n) > 0 and
-                  (args.engine == "trace" or (args.engine == "auto" and trace_routed(n, d, shots))))
-    odd_trace_used = (d != 2 and n <= TRACE_U8_MAX_QUDITS and
-                      (args.engine == "trace" or (args.engine == "auto" and trace_routed(n, d, shots))))
+    rows = bool(row_form_of(ctx, [enc], [shots], engine_flags)[0])
+    on_trace = args.engine in ("auto", "trace") and (trace_routed(n, d, shots, rows) or
+                                                     (args.engine == "trace" and trace_routed(n, d, TRACE_MIN_SHOTS)))
+    trace_used, odd_trace_used = on_trace and d == 2, on_trace and d != 2
 
     def step(extra=None):
         rc = ctx.lib.sdim_run_device(ctx.ptr, dp.ptr, 0, shot0, shots, out.data_ptr(), stream.cuda_stream,
@@ -723,7 +787,9 @@ def run_single(args, torch, dist, ws, rank, local):
             "scaling": "weak", "vs_baseline": None, "dtype": "u8 residues",
             "data": "synthetic (seeded circuit generator, Philox frame and noise stream)",
             "config": {"workload": desc, "shots_per_gpu": shots, "mode": "quick: frame route only"},
-            "route": "frame", "kernel_ms": kms, "gpu_launches": 2 * args.steps, "clocks": clk}
+            "route": "frame", "kernel_ms": kms,
+            "gpu_launches": frame_launches(ctx, enc, ref.enc, frame_planes(ctx, enc, shots)) * args.steps,
+            "clocks": clk}
     for _ in range(args.warmup):
         step()
     ctx.sync()
@@ -745,7 +811,7 @@ def run_single(args, torch, dist, ws, rank, local):
             "engine": args.engine, "kernel_ms": statistics.mean(kern_ms),
             "stages_ms": {"xz_pass": stages[0], "phase_pass": stages[1], "other_engines": stages[2]},
             "passes_ms": {"xz_pass": passes[0], "coin_pass": passes[1], "column_pass": passes[2]},
-            "gpu_launches": args.steps, "clocks": clk}
+            "gpu_launches": args.steps * step_launches(ctx, enc, rows, on_trace, passes), "clocks": clk}
 
     # per-shot engine (one warp, one full tableau per shot) on the same inputs
     step(_lib.FLAG_PER_SHOT)
@@ -862,11 +928,15 @@ def run_single(args, torch, dist, ws, rank, local):
         cpu = {"value": r, "unit": UNIT, "cores": threads, "kind": "port",
                "sample": f"{cshots} shots of the same workload in {cdt:.1f} s (C restatement of sdim's "
                          f"ExtendedTableau + shot loop, OpenMP over shots)"}
+    if on_trace:  # an equivalent rate: the trace engines do not move these bytes
+        frac_of = lambda rate: None  # noqa: E731
+    else:
+        frac_of = lambda rate: rate / peak  # noqa: E731
     kernel = {2: "k_group_warp<TGroupBits<WarpTeam>>"}.get(d, f"k_group_{'cta' if n >= 160 else 'warp'}"
                                                               f"<TGroupU8<{d}>>")
     if d == 2 and n >= 160:
         kernel = "k_group_cta<TGroupBits<CtaTeam>>"
-    group_model = {"bound": "smem", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+    group_model = {"bound": "smem", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": frac_of(achieved),
                    "kernel": kernel,
                    "peak_source": "shared-memory read bandwidth measured live by sdim_probe_smem_bandwidth",
                    "algorithmic_bytes_per_launch": gbytes,
@@ -901,8 +971,9 @@ def run_single(args, torch, dist, ws, rank, local):
         roofline = {"bound": "int-multiply (Philox4x32-10 blocks)", "achieved": ach / 1e9, "peak": prate / 1e9,
                     "unit": "Gblock/s", "frac": ach / prate,
                     "traffic": read_traffic("trace_engine_surface_L7.md") if args.workload == "surface" else None,
-                    "kernel": "trace engine step: k_rows_chain and k_rows_extra (x/z, a cluster of 8 CTAs) alongside "
-                              "k_coin_pass, then " +
+                    "kernel": "trace engine step: " +
+                              ("k_rows_chain and k_rows_extra" if rows else "k_trace_pass") +
+                              " (x/z) alongside k_coin_pass, then " +
                               (f"k_column_pass<{trace_words(n)}> and k_record_pass<{nw}>" if columns else
                                f"k_phase_pass<{trace_words(n)}>"),
                     "peak_source": "Philox throughput measured live by sdim_probe_philox_rate",
@@ -953,21 +1024,23 @@ def run_single(args, torch, dist, ws, rank, local):
         roofline = dict(group_model)
         roofline["traffic"] = None
         if odd_trace_used:
-            # the x / z pass updates one tableau per program on one CTA, a CTA
+            # a tableau pass updates one tableau per program on one CTA, a CTA
             # pair or a cluster of 8: its algorithmic shared-memory bytes
             # against the share of the measured shared-memory bandwidth of the
-            # SMs it runs on
+            # SMs it runs on.  The row form does not move those bytes: the rate
+            # is an equivalent one, without a fraction
             xz_ms = stages[0]
             sms, _ = u8_xz_layout(n, 1, ctx.smem_optin, ctx.num_sms, d)
-            rows = args.xz == "auto" and d in (3, 5, 7) and n <= 2048  # the row form: a cluster of 8 CTAs, or one
-            if rows:
+            if rows:  # a cluster of 8 CTAs, or one
                 sms = 8 if spec.num_measurements() > 62 else 1
             share = peak * sms / ctx.num_sms
             xz_ach = per_shot_bytes / (xz_ms / 1e3) / 1e9
             xz_kernel = "k_rows_chain" if rows else \
                 xz_kernel_name(ctx.lib.sdim_trace_xz_mode(n, d, 1, 0, ctx.smem_optin, ctx.num_sms))
-            roofline = {"bound": f"smem (x/z pass, latency-bound on {sms} CTA{'s' if sms > 1 else ''})",
-                        "achieved": xz_ach, "peak": share, "unit": "GB/s", "frac": xz_ach / share,
+            roofline = {"bound": f"latency (x/z pass in row form on {sms} CTA{'s' if sms > 1 else ''}: layers of gates, "
+                                 "then a dependent chain per random measurement); no byte bound" if rows else
+                                 f"smem (x/z pass, latency-bound on {sms} CTA{'s' if sms > 1 else ''})",
+                        "achieved": xz_ach, "peak": share, "unit": "GB/s", "frac": None if rows else xz_ach / share,
                         "traffic": read_traffic(f"trace_engine_{args.workload}.md"),
                         "traffic_source": "DRAM bytes of one step under ncu, read from profiles/ (not measured "
                                           "in this run)",
@@ -982,7 +1055,8 @@ def run_single(args, torch, dist, ws, rank, local):
                                                 "gates between them are walked in order"},
                         "peak_source": f"sdim_probe_smem_bandwidth x {sms}/{ctx.num_sms} SMs",
                         "algorithmic_bytes_per_launch": per_shot_bytes,
-                        "bytes_model": "per-instruction bytes of one tableau update (x/z pass: one tableau per program)",
+                        "bytes_model": "per-instruction bytes of one tableau update (x/z pass: one tableau per program)"
+                                       + ("; an equivalent rate, the row form does not move them" if rows else ""),
                         "kernel_ms": xz_ms,
                         "stages_ms": {"xz_pass": stages[0], "phase_pass": stages[1]},
                         "group_engine_model": group_model}
@@ -1013,7 +1087,7 @@ def run_single(args, torch, dist, ws, rank, local):
                          "frac": ps_achieved / peak, "algorithmic_bytes_per_shot": per_shot_bytes}},
         "roofline": roofline,
         "cpu_baseline": cpu,
-        "gpu_launches": args.steps * (3 if trace_used else 1),
+        "gpu_launches": args.steps * graph["kernel_nodes"],
         "clocks": clk,
         "engine": args.engine,
         "stages_ms": {"xz_pass": stages[0], "phase_pass": stages[1], "other_engines": stages[2]},
@@ -1052,6 +1126,23 @@ def plain_uneven(br, entries, budget_s):
         if spent > budget_s:
             break
     return units / est_s, used, len(sample), spent
+
+
+def batch_launches(ctx, entries, in_rows):
+    """Kernels of a batch's step: per (d, spread of a row) of its row-form programs
+    the x / z passes and the phase pass, at least one per (d, team) of the others."""
+    def spread(n, d):  # rows.cuh: row_slice
+        e = -(-n // 32)
+        return (1 if e <= 1 else 2 if e <= 2 else 4 if e <= 4 else 8 if e <= 8 else 24 if e <= 24 else 64)
+    groups = {}
+    for e, r in zip(entries, in_rows):
+        if r:
+            enc = e.program.enc
+            ns, infos = groups.setdefault((enc.d, spread(enc.n, enc.d)), ([], []))
+            ns.append(enc.n)
+            infos.append(row_program_of(ctx, enc))
+    rest = {(e.program.enc.d, e.program.enc.n >= 160) for e, r in zip(entries, in_rows) if not r}
+    return sum(1 + row_launches(ctx, d, ns, infos) for (d, _), (ns, infos) in groups.items()) + len(rest)
 
 
 def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
@@ -1106,7 +1197,8 @@ def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
                 "kernel_ms": statistics.mean(kern_ms),
                 "stages_ms": {"xz_pass_and_coin_pass": stages[0], "phase_pass": stages[1],
                               "shot_group_engines_alongside": stages[2]},
-                "gpu_launches": steps * len({(e.program.enc.d, e.program.enc.n >= 160) for e in entries}),
+                "gpu_launches": steps * batch_launches(ctx, entries, row_form_of(
+                    ctx, [e.program.enc for e in entries], [e.shots for e in entries])),
                 "clocks": clk}
 
     ps = None
@@ -1153,7 +1245,9 @@ def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
     peak = smem_peak(ctx)
     hbm = hbm_peak()
     l2 = l2_peak(ctx)
-    odd_trace = sum(1 for e in entries if e.program.enc.d != 2 and e.program.enc.n <= TRACE_U8_MAX_QUDITS
+    in_rows = row_form_of(ctx, [e.program.enc for e in entries], [e.shots for e in entries])
+    launches = batch_launches(ctx, entries, in_rows)
+    odd_trace = sum(1 for e, r in zip(entries, in_rows) if e.program.enc.d != 2 and not r
                     and trace_routed(e.program.enc.n, e.program.enc.d, e.shots))
     # t_packed: the same bound with the x / z bytes of d = 5, 7 trace programs
     # at the 4-bit lanes their batched x / z pass stores (half of the byte
@@ -1161,11 +1255,11 @@ def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
     # planes)
     packed_run = 2 * odd_trace >= ctx.num_sms
     gb, gb_packed, t_min, t_packed, streamed, in_l2 = 0.0, 0.0, 0.0, 0.0, 0.0, 0.0
-    for e, o in zip(entries, offs[:-1]):
+    for e, o, r in zip(entries, offs[:-1], in_rows):
         enc = e.program.enc
         nr = e.program.num_records
         det_row = (ref_out[int(o):int(o) + nr] >> 7).astype(bool)
-        on_trace = trace_routed(enc.n, enc.d, e.shots)
+        on_trace = trace_routed(enc.n, enc.d, e.shots, r)
         xz = algorithmic_bytes_per_shot(enc, det_row, enc.n, enc.d) * (1 if on_trace else -(-e.shots // 32))
         delta = e.shots * group_delta_bytes_per_shot(enc, det_row, 0.0, enc.n, enc.d)
         place = tableau_place(enc.n, enc.d, on_trace, ctx.smem_optin, odd_trace, ctx.num_sms)
@@ -1209,9 +1303,11 @@ def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
         cpu = {"value": r, "unit": UNIT, "cores": threads, "kind": "port",
                "sample": f"{used} programs, min(shots,4) shots each, in {cdt:.1f} s (C oracle, OpenMP)"}
         _leg("uneven: CPU oracle", t_leg)
+    by_rows = bool(in_rows.any())  # bytes that the row form does not move: no fraction
     return {
         "value": value, "unit": UNIT, "steps": steps, "warmup": warmup, "ms_per_step": total_ms / steps,
         "config": uneven_config(items, ws),
+        "row_form_programs": int(in_rows.sum()),
         "shots_per_s": br.total_shots() * ws * steps / (total_ms / 1e3),
         "latency_ms": {"p50": float(np.percentile(step_ms, 50)), "p99": float(np.percentile(step_ms, 99))},
         "kernel_ms": mean_kern,
@@ -1227,12 +1323,15 @@ def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
                               "times its shot count, smallest programs first within a time budget"},
         "batched_vs_plain": value / plain_rate,
         "per_shot_engine": ps,
-        "roofline": {"bound": "smem for resident tableaux, L2 for columns streamed by CTA clusters, HBM for "
+        "roofline": {"bound": "issue and latency of the row form's eliminations and row updates; no byte bound (the "
+                              "tableau figures are an equivalent rate)" if by_rows else
+                              "smem for resident tableaux, L2 for columns streamed by CTA clusters, HBM for "
                               "other streamed tableaux",
                      "achieved": gb_packed / (mean_kern / 1e3) / 1e9, "peak": gb_packed / t_packed / 1e9,
-                     "unit": "GB/s", "frac": t_packed * 1e3 / mean_kern, "traffic": None,
-                     "kernel": "trace engines (k_trace_pass*, k_phase_pass*) for n >= 160 or 128+ shots, "
-                               "k_group_warp / k_group_cta for the rest",
+                     "unit": "GB/s", "frac": None if by_rows else t_packed * 1e3 / mean_kern, "traffic": None,
+                     "kernel": "row form (k_rows_raw, k_rows_chain, k_rows_phase) where the run's estimate has it, of "
+                               "the rest trace engines (k_trace_pass*, k_phase_pass*) for n >= 160 or 128+ shots, "
+                               "k_group_warp / k_group_cta below",
                      "algorithmic_bytes_per_launch": gb_packed, "streamed_bytes": streamed, "l2_bytes": in_l2,
                      "kernel_ms": mean_kern, "bound_ms": t_packed * 1e3, "smem_peak_gbs": peak, "l2_peak_gbs": l2,
                      "hbm_peak_gbs": hbm,
@@ -1243,13 +1342,12 @@ def uneven_measure(args, torch, dist, ws, rank, local, sub=False):
                                     "at the residue width the library stores (bit planes for d = 2, 3; 4-bit lanes "
                                     "for d = 5, 7 in the batched packed x/z pass; bytes otherwise), plus per-shot "
                                     "phase-delta bytes; frac = bound_ms / kernel_ms",
-                     "byte_residues": {"bound_ms": t_min * 1e3, "frac": t_min * 1e3 / mean_kern,
+                     "byte_residues": {"bound_ms": t_min * 1e3, "frac": None if by_rows else t_min * 1e3 / mean_kern,
                                        "algorithmic_bytes": gb,
                                        "model": "the same bound with d = 5, 7 x/z rows at one byte per residue "
                                                 "(the per-gate byte table's figure for d >= 5)"}},
         "cpu_baseline": cpu,
-        # one persistent launch per (dimension, team kind) present in the batch
-        "gpu_launches": steps * len({(e.program.enc.d, e.program.enc.n >= 160) for e in entries}),
+        "gpu_launches": steps * launches,
         "clocks": clk,
         "graph_replay": graph,
         "autotune": tuned,

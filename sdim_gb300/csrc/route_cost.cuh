@@ -8,8 +8,8 @@
 // is the faster one therefore turns on how many programs share the device, on
 // the shots, and on measurements against qudits.  Measured on GB300, row form
 // and the other route (us):
-//     1 x   97 qubits, 385 measurements, 1 shot           102    550
-//     1 x    3 qudits of d = 7,  2,000 measurements      3969   5193
+//     1 x   49 qubits (a memory), 145 measurements, 1 shot 102    505
+//     1 x    3 qudits of d = 7, 2,000 measurements       3969   5193
 //     1 x    3 qudits of d = 7, 20,000 measurements    170496  51700
 //   300 x   31 qudits of d = 7, 200 measurements, 1 shot  587    848
 //   300 x    3 qudits of d = 7, 2,000 measurements      49678   5104
@@ -17,11 +17,11 @@
 //  4000 x   31 qubits, 31 measurements, 200 shots         979   1685
 // The constants below are fitted to 6,210 such pairs: d = 2, 3, 7, 3 to 400
 // qudits, 3 to 4,000 measurements, with noise and without, 1 to 2,000 shots, 1 to
-// 4,000 programs a run.  Four fifths of the estimates are within 35% of the
+// 4,000 programs a run.  Four fifths of the estimates are within 30% of the
 // measured time, and the choice (choose_row_form) costs at most 3% over the faster
-// of the two in 95% of the pairs and 1.3 times in 99%.  (The row form for all of
-// them: slower in 20% of the pairs, up to 29 times; for none: slower in 77%, up to
-// 52 times.)
+// of the two in 95% of the pairs, 1.3 times in 99% and 2 times at worst.  (The row
+// form for all of them: slower in 20% of the pairs, up to 29 times; for none: slower
+// in 77%, up to 52 times.)
 #pragma once
 #include <algorithm>
 #include <cmath>

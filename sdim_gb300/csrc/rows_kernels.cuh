@@ -58,7 +58,6 @@ struct El {
     if constexpr (D == 7) return make_uint4(~a.x, ~a.y, ~a.z, 0u);
     return make_uint4(a.z | (a.y & ~a.x), a.y, a.x & ~a.y, 0u);
   }
-  static __device__ __forceinline__ T sub(T a, T b) { return add(a, neg(b)); }
   static __device__ __forceinline__ T dbl(T a) {
     if constexpr (D == 7) return make_uint4(a.z, a.x, a.y, 0u);
     return make_uint4((a.x & a.y) | a.z, (a.x & ~a.y) | a.z, a.y & ~a.x, 0u);
@@ -195,7 +194,6 @@ struct El<3> {  // two planes (planes3.cuh)
   static __device__ __forceinline__ T zero() { return make_uint2(0u, 0u); }
   static __device__ __forceinline__ uint32_t nzw(T a) { return a.x | a.y; }
   static __device__ __forceinline__ T add(T a, T b) { return t(p3_add(p(a), p(b))); }
-  static __device__ __forceinline__ T sub(T a, T b) { return t(p3_sub(p(a), p(b))); }
   static __device__ __forceinline__ T neg(T a) { return make_uint2(a.y, a.x); }
   static __device__ __forceinline__ T mulc(T a, int c) { return c == 0 ? zero() : c == 1 ? a : neg(a); }
   static __device__ __forceinline__ T muladd(T v, T f, int c) {

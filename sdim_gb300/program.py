@@ -181,8 +181,9 @@ class Program:
         """Records of shots [shot0, shot0 + shots) as a (shots, records) uint8
         array, value | deterministic << 7 -- the fast path without Python objects.
 
-        ``engine`` picks the batched engine: None (by shot count and d),
-        "trace" (d = 2: one x / z pass, one lane per shot), "group" (32-shot
+        ``engine`` picks the batched engine: None (by the library's estimate
+        of the run), "trace" (one x / z pass, then a replay per shot; "rows" and
+        "tableau" name the pass's form), "group" (32-shot
         groups), "per_shot" (one warp per shot; same as ``per_shot=True``),
         "tuned" (the route the autotuner timed fastest for this program's
         class of d, n and shots; the first call of a class times them).

@@ -18,8 +18,8 @@
 // The constants below are fitted to 6,210 such pairs: d = 2, 3, 7, 3 to 400
 // qudits, 3 to 4,000 measurements, with noise and without, 1 to 2,000 shots, 1 to
 // 4,000 programs a run.  Four fifths of the estimates are within 30% of the
-// measured time, and the choice (choose_row_form) costs at most 3% over the faster
-// of the two in 95% of the pairs, 1.3 times in 99% and 2 times at worst.  (The row
+// measured time, and the choice (choose_row_form) costs at most 2% over the faster
+// of the two in 95% of the pairs, 1.24 times in 99% and 1.8 times at worst.  (The row
 // form for all of them: slower in 20% of the pairs, up to 29 times; for none: slower
 // in 77%, up to 52 times.)
 #pragma once
@@ -63,7 +63,7 @@ inline RouteCost row_cost(const RouteShape& p, long long programs, int num_sms) 
   const double updates = full * nm - 0.5 * kRowPanel * full * (full + 1);
   const double task = odd ? 1.8 * updates : (group == 1 ? 3.5 : 2.5) * updates * group / 32;
   RouteCost c;
-  c.latency = 26 + 0.27 * p.layers + (odd ? 0.71 : 0.50) * nm + task / warps;
+  c.latency = 20 + (p.nx ? 6 : 0) + 0.27 * p.layers + (odd ? 0.71 : 0.50) * nm + task / warps;
   c.work = (0.48 * p.layers + 0.71 * nm) * block / (32.0 * kRowWarps) + 0.09 * task + (odd ? 0.11 : 0.003) * p.nx +
            (double)p.shots * ((odd ? 0.0018 : 0.0008) * nm + (odd ? 0.0004 : 0.0001) * p.nn1);
   if (!batch) c.work = std::min(c.work, c.latency);  // an SM to itself
@@ -92,14 +92,16 @@ inline RouteCost other_cost(const RouteShape& p) {
 
 // Which programs of a run take the row form (programs[i]: how many share p[i]'s
 // launch).  A run's time is estimated as the longest latency and the work over
-// all SMs, added as squares, the descriptors, and kGroupLaunch where shot groups run (their work
-// queue's reset, descriptors and launches).  Tried are the row form for all and,
-// for each bound on the latency, for every program the route of less work and
-// descriptors within the bound; the row form for all is kept unless another split is 5% shorter
-// (engines beside one another take each other's SMs, which the estimate leaves
-// out: 384 uneven programs 3353 us, 3686 with 170 small ones as shot groups,
-// estimated 1.4% shorter).
-constexpr double kGroupLaunch = 12.0;
+// all SMs, added as squares, the descriptors, and kGroupLaunch where shot groups
+// run (their work queue's reset, descriptors and launches).  The row form is for
+// all or for none (none where that is 5% shorter), unless a split -- for a bound
+// on the latency, for every program the route of less work and descriptors within
+// the bound -- is half as long as either: engines beside one another take each
+// other's SMs, which the estimate leaves out.  Of 60 mixed batches (12 to 2,500
+// programs, 4 to 1,024 qudits, 1 to 600 shots) splits that were estimated up to a
+// third shorter than the row form for all took up to 2.2 times as long, and the
+// row form for all up to 29 times less than none.
+constexpr double kGroupLaunch = 4.0;
 
 inline std::vector<char> choose_row_form(const std::vector<RouteShape>& p, const std::vector<long long>& programs,
                                          int num_sms) {
@@ -118,16 +120,19 @@ inline std::vector<char> choose_row_form(const std::vector<RouteShape>& p, const
     const double w = s.work / num_sms;
     return std::sqrt(s.longest * s.longest + w * w) + s.host + (s.groups ? kGroupLaunch : 0.0);
   };
-  Sum all, least;  // the row form for all; the least of either route
+  Sum all, none, least;  // the row form for all, for none; the least of either
   double most = 0.0;
   for (size_t i = 0; i < k; ++i) {
     const RouteCost &r = row[i] = row_cost(p[i], programs[i], num_sms), &o = other[i] = other_cost(p[i]);
     all.add(r);
+    none.add(o);
+    none.groups |= !p[i].trace;
     least.add(RouteCost{std::min(r.latency, o.latency), std::min(r.work, o.work), std::min(r.host, o.host)});
     most = std::max(most, std::max(r.latency, o.latency));
   }
-  std::vector<char> best(k, 1), take(k);
-  double best_time = 0.95 * time(all);
+  const bool rows = time(none) >= 0.95 * time(all);
+  std::vector<char> best(k, rows), take(k);
+  double best_time = 0.5 * time(rows ? all : none);
   // (no split is shorter than `least`, none with a latency past `bound` than the bound)
   for (double bound = least.longest; time(least) < best_time && bound < best_time; bound *= 1.3) {
     Sum s;

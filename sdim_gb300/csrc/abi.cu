@@ -609,17 +609,23 @@ void choose_rows(std::vector<Job>& jobs, unsigned flags, int num_sms) {
     for (size_t i : at) jobs[i].rows = true;
     return;
   }
+  auto shape = [&](const Job& j) {
+    const sdim_circuit* c = j.c;
+    const bool trace = (flags & SDIM_FLAG_TRACE) || j.nshots >= kTraceMinShots || c->n >= kTraceMinQudits;
+    return RouteShape{c->n, c->d, c->nmeas, c->nn1, c->nops - c->nn1 - c->nmeas, c->rows.nlayers, c->rows.nx, j.nshots, trace};
+  };
+  if (at.size() == 1) {
+    jobs[at[0]].rows = row_form_alone(shape(jobs[at[0]]), num_sms);
+    return;
+  }
   auto launch = [&](const sdim_circuit* c) { return 64 * c->d + row_slice(row_elems(c->n), c->d); };
   long long share[64 * 8] = {};
   for (size_t i : at) ++share[launch(jobs[i].c)];
   std::vector<RouteShape> shapes;
   std::vector<long long> programs;
   for (size_t i : at) {
-    const sdim_circuit* c = jobs[i].c;
-    const bool trace = (flags & SDIM_FLAG_TRACE) || jobs[i].nshots >= kTraceMinShots || c->n >= kTraceMinQudits;
-    shapes.push_back(RouteShape{c->n, c->d, c->nmeas, c->nn1, c->nops - c->nn1 - c->nmeas, c->rows.nlayers, c->rows.nx,
-                                jobs[i].nshots, trace});
-    programs.push_back(share[launch(c)]);
+    shapes.push_back(shape(jobs[i]));
+    programs.push_back(share[launch(jobs[i].c)]);
   }
   const std::vector<char> take = choose_row_form(shapes, programs, num_sms);
   for (size_t i = 0; i < at.size(); ++i) jobs[at[i]].rows = take[i];

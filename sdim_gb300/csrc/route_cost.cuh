@@ -103,24 +103,34 @@ inline RouteCost other_cost(const RouteShape& p) {
 // row form for all up to 29 times less than none.
 constexpr double kGroupLaunch = 4.0;
 
+struct RunCost {  // of the programs' chosen routes
+  double longest = 0.0, work = 0.0, host = 0.0;
+  bool groups = false;
+  void add(const RouteCost& c) {
+    longest = std::max(longest, c.latency);
+    work += c.work;
+    host += c.host;
+  }
+  double time(int num_sms) const {
+    const double w = work / num_sms;
+    return std::sqrt(longest * longest + w * w) + host + (groups ? kGroupLaunch : 0.0);
+  }
+};
+
+// A run of one program.
+inline bool row_form_alone(const RouteShape& p, int num_sms) {
+  RunCost row, other;
+  row.add(row_cost(p, 1, num_sms));
+  other.add(other_cost(p));
+  other.groups = !p.trace;
+  return other.time(num_sms) >= 0.95 * row.time(num_sms);
+}
+
 inline std::vector<char> choose_row_form(const std::vector<RouteShape>& p, const std::vector<long long>& programs,
                                          int num_sms) {
   const size_t k = p.size();
   std::vector<RouteCost> row(k), other(k);
-  struct Sum {  // of the programs' chosen routes
-    double longest = 0.0, work = 0.0, host = 0.0;
-    bool groups = false;
-    void add(const RouteCost& c) {
-      longest = std::max(longest, c.latency);
-      work += c.work;
-      host += c.host;
-    }
-  };
-  auto time = [&](const Sum& s) {
-    const double w = s.work / num_sms;
-    return std::sqrt(s.longest * s.longest + w * w) + s.host + (s.groups ? kGroupLaunch : 0.0);
-  };
-  Sum all, none, least;  // the row form for all, for none; the least of either
+  RunCost all, none, least;  // the row form for all, for none; the least of either
   double most = 0.0;
   for (size_t i = 0; i < k; ++i) {
     const RouteCost &r = row[i] = row_cost(p[i], programs[i], num_sms), &o = other[i] = other_cost(p[i]);
@@ -130,12 +140,12 @@ inline std::vector<char> choose_row_form(const std::vector<RouteShape>& p, const
     least.add(RouteCost{std::min(r.latency, o.latency), std::min(r.work, o.work), std::min(r.host, o.host)});
     most = std::max(most, std::max(r.latency, o.latency));
   }
-  const bool rows = time(none) >= 0.95 * time(all);
+  const bool rows = none.time(num_sms) >= 0.95 * all.time(num_sms);
   std::vector<char> best(k, rows), take(k);
-  double best_time = 0.5 * time(rows ? all : none);
+  double best_time = 0.5 * (rows ? all : none).time(num_sms);
   // (no split is shorter than `least`, none with a latency past `bound` than the bound)
-  for (double bound = least.longest; time(least) < best_time && bound < best_time; bound *= 1.3) {
-    Sum s;
+  for (double bound = least.longest; least.time(num_sms) < best_time && bound < best_time; bound *= 1.3) {
+    RunCost s;
     for (size_t i = 0; i < k; ++i) {
       const RouteCost &r = row[i], &o = other[i];
       const double more = (r.work - o.work) / num_sms + r.host - o.host;  // of the row form, in the run's time
@@ -143,8 +153,8 @@ inline std::vector<char> choose_row_form(const std::vector<RouteShape>& p, const
       s.add(take[i] ? r : o);
       s.groups |= !take[i] && !p[i].trace;
     }
-    if (time(s) < best_time) {
-      best_time = time(s);
+    if (s.time(num_sms) < best_time) {
+      best_time = s.time(num_sms);
       best = take;
     }
     if (bound >= most) break;

@@ -19,7 +19,7 @@
 // qudits, 3 to 4,000 measurements, with noise and without, 1 to 2,000 shots, 1 to
 // 4,000 programs a run.  Four fifths of the estimates are within 30% of the
 // measured time, and the choice (choose_row_form) costs at most 2% over the faster
-// of the two in 95% of the pairs, 1.24 times in 99% and 1.8 times at worst.  (The row
+// of the two in 95% of the pairs, 1.23 times in 99% and 1.8 times at worst.  (The row
 // form for all of them: slower in 20% of the pairs, up to 29 times; for none: slower
 // in 77%, up to 52 times.)
 #pragma once
@@ -44,6 +44,9 @@ struct RouteCost {
   double latency, work, host;
 };
 
+// Replay of one shot, d = 2: much the same on both routes.
+inline double replay_us_d2(const RouteShape& p) { return 0.00016 * (p.nmeas * (1 + p.n / 64.0) + p.nn1); }
+
 // Row form, programs of its launch sharing the device.
 inline RouteCost row_cost(const RouteShape& p, long long programs, int num_sms) {
   const double nm = p.nmeas, full = std::floor(nm / kRowPanel);
@@ -64,9 +67,10 @@ inline RouteCost row_cost(const RouteShape& p, long long programs, int num_sms) 
   const double task = odd ? 1.8 * updates : (group == 1 ? 3.5 : 2.5) * updates * group / 32;
   RouteCost c;
   c.latency = 20 + (p.nx ? 6 : 0) + 0.27 * p.layers + (odd ? 0.71 : 0.50) * nm + task / warps;
-  c.work = (0.48 * p.layers + 0.71 * nm) * block / (32.0 * kRowWarps) + 0.09 * task + (odd ? 0.11 : 0.003) * p.nx +
-           (double)p.shots * ((odd ? 0.0018 : 0.0008) * nm + (odd ? 0.0004 : 0.0001) * p.nn1);
+  c.work = (0.48 * p.layers + 0.71 * nm) * block / (32.0 * kRowWarps) + 0.09 * task + (odd ? 0.11 : 0.003) * p.nx;
   if (!batch) c.work = std::min(c.work, c.latency);  // an SM to itself
+  c.work += (double)p.shots * (odd ? 0.003 + (p.d == 3 ? 0.00125 : 0.0017) * std::max(1.0, 0.35 * E) * nm + 0.0004 * p.nn1
+                                   : replay_us_d2(p));
   c.host = 0.17;
   return c;
 }
@@ -85,7 +89,8 @@ inline RouteCost other_cost(const RouteShape& p) {
     const double part = odd ? (p.d == 3 ? 0.12 : 0.23) * (1 + 3.2e-5 * n * n) : 0.53 * (1 + 0.0012 * n);
     c.latency = 26 + chain;
     c.host = 0.09;
-    c.work = chain * std::min(1.0, part) + shots * (odd ? 0.0018 : 0.00016) * (nm * (1 + n / 64) + p.nn1);
+    c.work = chain * std::min(1.0, part) +
+             shots * (odd ? 0.001 + std::max(0.0016, 3.2e-5 * n) * nm + 0.0018 * p.nn1 : replay_us_d2(p));
   }
   return c;
 }

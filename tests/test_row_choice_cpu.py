@@ -76,6 +76,15 @@ def test_a_wide_program_takes_it_beside_thousands_of_small_ones():
     assert got[:8].all() and not got[8:].any()
 
 
+def test_millions_of_shots_of_a_tiny_odd_d_program():
+    """The row form's replay costs more a shot there: 2 qudits of d = 7, 20,000 shots
+    28 and 30 us, 3,000,000 shots 168 and 86 us.  Not for qubits, or with noise."""
+    tiny = workloads.random_hpc(2, 7, 12, seed=2)
+    assert _choice([tiny], 20000)[0] == 1 and _choice([tiny], 3000000)[0] == 0
+    assert _choice([workloads.random_hpc(2, 2, 12, seed=2)], 3000000)[0] == 1
+    assert _choice([workloads.random_hpc(300, 7, 1800, seed=2)], 3000000)[0] == 1
+
+
 def test_mixed_sizes_keep_one_route():
     """Batches of many sizes, whose small programs would do as well as shot groups:
     splits took up to 2.2 times as long as the row form for all."""
